@@ -32,27 +32,6 @@ __global__ void scatter_i64_kernel(int64_t* dst, const int64_t* idx, const int64
   if (i < n) dst[idx[i]] = val[i];
 }
 
-// ---- the quantizer, many values under one reciprocal ---------------------------------------------
-// code = clamp(rne((x - mn) / scale), 0, levels) without a divide per value.  With y = RN(1 / scale) computed once,
-// q0 = RN(d * y), r = RN(d - scale * q0) (exact: one FMA) and q1 = RN(q0 + r * y), q1 IS the correctly rounded
-// quotient RN(d / scale) (Markstein's correction step; it needs y correctly rounded and the significand of the
-// divisor not all ones, and every scale here is an fp16 value).  q0 is capped at 512 first so that infinities and
-// overflowing quotients stay ordered through the correction (anything >= 255.5 clamps to `levels` anyway; NaN
-// clamps to 0 as on the divide route).  Adding 1.5 * 2^23 to the clamped quotient rounds it to the nearest-even
-// integer in the float's low mantissa bits (0 and levels are integers, so clamping before or after the rounding
-// gives the same code).
-constexpr float QMAGIC = 12582912.f;            // 1.5 * 2^23
-constexpr uint32_t QMAGIC_BITS = 0x4B400000u;   // its bit pattern; QMAGIC + code has bit pattern QMAGIC_BITS + code
-
-__device__ __forceinline__ uint32_t quant_u(float x, float mn, float scale, float rscale, float levels) {
-  const float d = __fsub_rn(x, mn);
-  const float q0 = fminf(__fmul_rn(d, rscale), 512.0f);
-  const float r = __fmaf_rn(-scale, q0, d);
-  const float q1 = __fmaf_rn(r, rscale, q0);
-  const float t = fminf(fmaxf(q1, 0.0f), levels);
-  return __float_as_uint(__fadd_rn(t, QMAGIC));
-}
-
 // 8 values of QMAGIC_BITS + code -> the 8 codes packed at BITS (element k at bit k * BITS): the shifted sum of
 // the words minus the shifted sum of the constant, modulo 2^32.
 template <int BITS>
