@@ -90,9 +90,15 @@ dequant_dense_kernel(LayoutDev L, ResidualDev R, const uint8_t* __restrict__ pag
   }
 }
 
-// The same for 16-bit outputs whose rows allow 16-byte stores and blocks of at most 64 tokens: one thread per
-// (token, 8 channels) loads the 8 codes of each side as one word and the K stats as two 16-byte vectors, and
-// stores 16 bytes of K and of V.  The arithmetic is dequant8's: code * scale + min in fp32, two roundings.
+// The same for 16-bit outputs whose rows allow 16-byte stores: one CTA per 16 tokens of a work item, one thread per
+// 8 channels and every (256 / (H * D / 8))-th of the tokens.  The arithmetic is dequant8's: code * scale + min in fp32, two
+// roundings, two values per instruction.
+//
+// Bound by its instructions, and for few blocks by the chain work item -> block table -> header -> rows, so a CTA is
+// as small as keeps that chain worth it (a 64-token block as one CTA left 34 CTAs of 32 rounds each for a 2,112-token context:
+// 60 us, now 6.5 us), a thread stays on its channels (its K group's statistics are read once) with four tokens' loads
+// in flight, and a code becomes a float with one byte permute.  8 x 8,704 tokens x 8 heads x 128 at INT4 / INT8
+// alternating: 88 us, 156 us before = 0.66 of the measured copy peak at INT4 + INT8's mean of 383 MB.
 template <typename T> __device__ __forceinline__ uint32_t pack2_rn(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2_rn<__half>(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
@@ -103,99 +109,145 @@ template <> __device__ __forceinline__ uint32_t pack2_rn<__nv_bfloat16>(float a,
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// 8 codes as floats.  A code c < 2^23 placed in the mantissa of 2^23 is the float 2^23 + c, and subtracting 2^23 is
-// exact: two full-rate instructions per code instead of an integer-to-float conversion.
-__device__ __forceinline__ float code_f32(uint32_t c) { return __uint_as_float(0x4B000000u | c) - 8388608.f; }
-__device__ __forceinline__ void load_codes8(const uint8_t* p, int bits, float (&q)[8]) {
-  if (bits == 8) {
-    const uint2 w = *reinterpret_cast<const uint2*>(p);
+// 8 codes as four float pairs.  A code c < 2^23 placed in the mantissa of 2^23 is the float 2^23 + c (one byte permute),
+// and subtracting 2^23 is exact.
+__device__ __forceinline__ float code_byte(uint32_t w, int k) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + k));
+}
+__device__ __forceinline__ float2 code_pair(uint32_t wa, int ka, uint32_t wb, int kb) {
+  return __fadd2_rn(make_float2(code_byte(wa, ka), code_byte(wb, kb)), make_float2(-8388608.f, -8388608.f));
+}
+template <int BITS> struct Codes8;  // 8 packed codes as loaded
+template <> struct Codes8<8> { using W = uint2; };
+template <> struct Codes8<4> { using W = uint32_t; };
+template <> struct Codes8<2> { using W = uint16_t; };
+template <int BITS>
+__device__ __forceinline__ void unpack8(const typename Codes8<BITS>::W& w, float2 (&q)[4]) {
+  if constexpr (BITS == 8) {
+    q[0] = code_pair(w.x, 0, w.x, 1); q[1] = code_pair(w.x, 2, w.x, 3);
+    q[2] = code_pair(w.y, 0, w.y, 1); q[3] = code_pair(w.y, 2, w.y, 3);
+  } else if constexpr (BITS == 4) {
+    const uint32_t e = w & 0x0F0F0F0Fu, o = (w >> 4) & 0x0F0F0F0Fu;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { q[i] = code_f32((w.x >> (8 * i)) & 0xFFu); q[4 + i] = code_f32((w.y >> (8 * i)) & 0xFFu); }
-  } else if (bits == 4) {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(p);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = code_f32((w >> (4 * i)) & 0xFu);
+    for (int i = 0; i < 4; ++i) q[i] = code_pair(e, i, o, i);
   } else {
-    const uint32_t w = *reinterpret_cast<const uint16_t*>(p);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = code_f32((w >> (2 * i)) & 0x3u);
+    const uint32_t x = w, c0 = x & 0x0303u, c1 = (x >> 2) & 0x0303u, c2 = (x >> 4) & 0x0303u, c3 = (x >> 6) & 0x0303u;
+    q[0] = code_pair(c0, 0, c1, 0); q[1] = code_pair(c2, 0, c3, 0);
+    q[2] = code_pair(c0, 1, c1, 1); q[3] = code_pair(c2, 1, c3, 1);
   }
 }
 
-constexpr int DENSE_MAX_BS = 64;
+constexpr int DENSE_TOK = 16;  // tokens per CTA
 
 template <typename T>
-__global__ void __launch_bounds__(256)
-dequant_dense_vec_kernel(LayoutDev L, ResidualDev R, const uint8_t* __restrict__ pages, const int32_t* __restrict__ work,
-                         const int32_t* __restrict__ bt, int64_t bt_s0, T* __restrict__ k_out, T* __restrict__ v_out,
-                         int64_t o_s0, int64_t o_s1) {
-  __shared__ int64_t s_row[DENSE_MAX_BS];
-  const int4 w = reinterpret_cast<const int4*>(work)[blockIdx.x];
-  const int req = w.x, bi = w.y, ctx = w.w;
-  const int64_t row0 = w.z;
-  const int64_t blk = bt[(int64_t)req * bt_s0 + bi];
-  const int nvalid = min(L.BS, ctx - bi * L.BS);
-  const uint8_t* page = pages + blk * L.PS;
-  int bits = page[0];
-  if (bits == 0) bits = 2;  // an unopened block reads as INT2, like the attention kernels
-  if ((int)threadIdx.x < nvalid) s_row[threadIdx.x] = row_offset(pages, L, blk, threadIdx.x, bits);
-  const int64_t slot = R.block_res[blk];
-  const int open_grp = slot >= 0 ? (int)R.res_group[slot] : -1;
-  __syncthreads();
+struct DenseArgs {
+  LayoutDev L;
+  ResidualDev R;
+  const uint8_t* pages;
+  const int32_t* work;
+  const int32_t* bt;
+  int64_t bt_s0;
+  T *k_out, *v_out;
+  int64_t o_s0, o_s1;
+  int slices;  // CTAs per block
+};
+
+// Tokens [t0, t1) of one block of tier BITS; `s_row`: byte offset of each token's row from the pool base.  The loads of
+// a batch of tokens are issued together; the K statistics are read again only where the K group changes.
+template <typename T, int BITS>
+__device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t* page, int64_t row0, int t0, int t1,
+                                           int64_t slot, int open_grp, const int64_t* s_row) {
+  using W = typename Codes8<BITS>::W;
+  constexpr int BATCH = 4;
+  const LayoutDev& L = A.L;
   const int cpt = (L.H * L.D) / 8, cph = L.D / 8;
-  const int side_bytes = (L.H * L.D * bits) / 8;
-  const __half* vs_p = reinterpret_cast<const __half*>(page + L.o_vs);
-  const __half* vm_p = reinterpret_cast<const __half*>(page + L.o_vm);
-  // (token, chunk) of this thread's items without a division per item: 256 items ahead is t_step tokens and
-  // c_step chunks further
-  const int t_step = 256 / cpt, c_step = 256 % cpt;
-  int t = (int)threadIdx.x / cpt, c = (int)threadIdx.x % cpt;
-  int h = c / cph, d0 = (c - h * cph) * 8;
-#pragma unroll 4
-  for (; t < nvalid; t += t_step) {
-    const uint8_t* krow = pages + s_row[t] + (c * bits);  // 8 channels * bits / 8 bytes per chunk of 8
-    float qk[8], qv[8];
-    load_codes8(krow + side_bytes, bits, qv);
-    const int64_t ve = ((int64_t)t * L.H + h) * L.NG + d0 / L.VG;
-    const float vs = __half2float(vs_p[ve]), vm = __half2float(vm_p[ve]);
-    const int grp = t / L.KG;
-    float k[8];
-    if (grp == open_grp) {
-      const int64_t o = slot * R.s_slot + (int64_t)(t - grp * L.KG) * R.s_pos + h * R.s_head + d0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) k[i] = ld_dt(R.base, R.dtype, o + i);
-    } else {
-      load_codes8(krow, bits, qk);
-      const int64_t ke = ((int64_t)grp * L.H + h) * L.D + d0;
+  const int side_bytes = (L.H * L.D * BITS) / 8;
+  const int lanes_t = cpt < 256 ? 256 / cpt : 1;  // tokens in work at once
+  const int t_off = cpt < 256 ? (int)threadIdx.x / cpt : 0;
+  if (t_off >= lanes_t) return;
+  for (int c = (int)threadIdx.x - t_off * cpt; c < cpt; c += 256) {
+    const int h = c / cph, d0 = (c - h * cph) * 8;
+    const __half* vs_p = reinterpret_cast<const __half*>(page + L.o_vs) + h * L.NG + d0 / L.VG;
+    const __half* vm_p = reinterpret_cast<const __half*>(page + L.o_vm) + h * L.NG + d0 / L.VG;
+    T* ko_p = A.k_out + row0 * A.o_s0 + h * A.o_s1 + d0;
+    T* vo_p = A.v_out + row0 * A.o_s0 + h * A.o_s1 + d0;
+    for (int g0 = t0; g0 < t1;) {  // tokens [g0, g1) share a K group
+      const int grp = g0 / L.KG, g1 = min(t1, (grp + 1) * L.KG);
+      const bool open = grp == open_grp;
+      const int ke = (grp * L.H + h) * L.D + d0;
       const uint4 s8 = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(page + L.o_ks) + ke);
       const uint4 m8 = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(page + L.o_km) + ke);
-      const __half2* sh = reinterpret_cast<const __half2*>(&s8);
-      const __half2* mh = reinterpret_cast<const __half2*>(&m8);
+      for (int tb = g0 + t_off; tb < g1; tb += BATCH * lanes_t) {
+        W kw[BATCH], vw[BATCH];
+        __half vs[BATCH], vm[BATCH];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 sc = __half22float2(sh[i]), mn = __half22float2(mh[i]);
-        k[2 * i] = __fadd_rn(__fmul_rn(qk[2 * i], sc.x), mn.x);
-        k[2 * i + 1] = __fadd_rn(__fmul_rn(qk[2 * i + 1], sc.y), mn.y);
+        for (int b = 0; b < BATCH; ++b) {
+          const int t = min(tb + b * lanes_t, g1 - 1);
+          const uint8_t* krow = A.pages + s_row[t - t0] + c * BITS;  // 8 channels * BITS / 8 bytes per chunk of 8
+          kw[b] = *reinterpret_cast<const W*>(krow);
+          vw[b] = *reinterpret_cast<const W*>(krow + side_bytes);
+          vs[b] = vs_p[t * L.H * L.NG];
+          vm[b] = vm_p[t * L.H * L.NG];
+        }
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b) {
+          const int t = tb + b * lanes_t;
+          if (t >= g1) break;
+          uint4 ko, vo;
+          uint32_t* ki = reinterpret_cast<uint32_t*>(&ko);
+          uint32_t* vi = reinterpret_cast<uint32_t*>(&vo);
+          float2 q[4];
+          if (open) {
+            const int64_t o = slot * A.R.s_slot + (int64_t)(t - grp * L.KG) * A.R.s_pos + h * A.R.s_head + d0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              ki[i] = pack2_rn<T>(ld_dt(A.R.base, A.R.dtype, o + 2 * i), ld_dt(A.R.base, A.R.dtype, o + 2 * i + 1));
+          } else {
+            unpack8<BITS>(kw[b], q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 ks = __half22float2(reinterpret_cast<const __half2*>(&s8)[i]);
+              const float2 km = __half22float2(reinterpret_cast<const __half2*>(&m8)[i]);
+              const float2 k = __fadd2_rn(__fmul2_rn(q[i], ks), km);
+              ki[i] = pack2_rn<T>(k.x, k.y);
+            }
+          }
+          unpack8<BITS>(vw[b], q);
+          const float fs = __half2float(vs[b]), fm = __half2float(vm[b]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 v = __fadd2_rn(__fmul2_rn(q[i], make_float2(fs, fs)), make_float2(fm, fm));
+            vi[i] = pack2_rn<T>(v.x, v.y);
+          }
+          *reinterpret_cast<uint4*>(ko_p + t * A.o_s0) = ko;
+          *reinterpret_cast<uint4*>(vo_p + t * A.o_s0) = vo;
+        }
       }
-    }
-    uint4 ko, vo;
-    uint32_t* kw = reinterpret_cast<uint32_t*>(&ko);
-    uint32_t* vw = reinterpret_cast<uint32_t*>(&vo);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      kw[i] = pack2_rn<T>(k[2 * i], k[2 * i + 1]);
-      vw[i] = pack2_rn<T>(__fadd_rn(__fmul_rn(qv[2 * i], vs), vm), __fadd_rn(__fmul_rn(qv[2 * i + 1], vs), vm));
-    }
-    const int64_t o = (row0 + t) * o_s0 + h * o_s1 + d0;
-    *reinterpret_cast<uint4*>(k_out + o) = ko;
-    *reinterpret_cast<uint4*>(v_out + o) = vo;
-    if (c_step) {
-      c += c_step;
-      if (c >= cpt) { c -= cpt; ++t; }
-      h = c / cph;
-      d0 = (c - h * cph) * 8;
+      g0 = g1;
     }
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) dequant_dense_vec_kernel(const DenseArgs<T> A) {
+  __shared__ int64_t s_row[DENSE_TOK];
+  const LayoutDev& L = A.L;
+  const int item = blockIdx.x / A.slices, t0 = (blockIdx.x - item * A.slices) * DENSE_TOK;
+  const int4 w = reinterpret_cast<const int4*>(A.work)[item];
+  const int req = w.x, bi = w.y, ctx = w.w;
+  const int t1 = min(min(L.BS, ctx - bi * L.BS), t0 + DENSE_TOK);
+  if (t0 >= t1) return;
+  const int64_t blk = A.bt[(int64_t)req * A.bt_s0 + bi];
+  const uint8_t* page = A.pages + blk * L.PS;
+  int bits = page[0];
+  if (bits == 0) bits = 2;  // an unopened block reads as INT2, like the attention kernels
+  const int64_t slot = A.R.block_res[blk];
+  const int open_grp = slot >= 0 ? (int)A.R.res_group[slot] : -1;
+  if (t0 + (int)threadIdx.x < t1) s_row[threadIdx.x] = row_offset(A.pages, L, blk, t0 + threadIdx.x, bits);
+  __syncthreads();
+  if (bits == 4) dense_rows<T, 4>(A, page, w.z, t0, t1, slot, open_grp, s_row);
+  else if (bits == 8) dense_rows<T, 8>(A, page, w.z, t0, t1, slot, open_grp, s_row);
+  else dense_rows<T, 2>(A, page, w.z, t0, t1, slot, open_grp, s_row);
 }
 
 // Demotion, phase 2: requantize a block's dequantized contents (scratch: K then V, float
@@ -313,15 +365,19 @@ int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages,
   dequant_dense_kernel<T><<<(unsigned)n_work, 256, 0, st>>>(L, R, (const uint8_t*)pages->base, work, block_table, \
                                                            bt_s0, (T*)k_out, (T*)v_out, out_s0, out_s1)
   // 16-byte loads and stores need the stat arrays, the rows of the outputs and 8-channel chunks aligned
-  const bool vec = out_dtype != ECHOKV_DT_F32 && L.BS <= DENSE_MAX_BS && L.D % 8 == 0 && L.VG % 8 == 0 &&
+  const int slices = (L.BS + DENSE_TOK - 1) / DENSE_TOK;
+  const bool vec = out_dtype != ECHOKV_DT_F32 && n_work * slices < (1ll << 31) && L.D % 8 == 0 && L.VG % 8 == 0 &&
                    ((L.o_ks | L.o_km | L.PS | L.o_data | L.CB) % 16) == 0 && (out_s0 % 8) == 0 && (out_s1 % 8) == 0 &&
                    ((reinterpret_cast<uintptr_t>(k_out) | reinterpret_cast<uintptr_t>(v_out) |
                      reinterpret_cast<uintptr_t>(pages->base) | reinterpret_cast<uintptr_t>(work)) % 16) == 0;
-#define LAUNCH_VEC(T)                                                                                              \
-  dequant_dense_vec_kernel<T><<<(unsigned)n_work, 256, 0, st>>>(L, R, (const uint8_t*)pages->base, work, block_table, \
-                                                               bt_s0, (T*)k_out, (T*)v_out, out_s0, out_s1)
+#define LAUNCH_VEC(T)                                                                                         \
+  {                                                                                                           \
+    DenseArgs<T> A = {L, R, (const uint8_t*)pages->base, work, block_table, bt_s0, (T*)k_out, (T*)v_out, out_s0, \
+                      out_s1, slices};                                                                        \
+    dequant_dense_vec_kernel<T><<<(unsigned)(n_work * slices), 256, 0, st>>>(A);                              \
+  }
   if (vec) {
-    if (out_dtype == ECHOKV_DT_F16) LAUNCH_VEC(__half); else LAUNCH_VEC(__nv_bfloat16);
+    if (out_dtype == ECHOKV_DT_F16) LAUNCH_VEC(__half) else LAUNCH_VEC(__nv_bfloat16)
     return check_launch("dequant_dense");
   }
 #undef LAUNCH_VEC
