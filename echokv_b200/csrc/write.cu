@@ -120,6 +120,16 @@ struct MinMax8 {
       }
     }
   }
+  __device__ __forceinline__ void merge(const MinMax8& o) {
+    using P = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const P a = __hmin2(*reinterpret_cast<const P*>(&mn[k]), *reinterpret_cast<const P*>(&o.mn[k]));
+      const P b = __hmax2(*reinterpret_cast<const P*>(&mx[k]), *reinterpret_cast<const P*>(&o.mx[k]));
+      mn[k] = *reinterpret_cast<const uint32_t*>(&a);
+      mx[k] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+  }
   __device__ __forceinline__ void finish(float (&lo)[8], float (&hi)[8]) const {
     cvt8<T>(make_uint4(mn[0], mn[1], mn[2], mn[3]), lo);
     cvt8<T>(make_uint4(mx[0], mx[1], mx[2], mx[3]), hi);
@@ -237,37 +247,68 @@ __device__ __forceinline__ void key_chunk(const TokArgs<T>& A, int64_t row, int 
   }
 }
 
-// One token row.  `row_in_cta`: row index this CTA / warp works on; `skip_residual`: the row's open-group key is
-// stored by someone else (see write_step_kernel).
+// Where a token row goes: everything the plan and the page headers say about it.
+struct RowMeta {
+  int64_t slot, blk, rowoff, rslot, kidx;
+  int off, bits;
+  bool sealed;
+};
+template <typename T>
+__device__ __forceinline__ RowMeta row_meta(const TokArgs<T>& A, int64_t row) {
+  const LayoutDev& L = A.L;
+  const Shifts sh = A.sh;
+  RowMeta m;
+  m.slot = A.tok[row];
+  m.rslot = A.tok[A.tok_s0 + row];
+  m.sealed = A.tok[2 * A.tok_s0 + row] != 0;
+  m.kidx = A.kref ? A.tok[3 * A.tok_s0 + row] : -1;
+  m.blk = sh.BS >= 0 ? m.slot >> sh.BS : m.slot / L.BS;
+  m.off = (int)(m.slot - m.blk * L.BS);
+  m.bits = block_bits(A.pages, L, m.blk);
+  RowWalk walk;
+  walk.start(A.pages, L, sh.BS, m.blk, m.off, m.bits);
+  m.rowoff = walk.offset();
+  return m;
+}
+
+// The 8 channels of a row's value and key that a thread works on first, as loaded (16-bit rows on 16-byte boundaries).
+struct RowRaw {
+  uint4 v, k;
+  bool on;
+  template <typename T>
+  __device__ __forceinline__ void load(const TokArgs<T>& A, int64_t row) {
+    const int c = threadIdx.x;
+    on = sizeof(T) == 2 && A.vec_in && c < (A.L.H * A.L.D) / 8;
+    v = k = make_uint4(0, 0, 0, 0);
+    if (on) {
+      const int h = qdiv(c * 8, A.L.D, A.sh.D), d0 = qmod(c * 8, A.L.D, A.sh.D);
+      v = *reinterpret_cast<const uint4*>(A.value + row * A.v_s0 + h * A.v_s1 + d0);
+      k = *reinterpret_cast<const uint4*>(A.key + row * A.k_s0 + h * A.k_s1 + d0);
+    }
+  }
+};
+
+// One token row that is stored (its slot is not negative).  `skip_residual`: the row's open-group key is stored by
+// someone else (see write_step_kernel).
 template <typename T, int MODE>
-__device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, bool skip_residual) {
+__device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, const RowMeta& M, const RowRaw& raw, bool skip_residual) {
   const LayoutDev& L = A.L;
   uint8_t* __restrict__ pages = A.pages;
-  const T* __restrict__ key = A.key;
   const T* __restrict__ value = A.value;
-  const int64_t* __restrict__ tok = A.tok;
-  const int64_t k_s0 = A.k_s0, k_s1 = A.k_s1, v_s0 = A.v_s0, v_s1 = A.v_s1, tok_s0 = A.tok_s0;
-  void* res = A.res;
-  const int res_dt = A.res_dt;
-  const int64_t r_s0 = A.r_s0, r_s1 = A.r_s1, r_s2 = A.r_s2, kref_s0 = A.kref_s0, kref_s1 = A.kref_s1;
-  float* __restrict__ kref = A.kref;
-  const bool vec_in = A.vec_in, res_raw = A.res_raw, kref_vec = A.kref_vec;
+  const int64_t v_s0 = A.v_s0, v_s1 = A.v_s1;
+  const bool vec_in = A.vec_in;
   const Shifts sh = A.sh;
   const int lane = threadIdx.x & 31;
-  const int64_t slot = tok[row];
-  if (slot < 0) return;  // padding, or a token that is not stored
-  const int64_t blk = sh.BS >= 0 ? slot >> sh.BS : slot / L.BS;
-  const int off = (int)(slot - blk * L.BS);
-  const int bits = block_bits(pages, L, blk);
+  const int off = M.off, bits = M.bits;
   const float levels = (float)((1 << bits) - 1);
-  RowWalk walk;
-  walk.start(pages, L, sh.BS, blk, off, bits);
-  const int64_t rowoff = walk.offset();
+  const int64_t rowoff = M.rowoff;
   const int side_bytes = (L.H * L.D * bits) / 8;
   const int head_bytes = (L.D * bits) / 8;
-  uint8_t* page = pages + blk * L.PS;
+  uint8_t* page = pages + M.blk * L.PS;
   const int units = (L.H * L.D) / 8;  // 8-channel pieces of a row
   const int first = MODE == 2 ? threadIdx.x : lane, step = MODE == 2 ? WT_WARPS * 32 : 32;
+  int64_t rslot = skip_residual ? -1 : M.rslot;
+  const bool key_early = MODE == 2 && rslot >= 0 && A.res_raw && A.vec_in && units <= step;  // the whole key row is in `raw`
 
   if constexpr (MODE != 0) {
     // V: per token, groups of VG along head_dim; VG / 8 neighbouring threads share a group.
@@ -279,7 +320,11 @@ __device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, bool
       float x[8];
       float mn = INFINITY, mx = -INFINITY;
       if (on) {
-        ld8<T>(value, row * v_s0 + h * v_s1 + d0, vec_in, x);
+        bool have = false;
+        if constexpr (MODE == 2 && sizeof(T) == 2) {
+          if (raw.on && u == first) { cvt8<T>(raw.v, x); have = true; }
+        }
+        if (!have) ld8<T>(value, row * v_s0 + h * v_s1 + d0, vec_in, x);
 #pragma unroll
         for (int k = 0; k < 8; ++k) { mn = fminf(mn, x[k]); mx = fmaxf(mx, x[k]); }
       }
@@ -327,11 +372,16 @@ __device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, bool
   }
 
   // K: residual row (open group), codes under stored stats (sealed group), K_ref ring row.
-  const int64_t rslot = skip_residual ? -1 : tok[tok_s0 + row];
-  const bool sealed = tok[2 * tok_s0 + row] != 0;
-  const int64_t kidx = kref ? tok[3 * tok_s0 + row] : -1;
-  if (rslot < 0 && !sealed && kidx < 0) return;
-  for (int c = first; c < units; c += step) key_chunk<T>(A, row, c, off, bits, rowoff, rslot, sealed, kidx);
+  if (key_early) {
+    if (raw.on) {
+      const int h = qdiv(first * 8, L.D, sh.D), d0 = qmod(first * 8, L.D, sh.D);
+      const int64_t ro = rslot * A.r_s0 + (int64_t)qmod(off, L.KG, sh.KG) * A.r_s1 + h * A.r_s2 + d0;
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(A.res) + ro) = raw.k;
+    }
+    rslot = -1;
+  }
+  if (rslot < 0 && !M.sealed && M.kidx < 0) return;
+  for (int c = first; c < units; c += step) key_chunk<T>(A, row, c, off, bits, rowoff, rslot, M.sealed, M.kidx);
 }
 
 // Many token rows, one thread per (row, KV head, group of 32 channels): the V group's 64 bytes are loaded once,
@@ -407,8 +457,11 @@ __global__ void __launch_bounds__(128, 8) write_tokens_bulk_kernel(const TokArgs
 template <typename T, int MODE>
 __global__ void __launch_bounds__(WT_WARPS * 32) write_tokens_kernel(const TokArgs<T> A) {
   const int64_t row = MODE == 2 ? (int64_t)blockIdx.x : blockIdx.x * (int64_t)WT_WARPS + (threadIdx.x >> 5);
-  if (row >= A.n_rows) return;
-  token_row<T, MODE>(A, row, false);
+  if (row >= A.n_rows || A.tok[row] < 0) return;  // past the end, padding, or a token that is not stored
+  RowRaw raw;
+  raw.on = false;
+  if constexpr (MODE == 2) raw.load<T>(A, row);
+  token_row<T, MODE>(A, row, row_meta<T>(A, row), raw, false);
 }
 
 // One CTA per completed K group; each thread owns 8 channels of one head over the KG tokens
@@ -551,6 +604,152 @@ __global__ void __launch_bounds__(256, 4) finalize_k_kernel(const FinArgs<T> A) 
   finalize_group<T, SEAL>(A, blockIdx.x);
 }
 
+// The same for the usual group sizes and 16-bit rows as loaded (raw16): a group's channels are spread over `parts`
+// CTAs of 128 threads and its tokens over SL neighbouring lanes, TPL tokens each, so that a thread has all its rows
+// in flight at once and keeps them in registers between the statistics and the codes.
+//
+// A group is KG * H * D * 2 bytes in and a quarter to a half of that out, far below what a launch costs: the time is
+// the chain list -> rows -> statistics -> codes, and with a thread walking all KG tokens twice (finalize_group) that
+// chain had 2 KG loads in a row.  350 groups of 32 x 8 heads x 128: 20 us, 24 us before; in a decode step see
+// write_step_kernel.
+template <typename T> struct SplitArgs { int n_take; const int* take; const TokArgs<T>* tok; };
+
+template <typename T, int SL, int TPL>
+__device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
+  const LayoutDev& L = A.L;
+  const Shifts sh = A.sh;
+  const int64_t* line = A.fin + f * (3 + L.KG);
+  const int64_t blk = line[0], rs = max(line[2], (int64_t)0);
+  const int grp = (int)line[1];
+  const int sub = threadIdx.x % SL, per = blockDim.x / SL;  // token lane, 8-channel pieces at a time
+  int rows[TPL];
+#pragma unroll
+  for (int i = 0; i < TPL; ++i) rows[i] = (int)line[3 + sub + SL * i];
+  uint8_t* page = A.pages + blk * L.PS;
+  const uint4 hd = *reinterpret_cast<const uint4*>(page);
+  const int bits = (hd.x & 0xff) == 0 ? 2 : (int)(hd.x & 0xff);
+  const float levels = (float)((1 << bits) - 1);
+  const int row_bytes = (2 * L.H * L.D * bits) / 8;
+  int64_t dst_row[TPL];  // byte offsets of this lane's token rows from the pool base
+#pragma unroll
+  for (int i = 0; i < TPL; ++i) {
+    const int t = grp * L.KG + sub + SL * i, sh_bits = bits == 2 ? 1 : (bits == 4 ? 2 : 3);
+    const int tpc = (2 * L.BS) >> sh_bits, j = qdiv(t, tpc, sh.BS >= 0 ? sh.BS + 1 - sh_bits : -1);
+    int64_t pg = blk, slot = 0;
+    if (j > 0) {
+      const int id = j == 1 ? (int)hd.y : (j == 2 ? (int)hd.z : (int)hd.w);
+      pg = id / L.KC;
+      slot = id - pg * L.KC;
+    }
+    dst_row[i] = pg * L.PS + L.o_data + slot * L.CB + (int64_t)(t - j * tpc) * row_bytes;
+  }
+  const int units = (L.H * L.D) / 8;
+  for (int base = part * per; base < units; base += parts * per) {
+    const int u = base + threadIdx.x / SL;
+    const bool on = u < units;
+    const int c = on ? u : 0;
+    const int h = qdiv(c * 8, L.D, sh.D), d0 = qmod(c * 8, L.D, sh.D);
+    const T* kcol = A.key + (h * A.k_s1 + d0);
+    const T* rcol = reinterpret_cast<const T*>(A.res) + (rs * A.r_s0 + h * A.r_s2 + d0);
+    uint4 raw[TPL];
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) {
+      const T* src = rows[i] >= 0 ? kcol + (int64_t)rows[i] * (int)A.k_s0 : rcol + (int64_t)(sub + SL * i) * (int)A.r_s1;
+      raw[i] = *reinterpret_cast<const uint4*>(src);
+    }
+    MinMax8<T> acc;
+    acc.init();
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) acc.update(raw[i]);
+#pragma unroll
+    for (int o = 1; o < SL; o <<= 1) {
+      MinMax8<T> other;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        other.mn[k] = __shfl_xor_sync(0xffffffffu, acc.mn[k], o);
+        other.mx[k] = __shfl_xor_sync(0xffffffffu, acc.mx[k], o);
+      }
+      acc.merge(other);
+    }
+    float mn[8], mx[8];
+    acc.finish(mn, mx);
+    // The SL lanes hold the same minima and maxima: each works out the statistics of 8 / SL channels for all.
+    constexpr int CH = 8 / SL;
+    uint32_t own[CH];  // scale, min as fp16 pair
+    float own_r[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      float lo = mn[i], hi = mx[i];
+#pragma unroll
+      for (int l = 1; l < SL; ++l) {
+        if (sub == l) { lo = mn[l * CH + i]; hi = mx[l * CH + i]; }
+      }
+      __half s, z;
+      group_stats(lo, hi, levels, s, z);
+      own[i] = (uint32_t)__half_as_ushort(s) | ((uint32_t)__half_as_ushort(z) << 16);
+      own_r[i] = __frcp_rn(__half2float(s));
+    }
+    __align__(16) __half s16[8], m16[8];
+    float sc[8], m[8], rsc[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int from = (threadIdx.x & 31 & ~(SL - 1)) + k / CH;
+      const uint32_t sm = __shfl_sync(0xffffffffu, own[k % CH], from);
+      rsc[k] = __shfl_sync(0xffffffffu, own_r[k % CH], from);
+      s16[k] = __ushort_as_half((unsigned short)(sm & 0xffff));
+      m16[k] = __ushort_as_half((unsigned short)(sm >> 16));
+      sc[k] = __half2float(s16[k]); m[k] = __half2float(m16[k]);
+    }
+    if (!on) continue;
+    if (sub == 0) {
+      const int e = (grp * L.H + h) * L.D + d0;
+      *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(page + L.o_ks) + e) = *reinterpret_cast<uint4*>(s16);
+      *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(page + L.o_km) + e) = *reinterpret_cast<uint4*>(m16);
+    }
+    uint8_t* col = A.pages + h * ((L.D * bits) / 8) + (d0 * bits) / 8;
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) {
+      float x[8];
+      cvt8<T>(raw[i], x);
+      quant_store8<true>(bits, col + dst_row[i], x, m, sc, rsc);
+    }
+    // Keys of a group that takes the slot over (write_step_kernel): every lane of these channels has its rows in registers.
+    for (int i = sub; i < S.n_take; i += SL) {
+      const TokArgs<T>& TA = *S.tok;
+      const int64_t row = S.take[i], tslot = TA.tok[row];
+      const int off = (int)(tslot - (sh.BS >= 0 ? tslot >> sh.BS : tslot / L.BS) * L.BS);
+      const int64_t ro = rs * A.r_s0 + (int64_t)qmod(off, L.KG, sh.KG) * A.r_s1 + h * A.r_s2 + d0;
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(TA.res) + ro) =
+          *reinterpret_cast<const uint4*>(TA.key + row * TA.k_s0 + h * TA.k_s1 + d0);
+    }
+  }
+}
+// The group sizes finalize_split is instantiated for (split_group_ok says which).
+template <typename T>
+__device__ __forceinline__ void finalize_split_any(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
+  if constexpr (sizeof(T) == 2) {
+    if (A.L.KG == 16) finalize_split<T, 4, 4>(A, f, part, parts, S);
+    else if (A.L.KG == 32) finalize_split<T, 8, 4>(A, f, part, parts, S);
+    else finalize_split<T, 8, 8>(A, f, part, parts, S);
+  }
+}
+static bool split_group_ok(const LayoutDev& L, bool raw16) { return raw16 && (L.KG == 16 || L.KG == 32 || L.KG == 64); }
+// CTAs per group: as many as the group's pieces fill, while the launch stays within about one round of the chip
+// (a captured step launches a group per row, and nearly all of them have nothing to do).
+static int split_parts(const LayoutDev& L, int64_t n_groups) {
+  const int per = 128 / (L.KG == 16 ? 4 : 8), need = (L.H * L.D / 8 + per - 1) / per;
+  const int64_t room = 1024 / (n_groups > 0 ? n_groups : 1);
+  return room < 1 ? 1 : (room < need ? (int)room : need);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(WT_WARPS * 32) finalize_split_kernel(const FinArgs<T> A, int parts) {
+  const int64_t f = blockIdx.x / parts;
+  if (f >= *A.fin_count) return;
+  const SplitArgs<T> none = {0, nullptr, nullptr};
+  finalize_split_any<T>(A, f, (int)(blockIdx.x - f * parts), parts, none);
+}
+
 // A step's writes of one layer in one launch: CTAs [0, n_rows) store the token rows, the next n_fin_launch CTAs
 // quantize the completed K groups (masked by the device-side count), the rest copy `stash_n` rows of `stash_src`
 // (the canary's query rows) to `stash_dst`.  Run one after the other, the group pass comes first because a
@@ -564,31 +763,38 @@ struct StashArgs {
 };
 constexpr int STEP_MAX_ROWS = 1024;
 
+//
+// A step's rows are a few hundred kilobytes: the time is the chain of dependent reads (token list -> page header ->
+// rows -> statistics -> codes), so a row's value and key are on their way while the header is looked up, and a
+// group's tokens are spread over lanes and CTAs (finalize_split).  Per layer: 12.4 -> 6.3 us at 64 sequences x 8 heads, 10.1 -> 5.6 us
+// at 16 sequences x 1 head, 20 -> 10 us at 575 rows.
 template <typename T>
 __global__ void __launch_bounds__(WT_WARPS * 32)
-write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, const StashArgs SA) {
+write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, int parts, const StashArgs SA) {
   __shared__ int take[STEP_MAX_ROWS];
   __shared__ int n_take;
   pdl_launch_dependents();
   pdl_wait();
   const LayoutDev& L = TA.L;
-  const int64_t b = blockIdx.x;
+  const int64_t b = blockIdx.x, n_fin_ctas = n_fin_launch * max(parts, 1);
   const int w = 3 + L.KG;
   if (b < TA.n_rows) {
     if (TA.tok[b] < 0) return;  // padding, or a token that is not stored
-    const int64_t rslot = TA.tok[TA.tok_s0 + b];
+    RowRaw raw;
+    raw.load<T>(TA, b);
+    const RowMeta M = row_meta<T>(TA, b);
     bool skip = false;
-    if (rslot >= 0) {
+    if (M.rslot >= 0) {
       const int64_t n_fin = n_fin_launch > 0 ? min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
       int hit = 0;
-      for (int64_t f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[f * w + 2] == rslot;
+      for (int64_t f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[f * w + 2] == M.rslot;
       skip = __syncthreads_or(hit) != 0;
     }
-    token_row<T, 2>(TA, b, skip);
+    token_row<T, 2>(TA, b, M, raw, skip);
     return;
   }
-  if (b < TA.n_rows + n_fin_launch) {
-    const int64_t f = b - TA.n_rows;
+  if (b < TA.n_rows + n_fin_ctas) {
+    const int64_t g = b - TA.n_rows, f = parts > 0 ? g / parts : g;
     if (f >= *FA.fin_count) return;
     const int64_t slot = FA.fin[f * w + 2];
     if (threadIdx.x == 0) n_take = 0;
@@ -598,6 +804,11 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
         if (TA.tok[r] >= 0 && TA.tok[TA.tok_s0 + r] == slot) take[atomicAdd(&n_take, 1)] = r;
     }
     __syncthreads();
+    if (parts > 0) {
+      const SplitArgs<T> S = {n_take, take, &TA};
+      finalize_split_any<T>(FA, f, (int)(g - f * parts), parts, S);
+      return;
+    }
     finalize_group<T, false>(FA, f);
     // Keys of the group that takes the slot over: each thread stores the channels it has just read for the last time.
     const int units = (L.H * L.D) / 8;
@@ -622,7 +833,7 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
     }
     return;
   }
-  const int64_t i = (b - TA.n_rows - n_fin_launch) * blockDim.x + threadIdx.x;
+  const int64_t i = (b - TA.n_rows - n_fin_ctas) * blockDim.x + threadIdx.x;
   if (i >= SA.n * SA.row16) return;
   const int64_t r = i / SA.row16;
   SA.dst[i] = SA.src[SA.rows[r] * SA.src_stride16 + (i - r * SA.row16)];
@@ -777,9 +988,15 @@ int echokv_finalize_k(const echokv_layout* layout, const echokv_pages* pages, co
   if (rc) return rc;
   if (!key || !fin || !fin_count) return set_error(ECHOKV_E_ARGUMENT, "finalize_k: null pointer");
   const int threads = (L.H * L.D / 8) < 256 ? ((L.H * L.D / 8 + 31) / 32 * 32) : 256;
+  const int parts = split_parts(L, n_launch);
   cudaStream_t st = (cudaStream_t)stream;
-#define LAUNCH(T) \
-  finalize_k_kernel<T, false><<<(unsigned)n_launch, threads, 0, st>>>(fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count))
+#define LAUNCH(T)                                                                                              \
+  {                                                                                                            \
+    const FinArgs<T> A = fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count);                            \
+    if (split_group_ok(L, A.raw16))                                                                            \
+      finalize_split_kernel<T><<<(unsigned)(n_launch * parts), WT_WARPS * 32, 0, st>>>(A, parts);              \
+    else finalize_k_kernel<T, false><<<(unsigned)n_launch, threads, 0, st>>>(A);                               \
+  }
   switch (kv_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;
     case ECHOKV_DT_F16: LAUNCH(__half); break;
@@ -843,12 +1060,16 @@ int echokv_write_step(const echokv_layout* layout, const echokv_pages* pages, co
   SA.src = (const uint4*)stash_src; SA.src_stride16 = stash_src_row_stride_bytes / 16; SA.rows = stash_rows;
   SA.n = stash_n; SA.dst = (uint4*)stash_dst; SA.row16 = (int)(stash_row_bytes / 16);
   const int64_t stash_ctas = (stash_n * SA.row16 + WT_WARPS * 32 - 1) / (WT_WARPS * 32);
-  const unsigned grid = (unsigned)(n_rows + n_fin_launch + stash_ctas);
   cudaStream_t st = (cudaStream_t)stream;
 #define LAUNCH(T)                                                                                                  \
-  launch_pdl(write_step_kernel<T>, dim3(grid), dim3(WT_WARPS * 32), 0, st,                                         \
-             tok_args<T>(L, pages, R, key, k_s0, k_s1, value, v_s0, v_s1, tok, tok_s0, kref, kref_s0, kref_s1, n_rows), \
-             fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count), n_fin_launch, SA)
+  {                                                                                                                \
+    const TokArgs<T> TA = tok_args<T>(L, pages, R, key, k_s0, k_s1, value, v_s0, v_s1, tok, tok_s0, kref, kref_s0, \
+                                      kref_s1, n_rows);                                                            \
+    const FinArgs<T> FA = fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count);                               \
+    const int parts = split_group_ok(L, FA.raw16 && TA.res_raw) ? split_parts(L, n_fin_launch) : 0;                \
+    const unsigned grid = (unsigned)(n_rows + n_fin_launch * (parts > 0 ? parts : 1) + stash_ctas);                \
+    launch_pdl(write_step_kernel<T>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin_launch, parts, SA);     \
+  }
   switch (kv_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;
     case ECHOKV_DT_F16: LAUNCH(__half); break;
