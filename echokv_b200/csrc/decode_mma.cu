@@ -73,6 +73,7 @@ struct alignas(16) TilePlan {
   const unsigned char* run[4];      // the tile's token rows lie in up to four runs (one per chunk it touches) of `TILE >> run_shift` rows
 };
 constexpr int UNIT = 16;         // tiles planned at a time (one per producer lane)
+constexpr int PREFETCH_TILES = 4;  // tiles a team brings into L2 while it waits for the kernel before (27 MB over all teams at most)
 constexpr int MAX_NS = 8;        // stage ring slots at most
 constexpr int HDR_BYTES = 256;   // 2 * MAX_NS mbarriers
 static_assert(sizeof(StageHeader) == 32 && sizeof(TilePlan) % 16 == 0, "16-byte copies of headers");
@@ -848,7 +849,9 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
   const int team = threadIdx.x / TEAM_THREADS, tid = threadIdx.x - team * TEAM_THREADS;
   const int warp = tid >> 5, lane = tid & 31;
   const int NS = P.NS;
-  const int n_items = P.num_seqs * A.num_splits;
+  // A team's first work item: consecutive items go to different SMs, so that a step with fewer items than teams has one
+  // team (half the contention for issue slots) per SM; the counter hands out the items after the first round.
+  const int item0 = blockIdx.x + gridDim.x * team;
   constexpr int SB = stage_bytes(H);
 #ifdef ECHOKV_PROFILE
   const unsigned long long cta_t0 = global_ns();
@@ -908,27 +911,35 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     int64_t seq_len = 0, bt_row = 0;
     bool have = false;
     const int bps_min = bps_floor(A);
-    // A team's first work item is its own index; the counter (which the merge kernel before this one may still be
-    // resetting when this runs ahead of `pdl_wait`) hands out the items after the first round.
     const int n_teams = gridDim.x * V;
-    bool first_claim = true;
+    // Items exist up to the longest sequence's split count: the grid of splits is sized for the longest sequence a step may
+    // ever have, and claiming its empty rest one atomic after the other held up every team's last item (64 splits in
+    // the grid, 9 in use: a dozen round trips per team).
+    int used_max = 0;
+    for (int i = lane; i < P.num_seqs; i += 32) {
+      const int nb = (int)((A.lens[i] + L.BS - 1) / L.BS), bps = max(bps_min, (nb + A.num_splits - 1) / A.num_splits);
+      used_max = max(used_max, (nb + bps - 1) / bps);
+    }
+    const int n_items = P.num_seqs * __reduce_max_sync(0xffffffffu, used_max);
     auto advance = [&]() {  // move to the next unit (claiming a new item when needed); false when there is no work left
       if (have && base + U < b_end) { base += U; return true; }
       for (;;) {
         int it = 0;
-        if (first_claim) {
-          it = blockIdx.x * V + team;
-          first_claim = false;
-        } else {
-          if (lane == 0) it = atomicAdd(P.counter, 1);
-          it = __shfl_sync(0xffffffffu, it, 0) + n_teams;
-        }
+        if (lane == 0) it = atomicAdd(P.counter, 1);
+        it = __shfl_sync(0xffffffffu, it, 0) + n_teams;
         if (it >= n_items) { have = false; return false; }
         if (item_range(P, bps_min, it, seq, split, seq_len, b_start, b_end)) {
           base = b_start; bt_row = A.bt_rows ? A.bt_rows[seq] : seq; have = true;
           return true;
         }
       }
+    };
+    // The dependency wait comes as late as it can: the first unit is planned and its first stage prepared ahead of it,
+    // down to the copies themselves, which read pages that the write step before this kernel may still be storing to.
+    // (The work counter, which the merge kernel before may still be resetting, is not touched before it either.)
+    bool waited = false;
+    auto wait_once = [&]() {
+      if (!waited) { pdl_wait(); waited = true; }
     };
     // Fill one stage: wait until the consumers have released it, write the header, start the copies.
     // `rows`: 1 = a whole INT4 / INT2 tile (token rows in pairs, all stats); 2 / 3 = the first / second half of an INT8
@@ -986,6 +997,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         mbar_expect_tx(bar, tx);
       }
       __syncwarp();
+      wait_once();
       if (c_bytes) bulk_copy(st_u + c_dst, c_src, c_bytes, bar, policy);
       ++fills;
       st = ring_next(st, NS);
@@ -1046,21 +1058,29 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         mbar_expect_tx(bar, tx);
       }
       __syncwarp();
+      wait_once();
       if (c_bytes) bulk_copy(st_u + c_dst, c_src, c_bytes, bar, policy);
       fills += 2;
       st = ring_next(stB, NS);
       return true;
     };
-    bool more = P.idle_producer ? false : advance();
+    // The first item may be empty (a short sequence's last split): then its successor comes from the counter.
+    bool more = false;
+    if (!P.idle_producer) {
+      if (item0 < n_items && item_range(P, bps_min, item0, seq, split, seq_len, b_start, b_end)) {
+        base = b_start; bt_row = A.bt_rows ? A.bt_rows[seq] : seq; have = true;
+        more = true;
+      } else {
+        wait_once();
+        more = advance();
+      }
+    }
     BlockMeta nxt = more ? load_meta(P, bt_row, lane < U ? base + lane : b_end, b_end) : BlockMeta{};
-    pdl_wait();  // pages and the work counter are final from here on
     while (more && ok) {
       const BlockMeta cur = nxt;
       const int u_base = base, u_end = b_end, u_seq = seq, u_split = split;
       const bool u_first = base == b_start, u_last = base + U >= b_end;
       const int64_t u_len = seq_len;
-      more = advance();
-      if (more) nxt = load_meta(P, bt_row, lane < U ? base + lane : b_end, b_end);
       const int nb = min(U, u_end - u_base);
       // tokens of the unit: all blocks are full except possibly the item's last one
       const int unit_tok = (int)min((int64_t)nb * L.BS, u_len - (int64_t)u_base * L.BS);
@@ -1108,7 +1128,30 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         pair_ok = __ballot_sync(0xffffffffu, can_pair);
         __syncwarp();
       }
-      for (int ti = 0; ti < unit_tiles && ok; ++ti) {
+      if (!waited) {
+        // Until then the unit's first tiles come into L2 (a prefetch is no read: a line stored to afterwards is updated
+        // there), which also takes the address translations of scattered pages off the first copies' path.
+        if (lane < min(unit_tiles, PREFETCH_TILES)) {
+          const TilePlan& d = plan[lane];
+          const int rows = min(TILE, (2 * L.BS) / d.hdr.bits);  // token rows per run
+          for (int rr = 0; rr < TILE / rows && rr * rows < d.hdr.n_valid; ++rr)
+            l2_prefetch(d.run[rr], (uint32_t)min(rows, d.hdr.n_valid - rr * rows) * 32u * H * d.hdr.bits);
+          l2_prefetch(d.stats[0], TILE * H * NG * 2);
+          l2_prefetch(d.stats[1], TILE * H * NG * 2);
+          l2_prefetch(d.stats[2], H * D * 2);
+          l2_prefetch(d.stats[3], H * D * 2);
+        }
+      }
+      // The next unit is claimed and its metadata requested (a chain of dependent reads) once this unit's first groups
+      // fill the ring, not before.
+      bool claimed = false;
+      auto claim_next = [&]() {
+        claimed = true;
+        more = advance();
+        if (more) nxt = load_meta(P, bt_row, lane < U ? base + lane : b_end, b_end);
+      };
+      for (int ti = 0, filled = 0; ti < unit_tiles && ok; ++ti, ++filled) {
+        if (filled == 2) claim_next();
         const TilePlan& d = plan[ti];
         const int bits = d.hdr.bits;
         if (bits == 8) {  // two stages: K side with the K stats, then V side with the V stats
@@ -1120,9 +1163,11 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
           ok = fill(d, 0, 1);
         }
       }
+      if (!claimed && ok) claim_next();
       __syncwarp();  // every lane is done reading the plans before the next unit overwrites them
       ok = !__any_sync(0xffffffffu, !ok);
     }
+    wait_once();
     if (ok && !P.idle_producer) {  // no more work: tell the consumers
       if (mbar_wait(empty_u + st * 8, (pph >> st) & 1, P.wait_ns)) {
         if (lane == 0) {
@@ -1231,8 +1276,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // resolves the item's blocks and the first copies are in flight.
     int preloaded = -1;
     {
-      const int item0 = blockIdx.x * V + team;
-      if (item0 < n_items) {
+      if (item0 < P.num_seqs * A.num_splits) {
         seq = item0 % P.num_seqs;
         load_queries();
         preloaded = seq;
@@ -1460,7 +1504,7 @@ int launch_decode_mma(const LayoutDev& L, const ResidualDev& R, const uint8_t* p
   const int smem_bytes = CTA_SHARED_BYTES + P.team_bytes * V;
   const int64_t n_items = num_seqs * (int64_t)A.num_splits;
   int64_t grid = dv->num_sms;
-  if (grid * V > n_items) grid = (n_items + V - 1) / V;
+  if (grid > n_items) grid = n_items;
   // The merge kernel leaves the counter at zero for the next call; a caller that cannot promise a zeroed state
   // gets it zeroed here.
   if (zero_counter && cudaMemsetAsync(counter, 0, sizeof(int), st) != cudaSuccess) return check_launch("decode (work counter)");
