@@ -52,6 +52,8 @@ struct Args {
   const int32_t* chunks;  // [n, 4]: q_start, q_end, ctx, dense_start
   int64_t q_s0, q_s1, kv_s0, kv_s1, o_s0, o_s1;
   int gqa, out_dtype, is_bf16;
+  int out_vec;   // output rows lie on 16-byte boundaries
+  int n_chunks;  // wide kernel: chunks in the table
   float scale_log2;
   int* status;
 };
@@ -144,6 +146,38 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi, bool bf16) {
   if (bf16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
+}
+
+// 32 consecutive channels of one output row, as 16-byte stores where the rows lie on 16-byte boundaries (a row belongs
+// to one thread, so a warp's store touches 32 rows: 4-byte stores made 64 instructions of 32 sectors each per row).
+__device__ __forceinline__ void store_out32(const Args& A, int64_t e, const float (&o)[32], float inv) {
+  if (A.out_dtype == ECHOKV_DT_F32) {
+    float* dst = reinterpret_cast<float*>(A.out) + e;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      if (A.out_vec) {
+        *reinterpret_cast<float4*>(dst + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
+      } else {
+        *reinterpret_cast<float2*>(dst + j) = make_float2(o[j] * inv, o[j + 1] * inv);
+        *reinterpret_cast<float2*>(dst + j + 2) = make_float2(o[j + 2] * inv, o[j + 3] * inv);
+      }
+    }
+  } else {
+    const bool bf16 = A.out_dtype == ECHOKV_DT_BF16;
+    uint16_t* dst = reinterpret_cast<uint16_t*>(A.out) + e;
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w[k] = pack16(o[j + 2 * k] * inv, o[j + 2 * k + 1] * inv, bf16);
+      if (A.out_vec) {
+        *reinterpret_cast<uint4*>(dst + j) = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint32_t*>(dst + j + 2 * k) = w[k];
+      }
+    }
+  }
 }
 
 __global__ void __launch_bounds__(UM, 2) prefill_umma_kernel(Args A) {
@@ -323,16 +357,7 @@ __global__ void __launch_bounds__(UM, 2) prefill_umma_kernel(Args A) {
       float o[32];
       tmem_ld32(t_row + O_COL + c0, o);
       if (live) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float x0 = o[j] * inv, x1 = o[j + 1] * inv;
-          const int d = c0 + j;
-          if (A.out_dtype == ECHOKV_DT_F32) {
-            *reinterpret_cast<float2*>(reinterpret_cast<float*>(A.out) + base_o + d) = make_float2(x0, x1);
-          } else {
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(A.out) + base_o + d) = pack16(x0, x1, A.out_dtype == ECHOKV_DT_BF16);
-          }
-        }
+        store_out32(A, base_o + c0, o, inv);
       }
     }
   }
@@ -630,16 +655,7 @@ __global__ void __launch_bounds__(UM * G + (TMA ? 64 : 32), 1) prefill_umma_pipe
         float o[32];
         tmem_ld32(t_row + O_COL + c0, o);
         if (live) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float x0 = o[j] * inv, x1 = o[j + 1] * inv;
-            const int d = c0 + j;
-            if (A.out_dtype == ECHOKV_DT_F32) {
-              *reinterpret_cast<float2*>(reinterpret_cast<float*>(A.out) + base_o + d) = make_float2(x0, x1);
-            } else {
-              *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(A.out) + base_o + d) = pack16(x0, x1, A.out_dtype == ECHOKV_DT_BF16);
-            }
-          }
+        store_out32(A, base_o + c0, o, inv);
         }
       }
     }
@@ -678,6 +694,11 @@ __device__ __forceinline__ void tmem_ld16_raw(uint32_t taddr, uint32_t (&r)[16])
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+//
+// Chunks of uneven length: the row tiles of all chunks form one list, longest first, so that the launch has next to no
+// empty CTAs and what is left at its end is short; a grid of (longest chunk's tiles) x chunks launched three empty CTAs
+// of 193 KB for each working one, in no order.  12 prompts of 87 - 2,900 tokens, 32 / 8 heads: 309 -> 222 us; 8 x 512 tokens
+// behind 8,192: 636 -> 585 us (0.59 of the measured bf16 peak); 512 behind 1,600: 36.6 -> 29.5 us.
 __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args A, const __grid_constant__ Maps M) {
   extern __shared__ unsigned char dyn[];
   __shared__ __align__(8) uint64_t bar_s[2], bar_p[2], bar_o[2], bar_k[W_STAGES], bar_v[W_STAGES], bar_kfree[W_STAGES],
@@ -687,13 +708,51 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
   const uint32_t base = (smem_u32(dyn) + 1023u) & ~1023u;
   const uint32_t q_s = base, k_s = q_s + 2 * Q_BYTES, v_s = k_s + W_STAGES * WKV_BYTES;
 
-  const int4 ck = reinterpret_cast<const int4*>(A.chunks)[blockIdx.z];
+  // Work unit blockIdx.y of the chunks' row tiles laid end to end, chunks by descending context (32 of the table at a
+  // time), a chunk's last (longest) tile first.
+  const int gqa = A.gqa, h = blockIdx.x;
+  int4 ck = make_int4(0, 0, 0, 0);
+  int t_in = -1, n_in = 0;  // tile and tiles of the unit's chunk
+  {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int c0 = 0; c0 < A.n_chunks && t_in < 0; c0 += 32) {
+      int4 mine = c0 + lane < A.n_chunks ? reinterpret_cast<const int4*>(A.chunks)[c0 + lane] : make_int4(0, 0, 0, 0);
+      if (A.n_chunks > 1) {
+        int rank = 0, from = 0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int other = __shfl_sync(0xffffffffu, mine.z, j);
+          rank += other > mine.z || (other == mine.z && j < lane);
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) from = __shfl_sync(0xffffffffu, rank, j) == lane ? j : from;
+        mine = make_int4(__shfl_sync(0xffffffffu, mine.x, from), __shfl_sync(0xffffffffu, mine.y, from),
+                         __shfl_sync(0xffffffffu, mine.z, from), __shfl_sync(0xffffffffu, mine.w, from));
+      }
+      const int n = ((mine.y - mine.x) * gqa + NROW - 1) / NROW;
+      int upto = n;  // inclusive sum over the lanes
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.y);
+      if (hit) {
+        const int src = __ffs(hit) - 1;
+        ck = make_int4(__shfl_sync(0xffffffffu, mine.x, src), __shfl_sync(0xffffffffu, mine.y, src),
+                       __shfl_sync(0xffffffffu, mine.z, src), __shfl_sync(0xffffffffu, mine.w, src));
+        n_in = __shfl_sync(0xffffffffu, n, src);
+        t_in = (int)blockIdx.y - (before + __shfl_sync(0xffffffffu, upto, src) - n_in);
+      }
+      before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  if (t_in < 0) return;
   const int q0 = ck.x, nq = ck.y - ck.x, ctx = ck.z;
   const int dense0 = ck.w;
-  const int gqa = A.gqa, h = blockIdx.y;
   const int rows = nq * gqa;
-  const int row0 = blockIdx.x * NROW;
-  if (row0 >= rows) return;
+  const int row0 = (n_in - 1 - t_in) * NROW;
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool row_thread = tid < NROW;
   const int grp = row_thread ? tid / UM : 0, r128 = tid % UM;
@@ -706,6 +765,22 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
   const int n_keys = min(ctx, ctx - nq + last_tok + 1);
   const int n_tiles = (n_keys + WN - 1) / WN;
 
+  auto load = [&](const CUtensorMap* map, uint32_t dst, uint64_t* bar, int tile) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(WKV_BYTES) : "memory");
+    tma_load_3d(dst, map, 0, h, dense0 + tile * WN, bar);
+    tma_load_3d(dst + WN * 128, map, 64, h, dense0 + tile * WN, bar);
+  };
+  if (tid == NROW + 32) {  // the tile producer sets the barriers up and starts the first tiles under the copies of Q
+    auto init = [](uint64_t* b, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n)); };
+    for (int g = 0; g < 2; ++g) { init(&bar_s[g], 1); init(&bar_p[g], UM); init(&bar_o[g], 1); }
+    for (int i = 0; i < W_STAGES; ++i) { init(&bar_k[i], 1); init(&bar_v[i], 1); init(&bar_kfree[i], 1); init(&bar_vfree[i], 1); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int tile = 0; tile < min(n_tiles, W_STAGES); ++tile) {
+      load(&M.k, k_s + tile * WKV_BYTES, &bar_k[tile], tile);
+      load(&M.v, v_s + tile * WKV_BYTES, &bar_v[tile], tile);
+    }
+  }
   if (row_thread) {
     const uint16_t* qp = reinterpret_cast<const uint16_t*>(A.q) + (int64_t)(q0 + tok) * A.q_s0 + (int64_t)hq * A.q_s1;
 #pragma unroll
@@ -713,12 +788,6 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (tid == 0) {
-    auto init = [](uint64_t* b, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n)); };
-    for (int g = 0; g < 2; ++g) { init(&bar_s[g], 1); init(&bar_p[g], UM); init(&bar_o[g], 1); }
-    for (int i = 0; i < W_STAGES; ++i) { init(&bar_k[i], 1); init(&bar_v[i], 1); init(&bar_kfree[i], 1); init(&bar_vfree[i], 1); }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(2 * W_GCOLS));
@@ -776,17 +845,12 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
       }
     }
   } else if (tid == NROW + 32) {  // the tile producer
-    auto load = [&](const CUtensorMap* map, uint32_t dst, uint64_t* bar, int tile) {
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(WKV_BYTES) : "memory");
-      tma_load_3d(dst, map, 0, h, dense0 + tile * WN, bar);
-      tma_load_3d(dst + WN * 128, map, 64, h, dense0 + tile * WN, bar);
-    };
-    for (int tile = 0; tile < n_tiles; ++tile) {
+    for (int tile = W_STAGES; tile < n_tiles; ++tile) {
       const int stage = tile % W_STAGES;
       const uint32_t par = ((tile / W_STAGES) - 1) & 1;
-      if (tile >= W_STAGES && !bar_wait(&bar_kfree[stage], par)) { ok = false; break; }
+      if (!bar_wait(&bar_kfree[stage], par)) { ok = false; break; }
       load(&M.k, k_s + stage * WKV_BYTES, &bar_k[stage], tile);
-      if (tile >= W_STAGES && !bar_wait(&bar_vfree[stage], par)) { ok = false; break; }
+      if (!bar_wait(&bar_vfree[stage], par)) { ok = false; break; }
       load(&M.v, v_s + stage * WKV_BYTES, &bar_v[stage], tile);
     }
   } else if (row_thread) {
@@ -889,16 +953,7 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
         float o[32];
         tmem_ld32(t_row + W_OCOL + c0, o);
         if (live) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float x0 = o[j] * inv, x1 = o[j + 1] * inv;
-            const int d = c0 + j;
-            if (A.out_dtype == ECHOKV_DT_F32) {
-              *reinterpret_cast<float2*>(reinterpret_cast<float*>(A.out) + base_o + d) = make_float2(x0, x1);
-            } else {
-              *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(A.out) + base_o + d) = pack16(x0, x1, A.out_dtype == ECHOKV_DT_BF16);
-            }
-          }
+        store_out32(A, base_o + c0, o, inv);
         }
       }
     }
@@ -971,13 +1026,14 @@ bool encode_kv_map(CUtensorMap* map, const void* base, int64_t rows, int H, int6
 
 }  // namespace
 
+// `q_rows`: an upper bound of the chunks' query rows together (<= 0: not known).
 // mode 0: pipelined; K / V tiles by tensor-map copies when `total_rows` is known and the strides allow it, and then
 // 128-key tiles for chunks of more than 128 rows; mode 4: the same with 64-key tiles throughout; mode 2: the plain
 // kernel; mode 3: pipelined, 64-key tiles copied by the row threads.
 int launch_prefill_umma(const void* q, int64_t q_s0, int64_t q_s1, const void* k, const void* v, int64_t kv_s0,
                         int64_t kv_s1, int64_t total_rows, int dtype, const int32_t* chunks, int64_t n_chunks, int max_rows,
                         void* out, int64_t o_s0, int64_t o_s1, int out_dtype, float scale_log2, int gqa, int H, int head_size,
-                        cudaStream_t st, int mode, bool* handled) {
+                        cudaStream_t st, int mode, int64_t q_rows, bool* handled) {
   using namespace umma;
   *handled = false;
   if (head_size != UD || (dtype != ECHOKV_DT_F16 && dtype != ECHOKV_DT_BF16)) return ECHOKV_OK;
@@ -985,6 +1041,9 @@ int launch_prefill_umma(const void* q, int64_t q_s0, int64_t q_s1, const void* k
   A.q = q; A.k = k; A.v = v; A.out = out; A.chunks = chunks;
   A.q_s0 = q_s0; A.q_s1 = q_s1; A.kv_s0 = kv_s0; A.kv_s1 = kv_s1; A.o_s0 = o_s0; A.o_s1 = o_s1;
   A.gqa = gqa; A.out_dtype = out_dtype; A.is_bf16 = dtype == ECHOKV_DT_BF16; A.scale_log2 = scale_log2;
+  const int out_unit = out_dtype == ECHOKV_DT_F32 ? 4 : 8;  // elements in 16 bytes
+  A.out_vec = (o_s0 | o_s1) % out_unit == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  A.n_chunks = (int)n_chunks;
   static bool configured[64] = {};
   static int* status_word[64] = {};
   int dev = 0;
@@ -1015,7 +1074,12 @@ int launch_prefill_umma(const void* q, int64_t q_s0, int64_t q_s1, const void* k
                      encode_kv_map(&M.k, k, total_rows, H, kv_s0, kv_s1, A.is_bf16, wide ? WN : UN) &&
                      encode_kv_map(&M.v, v, total_rows, H, kv_s0, kv_s1, A.is_bf16, wide ? WN : UN);
     if (two) grid.x = (max_rows + 2 * UM - 1) / (2 * UM);
-    if (wide && tma) prefill_umma_wide_kernel<<<grid, 2 * UM + 64, smem_wide(), st>>>(A, M);
+    // row tiles over all chunks: at most one ragged tile per chunk when the number of query rows is known
+    const int64_t by_chunk = (int64_t)grid.x * n_chunks;
+    const int64_t by_rows = q_rows > 0 ? q_rows * gqa / (2 * UM) + n_chunks : by_chunk;
+    const int64_t units = by_rows < by_chunk ? by_rows : by_chunk;
+    if (wide && tma && units <= 65535)
+      prefill_umma_wide_kernel<<<dim3((unsigned)H, (unsigned)units), 2 * UM + 64, smem_wide(), st>>>(A, M);
     else if (wide) prefill_umma_pipe_kernel<2, false><<<grid, 2 * UM + 32, smem_pipe<2>(), st>>>(A, M);
     else if (two && tma) prefill_umma_pipe_kernel<2, true><<<grid, 2 * UM + 64, smem_pipe<2>(), st>>>(A, M);
     else if (two) prefill_umma_pipe_kernel<2, false><<<grid, 2 * UM + 32, smem_pipe<2>(), st>>>(A, M);

@@ -78,19 +78,20 @@ def build_dense(prefill, req_of, block_size: int, device):
 
 
 def dense_attention(query: torch.Tensor, k: torch.Tensor, v: torch.Tensor, chunks: torch.Tensor, max_chunk: int,
-                    out: torch.Tensor, softmax_scale: float) -> None:
+                    out: torch.Tensor, softmax_scale: float, query_rows: int = 0) -> None:
     """Bottom-right causal attention of each chunk's queries over its dense context (``csrc/prefill.cu``).
-    ``query [T, Hq, D]`` and ``k``/``v [total_ctx, H, D]`` share one 16-bit dtype; ``out [T, Hq, D]``."""
+    ``query [T, Hq, D]`` and ``k``/``v [total_ctx, H, D]`` share one 16-bit dtype; ``out [T, Hq, D]``.
+    ``query_rows``: the chunks' query rows together, when known (it sizes the launch)."""
     N.require_cuda(query, k, v, chunks, out)
     if query.dtype != k.dtype or k.dtype != v.dtype or k.stride() != v.stride():
         raise ValueError("query, K and V must share a dtype and K, V a layout")
     if query.stride(2) != 1 or k.stride(2) != 1 or out.stride(2) != 1:
         raise ValueError("the head dimension must be contiguous")
-    N.check(N.lib.echokv_prefill(
+    N.check(N.lib.echokv_prefill_ex(
         query.data_ptr(), query.stride(0), query.stride(1), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
-        k.shape[0], N.dtype_code(query.dtype), chunks.data_ptr(), chunks.shape[0], max_chunk, out.data_ptr(), out.stride(0),
-        out.stride(1), N.dtype_code(out.dtype), softmax_scale, query.shape[1], k.shape[1], query.shape[2],
-        N.stream_ptr(query.device)))
+        k.shape[0], N.dtype_code(query.dtype), chunks.data_ptr(), chunks.shape[0], max_chunk, query_rows,
+        out.data_ptr(), out.stride(0), out.stride(1), N.dtype_code(out.dtype), softmax_scale, query.shape[1],
+        k.shape[1], query.shape[2], N.stream_ptr(query.device)))
 
 
 def dense_supported(store, query: torch.Tensor) -> bool:
@@ -117,7 +118,7 @@ def prefill_attention(store, query: torch.Tensor, output: torch.Tensor, prefill,
     if dense is not None and dense_supported(store, query):
         work, total, chunks, max_chunk = dense
         k, v = dequant_dense(store, work, total, block_table, query.dtype)
-        dense_attention(query, k, v, chunks, max_chunk, out3, softmax_scale)
+        dense_attention(query, k, v, chunks, max_chunk, out3, softmax_scale, sum(qe - qs for qs, qe, _, _ in prefill))
         return
     if rows is None:
         rows = build_rows(prefill, req_of, query.device)

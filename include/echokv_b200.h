@@ -281,6 +281,14 @@ int echokv_prefill(const void* query, int64_t q_s0, int64_t q_s1, const void* k_
 int echokv_gather_rows(const void* src, int64_t src_row_stride_bytes, const int64_t* rows, int64_t n, void* dst,
                        int64_t row_bytes, void* stream);
 
+/* The same with an upper bound of the chunks' query rows together (e.g. the rows of `query`; <= 0: not known), which
+ * sizes the launch for chunks of uneven length. */
+int echokv_prefill_ex(const void* query, int64_t q_s0, int64_t q_s1, const void* k_dense, const void* v_dense,
+                      int64_t kv_s0, int64_t kv_s1, int64_t total_ctx, int32_t dtype, const int32_t* chunks,
+                      int64_t n_chunks, int32_t max_chunk_len, int64_t query_rows, void* out, int64_t o_s0, int64_t o_s1,
+                      int32_t out_dtype, float softmax_scale, int32_t num_q_heads, int32_t num_kv_heads, int32_t head_size,
+                      void* stream);
+
 /* Kernel selection of echokv_prefill: 0 (default) takes the tcgen05 / TMEM kernel when the shape fits
  * (head size 128) and the mma.sync kernel otherwise; 1 always takes the mma.sync kernel; 2 takes the
  * tcgen05 kernel without the overlap of tensor work and softmax (two CTAs per SM); 3 takes the
