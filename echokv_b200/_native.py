@@ -87,6 +87,7 @@ _SIGS = {
                        _I32, _I32, _P],
     "echokv_prefill_ex": [_P, _I64, _I64, _P, _P, _I64, _I64, _I64, _I32, _P, _I64, _I32, _I64, _P, _I64, _I64, _I32, _F,
                           _I32, _I32, _I32, _P],
+    "echokv_write_headers_many": [_PP, C.POINTER(_P), C.POINTER(_P), C.POINTER(_I64), _I32, _P],
     "echokv_set_decode_events": [_P, _P],
     "echokv_gather_rows": [_P, _I64, _P, _I64, _P, _I64, _P],
     "echokv_canary_kl": [_P, _I32, _I64, _I64, _I64, _P, _I64, _I64, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _I32,
@@ -134,7 +135,9 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 def stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the current stream of ``device`` (without building a Stream object: this runs once per launch)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

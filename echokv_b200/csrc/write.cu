@@ -17,6 +17,20 @@ __global__ void write_headers_kernel(uint8_t* pages, int64_t ps, const int64_t* 
   *reinterpret_cast<uint4*>(pages + blocks[i] * ps) = h;
 }
 
+// The headers of several pools (the layers of a group) in one launch; blockIdx.y = pool.
+constexpr int HEADER_POOLS = 32;
+struct HeaderPools {
+  uint8_t* pages[HEADER_POOLS];
+  const int64_t* blocks[HEADER_POOLS];
+  const uint4* headers[HEADER_POOLS];
+  int64_t ps[HEADER_POOLS], n[HEADER_POOLS];
+};
+__global__ void write_headers_many_kernel(const __grid_constant__ HeaderPools P) {
+  const int k = blockIdx.y;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < P.n[k]) *reinterpret_cast<uint4*>(P.pages[k] + P.blocks[k][i] * P.ps[k]) = P.headers[k][i];
+}
+
 // dst row i = src row rows[i], 16 bytes per thread.
 __global__ void gather_rows_kernel(const uint4* __restrict__ src, int64_t src_stride16, const int64_t* __restrict__ rows,
                                    uint4* __restrict__ dst, int64_t n, int row16) {
@@ -926,6 +940,34 @@ int echokv_write_headers(const echokv_pages* pages, const int64_t* blocks, const
   write_headers_kernel<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
       (uint8_t*)pages->base, pages->page_stride_bytes, blocks, headers, n);
   return check_launch("write_headers");
+}
+
+int echokv_write_headers_many(const echokv_pages* pages, const int64_t* const* blocks, const uint8_t* const* headers,
+                              const int64_t* n, int32_t count, void* stream) {
+  if (count <= 0) return ECHOKV_OK;
+  if (!pages || !blocks || !headers || !n) return set_error(ECHOKV_E_ARGUMENT, "write_headers_many: null pointer");
+  for (int32_t i = 0; i < count; ++i) {
+    if (n[i] <= 0) continue;
+    if (!pages[i].base || !blocks[i] || !headers[i]) return set_error(ECHOKV_E_ARGUMENT, "write_headers_many: null pointer");
+    if (!aligned16(headers[i]) || !aligned16(pages[i].base) || pages[i].page_stride_bytes % 16)
+      return set_error(ECHOKV_E_ARGUMENT, "write_headers_many: headers and pages must be 16-byte aligned");
+  }
+  for (int32_t at = 0; at < count; at += HEADER_POOLS) {
+    const int32_t k = count - at < HEADER_POOLS ? count - at : HEADER_POOLS;
+    HeaderPools P = {};
+    int64_t most = 0;
+    for (int32_t i = 0; i < k; ++i) {
+      P.pages[i] = (uint8_t*)pages[at + i].base;
+      P.ps[i] = pages[at + i].page_stride_bytes;
+      P.blocks[i] = blocks[at + i];
+      P.headers[i] = (const uint4*)headers[at + i];
+      P.n[i] = n[at + i] > 0 ? n[at + i] : 0;
+      if (P.n[i] > most) most = P.n[i];
+    }
+    if (most == 0) continue;
+    write_headers_many_kernel<<<dim3((unsigned)((most + 127) / 128), (unsigned)k), 128, 0, (cudaStream_t)stream>>>(P);
+  }
+  return check_launch("write_headers_many");
 }
 
 int echokv_scatter_i64(int64_t* dst, const int64_t* idx, const int64_t* val, int64_t n, void* stream) {

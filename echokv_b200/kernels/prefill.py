@@ -17,8 +17,7 @@ Two device paths:
 
 from __future__ import annotations
 
-import itertools
-
+import numpy as np
 import torch
 
 from echokv_b200 import _native as N
@@ -31,9 +30,15 @@ ROW_PATH_MAX_CHUNK = 64  # longer chunks take the dense path when it is availabl
 def build_dequant_work(prefill, req_of, block_size: int, device) -> torch.Tensor:
     """Work list ``[n, 4]`` int32: (request, block index, dense row of the block's first token, ctx);
     contexts are packed back to back in ``prefill`` order."""
-    rows = [(r, bi, g0 + bi * block_size, ctx)
-            for (_, _, ctx, g0), r in zip(prefill, req_of) for bi in range(-(-ctx // block_size))]
-    return to_device(torch.tensor(rows, dtype=torch.int32).reshape(-1, 4), device)
+    pairs = list(zip(prefill, req_of))
+    ctx = np.array([p[2] for p, _ in pairs], dtype=np.int64)
+    count = -(-ctx // block_size)
+    rows = np.empty((int(count.sum()), 4), dtype=np.int32)
+    rows[:, 0] = np.repeat(np.array([r for _, r in pairs], dtype=np.int64), count)
+    rows[:, 1] = np.arange(rows.shape[0]) - np.repeat(np.cumsum(count) - count, count)
+    rows[:, 2] = np.repeat(np.array([p[3] for p, _ in pairs], dtype=np.int64), count) + rows[:, 1].astype(np.int64) * block_size
+    rows[:, 3] = np.repeat(ctx, count)
+    return to_device(torch.from_numpy(rows), device)
 
 
 def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.Tensor, dtype):
@@ -54,14 +59,17 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
 
 def build_rows(prefill, req_of, device):
     """Row-path metadata: per query token its row, its request and its causal limit (device int64)."""
-    q_rows, reqs, lens = [], [], []
-    for (qs, qe, ctx, _), r in zip(prefill, req_of):
-        nq = qe - qs
-        q_rows.extend(range(qs, qe))
-        reqs.extend([r] * nq)
-        lens.extend(range(ctx - nq + 1, ctx + 1))
-    packed = to_device(torch.tensor([q_rows, reqs, lens], dtype=torch.long), device)
-    return packed[0], packed[1], packed[2], (max(lens) if lens else 0)
+    pairs = list(zip(prefill, req_of))
+    start = np.array([p[0] for p, _ in pairs], dtype=np.int64)
+    nq = np.array([max(p[1] - p[0], 0) for p, _ in pairs], dtype=np.int64)
+    ctx = np.array([p[2] for p, _ in pairs], dtype=np.int64)
+    rows = np.empty((3, int(nq.sum())), dtype=np.int64)
+    at = np.arange(rows.shape[1]) - np.repeat(np.cumsum(nq) - nq, nq)  # place in the chunk
+    rows[0] = np.repeat(start, nq) + at
+    rows[1] = np.repeat(np.array([r for _, r in pairs], dtype=np.int64), nq)
+    rows[2] = np.repeat(ctx - nq + 1, nq) + at
+    packed = to_device(torch.from_numpy(rows), device)
+    return packed[0], packed[1], packed[2], int(rows[2].max(initial=0))
 
 
 def build_dense(prefill, req_of, block_size: int, device):

@@ -15,11 +15,13 @@ the benchmark drives it directly.
 
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass
 
 import numpy as np
 import torch
 
+from echokv_b200 import _native as N
 from echokv_b200.canary import canary_kl_ring, tp_mean
 from echokv_b200.controller import LayerController
 from echokv_b200.quant import SUPPORTED_BITS
@@ -82,7 +84,7 @@ class Staging:
         else:
             cd, ct, cf = s + (s & 1), t + (t & 1), n_fin
             total = self._offsets(cd, ct, cf)[2] + sum(tail_sizes)
-            hbuf = torch.zeros(total, dtype=torch.long).pin_memory()
+            hbuf = torch.empty(total, dtype=torch.long, pin_memory=True)
             h = hbuf.numpy()
         o_tok, o_fin, o_tail = self._offsets(cd, ct, cf)
         h[0], h[1] = n_fin, bps
@@ -95,7 +97,7 @@ class Staging:
         end = o_tail
         tail_dev = None
         if tail_own:
-            th = torch.zeros(sum(tail_sizes), dtype=torch.long).pin_memory()
+            th = torch.empty(sum(tail_sizes), dtype=torch.long, pin_memory=True)
             o = 0
             for a, n in zip(tail, tail_sizes):
                 th.numpy()[o: o + a.size] = a.reshape(-1)
@@ -172,6 +174,7 @@ class GroupRunner:
             self.stores.append(TieredKVCache(layout, pages, residual=res, shared=self.shared))
             self.krefs.append(krefs[i] if krefs else self._kref_all[i])
             self.stashes.append(stashes[i] if stashes else self._stash_all[i])
+        self._c_pages = (N.Pages * len(self.stores))(*[st._c_pages for st in self.stores])
         self.canary_max_q = canary_max_q
         self.cap = cap
         tail = cap * (4 + 3 * len(caches)) + 64
@@ -216,12 +219,20 @@ class GroupRunner:
         fin_count, canary_rows, dviews, tok, fin, views, bps_dev = self.staging.stage(
             plan.n_fin, can, dec, (plan.tok_slot, plan.tok_res, plan.tok_sealed, plan.tok_kref), plan.fin, tail, bps)
         shared.apply_res_map(*views[:4])
-        for st, ids, hdr in zip(self.stores, views[4::2], views[5::2]):
-            st.write_headers(ids, hdr.view(torch.uint8).view(-1, 16))
+        if opened:
+            self._write_headers([v.data_ptr() for v in views[4::2]], [v.data_ptr() for v in views[5::2]],
+                                [blocks.size for blocks, _ in opened])
         write = WriteMeta(tok=tok, fin=fin, fin_count=fin_count, n_rows=plan.n_rows, n_fin=plan.n_fin)
         has_dec = decode is not None and dec[0].size > 0
         return StepMeta(write, canary_rows, dviews[0] if has_dec else None, dviews[1] if has_dec else None,
                         dviews[2] if has_dec else None, self.num_splits, bps_dev)
+
+    def _write_headers(self, blocks: list[int], headers: list[int], counts: list[int]) -> None:
+        """Every layer's opened page headers (device addresses of block ids and headers) in one launch."""
+        n = len(counts)
+        N.check(N.lib.echokv_write_headers_many(
+            self._c_pages, (C.c_void_p * n)(*blocks), (C.c_void_p * n)(*headers), (C.c_int64 * n)(*counts), n,
+            N.stream_ptr(self.device)))
 
     # -- canary (reference: EchoKVMetadataBuilder._run_canary, backend.py:314-333) --------------
     def stash_queries(self, layer: int, query: torch.Tensor, meta: StepMeta) -> None:

@@ -110,6 +110,12 @@ class TieredLayout:
         return N.Layout(self.num_kv_heads, self.head_size, self.block_size, self.mem_bits, self.k_group, self.v_group)
 
 
+_NEXTRA_OF = np.zeros(9, dtype=np.int64)  # extra chunks of a block by its tier
+for _bits, _n in NEXTRA.items():
+    _NEXTRA_OF[_bits] = _n
+_SLOT = np.arange(3)
+
+
 class ChunkPool:
     """Host free list of the spare chunk slots (1 .. k_c-1 of every page) of one layer.
 
@@ -130,6 +136,13 @@ class ChunkPool:
         n = NEXTRA.get(int(self.tier[block]), 0)
         self.free.extend(self.table[block, :n].tolist())
         self.tier[block] = new_tier
+
+    def release_many(self, blocks: np.ndarray, new_tier: int) -> None:
+        """``release`` of every block in order."""
+        n = _NEXTRA_OF[self.tier[blocks]]
+        if n.any():
+            self.free.extend(self.table[blocks][_SLOT < n[:, None]].tolist())
+        self.tier[blocks] = new_tier
 
     def allot(self, blocks: np.ndarray, target_bits: int) -> np.ndarray:
         """Greedy in block order: as many blocks as fit at the target tier, then the next tier down."""
@@ -293,18 +306,16 @@ class TieredKVCache:
             blocks = blocks.cpu().numpy()
         blocks = np.asarray(blocks, dtype=np.int64)
         self._settle(blocks)
-        for b in blocks.tolist():
-            self.pool.release(b, 0)
+        self.pool.release_many(blocks, 0)
         short = NEXTRA[target_bits] * blocks.size - len(self.pool.free)
         if short > 0:
-            keep = set(blocks.tolist())
-            if protect is not None:
-                keep |= set(np.asarray(protect).tolist())
+            keep = blocks if protect is None else np.concatenate([blocks, np.asarray(protect, dtype=np.int64).reshape(-1)])
             self._demote_lru(short, keep)
         tiers = self.pool.allot(blocks, target_bits)
+        count = np.bincount(tiers, minlength=9).tolist()
         for bits in SUPPORTED_BITS:
-            self.blocks_opened[bits] += int((tiers == bits).sum())
-        self.downgraded_blocks += int((tiers < target_bits).sum())
+            self.blocks_opened[bits] += count[bits]
+        self.downgraded_blocks += sum(count[:target_bits])
         return blocks, self.pool.headers(blocks)
 
     def write_headers(self, blocks: torch.Tensor, headers: torch.Tensor) -> None:
@@ -312,30 +323,23 @@ class TieredKVCache:
         N.check(N.lib.echokv_write_headers(self.c_pages, blocks.data_ptr(), headers.data_ptr(), blocks.numel(),
                                            N.stream_ptr(self.device)))
 
-    def _demote_lru(self, chunks_needed: int, keep: set) -> None:
+    def _demote_lru(self, chunks_needed: int, keep: np.ndarray) -> None:
         """Requantize the least recently written full INT4/INT8 blocks to INT2, freeing their chunks."""
         tier = self.pool.tier
         full = np.flatnonzero((tier >= 4) & (self.shared.fill_h == self.layout.block_size))
         ranked = full[np.argsort(self.shared.last_h[full], kind="stable")]
-        victims, freed = [], 0
-        for b in ranked.tolist():
-            if freed >= chunks_needed:
-                break
-            if b in keep:
-                continue
-            victims.append(b)
-            freed += NEXTRA[int(tier[b])]
-        if not victims:
+        ranked = ranked[~np.isin(ranked, keep)]
+        freed = np.cumsum(_NEXTRA_OF[tier[ranked]])
+        victims = ranked[: int(np.searchsorted(freed, chunks_needed)) + 1]  # up to the one that frees enough
+        if not victims.size:
             return
-        vb = to_device(torch.tensor(victims, dtype=torch.long), self.device)
+        vb = to_device(torch.from_numpy(victims), self.device)
         nbytes = N.lib.echokv_demote_scratch_bytes(self.c_layout, len(victims))
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         N.check(N.lib.echokv_demote_blocks(self.c_layout, self.c_pages, self.c_res, vb.data_ptr(), len(victims),
                                            scratch.data_ptr(), nbytes, N.stream_ptr(self.device)))
-        varr = np.asarray(victims, dtype=np.int64)
-        self._settle(varr)
-        for b in victims:
-            self.pool.release(b, 2)
+        self._settle(victims)
+        self.pool.release_many(victims, 2)
         self.demoted_blocks += len(victims)
 
     # -- write ------------------------------------------------------------

@@ -97,6 +97,11 @@ int echokv_layout_describe(const echokv_layout* layout, echokv_layout_info* out)
 int echokv_write_headers(const echokv_pages* pages, const int64_t* blocks, const uint8_t* headers,
                          int64_t n, void* stream);
 
+/* The same for `count` pools in one launch (every layer of a KV-cache group opens blocks in the same step): entry i
+ * writes n[i] headers.  The four arrays are host memory, blocks[i] / headers[i] device memory. */
+int echokv_write_headers_many(const echokv_pages* pages, const int64_t* const* blocks, const uint8_t* const* headers,
+                              const int64_t* n, int32_t count, void* stream);
+
 /* dst[idx[i]] = val[i] -- SharedState.apply_res_map (write_plan.py:266-271). */
 int echokv_scatter_i64(int64_t* dst, const int64_t* idx, const int64_t* val, int64_t n, void* stream);
 
