@@ -149,7 +149,7 @@ struct DenseArgs {
   int64_t bt_s0;
   T *k_out, *v_out;
   int64_t o_s0, o_s1;
-  int slices;  // CTAs per block
+  int slices;  // CTAs per block; 0: the work list is in slices of DENSE_TOK tokens instead of blocks
 };
 
 // Tokens [t0, t1) of one block of tier BITS; `s_row`: byte offset of each token's row from the pool base.  The loads of
@@ -232,9 +232,19 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_dense_vec_kernel(const DenseArgs<T> A) {
   __shared__ int64_t s_row[DENSE_TOK];
   const LayoutDev& L = A.L;
-  const int item = blockIdx.x / A.slices, t0 = (blockIdx.x - item * A.slices) * DENSE_TOK;
+  int item = blockIdx.x, t0 = 0;
+  if (A.slices > 0) {
+    item = blockIdx.x / A.slices;
+    t0 = (blockIdx.x - item * A.slices) * DENSE_TOK;
+  }
   const int4 w = reinterpret_cast<const int4*>(A.work)[item];
-  const int req = w.x, bi = w.y, ctx = w.w;
+  const int req = w.x, ctx = w.w;
+  int bi = w.y, row0 = w.z;  // block of the context, dense row of its first token
+  if (A.slices == 0) {  // w.y: slice of the context, w.z: dense row of its first token
+    bi = w.y * DENSE_TOK / L.BS;
+    t0 = w.y * DENSE_TOK - bi * L.BS;
+    row0 -= t0;
+  }
   const int t1 = min(min(L.BS, ctx - bi * L.BS), t0 + DENSE_TOK);
   if (t0 >= t1) return;
   const int64_t blk = A.bt[(int64_t)req * A.bt_s0 + bi];
@@ -245,9 +255,9 @@ __global__ void __launch_bounds__(256) dequant_dense_vec_kernel(const DenseArgs<
   const int open_grp = slot >= 0 ? (int)A.R.res_group[slot] : -1;
   if (t0 + (int)threadIdx.x < t1) s_row[threadIdx.x] = row_offset(A.pages, L, blk, t0 + threadIdx.x, bits);
   __syncthreads();
-  if (bits == 4) dense_rows<T, 4>(A, page, w.z, t0, t1, slot, open_grp, s_row);
-  else if (bits == 8) dense_rows<T, 8>(A, page, w.z, t0, t1, slot, open_grp, s_row);
-  else dense_rows<T, 2>(A, page, w.z, t0, t1, slot, open_grp, s_row);
+  if (bits == 4) dense_rows<T, 4>(A, page, row0, t0, t1, slot, open_grp, s_row);
+  else if (bits == 8) dense_rows<T, 8>(A, page, row0, t0, t1, slot, open_grp, s_row);
+  else dense_rows<T, 2>(A, page, row0, t0, t1, slot, open_grp, s_row);
 }
 
 // Demotion, phase 2: requantize a block's dequantized contents (scratch: K then V, float
@@ -485,9 +495,9 @@ int echokv_gather(const echokv_layout* layout, const echokv_pages* pages, const 
   return check_launch("gather");
 }
 
-int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
-                         const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
-                         void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream) {
+static int dequant_dense_impl(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                              const int32_t* work, int64_t n_work, bool by_slice, const int32_t* block_table, int64_t bt_s0,
+                              void* k_out, void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream) {
   if (n_work <= 0) return ECHOKV_OK;
   LayoutDev L;
   ResidualDev R;
@@ -501,8 +511,9 @@ int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages,
   dequant_dense_kernel<T><<<(unsigned)n_work, 256, 0, st>>>(L, R, (const uint8_t*)pages->base, work, block_table, \
                                                            bt_s0, (T*)k_out, (T*)v_out, out_s0, out_s1)
   // 16-byte loads and stores need the stat arrays, the rows of the outputs and 8-channel chunks aligned
-  const int slices = (L.BS + DENSE_TOK - 1) / DENSE_TOK;
-  const bool vec = out_dtype != ECHOKV_DT_F32 && n_work * slices < (1ll << 31) && L.D % 8 == 0 && L.VG % 8 == 0 &&
+  const int slices = by_slice ? 0 : (L.BS + DENSE_TOK - 1) / DENSE_TOK;
+  const int64_t ctas = by_slice ? n_work : n_work * slices;
+  const bool vec = out_dtype != ECHOKV_DT_F32 && ctas < (1ll << 31) && L.D % 8 == 0 && L.VG % 8 == 0 &&
                    ((L.o_ks | L.o_km | L.PS | L.o_data | L.CB) % 16) == 0 && (out_s0 % 8) == 0 && (out_s1 % 8) == 0 &&
                    ((reinterpret_cast<uintptr_t>(k_out) | reinterpret_cast<uintptr_t>(v_out) |
                      reinterpret_cast<uintptr_t>(pages->base) | reinterpret_cast<uintptr_t>(work)) % 16) == 0;
@@ -510,13 +521,14 @@ int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages,
   {                                                                                                           \
     DenseArgs<T> A = {L, R, (const uint8_t*)pages->base, work, block_table, bt_s0, (T*)k_out, (T*)v_out, out_s0, \
                       out_s1, slices};                                                                        \
-    dequant_dense_vec_kernel<T><<<(unsigned)(n_work * slices), 256, 0, st>>>(A);                              \
+    dequant_dense_vec_kernel<T><<<(unsigned)ctas, 256, 0, st>>>(A);                                           \
   }
   if (vec) {
     if (out_dtype == ECHOKV_DT_F16) LAUNCH_VEC(__half) else LAUNCH_VEC(__nv_bfloat16)
     return check_launch("dequant_dense");
   }
 #undef LAUNCH_VEC
+  if (by_slice) return set_error(ECHOKV_E_UNSUPPORTED, "dequant_dense_slices: 16-bit outputs with 16-byte aligned rows only");
   switch (out_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;
     case ECHOKV_DT_F16: LAUNCH(__half); break;
@@ -525,6 +537,22 @@ int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages,
   }
 #undef LAUNCH
   return check_launch("dequant_dense");
+}
+
+int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                         const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
+                         void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream) {
+  return dequant_dense_impl(layout, pages, residual, work, n_work, false, block_table, bt_s0, k_out, v_out, out_s0, out_s1,
+                            out_dtype, stream);
+}
+
+int echokv_dequant_dense_slices(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                                const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
+                                void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream) {
+  if (layout && layout->block_size % DENSE_TOK)
+    return set_error(ECHOKV_E_UNSUPPORTED, "dequant_dense_slices: block size %d is not a multiple of %d", layout->block_size, DENSE_TOK);
+  return dequant_dense_impl(layout, pages, residual, work, n_work, true, block_table, bt_s0, k_out, v_out, out_s0, out_s1,
+                            out_dtype, stream);
 }
 
 int64_t echokv_demote_scratch_bytes(const echokv_layout* layout, int64_t n) {
