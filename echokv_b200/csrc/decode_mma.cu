@@ -59,7 +59,7 @@ constexpr unsigned long long WAIT_NS = 2000000000ull;  // a wait gives up after 
 // What the producer tells the consumers about a staged group (stored at `o_hdr` of its first stage).
 constexpr int F_RES = 1, F_FIRST = 2, F_LAST = 4;  // K from the residual buffer / first / last group of a work item
 constexpr int F_PAIR = 8;                          // the next stage holds a second full tile of the same tier
-constexpr int RT_LOG_SHIFT = 8;                    // plan entries only: bits 8..11 = log2(token rows per run), 15 = not a power of two
+constexpr int RT_LOG_SHIFT = 8;                    // plan entries only: bits 8..11 = log2(token rows per run)
 constexpr int F_MASK = 0xff;                       // the flag bits a stage header carries
 struct alignas(16) StageHeader {
   int bits, n_valid, flags, pos0;   // n_valid: 1..16 tokens, -1 = no more work
@@ -972,9 +972,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
       const uint32_t k_stats = 2u * H * D * 2, v_stats = 2u * TILE * H * NG * 2;
       const int rt_log = (h0.z >> RT_LOG_SHIFT) & 15;           // token rows per run (see TilePlan) = 1 << rt_log
       auto row_src = [&](int t) {
-        if (rt_log != 15) return d.run[t >> rt_log] + (uint32_t)(t & ((1 << rt_log) - 1)) * 2u * side;
-        const int rt = min((2 * L.BS) / h0.x, TILE);
-        return d.run[t / rt] + (uint32_t)(t % rt) * 2u * side;
+        return d.run[t >> rt_log] + (uint32_t)(t & ((1 << rt_log) - 1)) * 2u * side;
       };
       const int half0 = rows == 3 ? TILE / 2 : 0;               // first token of an INT8 half
       const int nh = rows == 1 ? nv : max(0, min(nv - half0, TILE / 2));  // token rows this stage receives
@@ -1033,9 +1031,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
       const uint32_t k_stats = 2u * H * D * 2, v_stats = 2u * TILE * H * NG * 2;
       const int rt_log = (h0.z >> RT_LOG_SHIFT) & 15;           // token rows per run (see TilePlan) = 1 << rt_log
       auto row_src = [&](int t) {
-        if (rt_log != 15) return d.run[t >> rt_log] + (uint32_t)(t & ((1 << rt_log) - 1)) * 2u * side;
-        const int rt = min((2 * L.BS) / h0.x, TILE);
-        return d.run[t / rt] + (uint32_t)(t % rt) * 2u * side;
+        return d.run[t >> rt_log] + (uint32_t)(t & ((1 << rt_log) - 1)) * 2u * side;
       };
       const int half0 = rows == 3 ? TILE / 2 : 0;
       const int nh = rows == 1 ? nv : max(0, min(nv - half0, TILE / 2));
@@ -1132,7 +1128,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
           }
           const int nv = min(TILE, blk_tok - t0);
           d.hdr.bits = bits; d.hdr.n_valid = nv;
-          const int rt_log = (rt & (rt - 1)) == 0 ? 31 - __clz(rt) : 15;  // for the fills: a run's rows by shift and mask
+          const int rt_log = 31 - __clz(rt);                // for the fills: a run's rows by shift and mask
           d.hdr.flags = (in_res ? F_RES : 0) | (u_first && lane == 0 ? F_FIRST : 0) |
                         (u_last && lane == unit_tiles - 1 ? F_LAST : 0) | (rt_log << RT_LOG_SHIFT);
           d.hdr.pos0 = t0 - grp * L.KG; d.hdr.res_slot = ks_slot; d.hdr.seq = u_seq; d.hdr.split = u_split;
@@ -1478,7 +1474,9 @@ static bool team_shape(const DecodeDevice& dv, int H, int gqa, TeamShape* out) {
 
 static bool mma_shape_ok(int H, int D_, int VG, int KG, int BS, int gqa) {
   using namespace mma;
-  return D_ == D && VG == 32 && KG % TILE == 0 && BS % TILE == 0 && gqa <= 8 && (H == 1 || H == 2 || H == 4 || H == 8);
+  // a block of a power of two of tokens: only then does a tile's run of rows never cross from one chunk to the next
+  return D_ == D && VG == 32 && KG % TILE == 0 && BS % TILE == 0 && (BS & (BS - 1)) == 0 && gqa <= 8 &&
+         (H == 1 || H == 2 || H == 4 || H == 8);
 }
 
 // Teams of the tensor-core kernel on the current device for this shape (0: the generic kernel takes it, or no device).
