@@ -13,7 +13,9 @@ Two device paths:
     trade-off, kernels/prefill.py:10-13).  Where that re-reading costs more than
     it saves (`short_chunks_as_dense`), the contexts are dequantized to fp16 and
     the tensor-core attention kernel runs on fp16 operands -- the precision of the
-    decode kernel's operands, which the model's bf16 would not give.
+    decode kernel's operands, which the model's bf16 would not give.  One vector
+    per context and head is subtracted from its keys first, so that channels far
+    from zero keep that precision too.
   * dense path: dequantize every context once into ``[total_ctx, H, D]`` in the
     model dtype, then run the tensor-core attention kernel over it.
 """
@@ -46,9 +48,10 @@ def build_dequant_work(prefill, req_of, block_size: int, device) -> torch.Tensor
     return to_device(torch.from_numpy(rows), device)
 
 
-def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.Tensor, dtype, by_slice: bool = False):
+def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.Tensor, dtype, by_slice: bool = False,
+                  center: bool = False):
     """Dense ``[total_ctx, H, D]`` K and V (``dtype``) of the contexts in ``work`` (entries per block, or per
-    ``SLICE`` tokens with ``by_slice``)."""
+    ``SLICE`` tokens with ``by_slice``, then optionally ``center``: K minus a constant per request, head and channel)."""
     L = store.layout
     k = torch.empty(total_ctx, L.num_kv_heads, L.head_size, device=store.device, dtype=dtype)
     v = torch.empty_like(k)
@@ -57,10 +60,11 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
         if block_table.dtype != torch.int32 or block_table.stride(1) != 1:
             block_table = block_table.to(torch.int32).contiguous()
         launch = N.lib.echokv_dequant_dense_slices if by_slice else N.lib.echokv_dequant_dense
+        extra = (int(center),) if by_slice else ()
         N.check(launch(
             store.c_layout, store.c_pages, store.c_res, work.data_ptr(), work.shape[0],
             block_table.data_ptr(), block_table.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
-            N.dtype_code(dtype), N.stream_ptr(store.device)))
+            N.dtype_code(dtype), *extra, N.stream_ptr(store.device)))
     return k, v
 
 
@@ -119,8 +123,8 @@ def short_chunks_as_dense(prefill, num_kv_heads: int, num_q_heads: int) -> bool:
     and 8 heads once the chip is full, 15 us around it.  Dense: 0.9 ns per context token and 8 heads to dequantize,
     12 us for that and the query's conversion; the attention kernel's CTAs (128 rows of query token x head; 256 when
     a chunk has more) each walk 128 keys in 2.2 us, one CTA per SM.  Measured, row / dense: 16 chunks of 33 behind
-    1,472 216 / 74 us, 4 of 50 behind 4,000 303 / 104, 8 of 40 behind 3,000 at one head per KV head 320 / 84, 16 of 8
-    behind 1,472 65 / 57, one of 33 behind 1,472 32 / 49, 8 of 30 behind 100 29 / 32.  The margin keeps a step on the
+    1,472 217 / 81 us, 4 of 50 behind 4,000 300 / 105, 8 of 40 behind 3,000 at one head per KV head 320 / 94, 16 of 8
+    behind 1,472 65 / 66, one of 33 behind 1,472 32 / 50, 8 of 30 behind 100 28 / 32.  The margin keeps a step on the
     row path where the two are close.  Against 64-bit attention over the stored values the dense side's relative
     error is the smaller one wherever it is chosen (16 x 33: 0.7e-3, row path 1.1e-3).
     """
@@ -196,7 +200,7 @@ def prefill_attention(store, query: torch.Tensor, output: torch.Tensor, prefill,
     if isinstance(rows, Rows) and dense_supported(store, query) and L.block_size % SLICE == 0 and L.head_size == 128 and \
             query.shape[1] // L.num_kv_heads <= 8 and short_chunks_as_dense(prefill, L.num_kv_heads, query.shape[1]):
         work, total, chunks, max_chunk = rows.dense
-        k, v = dequant_dense(store, work, total, block_table, torch.float16, by_slice=True)
+        k, v = dequant_dense(store, work, total, block_table, torch.float16, by_slice=True, center=True)
         dense_attention(query.to(torch.float16), k, v, chunks, max_chunk, out3, softmax_scale,
                         sum(qe - qs for qs, qe, _, _ in prefill))
         return
