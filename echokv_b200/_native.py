@@ -87,7 +87,6 @@ _SIGS = {
                        _I32, _I32, _P],
     "echokv_prefill_ex": [_P, _I64, _I64, _P, _P, _I64, _I64, _I64, _I32, _P, _I64, _I32, _I64, _P, _I64, _I64, _I32, _F,
                           _I32, _I32, _I32, _P],
-    "echokv_dequant_dense_slices": [_LP, _PP, _RP, _P, _I64, _P, _I64, _P, _P, _I64, _I64, _I32, _I32, _P],
     "echokv_write_headers_many": [_PP, C.POINTER(_P), C.POINTER(_P), C.POINTER(_I64), _I32, _P],
     "echokv_set_decode_events": [_P, _P],
     "echokv_gather_rows": [_P, _I64, _P, _I64, _P, _I64, _P],

@@ -149,45 +149,14 @@ struct DenseArgs {
   int64_t bt_s0;
   T *k_out, *v_out;
   int64_t o_s0, o_s1;
-  int slices;  // CTAs per block; 0: the work list is in slices of DENSE_TOK tokens instead of blocks
-  int center;  // subtract a per-channel constant of the context from K (see k_center)
+  int slices;  // CTAs per block
 };
-
-// A constant per context, head and channel: the middle of the range of the context's first K group (its first key while
-// that group is open).  Attention weights do not change when the same vector is subtracted from every key of a
-// context, and a channel that sits far from zero then loses nothing when it is rounded to 16 bits.
-template <typename T>
-__device__ __forceinline__ void k_center(const DenseArgs<T>& A, int req, int h, int d0, float2 (&c)[4]) {
-  const LayoutDev& L = A.L;
-  const int64_t blk = A.bt[(int64_t)req * A.bt_s0];
-  const uint8_t* page = A.pages + blk * L.PS;
-  const int64_t slot = A.R.block_res[blk];
-  const bool open = slot >= 0 && A.R.res_group[slot] == 0;
-  const int bits = page[0] == 0 ? 2 : page[0];
-  const float half = 0.5f * (float)((1 << bits) - 1);
-  float x[8];
-  if (open) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = ld_dt(A.R.base, A.R.dtype, slot * A.R.s_slot + h * A.R.s_head + d0 + k);
-  } else {
-    const int e = h * L.D + d0;
-    const uint4 s8 = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(page + L.o_ks) + e);
-    const uint4 m8 = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(page + L.o_km) + e);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      x[k] = __half2float(reinterpret_cast<const __half*>(&s8)[k]) * half + __half2float(reinterpret_cast<const __half*>(&m8)[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) x[k] = fabsf(x[k]) <= 65504.f ? x[k] : 0.f;  // infinities and NaN stay where they are
-#pragma unroll
-  for (int k = 0; k < 4; ++k) c[k] = make_float2(-x[2 * k], -x[2 * k + 1]);
-}
 
 // Tokens [t0, t1) of one block of tier BITS; `s_row`: byte offset of each token's row from the pool base.  The loads of
 // a batch of tokens are issued together; the K statistics are read again only where the K group changes.
 template <typename T, int BITS>
-__device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t* page, int req, int64_t row0, int t0, int t1,
-                                           int64_t slot, int open_grp, const int64_t* s_row) {
+__device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t* page, int64_t row0, int t0, int t1, int64_t slot,
+                                           int open_grp, const int64_t* s_row) {
   using W = typename Codes8<BITS>::W;
   constexpr int BATCH = 4;
   const LayoutDev& L = A.L;
@@ -202,8 +171,6 @@ __device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t*
     const __half* vm_p = reinterpret_cast<const __half*>(page + L.o_vm) + h * L.NG + d0 / L.VG;
     T* ko_p = A.k_out + row0 * A.o_s0 + h * A.o_s1 + d0;
     T* vo_p = A.v_out + row0 * A.o_s0 + h * A.o_s1 + d0;
-    float2 shift[4] = {};
-    if (A.center) k_center<T>(A, req, h, d0, shift);
     for (int g0 = t0; g0 < t1;) {  // tokens [g0, g1) share a K group
       const int grp = g0 / L.KG, g1 = min(t1, (grp + 1) * L.KG);
       const bool open = grp == open_grp;
@@ -234,9 +201,7 @@ __device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t*
             const int64_t o = slot * A.R.s_slot + (int64_t)(t - grp * L.KG) * A.R.s_pos + h * A.R.s_head + d0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              float2 k = make_float2(ld_dt(A.R.base, A.R.dtype, o + 2 * i), ld_dt(A.R.base, A.R.dtype, o + 2 * i + 1));
-              if (A.center) k = __fadd2_rn(k, shift[i]);
-              ki[i] = pack2_rn<T>(k.x, k.y);
+              ki[i] = pack2_rn<T>(ld_dt(A.R.base, A.R.dtype, o + 2 * i), ld_dt(A.R.base, A.R.dtype, o + 2 * i + 1));
             }
           } else {
             unpack8<BITS>(kw[b], q);
@@ -244,8 +209,7 @@ __device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t*
             for (int i = 0; i < 4; ++i) {
               const float2 ks = __half22float2(reinterpret_cast<const __half2*>(&s8)[i]);
               const float2 km = __half22float2(reinterpret_cast<const __half2*>(&m8)[i]);
-              float2 k = __fadd2_rn(__fmul2_rn(q[i], ks), km);
-              if (A.center) k = __fadd2_rn(k, shift[i]);
+              const float2 k = __fadd2_rn(__fmul2_rn(q[i], ks), km);
               ki[i] = pack2_rn<T>(k.x, k.y);
             }
           }
@@ -269,19 +233,9 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_dense_vec_kernel(const DenseArgs<T> A) {
   __shared__ int64_t s_row[DENSE_TOK];
   const LayoutDev& L = A.L;
-  int item = blockIdx.x, t0 = 0;
-  if (A.slices > 0) {
-    item = blockIdx.x / A.slices;
-    t0 = (blockIdx.x - item * A.slices) * DENSE_TOK;
-  }
+  const int item = blockIdx.x / A.slices, t0 = (blockIdx.x - item * A.slices) * DENSE_TOK;
   const int4 w = reinterpret_cast<const int4*>(A.work)[item];
-  const int req = w.x, ctx = w.w;
-  int bi = w.y, row0 = w.z;  // block of the context, dense row of its first token
-  if (A.slices == 0) {  // w.y: slice of the context, w.z: dense row of its first token
-    bi = w.y * DENSE_TOK / L.BS;
-    t0 = w.y * DENSE_TOK - bi * L.BS;
-    row0 -= t0;
-  }
+  const int req = w.x, bi = w.y, row0 = w.z, ctx = w.w;  // block of the context, dense row of its first token
   const int t1 = min(min(L.BS, ctx - bi * L.BS), t0 + DENSE_TOK);
   if (t0 >= t1) return;
   const int64_t blk = A.bt[(int64_t)req * A.bt_s0 + bi];
@@ -292,9 +246,9 @@ __global__ void __launch_bounds__(256) dequant_dense_vec_kernel(const DenseArgs<
   const int open_grp = slot >= 0 ? (int)A.R.res_group[slot] : -1;
   if (t0 + (int)threadIdx.x < t1) s_row[threadIdx.x] = row_offset(A.pages, L, blk, t0 + threadIdx.x, bits);
   __syncthreads();
-  if (bits == 4) dense_rows<T, 4>(A, page, req, row0, t0, t1, slot, open_grp, s_row);
-  else if (bits == 8) dense_rows<T, 8>(A, page, req, row0, t0, t1, slot, open_grp, s_row);
-  else dense_rows<T, 2>(A, page, req, row0, t0, t1, slot, open_grp, s_row);
+  if (bits == 4) dense_rows<T, 4>(A, page, row0, t0, t1, slot, open_grp, s_row);
+  else if (bits == 8) dense_rows<T, 8>(A, page, row0, t0, t1, slot, open_grp, s_row);
+  else dense_rows<T, 2>(A, page, row0, t0, t1, slot, open_grp, s_row);
 }
 
 // Demotion, phase 2: requantize a block's dequantized contents (scratch: K then V, float
@@ -532,10 +486,9 @@ int echokv_gather(const echokv_layout* layout, const echokv_pages* pages, const 
   return check_launch("gather");
 }
 
-static int dequant_dense_impl(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
-                              const int32_t* work, int64_t n_work, bool by_slice, int center, const int32_t* block_table,
-                              int64_t bt_s0, void* k_out, void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype,
-                              void* stream) {
+int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                         const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
+                         void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream) {
   if (n_work <= 0) return ECHOKV_OK;
   LayoutDev L;
   ResidualDev R;
@@ -549,8 +502,8 @@ static int dequant_dense_impl(const echokv_layout* layout, const echokv_pages* p
   dequant_dense_kernel<T><<<(unsigned)n_work, 256, 0, st>>>(L, R, (const uint8_t*)pages->base, work, block_table, \
                                                            bt_s0, (T*)k_out, (T*)v_out, out_s0, out_s1)
   // 16-byte loads and stores need the stat arrays, the rows of the outputs and 8-channel chunks aligned
-  const int slices = by_slice ? 0 : (L.BS + DENSE_TOK - 1) / DENSE_TOK;
-  const int64_t ctas = by_slice ? n_work : n_work * slices;
+  const int slices = (L.BS + DENSE_TOK - 1) / DENSE_TOK;
+  const int64_t ctas = n_work * slices;
   const bool vec = out_dtype != ECHOKV_DT_F32 && ctas < (1ll << 31) && L.D % 8 == 0 && L.VG % 8 == 0 &&
                    ((L.o_ks | L.o_km | L.PS | L.o_data | L.CB) % 16) == 0 && (out_s0 % 8) == 0 && (out_s1 % 8) == 0 &&
                    ((reinterpret_cast<uintptr_t>(k_out) | reinterpret_cast<uintptr_t>(v_out) |
@@ -558,7 +511,7 @@ static int dequant_dense_impl(const echokv_layout* layout, const echokv_pages* p
 #define LAUNCH_VEC(T)                                                                                         \
   {                                                                                                           \
     DenseArgs<T> A = {L, R, (const uint8_t*)pages->base, work, block_table, bt_s0, (T*)k_out, (T*)v_out, out_s0, \
-                      out_s1, slices, center};                                                                        \
+                      out_s1, slices};                                                                                \
     dequant_dense_vec_kernel<T><<<(unsigned)ctas, 256, 0, st>>>(A);                                           \
   }
   if (vec) {
@@ -566,7 +519,6 @@ static int dequant_dense_impl(const echokv_layout* layout, const echokv_pages* p
     return check_launch("dequant_dense");
   }
 #undef LAUNCH_VEC
-  if (by_slice) return set_error(ECHOKV_E_UNSUPPORTED, "dequant_dense_slices: 16-bit outputs with 16-byte aligned rows only");
   switch (out_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;
     case ECHOKV_DT_F16: LAUNCH(__half); break;
@@ -575,22 +527,6 @@ static int dequant_dense_impl(const echokv_layout* layout, const echokv_pages* p
   }
 #undef LAUNCH
   return check_launch("dequant_dense");
-}
-
-int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
-                         const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
-                         void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream) {
-  return dequant_dense_impl(layout, pages, residual, work, n_work, false, 0, block_table, bt_s0, k_out, v_out, out_s0, out_s1,
-                            out_dtype, stream);
-}
-
-int echokv_dequant_dense_slices(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
-                                const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
-                                void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, int32_t center, void* stream) {
-  if (layout && layout->block_size % DENSE_TOK)
-    return set_error(ECHOKV_E_UNSUPPORTED, "dequant_dense_slices: block size %d is not a multiple of %d", layout->block_size, DENSE_TOK);
-  return dequant_dense_impl(layout, pages, residual, work, n_work, true, center, block_table, bt_s0, k_out, v_out, out_s0,
-                            out_s1, out_dtype, stream);
 }
 
 int64_t echokv_demote_scratch_bytes(const echokv_layout* layout, int64_t n) {

@@ -10,12 +10,7 @@ Two device paths:
   * row path: every query token is handed to the split-K decode kernel as a
     sequence whose length is its causal limit.  Each token re-reads its context,
     so this is for short chunks (the reference's fused path has the same
-    trade-off, kernels/prefill.py:10-13).  Where that re-reading costs more than
-    it saves (`short_chunks_as_dense`), the contexts are dequantized to fp16 and
-    the tensor-core attention kernel runs on fp16 operands -- the precision of the
-    decode kernel's operands, which the model's bf16 would not give.  One vector
-    per context and head is subtracted from its keys first, so that channels far
-    from zero keep that precision too.
+    trade-off, kernels/prefill.py:10-13).
   * dense path: dequantize every context once into ``[total_ctx, H, D]`` in the
     model dtype, then run the tensor-core attention kernel over it.
 """
@@ -31,7 +26,6 @@ from echokv_b200.kernels.decode import (BLOCKS_PER_SPLIT, EAGER_MAX_SPLITS, choo
                                         decode_parallelism)
 
 ROW_PATH_MAX_CHUNK = 64  # longer chunks take the dense path when it is available
-SLICE = 16               # tokens per entry of the row path's dequantization work list
 
 
 def build_dequant_work(prefill, req_of, block_size: int, device) -> torch.Tensor:
@@ -48,10 +42,8 @@ def build_dequant_work(prefill, req_of, block_size: int, device) -> torch.Tensor
     return to_device(torch.from_numpy(rows), device)
 
 
-def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.Tensor, dtype, by_slice: bool = False,
-                  center: bool = False):
-    """Dense ``[total_ctx, H, D]`` K and V (``dtype``) of the contexts in ``work`` (entries per block, or per
-    ``SLICE`` tokens with ``by_slice``, then optionally ``center``: K minus a constant per request, head and channel)."""
+def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.Tensor, dtype):
+    """Dense ``[total_ctx, H, D]`` K and V (``dtype``) of the contexts in ``work``."""
     L = store.layout
     k = torch.empty(total_ctx, L.num_kv_heads, L.head_size, device=store.device, dtype=dtype)
     v = torch.empty_like(k)
@@ -59,21 +51,18 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
         N.require_cuda(work, block_table)
         if block_table.dtype != torch.int32 or block_table.stride(1) != 1:
             block_table = block_table.to(torch.int32).contiguous()
-        launch = N.lib.echokv_dequant_dense_slices if by_slice else N.lib.echokv_dequant_dense
-        extra = (int(center),) if by_slice else ()
-        N.check(launch(
+        N.check(N.lib.echokv_dequant_dense(
             store.c_layout, store.c_pages, store.c_res, work.data_ptr(), work.shape[0],
             block_table.data_ptr(), block_table.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
-            N.dtype_code(dtype), *extra, N.stream_ptr(store.device)))
+            N.dtype_code(dtype), N.stream_ptr(store.device)))
     return k, v
 
 
 class Rows(tuple):
-    """Row-path metadata ``(query rows, requests, causal limits, longest limit)``; ``dense`` holds what running the same
-    chunks over dense contexts takes: the work list in 16-token slices, context rows, chunk table, longest chunk.
-    ``host_lens``: the causal limits on the host, which size the row path's splits."""
+    """Row-path metadata ``(query rows, requests, causal limits, longest limit)``; ``host_lens``: the causal limits on the
+    host, which size the row path's splits."""
 
-    dense = host_lens = None
+    host_lens = None
     _blocks = (None, 0)
 
     def blocks_per_split(self, block_size: int, slots: int) -> int:
@@ -89,53 +78,15 @@ def build_rows(prefill, req_of, device):
     start = np.array([p[0] for p, _ in pairs], dtype=np.int64)
     nq = np.array([max(p[1] - p[0], 0) for p, _ in pairs], dtype=np.int64)
     ctx = np.array([p[2] for p, _ in pairs], dtype=np.int64)
-    n = int(nq.sum())
-    count = -(-ctx // SLICE) if ctx.size else ctx
-    slices = int(count.sum())
-    buf = np.empty(3 * n + (n & 1) + 2 * (slices + len(pairs)), dtype=np.int64)  # one upload: rows, slices, chunks
-    rows = buf[: 3 * n].reshape(3, n)
+    rows = np.empty((3, int(nq.sum())), dtype=np.int64)
     at = np.arange(rows.shape[1]) - np.repeat(np.cumsum(nq) - nq, nq)  # place in the chunk
     rows[0] = np.repeat(start, nq) + at
     rows[1] = np.repeat(np.array([r for _, r in pairs], dtype=np.int64), nq)
     rows[2] = np.repeat(ctx - nq + 1, nq) + at
-    o_work = 3 * n + (n & 1)  # 16-byte aligned
-    work = buf[o_work: o_work + 2 * slices].view(np.int32).reshape(slices, 4)
-    chunks = buf[o_work + 2 * slices:].view(np.int32).reshape(len(pairs), 4)
-    first = np.cumsum(ctx) - ctx
-    work[:, 0] = np.repeat(np.array([r for _, r in pairs], dtype=np.int64), count)
-    work[:, 1] = np.arange(slices) - np.repeat(np.cumsum(count) - count, count)
-    work[:, 2] = np.repeat(first, count) + work[:, 1].astype(np.int64) * SLICE
-    work[:, 3] = np.repeat(ctx, count)
-    chunks[:, 0], chunks[:, 1], chunks[:, 2], chunks[:, 3] = start, start + nq, ctx, first
-    dev = to_device(torch.from_numpy(buf), device)
-    packed = dev[: 3 * n].view(3, n)
+    packed = to_device(torch.from_numpy(rows), device)
     out = Rows((packed[0], packed[1], packed[2], int(rows[2].max(initial=0))))
-    out.dense = (dev[o_work: o_work + 2 * slices].view(torch.int32).view(slices, 4), int(ctx.sum()),
-                 dev[o_work + 2 * slices:].view(torch.int32).view(len(pairs), 4), int(nq.max(initial=0)))
     out.host_lens = rows[2]
     return out
-
-
-def short_chunks_as_dense(prefill, num_kv_heads: int, num_q_heads: int) -> bool:
-    """Whether chunks short enough for the row path are cheaper over dense fp16 contexts.
-
-    Both sides in microseconds per layer on B200.  Row path: every token walks its context, 5.5 ns per 16 tokens
-    and 8 heads once the chip is full, 15 us around it.  Dense: 0.9 ns per context token and 8 heads to dequantize,
-    12 us for that and the query's conversion; the attention kernel's CTAs (128 rows of query token x head; 256 when
-    a chunk has more) each walk 128 keys in 2.2 us, one CTA per SM.  Measured, row / dense: 16 chunks of 33 behind
-    1,472 217 / 81 us, 4 of 50 behind 4,000 300 / 105, 8 of 40 behind 3,000 at one head per KV head 320 / 94, 16 of 8
-    behind 1,472 65 / 66, one of 33 behind 1,472 32 / 50, 8 of 30 behind 100 28 / 32.  The margin keeps a step on the
-    row path where the two are close.  Against 64-bit attention over the stored values the dense side's relative
-    error is the smaller one wherever it is chosen (16 x 33: 0.7e-3, row path 1.1e-3).
-    """
-    gqa = num_q_heads // num_kv_heads
-    longest = max(qe - qs for qs, qe, _, _ in prefill) * gqa
-    tile = 256 if longest > 128 else 128
-    row = 15.0 + sum((qe - qs) * ctx for qs, qe, ctx, _ in prefill) / 16 * 0.0055 * num_kv_heads / 8
-    ctx_all = sum(ctx for _, _, ctx, _ in prefill)
-    walk = sum(-(-(qe - qs) * gqa // tile) * (ctx / 128 * 2.2 + 5) for qs, qe, ctx, _ in prefill) * num_kv_heads / 148
-    dense = 12.0 + 0.0009 * ctx_all * num_kv_heads / 8 + max(walk, max(ctx for _, _, ctx, _ in prefill) / 128 * 2.2 + 5)
-    return dense < 0.8 * row
 
 
 def build_dense(prefill, req_of, block_size: int, device):
@@ -197,13 +148,6 @@ def prefill_attention(store, query: torch.Tensor, output: torch.Tensor, prefill,
     if rows is None:
         rows = build_rows(prefill, req_of, query.device)
     L = store.layout
-    if isinstance(rows, Rows) and dense_supported(store, query) and L.block_size % SLICE == 0 and L.head_size == 128 and \
-            query.shape[1] // L.num_kv_heads <= 8 and short_chunks_as_dense(prefill, L.num_kv_heads, query.shape[1]):
-        work, total, chunks, max_chunk = rows.dense
-        k, v = dequant_dense(store, work, total, block_table, torch.float16, by_slice=True, center=True)
-        dense_attention(query.to(torch.float16), k, v, chunks, max_chunk, out3, softmax_scale,
-                        sum(qe - qs for qs, qe, _, _ in prefill))
-        return
     q_rows, reqs, lens, max_len = rows
     # Splits sized for the rows at hand: the fixed default (16 blocks, 1,024 tokens at block 64) left short chunks to a few
     # dozen serial tiles per item.

@@ -266,14 +266,6 @@ int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages,
                          const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0,
                          void* k_out, void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, void* stream);
 
-/* The same from a work list in slices of 16 tokens (request, slice of the context, dense row of its first token, ctx),
- * which does not depend on the block size; block_size must be a multiple of 16, the outputs 16-bit with 16-byte aligned
- * rows.  `center` != 0 subtracts one constant per request, head and channel from every key (attention weights do not
- * change; channels far from zero keep their precision). */
-int echokv_dequant_dense_slices(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
-                                const int32_t* work, int64_t n_work, const int32_t* block_table, int64_t bt_s0, void* k_out,
-                                void* v_out, int64_t out_s0, int64_t out_s1, int32_t out_dtype, int32_t center, void* stream);
-
 /* Chunked-prefill attention over dense contexts: the attention step of the dense path of
  * prefill_attention (kernels/prefill.py:118-167; the reference calls a flash-attention library
  * there, :145-153; oracle :210-236).  k_dense / v_dense [total_ctx, H, D] are what
