@@ -22,8 +22,7 @@ import torch
 
 from echokv_b200 import _native as N
 from echokv_b200._util import to_device
-from echokv_b200.kernels.decode import (BLOCKS_PER_SPLIT, EAGER_MAX_SPLITS, choose_blocks_per_split, decode_attention,
-                                        decode_parallelism)
+from echokv_b200.kernels.decode import decode_attention
 
 ROW_PATH_MAX_CHUNK = 64  # longer chunks take the dense path when it is available
 
@@ -58,20 +57,6 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
     return k, v
 
 
-class Rows(tuple):
-    """Row-path metadata ``(query rows, requests, causal limits, longest limit)``; ``host_lens``: the causal limits on the
-    host, which size the row path's splits."""
-
-    host_lens = None
-    _blocks = (None, 0)
-
-    def blocks_per_split(self, block_size: int, slots: int) -> int:
-        """Blocks per split of the row path for the step (worked out by its first layer)."""
-        if self._blocks[0] != (block_size, slots):
-            self._blocks = ((block_size, slots), choose_blocks_per_split(self.host_lens, block_size, EAGER_MAX_SPLITS, slots))
-        return self._blocks[1]
-
-
 def build_rows(prefill, req_of, device):
     """Row-path metadata: per query token its row, its request and its causal limit (device int64)."""
     pairs = list(zip(prefill, req_of))
@@ -84,9 +69,7 @@ def build_rows(prefill, req_of, device):
     rows[1] = np.repeat(np.array([r for _, r in pairs], dtype=np.int64), nq)
     rows[2] = np.repeat(ctx - nq + 1, nq) + at
     packed = to_device(torch.from_numpy(rows), device)
-    out = Rows((packed[0], packed[1], packed[2], int(rows[2].max(initial=0))))
-    out.host_lens = rows[2]
-    return out
+    return packed[0], packed[1], packed[2], int(rows[2].max(initial=0))
 
 
 def build_dense(prefill, req_of, block_size: int, device):
@@ -147,12 +130,7 @@ def prefill_attention(store, query: torch.Tensor, output: torch.Tensor, prefill,
         return
     if rows is None:
         rows = build_rows(prefill, req_of, query.device)
-    L = store.layout
     q_rows, reqs, lens, max_len = rows
-    # Splits sized for the rows at hand: the fixed default (16 blocks, 1,024 tokens at block 64) left short chunks to a few
-    # dozen serial tiles per item.
-    blocks, slots = BLOCKS_PER_SPLIT, decode_parallelism(store, query.shape[1]) if isinstance(rows, Rows) else 0
-    if slots > 0 and max_len > 0:
-        blocks = rows.blocks_per_split(L.block_size, slots)
-    decode_attention(store, query, block_table, lens, softmax_scale, blocks, q_rows=q_rows, bt_rows=reqs, out=out3,
+    # Splits of the default size: a token's split then follows from its own context, and its bits from the request alone.
+    decode_attention(store, query, block_table, lens, softmax_scale, q_rows=q_rows, bt_rows=reqs, out=out3,
                      max_len=max_len)

@@ -1,5 +1,5 @@
-"""Short prompt chunks (at most 64 tokens): what a call accepts, allocates and can represent does not depend on how many
-chunks share the step."""
+"""Short prompt chunks (at most 64 tokens): what a call returns, accepts and allocates follows from the chunk itself, not
+from the chunks it shares a step with."""
 
 import numpy as np
 import pytest
@@ -49,6 +49,28 @@ def _attend(store, query, table, chunks, out=None):
     out = torch.zeros_like(query) if out is None else out
     prefill_attention(store, query, out, prefill, req_of, table, D ** -0.5, rows=build_rows(prefill, req_of, query.device))
     return out
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+def test_a_chunk_does_not_depend_on_its_neighbours(dtype):
+    """The same bits alone, among chunks that fill the chip, and token by token through decode attention."""
+    import torch
+    from echokv_b200.kernels.decode import decode_attention
+
+    dt = getattr(torch, dtype)
+    store, table = _store(4000, dt)
+    chunks = [(33, 1472)] + [(40 + i, 4000 - 17 * i) for i in range(16)]
+    q = _query(sum(n for n, _ in chunks), 4, dt)
+    together = _attend(store, q, table, chunks)
+    at = 0
+    for n, ctx in chunks[:3]:
+        alone = _attend(store, q[at: at + n], table, [(n, ctx)])
+        assert torch.equal(alone, together[at: at + n])
+        lens = torch.arange(ctx - n + 1, ctx + 1, device="cuda")
+        want = torch.zeros_like(alone)
+        decode_attention(store, q[at: at + n], table, lens, D ** -0.5, bt_rows=torch.zeros_like(lens), out=want, max_len=ctx)
+        assert torch.equal(alone, want)
+        at += n
 
 
 @pytest.mark.parametrize("form", ["odd output stride", "output off 16 bytes", "query off 16 bytes", "odd query stride",
