@@ -369,7 +369,7 @@ class EchoKVAttentionImpl(AttentionImpl[EchoKVMetadata]):
             decode_attention(self.store, query, md.block_table, md.decode_lens, self.scale, md.split_floor,
                              q_rows=md.decode_rows, bt_rows=md.decode_reqs,
                              out=output.view(output.shape[0], -1, query.shape[-1]), num_splits=md.num_splits,
-                             bps_dev=md.bps_dev)
+                             bps_dev=md.bps_dev, planned=md.write.launched)
         # A graph captures the copy unconditionally: its row indices are valid either way.
         if md.fire or _capturing(query):
             gather_rows(query, md.canary_rows, self.stash)

@@ -39,22 +39,34 @@ int check_launch(const char* what);
 // ---- programmatic dependent launch ---------------------------------------------------------
 // A kernel launched with `launch_pdl` may be scheduled while the kernel before it on the stream still runs: its
 // CTAs take their places as SMs free up and run whatever precedes `pdl_wait()`, which returns once the earlier
-// kernel has completed and its writes are visible.  Every CTA calls `pdl_wait()` before it reads or writes
-// anything another kernel touches (so completion of this kernel implies completion of the one before it), and
-// `pdl_launch_dependents()` lets the next such kernel start being scheduled.  Launched the ordinary way, or after
-// something that is not a kernel, both are no-ops.
+// kernel has completed and its writes are visible.  `pdl_launch_dependents()` lets the next such kernel start being
+// scheduled; a kernel that does not call it lets its dependents start as its last CTAs exit, which says nothing about
+// the visibility of its writes.  Every CTA calls `pdl_wait()` before it writes anything another kernel touches (so
+// completion of this kernel implies completion of the one before it).  One kernel reads ahead of its wait: the split
+// kernel of a planned decode step (echokv_decode_step), whose lengths, rows, block table, page headers and residual map
+// were written by kernels and copies ahead of the step's first write.  All kernels of a step trigger at their start, so
+// nothing in their chain would hold the split kernel back until those writers have completed, were it not that the
+// step's first write (echokv_write_step, as opposed to echokv_write_step_next) is launched the ordinary way: it starts
+// when everything before it has completed and is visible, and what follows starts after it.  A trigger after the
+// wait in every write step would do too, but put the split kernel's launch back onto the critical path (1 sequence of 500
+// tokens x 32 layers 540 -> 640 us a step).  Launched the ordinary way, or after something that is not a kernel, both
+// are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+cudaError_t launch_after(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  return launch_after(true, kernel, grid, block, smem, st, args...);
 }
 
 // ---- element access by runtime dtype ----------------------------------------------------

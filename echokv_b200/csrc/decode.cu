@@ -134,8 +134,8 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
                        const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
                        void* scratch, int64_t scratch_bytes, void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
                        float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
-                       const int32_t* blocks_per_split_dev, bool zero_state, int64_t num_seqs, int32_t num_q_heads,
-                       void* stream) {
+                       const int32_t* blocks_per_split_dev, bool zero_state, bool planned, int64_t num_seqs,
+                       int32_t num_q_heads, void* stream) {
   if (num_seqs <= 0) return ECHOKV_OK;
   LayoutDev L;
   ResidualDev R;
@@ -164,6 +164,7 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
   A.scale_log2e = softmax_scale * 1.4426950408889634f;
   A.num_splits = num_splits; A.bps_min = blocks_per_split; A.gqa = gqa; A.Hq = num_q_heads;
   A.bps_dev = blocks_per_split_dev;
+  A.planned = planned;
   cudaStream_t st = (cudaStream_t)stream;
   const uint8_t* pg = (const uint8_t*)pages->base;
 
@@ -199,7 +200,18 @@ int echokv_decode_ex(const echokv_layout* layout, const echokv_pages* pages, con
                      const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream) {
   return decode_impl(layout, pages, residual, query, q_s0, q_s1, q_dtype, q_rows, block_table, bt_s0, bt_rows, lens, scratch,
                      scratch_bytes, out, o_s0, o_s1, out_dtype, softmax_scale, num_splits, blocks_per_split,
-                     blocks_per_split_dev, false, num_seqs, num_q_heads, stream);
+                     blocks_per_split_dev, false, false, num_seqs, num_q_heads, stream);
+}
+
+int echokv_decode_step(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                       const void* query, int64_t q_s0, int64_t q_s1, int32_t q_dtype, const int64_t* q_rows,
+                       const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
+                       void* scratch, int64_t scratch_bytes, void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
+                       float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
+                       const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream) {
+  return decode_impl(layout, pages, residual, query, q_s0, q_s1, q_dtype, q_rows, block_table, bt_s0, bt_rows, lens, scratch,
+                     scratch_bytes, out, o_s0, o_s1, out_dtype, softmax_scale, num_splits, blocks_per_split,
+                     blocks_per_split_dev, false, true, num_seqs, num_q_heads, stream);
 }
 
 int echokv_decode(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
@@ -209,7 +221,7 @@ int echokv_decode(const echokv_layout* layout, const echokv_pages* pages, const 
                   float softmax_scale, int32_t num_splits, int32_t blocks_per_split, int64_t num_seqs,
                   int32_t num_q_heads, void* stream) {
   return decode_impl(layout, pages, residual, query, q_s0, q_s1, q_dtype, q_rows, block_table, bt_s0, bt_rows, lens, scratch,
-                     scratch_bytes, out, o_s0, o_s1, out_dtype, softmax_scale, num_splits, blocks_per_split, nullptr, true,
+                     scratch_bytes, out, o_s0, o_s1, out_dtype, softmax_scale, num_splits, blocks_per_split, nullptr, true, false,
                      num_seqs, num_q_heads, stream);
 }
 

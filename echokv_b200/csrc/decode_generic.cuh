@@ -27,6 +27,7 @@ struct DecodeArgs {
   float scale_log2e;
   int num_splits, bps_min, gqa, Hq;
   const int32_t* bps_dev;  // optional: blocks per split chosen by the host for this step, read at run time
+  int planned;             // the step's metadata was final before the kernel in front of the split kernel (echokv_decode_step)
   int out_vec;             // the merge can store a lane's channels of `out` at once (its launcher sets it)
   int* state;              // work-queue state at the start of the scratch: [0] = the split kernel's item counter
 };

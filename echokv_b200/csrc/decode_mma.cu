@@ -903,9 +903,10 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
   }
   __syncthreads();
   // Barriers and ring are set up.  From here on the consumers read what the kernels before this one wrote (queries,
-  // pages, split partials); the producer first resolves its first work item's metadata, which no kernel of the step
-  // writes (lengths, block table, page headers and the residual map are set before the step's kernels start).
-  if (warp != H) pdl_wait();
+  // pages, split partials).  In a planned step the producer first resolves its first work item's metadata (lengths, block
+  // table, page headers and the residual map were final before the write step started, see common.cuh); in any other
+  // call a kernel right before this one may have written them, and it waits too.
+  if (warp != H || !A.planned) pdl_wait();
 
   bool ok = true;
   if (warp == H) {
@@ -954,7 +955,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // The dependency wait comes as late as it can: the first unit is planned and its first stage prepared ahead of it,
     // down to the copies themselves, which read pages that the write step before this kernel may still be storing to.
     // (The work counter, which the merge kernel before may still be resetting, is not touched before it either.)
-    bool waited = false;
+    bool waited = !A.planned;
     auto wait_once = [&]() {
       if (!waited) { pdl_wait(); waited = true; }
     };

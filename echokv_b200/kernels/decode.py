@@ -90,7 +90,8 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
                      softmax_scale: float, blocks_per_split: int = BLOCKS_PER_SPLIT,
                      q_rows: torch.Tensor | None = None, bt_rows: torch.Tensor | None = None,
                      out: torch.Tensor | None = None, max_len: int | None = None,
-                     num_splits: int | None = None, bps_dev: torch.Tensor | None = None) -> torch.Tensor:
+                     num_splits: int | None = None, bps_dev: torch.Tensor | None = None,
+                     planned: bool = False) -> torch.Tensor:
     """Attention of one query token per sequence over each sequence's cache.
 
     Sequence ``i`` uses query row ``q_rows[i]`` and block-table row ``bt_rows[i]``
@@ -101,9 +102,12 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
     splits of ``max(blocks_per_split, ceil(blocks / num_splits))`` blocks -- a
     function of the sequence alone, so results are batch-invariant.  ``bps_dev`` (one int32 on the
     device, or the low half of an int64) raises ``blocks_per_split`` at run time: a captured graph
-    keeps reading it, so the host can size the splits for every replayed step.
+    keeps reading it, so the host can size the splits for every replayed step.  ``planned``: a write of the
+    same step is ahead on the stream, and everything but the queries and the pages' rows was final before it, so the
+    kernel may read that while the kernel before it still runs.
     """
     L = store.layout
+    given = (block_table, seq_lens, q_rows, bt_rows)
     N.require_cuda(query, block_table, seq_lens, out)
     if query.dim() != 3 or query.shape[2] != L.head_size:
         raise ValueError("query must be [T, Hq, D]")
@@ -135,7 +139,10 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
         N.require_cuda(bps_dev)
         if bps_dev.dtype not in (torch.int32, torch.int64) or bps_dev.numel() < 1:
             raise TypeError("bps_dev must hold one int32 / int64 on the device")
-    N.check(N.lib.echokv_decode_ex(
+    # a conversion above is itself the kernel before this one
+    planned = planned and given[0] is block_table and given[1] is lens and given[2] is q_rows and given[3] is bt_rows
+    launch = N.lib.echokv_decode_step if planned else N.lib.echokv_decode_ex
+    N.check(launch(
         store.c_layout, store.c_pages, store.c_res,
         query.data_ptr(), query.stride(0), query.stride(1), N.dtype_code(query.dtype), N.ptr(q_rows),
         block_table.data_ptr(), block_table.stride(0), N.ptr(bt_rows), lens.data_ptr(),

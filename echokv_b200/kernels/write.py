@@ -73,7 +73,7 @@ def write_step(store, key: torch.Tensor, value: torch.Tensor, meta, kref: torch.
 
     ``stash`` = (source rows, int64 row indices on the device, destination): the canary's query
     rows.  Stores the same bytes as the three calls in that order (which is how steps of more than
-    1,024 rows run inside the library).
+    1,024 rows run inside the library).  ``meta.launched``: an earlier layer's write of the step is ahead on the stream.
     """
     if stash is not None and not _stash_vector_ok(*stash):
         write_step(store, key, value, meta, kref, full_grid, None)
@@ -96,13 +96,15 @@ def write_step(store, key: torch.Tensor, value: torch.Tensor, meta, kref: torch.
         N.require_cuda(src, rows, out)
         s_args = (src.data_ptr(), src.stride(0) * src.element_size(), rows.data_ptr(), out.shape[0], out.data_ptr(),
                   out[0].numel() * out.element_size())
-    N.check(N.lib.echokv_write_step(
+    launch = N.lib.echokv_write_step_next if meta.launched else N.lib.echokv_write_step
+    N.check(launch(
         store.c_layout, store.c_pages,
         key.data_ptr(), key.stride(0), key.stride(1), value.data_ptr(), value.stride(0), value.stride(1),
         N.dtype_code(key.dtype), tok.data_ptr(), tok.stride(0), store.c_res,
         N.ptr(kref), 0 if kref is None else kref.stride(0), 0 if kref is None else kref.stride(1),
         meta.n_rows, N.ptr(meta.fin) if n_fin else None, N.ptr(meta.fin_count) if n_fin else None, n_fin,
         *s_args, N.stream_ptr(key.device)))
+    meta.launched = meta.launched or meta.n_rows > 0
 
 
 def gather_rows(src: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) -> None:

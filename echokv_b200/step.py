@@ -286,6 +286,7 @@ class GroupRunner:
 
     def decode(self, layer: int, query: torch.Tensor, block_table: torch.Tensor, out: torch.Tensor,
                meta: StepMeta) -> None:
+        """Attention of the step's decode rows.  ``block_table`` is final before the step's first ``write``."""
         decode_attention(self.stores[layer], query, block_table, meta.decode_lens, self.scale, self.split_floor,
                          q_rows=meta.decode_rows, bt_rows=meta.decode_reqs, out=out, num_splits=meta.num_splits,
-                         bps_dev=meta.bps_dev)
+                         bps_dev=meta.bps_dev, planned=meta.write.launched)

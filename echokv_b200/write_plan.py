@@ -365,6 +365,7 @@ class WriteMeta:
     fin_count: torch.Tensor  # [1] int64: masks a full-grid (graph-captured) finalize
     n_rows: int
     n_fin: int
+    launched: bool = False  # a layer's write of the step is on the stream (see `write_step` and `decode_attention`)
 
 
 def stage_plan(plan: WritePlan, device, opened=None):

@@ -167,6 +167,18 @@ int echokv_write_step(const echokv_layout* layout, const echokv_pages* pages,
                       const void* stash_src, int64_t stash_src_row_stride_bytes, const int64_t* stash_rows,
                       int64_t stash_n, void* stash_dst, int64_t stash_row_bytes, void* stream);
 
+/* echokv_write_step of a further layer: the same stored bytes.  Where an echokv_write_step of the same step is ahead of
+ * it on the stream, and nothing since has written the step's plan or page headers, this launch may overlap the kernel
+ * before it; the step's first write starts only when everything before it has completed. */
+int echokv_write_step_next(const echokv_layout* layout, const echokv_pages* pages,
+                           const void* key, int64_t k_s0, int64_t k_s1,
+                           const void* value, int64_t v_s0, int64_t v_s1, int32_t kv_dtype,
+                           const int64_t* tok, int64_t tok_s0, const echokv_residual* residual,
+                           float* kref, int64_t kref_s0, int64_t kref_s1, int64_t n_rows,
+                           const int64_t* fin, const int64_t* fin_count, int64_t n_fin_launch,
+                           const void* stash_src, int64_t stash_src_row_stride_bytes, const int64_t* stash_rows,
+                           int64_t stash_n, void* stash_dst, int64_t stash_row_bytes, void* stream);
+
 /* Requantize full INT4/INT8 blocks to INT2 in place -- TieredKVCache._demote_lru
  * (tiered_cache.py:309-346).  `victims` int64 [n] on the device; `scratch` holds the blocks'
  * dequantized contents between the read and the rewrite (echokv_demote_scratch_bytes). */
@@ -218,6 +230,18 @@ int echokv_decode_ex(const echokv_layout* layout, const echokv_pages* pages, con
                      void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
                      float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
                      const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream);
+
+/* echokv_decode_ex behind an echokv_write_step of the same step (any layer's) on the same stream, where lens, q_rows,
+ * bt_rows, block_table, the split-size word, the page headers and the residual map were all written ahead of that
+ * write and nothing has changed them since.  The split kernel then resolves its first work items while the kernel
+ * before it still runs.  Call echokv_decode_ex otherwise. */
+int echokv_decode_step(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                       const void* query, int64_t q_s0, int64_t q_s1, int32_t q_dtype, const int64_t* q_rows,
+                       const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
+                       void* scratch, int64_t scratch_bytes,
+                       void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
+                       float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
+                       const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream);
 
 /* How many work items (sequence, split) the split kernel works on at the same time on the current device for
  * this layout and number of query heads, or 0 when the shape takes the generic kernel (one CTA per item and KV
