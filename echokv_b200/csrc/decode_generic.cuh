@@ -32,9 +32,10 @@ struct DecodeArgs {
   int* state;              // work-queue state at the start of the scratch: [0] = the split kernel's item counter
 };
 
-// Lower bound of a split's size in blocks: the call's argument, raised by the run-time value when there is one.
+// Lower bound of a split's size in blocks: the call's argument, raised by the run-time value when there is one (an
+// ordinary load: the word may have been written while a kernel launched ahead of time was already resident).
 __device__ __forceinline__ int bps_floor(const DecodeArgs& A) {
-  return A.bps_dev ? max(A.bps_min, (int)__ldg(A.bps_dev)) : A.bps_min;
+  return A.bps_dev ? max(A.bps_min, *A.bps_dev) : A.bps_min;
 }
 
 __device__ __forceinline__ float warp_max(float v) {

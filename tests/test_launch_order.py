@@ -31,6 +31,11 @@ def test_the_first_write_of_a_step_starts_when_everything_before_it_has_complete
     assert "cfg.numAttrs = early ? 1 : 0;" in (CSRC / "common.cuh").read_text()
 
 
+def test_no_load_that_may_be_moved_ahead_of_the_wait():
+    """``__ldg`` promises that nobody writes the word during the kernel's lifetime, which begins ahead of the wait."""
+    assert not [f.name for f in CSRC.glob("decode*.cu*") if "__ldg" in f.read_text()]
+
+
 def test_which_launches_a_step_makes(monkeypatch):
     """First write, further writes, decodes with and without a write ahead of them, and with tensors the call converts."""
     import torch
@@ -81,7 +86,8 @@ def test_split_kernel_waits_first_unless_the_step_was_planned():
 
 @pytest.mark.gpu
 def test_metadata_written_by_the_kernel_right_before():
-    """Lengths, rows and tables that a kernel just produced, or that the call itself converts, give the bits of settled ones."""
+    """Lengths, rows, tables and split sizes that a kernel just produced, or that the call itself converts, give the bits of
+    settled ones."""
     import torch
     from test_gpu_short_chunks import D, _query, _store
 
@@ -94,11 +100,12 @@ def test_metadata_written_by_the_kernel_right_before():
     for i in range(40):
         lens = torch.randint(1, 1001, (12,), device="cuda", generator=gen)
         perm = torch.randperm(12, device="cuda", generator=gen)
+        size = torch.tensor([2 + i % 7], device="cuda")
         torch.cuda.synchronize()
-        want = decode_attention(store, q, tables, lens, D ** -0.5, q_rows=perm)
+        want = decode_attention(store, q, tables, lens, D ** -0.5, 1, q_rows=perm, bps_dev=size)
         torch.cuda.synchronize()
         got = decode_attention(store, q, tables.long() if i % 2 else tables + 0, lens.int() if i % 3 else lens + zero, D ** -0.5,
-                               q_rows=perm.int() if i % 5 else perm + zero, planned=bool(i % 2))
+                               1, q_rows=perm.int() if i % 5 else perm + zero, bps_dev=size + 0, planned=bool(i % 2))
         assert torch.equal(got, want)
 
 
