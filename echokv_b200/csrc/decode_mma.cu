@@ -906,11 +906,12 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
   // pages, split partials).  In a planned step the producer first resolves its first work item's metadata (lengths, block
   // table, page headers and the residual map were final before the write step started, see common.cuh); in any other
   // call a kernel right before this one may have written them, and it waits too.
-  if (warp != H || !A.planned) pdl_wait();
+  if (warp != H) pdl_wait();
 
   bool ok = true;
   if (warp == H) {
     // ===================== producer warp =====================
+    if (!A.planned) pdl_wait();
     const int tpb = L.BS / TILE;                     // tiles per block
     const int U = tpb >= UNIT ? 1 : UNIT / tpb;      // blocks per unit
     const bool contig = L.BS == TILE && L.KG == TILE;  // a tile's four stats arrays form one run in the page
@@ -955,7 +956,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // The dependency wait comes as late as it can: the first unit is planned and its first stage prepared ahead of it,
     // down to the copies themselves, which read pages that the write step before this kernel may still be storing to.
     // (The work counter, which the merge kernel before may still be resetting, is not touched before it either.)
-    bool waited = !A.planned;
+    bool waited = false;
     auto wait_once = [&]() {
       if (!waited) { pdl_wait(); waited = true; }
     };
