@@ -1476,8 +1476,9 @@ static bool team_shape(const DecodeDevice& dv, int H, int gqa, TeamShape* out) {
 
 static bool mma_shape_ok(int H, int D_, int VG, int KG, int BS, int gqa) {
   using namespace mma;
-  // a block of a power of two of tokens: only then does a tile's run of rows never cross from one chunk to the next
-  return D_ == D && VG == 32 && KG % TILE == 0 && BS % TILE == 0 && (BS & (BS - 1)) == 0 && gqa <= 8 &&
+  // a block of a power of two of tokens: only then does a tile's run of rows never cross from one chunk to the next;
+  // of at most UNIT tiles: the producer plans at least one whole block at a time
+  return D_ == D && VG == 32 && KG % TILE == 0 && BS % TILE == 0 && (BS & (BS - 1)) == 0 && BS <= UNIT * TILE && gqa <= 8 &&
          (H == 1 || H == 2 || H == 4 || H == 8);
 }
 

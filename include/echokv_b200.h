@@ -270,8 +270,9 @@ int echokv_decode_static(const echokv_layout* layout, const echokv_pages* pages,
                          int64_t num_seqs, int32_t num_q_heads, void* stream);
 
 /* Kernel selection of echokv_decode: 0 (default) picks the tensor-core kernel when the shape fits
- * (head_size 128, v_group 32, 1/2/4/8 KV heads, <= 8 query heads per KV head, block_size and k_group
- * multiples of 16) and the generic CUDA-core kernel otherwise; 1 always takes the generic kernel.  Returns the previous setting.
+ * (head_size 128, v_group 32, 1/2/4/8 KV heads, <= 8 query heads per KV head, k_group a
+ * multiple of 16, block_size a power of two from 16 to 256) and the generic CUDA-core kernel otherwise; 1 always takes the
+ * generic kernel.  Returns the previous setting.
  * No counterpart in the reference (its Triton autotuner plays this role, kernels/decode.py:265-280). */
 int echokv_set_decode_path(int path);
 

@@ -105,6 +105,18 @@ def test_dense_attention_of_many_uneven_chunks(pad):
             assert (out[qs:qe].float() - want.transpose(0, 1)).abs().max().item() <= 2e-2
 
 
+@pytest.mark.parametrize("bs,kg", [(128, 64), (256, 64), (512, 64), (1024, 128)])
+def test_decode_of_large_blocks(bs, kg):
+    """Blocks of up to 256 tokens are what one plan of the tensor-core kernel holds; larger ones take the generic kernel."""
+    from cuda_runner import run_cuda
+    from echokv_b200.kernels.decode import decode_parallelism
+
+    sc = S.build_attention(f"bs{bs}", 2, 128, bs, 8, [700, bs, 33, 2 * bs + 5], [4, 8], seed=8, kg=kg, dtype="f16", gqa=4)
+    got = run_cuda(sc)
+    assert (decode_parallelism(got["_store"], 8) > 0) == (bs <= 256)
+    assert np.abs(got["attn_out"] - run_oracle(sc)["attn_out"]).max() <= 5e-3
+
+
 @pytest.mark.parametrize("h,d,bs,kg,dtype,rows", [(1, 128, 64, 64, "bf16", 7), (3, 64, 32, 32, "f16", 5), (8, 128, 16, 16, "bf16", 16),
                                                   (5, 128, 64, 32, "bf16", 41), (2, 128, 48, 48, "f16", 20), (2, 64, 16, 16, "bf16", 600)])
 @pytest.mark.parametrize("graph_semantics", [False, True])
