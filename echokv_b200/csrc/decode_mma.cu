@@ -933,13 +933,19 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     const int n_teams = gridDim.x * V;
     // Items exist up to the longest sequence's split count: the grid of splits is sized for the longest sequence a step may
     // ever have, and claiming its empty rest one atomic after the other held up every team's last item (64 splits in
-    // the grid, 9 in use: a dozen round trips per team).
-    int used_max = 0;
-    for (int i = lane; i < P.num_seqs; i += 32) {
-      const int nb = (int)((A.lens[i] + L.BS - 1) / L.BS), bps = max(bps_min, (nb + A.num_splits - 1) / A.num_splits);
-      used_max = max(used_max, (nb + bps - 1) / bps);
+    // the grid, 9 in use: a dozen round trips per team).  A sequence of n blocks uses at most min(num_splits,
+    // ceil(n / bps_min)) splits, so the longest one bounds the items.  Every producer of the grid runs the loop: with
+    // the split rule's divisions per sequence in it, 4,096 rows of 40 tokens at one KV head took 97 us, now 51 us, and
+    // 256 of 1,000 took 31.4, now 29.6 us.
+    int used_max = 1;
+    if (A.num_splits > 1) {
+      int longest = 0;
+#pragma unroll 4
+      for (int i = lane; i < P.num_seqs; i += 32) longest = max(longest, (int)A.lens[i]);
+      longest = __reduce_max_sync(0xffffffffu, longest);
+      used_max = min(A.num_splits, ((longest + L.BS - 1) / L.BS + bps_min - 1) / bps_min);
     }
-    const int n_items = P.num_seqs * __reduce_max_sync(0xffffffffu, used_max);
+    const int n_items = P.num_seqs * used_max;
     auto advance = [&]() {  // move to the next unit (claiming a new item when needed); false when there is no work left
       if (have && base + U < b_end) { base += U; return true; }
       for (;;) {
