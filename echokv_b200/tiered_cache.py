@@ -116,6 +116,12 @@ for _bits, _n in NEXTRA.items():
 _SLOT = np.arange(3)
 
 
+def block_ids(blocks) -> np.ndarray:
+    """Block ids as int64 ``[n]``: an array, a tensor or any iterable of them (a set too, which numpy takes for one object)."""
+    ids = np.asarray(blocks)
+    return np.asarray(list(set(ids.tolist())) if ids.dtype == object else ids, dtype=np.int64).reshape(-1)
+
+
 class ChunkPool:
     """Host free list of the spare chunk slots (1 .. k_c-1 of every page) of one layer.
 
@@ -309,7 +315,7 @@ class TieredKVCache:
         self.pool.release_many(blocks, 0)
         short = NEXTRA[target_bits] * blocks.size - len(self.pool.free)
         if short > 0:
-            keep = blocks if protect is None else np.concatenate([blocks, np.asarray(protect, dtype=np.int64).reshape(-1)])
+            keep = blocks if protect is None else np.concatenate([blocks, block_ids(protect)])
             self._demote_lru(short, keep)
         tiers = self.pool.allot(blocks, target_bits)
         count = np.bincount(tiers, minlength=9).tolist()
