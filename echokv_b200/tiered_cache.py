@@ -138,13 +138,8 @@ class ChunkPool:
         self.tier = np.zeros(num_blocks, dtype=np.int64)  # host copy of every block's tier
         self.table = np.zeros((num_blocks, 3), dtype=np.int64)  # extra chunk ids per block
 
-    def release(self, block: int, new_tier: int) -> None:
-        n = NEXTRA.get(int(self.tier[block]), 0)
-        self.free.extend(self.table[block, :n].tolist())
-        self.tier[block] = new_tier
-
     def release_many(self, blocks: np.ndarray, new_tier: int) -> None:
-        """``release`` of every block in order."""
+        """Every block (unique ids), in order: its extra chunks return to the pool, it becomes ``new_tier``."""
         n = _NEXTRA_OF[self.tier[blocks]]
         if n.any():
             self.free.extend(self.table[blocks][_SLOT < n[:, None]].tolist())
@@ -175,6 +170,16 @@ class ChunkPool:
         hdr[:, 0] = self.tier[blocks]
         hdr[:, 4:] = np.ascontiguousarray(self.table[blocks].astype(np.int32)).view(np.uint8)
         return hdr
+
+
+def lru_victims(tier: np.ndarray, full: np.ndarray, last: np.ndarray, chunks_needed: int, keep: np.ndarray) -> np.ndarray:
+    """The least recently written INT4/INT8 blocks (``full``: mask of full blocks, ``last``: step of the last write; ties by
+    block id) without those in ``keep``, up to the one whose extra chunks make ``chunks_needed``, or all there are."""
+    ranked = np.flatnonzero((tier >= 4) & full)
+    ranked = ranked[np.argsort(last[ranked], kind="stable")]
+    ranked = ranked[~np.isin(ranked, keep)]
+    freed = np.cumsum(_NEXTRA_OF[tier[ranked]])
+    return ranked[: int(np.searchsorted(freed, chunks_needed)) + 1]
 
 
 class TieredKVCache:
@@ -331,12 +336,7 @@ class TieredKVCache:
 
     def _demote_lru(self, chunks_needed: int, keep: np.ndarray) -> None:
         """Requantize the least recently written full INT4/INT8 blocks to INT2, freeing their chunks."""
-        tier = self.pool.tier
-        full = np.flatnonzero((tier >= 4) & (self.shared.fill_h == self.layout.block_size))
-        ranked = full[np.argsort(self.shared.last_h[full], kind="stable")]
-        ranked = ranked[~np.isin(ranked, keep)]
-        freed = np.cumsum(_NEXTRA_OF[tier[ranked]])
-        victims = ranked[: int(np.searchsorted(freed, chunks_needed)) + 1]  # up to the one that frees enough
+        victims = lru_victims(self.pool.tier, self.shared.fill_h == self.layout.block_size, self.shared.last_h, chunks_needed, keep)
         if not victims.size:
             return
         vb = to_device(torch.from_numpy(victims), self.device)

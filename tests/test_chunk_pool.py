@@ -21,6 +21,46 @@ def test_block_ids_of_a_tensor():
     assert block_ids(torch.tensor([4, 2])).tolist() == [4, 2]
 
 
+@pytest.mark.parametrize("seed", range(6))
+def test_release_of_blocks_of_mixed_tiers(seed):
+    """Chunks return in block order, each block's first chunk first, whatever tiers the blocks hold."""
+    from echokv_b200.tiered_cache import NEXTRA, ChunkPool
+
+    rng = np.random.default_rng(seed)
+    pool = ChunkPool(24, 4)
+    for _ in range(4):
+        pool.allot(rng.permutation(np.flatnonzero(pool.tier == 0))[:5], int(rng.choice([2, 4, 8])))
+    blocks = rng.permutation(24)[:16]
+    want, tier = list(pool.free), pool.tier.copy()
+    for b in blocks.tolist():
+        want += pool.table[b, : NEXTRA.get(int(tier[b]), 0)].tolist()
+    assert len(set(tier.tolist())) > 2
+    pool.release_many(blocks, 2)
+    assert pool.free == want and (pool.tier[blocks] == 2).all()
+    rest = np.setdiff1d(np.arange(24), blocks)
+    assert np.array_equal(pool.tier[rest], tier[rest])
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_victims_are_those_of_the_sequential_loop(seed):
+    """Every shortage from one chunk to more than there are, exact fits among them; blocks written in the same step, blocks
+    that are not full, protected ones."""
+    from echokv_b200.tiered_cache import NEXTRA, lru_victims
+
+    rng = np.random.default_rng(seed)
+    n = 20
+    tier, full = rng.choice([0, 2, 4, 8], size=n), rng.random(n) < 0.7
+    last, keep = rng.integers(0, 6, size=n), rng.permutation(n)[: int(rng.integers(0, 5))]
+    for needed in range(1, 3 * n):
+        want, freed = [], 0
+        for b in sorted((b for b in range(n) if tier[b] >= 4 and full[b] and b not in keep), key=lambda b: (last[b], b)):
+            if freed >= needed:
+                break
+            want.append(b)
+            freed += NEXTRA[int(tier[b])]
+        assert lru_victims(tier, full, last, needed, keep).tolist() == want
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", [set, list, np.array])
 def test_protected_blocks_of_every_form_stay(form):

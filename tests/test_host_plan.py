@@ -81,8 +81,7 @@ def test_chunk_pool_matches_oracle_order():
     for _ in range(60):
         blocks = np.unique(rng.integers(0, n, size=int(rng.integers(1, 6))))
         target = int(rng.choice([2, 4, 8]))
-        for b in blocks.tolist():
-            pool.release(b, 0)
+        pool.release_many(blocks, 0)
         tiers = pool.allot(blocks, target)
         _, hdr = ost.open_blocks(blocks, target)  # no full blocks: nothing to demote
         assert np.array_equal(pool.headers(blocks), hdr) and np.array_equal(tiers, ost.tag_h[blocks])
