@@ -46,7 +46,7 @@ int check_launch(const char* what);
 // kernel of a planned decode step (echokv_decode_step), whose lengths, rows, block table, page headers and residual map
 // were written by kernels and copies ahead of the step's first write.  All kernels of a step trigger at their start, so
 // nothing in their chain would hold the split kernel back until those writers have completed, were it not that the
-// step's first write (echokv_write_step, as opposed to echokv_write_step_next) is launched the ordinary way: it starts
+// step's first write (echokv_write_step_first) is launched the ordinary way: it starts
 // when everything before it has completed and is visible, and what follows starts after it.  A trigger after the
 // wait in every write step would do too, but put the split kernel's launch back onto the critical path (1 sequence of 500
 // tokens x 32 layers 540 -> 640 us a step).  Launched the ordinary way, or after something that is not a kernel, both

@@ -1071,14 +1071,14 @@ int echokv_seal_group(const echokv_layout* layout, const echokv_pages* pages, co
   return check_launch("seal_group");
 }
 
-// `next`: behind another write of the same step (see common.cuh).
+// `first`: the first write of a planned step (see common.cuh).
 static int write_step_impl(const echokv_layout* layout, const echokv_pages* pages, const void* key, int64_t k_s0,
                            int64_t k_s1, const void* value, int64_t v_s0, int64_t v_s1, int32_t kv_dtype,
                            const int64_t* tok, int64_t tok_s0, const echokv_residual* residual, float* kref,
                            int64_t kref_s0, int64_t kref_s1, int64_t n_rows, const int64_t* fin, const int64_t* fin_count,
                            int64_t n_fin_launch, const void* stash_src, int64_t stash_src_row_stride_bytes,
                            const int64_t* stash_rows, int64_t stash_n, void* stash_dst, int64_t stash_row_bytes,
-                           bool next, void* stream) {
+                           bool first, void* stream) {
   LayoutDev L;
   ResidualDev R;
   int rc = make_layout(layout, pages, &L);
@@ -1111,7 +1111,7 @@ static int write_step_impl(const echokv_layout* layout, const echokv_pages* page
     const FinArgs<T> FA = fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count);                               \
     const int parts = split_group_ok(L, FA.raw16 && TA.res_raw) ? split_parts(L, n_fin_launch) : 0;                \
     const unsigned grid = (unsigned)(n_rows + n_fin_launch * (parts > 0 ? parts : 1) + stash_ctas);                \
-    launch_after(next, write_step_kernel<T>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin_launch, parts, SA); \
+    launch_after(!first, write_step_kernel<T>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin_launch, parts, SA); \
   }
   switch (kv_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;
@@ -1135,13 +1135,13 @@ int echokv_write_step(const echokv_layout* layout, const echokv_pages* pages, co
                          stash_dst, stash_row_bytes, false, stream);
 }
 
-int echokv_write_step_next(const echokv_layout* layout, const echokv_pages* pages, const void* key, int64_t k_s0,
-                           int64_t k_s1, const void* value, int64_t v_s0, int64_t v_s1, int32_t kv_dtype,
-                           const int64_t* tok, int64_t tok_s0, const echokv_residual* residual, float* kref,
-                           int64_t kref_s0, int64_t kref_s1, int64_t n_rows, const int64_t* fin, const int64_t* fin_count,
-                           int64_t n_fin_launch, const void* stash_src, int64_t stash_src_row_stride_bytes,
-                           const int64_t* stash_rows, int64_t stash_n, void* stash_dst, int64_t stash_row_bytes,
-                           void* stream) {
+int echokv_write_step_first(const echokv_layout* layout, const echokv_pages* pages, const void* key, int64_t k_s0,
+                            int64_t k_s1, const void* value, int64_t v_s0, int64_t v_s1, int32_t kv_dtype,
+                            const int64_t* tok, int64_t tok_s0, const echokv_residual* residual, float* kref,
+                            int64_t kref_s0, int64_t kref_s1, int64_t n_rows, const int64_t* fin, const int64_t* fin_count,
+                            int64_t n_fin_launch, const void* stash_src, int64_t stash_src_row_stride_bytes,
+                            const int64_t* stash_rows, int64_t stash_n, void* stash_dst, int64_t stash_row_bytes,
+                            void* stream) {
   return write_step_impl(layout, pages, key, k_s0, k_s1, value, v_s0, v_s1, kv_dtype, tok, tok_s0, residual, kref, kref_s0, kref_s1,
                          n_rows, fin, fin_count, n_fin_launch, stash_src, stash_src_row_stride_bytes, stash_rows, stash_n,
                          stash_dst, stash_row_bytes, true, stream);

@@ -96,7 +96,7 @@ def write_step(store, key: torch.Tensor, value: torch.Tensor, meta, kref: torch.
         N.require_cuda(src, rows, out)
         s_args = (src.data_ptr(), src.stride(0) * src.element_size(), rows.data_ptr(), out.shape[0], out.data_ptr(),
                   out[0].numel() * out.element_size())
-    launch = N.lib.echokv_write_step_next if meta.launched else N.lib.echokv_write_step
+    launch = N.lib.echokv_write_step if meta.launched else N.lib.echokv_write_step_first
     N.check(launch(
         store.c_layout, store.c_pages,
         key.data_ptr(), key.stride(0), key.stride(1), value.data_ptr(), value.stride(0), value.stride(1),

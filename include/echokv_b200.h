@@ -167,17 +167,17 @@ int echokv_write_step(const echokv_layout* layout, const echokv_pages* pages,
                       const void* stash_src, int64_t stash_src_row_stride_bytes, const int64_t* stash_rows,
                       int64_t stash_n, void* stash_dst, int64_t stash_row_bytes, void* stream);
 
-/* echokv_write_step of a further layer: the same stored bytes.  Where an echokv_write_step of the same step is ahead of
- * it on the stream, and nothing since has written the step's plan or page headers, this launch may overlap the kernel
- * before it; the step's first write starts only when everything before it has completed. */
-int echokv_write_step_next(const echokv_layout* layout, const echokv_pages* pages,
-                           const void* key, int64_t k_s0, int64_t k_s1,
-                           const void* value, int64_t v_s0, int64_t v_s1, int32_t kv_dtype,
-                           const int64_t* tok, int64_t tok_s0, const echokv_residual* residual,
-                           float* kref, int64_t kref_s0, int64_t kref_s1, int64_t n_rows,
-                           const int64_t* fin, const int64_t* fin_count, int64_t n_fin_launch,
-                           const void* stash_src, int64_t stash_src_row_stride_bytes, const int64_t* stash_rows,
-                           int64_t stash_n, void* stash_dst, int64_t stash_row_bytes, void* stream);
+/* echokv_write_step of the first layer of a step whose decodes are echokv_decode_step calls: the same stored bytes, but
+ * the launch starts only when everything before it on the stream has completed (echokv_write_step's may overlap the
+ * kernel before it), so that what follows may read what was written before it without waiting for it. */
+int echokv_write_step_first(const echokv_layout* layout, const echokv_pages* pages,
+                            const void* key, int64_t k_s0, int64_t k_s1,
+                            const void* value, int64_t v_s0, int64_t v_s1, int32_t kv_dtype,
+                            const int64_t* tok, int64_t tok_s0, const echokv_residual* residual,
+                            float* kref, int64_t kref_s0, int64_t kref_s1, int64_t n_rows,
+                            const int64_t* fin, const int64_t* fin_count, int64_t n_fin_launch,
+                            const void* stash_src, int64_t stash_src_row_stride_bytes, const int64_t* stash_rows,
+                            int64_t stash_n, void* stash_dst, int64_t stash_row_bytes, void* stream);
 
 /* Requantize full INT4/INT8 blocks to INT2 in place -- TieredKVCache._demote_lru
  * (tiered_cache.py:309-346).  `victims` int64 [n] on the device; `scratch` holds the blocks'
@@ -231,7 +231,7 @@ int echokv_decode_ex(const echokv_layout* layout, const echokv_pages* pages, con
                      float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
                      const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream);
 
-/* echokv_decode_ex behind an echokv_write_step of the same step (any layer's) on the same stream, where lens, q_rows,
+/* echokv_decode_ex behind an echokv_write_step_first of the same step (any layer's) on the same stream, where lens, q_rows,
  * bt_rows, block_table, the split-size word, the page headers and the residual map were all written ahead of that
  * write and nothing has changed them since.  The split kernel then resolves its first work items while the kernel
  * before it still runs.  Call echokv_decode_ex otherwise. */

@@ -24,10 +24,10 @@ def _body(file: str, name: str) -> str:
 def test_the_first_write_of_a_step_starts_when_everything_before_it_has_completed():
     """Its launch carries no programmatic attribute; the writes of further layers may overlap the kernel before them."""
     text = (CSRC / "write.cu").read_text()
-    assert "launch_after(next, write_step_kernel<T>" in text
-    first, nxt = (text[text.index(f"int {name}("):] for name in ("echokv_write_step", "echokv_write_step_next"))
-    assert "stash_dst, stash_row_bytes, false, stream);" in first[: first.index("\n}\n")]
-    assert "stash_dst, stash_row_bytes, true, stream);" in nxt[: nxt.index("\n}\n")]
+    assert "launch_after(!first, write_step_kernel<T>" in text
+    first, nxt = (text[text.index(f"int {name}("):] for name in ("echokv_write_step_first", "echokv_write_step"))
+    assert "stash_dst, stash_row_bytes, true, stream);" in first[: first.index("\n}\n")]
+    assert "stash_dst, stash_row_bytes, false, stream);" in nxt[: nxt.index("\n}\n")]
     assert "cfg.numAttrs = early ? 1 : 0;" in (CSRC / "common.cuh").read_text()
 
 
@@ -71,7 +71,7 @@ def test_which_launches_a_step_makes(monkeypatch):
     empty = WriteMeta(tok=meta.tok, fin=meta.fin, fin_count=one, n_rows=0, n_fin=0)
     write.write_step(store, kv[:0], kv[:0], empty)
     assert not empty.launched
-    assert made == ["echokv_decode_ex", "echokv_write_step", "echokv_decode_step", "echokv_write_step_next", "echokv_decode_step"] + \
+    assert made == ["echokv_decode_ex", "echokv_write_step_first", "echokv_decode_step", "echokv_write_step", "echokv_decode_step"] + \
         ["echokv_decode_ex"] * 3
 
 
