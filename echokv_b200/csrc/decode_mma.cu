@@ -73,7 +73,7 @@ struct alignas(16) TilePlan {
   const unsigned char* run[4];      // the tile's token rows lie in up to four runs (one per chunk it touches) of `TILE >> run_shift` rows
 };
 constexpr int UNIT = 16;         // tiles planned at a time (one per producer lane)
-constexpr int PREFETCH_TILES = 4;  // tiles a team brings into L2 while it waits for the kernel before (27 MB over all teams at most)
+constexpr int PREFETCH_TILES = 4;  // tiles a team brings into L2 while it waits for the kernel before (over all teams 27 MB at INT4, 46 MB at INT8, at 8 or 4 KV heads)
 constexpr int MAX_NS = 8;        // stage ring slots at most
 constexpr int HDR_BYTES = 256;   // 2 * MAX_NS mbarriers
 static_assert(sizeof(StageHeader) == 32 && sizeof(TilePlan) % 16 == 0, "16-byte copies of headers");
@@ -905,7 +905,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
   // Barriers and ring are set up.  From here on the consumers read what the kernels before this one wrote (queries,
   // pages, split partials).  In a planned step the producer first resolves its first work item's metadata (lengths, block
   // table, page headers and the residual map were final before the write step started, see common.cuh); in any other
-  // call a kernel right before this one may have written them, and it waits too.
+  // call a kernel right before this one may have written them, and it waits too (5 us a layer at one sequence of 500 tokens).
   if (warp != H) pdl_wait();
 
   bool ok = true;

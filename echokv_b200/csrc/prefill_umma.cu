@@ -356,9 +356,7 @@ __global__ void __launch_bounds__(UM, 2) prefill_umma_kernel(Args A) {
     for (int c0 = 0; c0 < UD; c0 += 32) {
       float o[32];
       tmem_ld32(t_row + O_COL + c0, o);
-      if (live) {
-        store_out32(A, base_o + c0, o, inv);
-      }
+      if (live) store_out32(A, base_o + c0, o, inv);
     }
   }
   if (!ok && tid == 0 && A.status) atomicExch(A.status, 1);
@@ -654,9 +652,7 @@ __global__ void __launch_bounds__(UM * G + (TMA ? 64 : 32), 1) prefill_umma_pipe
       for (int c0 = 0; c0 < UD; c0 += 32) {
         float o[32];
         tmem_ld32(t_row + O_COL + c0, o);
-        if (live) {
-        store_out32(A, base_o + c0, o, inv);
-        }
+        if (live) store_out32(A, base_o + c0, o, inv);
       }
     }
   }
@@ -694,7 +690,6 @@ __device__ __forceinline__ void tmem_ld16_raw(uint32_t taddr, uint32_t (&r)[16])
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-//
 // Chunks of uneven length: the row tiles of all chunks form one list, longest first, so that the launch has next to no
 // empty CTAs and what is left at its end is short; a grid of (longest chunk's tiles) x chunks launched three empty CTAs
 // of 193 KB for each working one, in no order.  12 prompts of 87 - 2,900 tokens, 32 / 8 heads: 309 -> 222 us; 8 x 512 tokens
@@ -952,9 +947,7 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
       for (int c0 = 0; c0 < UD; c0 += 32) {
         float o[32];
         tmem_ld32(t_row + W_OCOL + c0, o);
-        if (live) {
-        store_out32(A, base_o + c0, o, inv);
-        }
+        if (live) store_out32(A, base_o + c0, o, inv);
       }
     }
   }

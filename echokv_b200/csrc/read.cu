@@ -98,7 +98,7 @@ dequant_dense_kernel(LayoutDev L, ResidualDev R, const uint8_t* __restrict__ pag
 // as small as keeps that chain worth it (a 64-token block as one CTA left 34 CTAs of 32 rounds each for a 2,112-token context:
 // 60 us, now 6.5 us), a thread stays on its channels (its K group's statistics are read once) with four tokens' loads
 // in flight, and a code becomes a float with one byte permute.  8 x 8,704 tokens x 8 heads x 128 at INT4 / INT8
-// alternating: 88 us, 156 us before = 0.66 of the measured copy peak at INT4 + INT8's mean of 383 MB.
+// alternating: 96 us, 156 us before = 0.61 of the measured copy peak at INT4 + INT8's mean of 383 MB.
 template <typename T> __device__ __forceinline__ uint32_t pack2_rn(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2_rn<__half>(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
