@@ -137,7 +137,8 @@ __device__ __forceinline__ void unpack8(const typename Codes8<BITS>::W& w, float
   }
 }
 
-constexpr int DENSE_TOK = 16;  // tokens per CTA
+constexpr int DENSE_TOK = 16;   // tokens per CTA
+constexpr int DENSE_BATCH = 4;  // of which a thread has this many in flight
 
 template <typename T>
 struct DenseArgs {
@@ -158,14 +159,14 @@ template <typename T, int BITS>
 __device__ __forceinline__ void dense_rows(const DenseArgs<T>& A, const uint8_t* page, int64_t row0, int t0, int t1, int64_t slot,
                                            int open_grp, const int64_t* s_row) {
   using W = typename Codes8<BITS>::W;
-  constexpr int BATCH = 4;
+  constexpr int BATCH = DENSE_BATCH;
   const LayoutDev& L = A.L;
   const int cpt = (L.H * L.D) / 8, cph = L.D / 8;
   const int side_bytes = (L.H * L.D * BITS) / 8;
-  const int lanes_t = cpt < 256 ? 256 / cpt : 1;  // tokens in work at once
-  const int t_off = cpt < 256 ? (int)threadIdx.x / cpt : 0;
+  const int threads = blockDim.x, lanes_t = cpt < threads ? threads / cpt : 1;  // tokens in work at once
+  const int t_off = cpt < threads ? (int)threadIdx.x / cpt : 0;
   if (t_off >= lanes_t) return;
-  for (int c = (int)threadIdx.x - t_off * cpt; c < cpt; c += 256) {
+  for (int c = (int)threadIdx.x - t_off * cpt; c < cpt; c += threads) {
     const int h = c / cph, d0 = (c - h * cph) * 8;
     const __half* vs_p = reinterpret_cast<const __half*>(page + L.o_vs) + h * L.NG + d0 / L.VG;
     const __half* vm_p = reinterpret_cast<const __half*>(page + L.o_vm) + h * L.NG + d0 / L.VG;
@@ -508,11 +509,17 @@ int echokv_dequant_dense(const echokv_layout* layout, const echokv_pages* pages,
                    ((L.o_ks | L.o_km | L.PS | L.o_data | L.CB) % 16) == 0 && (out_s0 % 8) == 0 && (out_s1 % 8) == 0 &&
                    ((reinterpret_cast<uintptr_t>(k_out) | reinterpret_cast<uintptr_t>(v_out) |
                      reinterpret_cast<uintptr_t>(pages->base) | reinterpret_cast<uintptr_t>(work)) % 16) == 0;
+  // Threads for DENSE_TOK / DENSE_BATCH tokens at once where the rows are so short that 256 threads would have a token each
+  // (and three repeated loads) and there are more CTAs than run at once (two per SM): one KV head of 128 channels, 16 x 500
+  // tokens 6.5 -> 4.2 us, 8 x 8,704 tokens 31 -> 13 us.  With fewer CTAs a token per thread is the shorter chain (700 tokens 3.6 us
+  // against 4.2).
+  const int chunks = L.H * L.D / 8 * (DENSE_TOK / DENSE_BATCH);
+  const unsigned threads = chunks < 256 && ctas > 2 * 148 ? (unsigned)(chunks + 31) / 32 * 32 : 256u;
 #define LAUNCH_VEC(T)                                                                                         \
   {                                                                                                           \
     DenseArgs<T> A = {L, R, (const uint8_t*)pages->base, work, block_table, bt_s0, (T*)k_out, (T*)v_out, out_s0, \
                       out_s1, slices};                                                                                \
-    dequant_dense_vec_kernel<T><<<(unsigned)ctas, 256, 0, st>>>(A);                                           \
+    dequant_dense_vec_kernel<T><<<(unsigned)ctas, threads, 0, st>>>(A);                                       \
   }
   if (vec) {
     if (out_dtype == ECHOKV_DT_F16) LAUNCH_VEC(__half) else LAUNCH_VEC(__nv_bfloat16)

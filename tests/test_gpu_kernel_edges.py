@@ -163,6 +163,26 @@ def test_demotion_across_block_shapes(h, d, bs, kg, bits):
     compare_store(sc, got, run_oracle(sc))
 
 
+@pytest.mark.parametrize("h,d,bs,kg,dtype", [(1, 64, 16, 16, "bf16"), (1, 128, 64, 32, "f16"), (3, 96, 48, 16, "bf16"), (2, 128, 32, 16, "f16")])
+def test_dense_dequantization_of_short_rows(h, d, bs, kg, dtype):
+    """Rows so short that a CTA has fewer than 256 threads once there are many of them (contexts of 5,000 tokens: 313 CTAs and
+    more), and with few CTAs; against the fp32 dequantization rounded to 16 bits, same bits."""
+    import torch
+    from cuda_runner import run_cuda
+    from echokv_b200.kernels.prefill import build_dense, dequant_dense
+
+    for lens in ([5003, 17], [79]):
+        sc = S.build_attention("short rows", h, d, bs, 8, lens, [8, 2, 4], seed=6, kg=kg, dtype=dtype, gqa=1, chunks=[1] * len(lens))
+        sc.prefill, prefill, sc.query = None, sc.prefill, None
+        store = run_cuda(sc)["_store"]
+        table = torch.from_numpy(sc.block_table).cuda()
+        work, total, _, _ = build_dense(prefill, sc.req_of, bs, "cuda")
+        want = dequant_dense(store, work, total, table, torch.float32)
+        for dt in (torch.float16, torch.bfloat16):
+            for a, b in zip(dequant_dense(store, work, total, table, dt), want):
+                assert torch.equal(a, b.to(dt))
+
+
 def test_headers_of_many_pools_in_one_launch():
     """More pools than one launch takes, empty entries among them."""
     import torch
