@@ -756,6 +756,16 @@ static int split_parts(const LayoutDev& L, int64_t n_groups) {
   return room < 1 ? 1 : (room < need ? (int)room : need);
 }
 
+// CTAs per group of write_step_kernel, or 0: a thread owns 8 channels over the group's tokens (finalize_group), which keeps more
+// CTAs on an SM.  That is the better route where a launch has far more groups than the chip works on at once: captured steps of
+// 1,024 rows x 8 heads x 128, us a layer, split / not: no group of 32 tokens complete 5.1 / 4.4, 62 complete 22.7 / 25.2,
+// all 54 / 43; at 512 rows 3.1 / 3.8, 10.2 / 19.7, 28 / 25.  At 64 tokens per group (all of 1,024: 88 / 94) and with short rows
+// (two heads of 64, 62 of 1,024: 10.6 / 18.6) the split is ahead throughout.
+constexpr int64_t SPLIT_MAX_GROUPS = 512;
+static int step_split(const LayoutDev& L, bool raw16, int64_t n_groups) {
+  return n_groups > 0 && split_group_ok(L, raw16) && (n_groups <= SPLIT_MAX_GROUPS || L.KG == 64 || L.H * L.D < 512) ? split_parts(L, n_groups) : 0;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(WT_WARPS * 32) finalize_split_kernel(const FinArgs<T> A, int parts) {
   const int64_t f = blockIdx.x / parts;
@@ -780,16 +790,17 @@ constexpr int STEP_MAX_ROWS = 1024;
 // A step's rows are a few hundred kilobytes: the time is the chain of dependent reads (token list -> page header ->
 // rows -> statistics -> codes), so a row's value and key are on their way while the header is looked up, and a
 // group's tokens are spread over lanes and CTAs (finalize_split).  Per layer: 12.4 -> 6.3 us at 64 sequences x 8 heads, 10.1 -> 5.6 us
-// at 16 sequences x 1 head, 20 -> 10 us at 575 rows.
-template <typename T>
-__global__ void __launch_bounds__(WT_WARPS * 32)
+// at 16 sequences x 1 head, 20 -> 10 us at 575 rows.  Four CTAs of the split pass fit an SM (with the 168 registers it would
+// take it is three: 512 groups of 32 tokens complete 35 us, now 28).
+template <typename T, bool SPLIT>
+__global__ void __launch_bounds__(WT_WARPS * 32, SPLIT ? 4 : (sizeof(T) == 2 ? 7 : 6))
 write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, int parts, const StashArgs SA) {
   __shared__ int take[STEP_MAX_ROWS];
   __shared__ int n_take;
   pdl_launch_dependents();
   pdl_wait();
   const LayoutDev& L = TA.L;
-  const int64_t b = blockIdx.x, n_fin_ctas = n_fin_launch * max(parts, 1);
+  const int64_t b = blockIdx.x, n_fin_ctas = n_fin_launch * (SPLIT ? parts : 1);
   const int w = 3 + L.KG;
   if (b < TA.n_rows) {
     if (TA.tok[b] < 0) return;  // padding, or a token that is not stored
@@ -807,7 +818,7 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
     return;
   }
   if (b < TA.n_rows + n_fin_ctas) {
-    const int64_t g = b - TA.n_rows, f = parts > 0 ? g / parts : g;
+    const int64_t g = b - TA.n_rows, f = SPLIT ? g / parts : g;
     if (f >= *FA.fin_count) return;
     const int64_t slot = FA.fin[f * w + 2];
     if (threadIdx.x == 0) n_take = 0;
@@ -817,7 +828,7 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
         if (TA.tok[r] >= 0 && TA.tok[TA.tok_s0 + r] == slot) take[atomicAdd(&n_take, 1)] = r;
     }
     __syncthreads();
-    if (parts > 0) {
+    if constexpr (SPLIT) {
       const SplitArgs<T> S = {n_take, take, &TA};
       finalize_split_any<T>(FA, f, (int)(g - f * parts), parts, S);
       return;
@@ -914,6 +925,18 @@ static FinArgs<T> fin_args(const LayoutDev& L, const echokv_pages* pages, const 
 }  // namespace echokv
 
 using namespace echokv;
+
+template <typename T>
+static void launch_write_step(bool first, int parts, unsigned grid, cudaStream_t st, const TokArgs<T>& TA, const FinArgs<T>& FA,
+                              int64_t n_fin, const StashArgs& SA) {
+  if constexpr (sizeof(T) == 2) {
+    if (parts > 0) {
+      launch_after(!first, write_step_kernel<T, true>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, parts, SA);
+      return;
+    }
+  }
+  launch_after(!first, write_step_kernel<T, false>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, 0, SA);
+}
 
 extern "C" {
 
@@ -1108,9 +1131,9 @@ static int write_step_impl(const echokv_layout* layout, const echokv_pages* page
     const TokArgs<T> TA = tok_args<T>(L, pages, R, key, k_s0, k_s1, value, v_s0, v_s1, tok, tok_s0, kref, kref_s0, \
                                       kref_s1, n_rows);                                                            \
     const FinArgs<T> FA = fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count);                               \
-    const int parts = split_group_ok(L, FA.raw16 && TA.res_raw) ? split_parts(L, n_fin_launch) : 0;                \
+    const int parts = step_split(L, FA.raw16 && TA.res_raw, n_fin_launch);                                         \
     const unsigned grid = (unsigned)(n_rows + n_fin_launch * (parts > 0 ? parts : 1) + stash_ctas);                \
-    launch_after(!first, write_step_kernel<T>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin_launch, parts, SA); \
+    launch_write_step<T>(first, parts, grid, st, TA, FA, n_fin_launch, SA);                                        \
   }
   switch (kv_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;

@@ -143,6 +143,13 @@ def test_groups_completed_across_steps(h, d, bs, kg, dtype, rows, graph_semantic
     compare_store(sc, run_cuda(sc, graph_semantics=graph_semantics), run_oracle(sc))
 
 
+@pytest.mark.parametrize("h,d,bs,kg", [(8, 64, 16, 16), (8, 64, 32, 32), (2, 64, 16, 16), (4, 128, 64, 64)])
+def test_steps_of_more_than_512_rows(h, d, bs, kg):
+    """Captured steps launch a group pass per row: above 512 rows the groups of 16 and 32 tokens of long rows take the pass with
+    a thread per channel piece, those of short rows and of 64 tokens stay spread over lanes."""
+    test_groups_completed_across_steps(h, d, bs, kg, "bf16", 200, True)
+
+
 @pytest.mark.parametrize("h,d,bs,kg", [(2, 64, 16, 16), (1, 128, 32, 16), (8, 128, 64, 32), (8, 128, 128, 64)])
 @pytest.mark.parametrize("bits", [8, 4])
 def test_demotion_across_block_shapes(h, d, bs, kg, bits):

@@ -24,7 +24,7 @@ def _body(file: str, name: str) -> str:
 def test_the_first_write_of_a_step_starts_when_everything_before_it_has_completed():
     """Its launch carries no programmatic attribute; the writes of further layers may overlap the kernel before them."""
     text = (CSRC / "write.cu").read_text()
-    assert "launch_after(!first, write_step_kernel<T>" in text
+    assert text.count("launch_after(!first, write_step_kernel<T,") == 2 == text.count("write_step_kernel<T,")
     first, nxt = (text[text.index(f"int {name}("):] for name in ("echokv_write_step_first", "echokv_write_step"))
     assert "stash_dst, stash_row_bytes, true, stream);" in first[: first.index("\n}\n")]
     assert "stash_dst, stash_row_bytes, false, stream);" in nxt[: nxt.index("\n}\n")]
