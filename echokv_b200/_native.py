@@ -84,6 +84,8 @@ _SIGS = {
                          _F, _I32, _I32, _P, _I64, _I32, _P],
     "echokv_decode_step": [_LP, _PP, _RP, _P, _I64, _I64, _I32, _P, _P, _I64, _P, _P, _P, _I64, _P, _I64, _I64, _I32,
                            _F, _I32, _I32, _P, _I64, _I32, _P],
+    "echokv_decode_chunks": [_LP, _PP, _RP, _P, _I64, _I64, _I32, _P, _P, _I64, _P, _P, _P, _I64, _P, _I64, _I64, _I32,
+                             _F, _I32, _I32, _P, _I64, _I64, _I32, _P],
     "echokv_decode_static": [_LP, _PP, _RP, _P, _I64, _I64, _I32, _P, _P, _I64, _P, _P, _P, _I64, _I64, _I32,
                              _F, _I32, _I32, _I64, _I32, _P],
     "echokv_dequant_dense": [_LP, _PP, _RP, _P, _I64, _P, _I64, _P, _P, _I64, _I64, _I32, _P],

@@ -60,7 +60,8 @@ constexpr unsigned long long WAIT_NS = 2000000000ull;  // a wait gives up after 
 constexpr int F_RES = 1, F_FIRST = 2, F_LAST = 4;  // K from the residual buffer / first / last group of a work item
 constexpr int F_PAIR = 8;                          // the next stage holds a second full tile of the same tier
 constexpr int RT_LOG_SHIFT = 8;                    // plan entries only: bits 8..11 = log2(token rows per run)
-constexpr int F_MASK = 0xff;                       // the flag bits a stage header carries
+constexpr int REM_SHIFT = 16, MAX_REM = 4095;      // bits 16 and up: tokens of the sequence from the tile's first on
+constexpr int F_MASK = 0xff | MAX_REM << REM_SHIFT;  // the flag bits a stage header carries
 struct alignas(16) StageHeader {
   int bits, n_valid, flags, pos0;   // n_valid: 1..16 tokens, -1 = no more work
   long long res_slot;
@@ -373,6 +374,8 @@ struct Lane {
   uint32_t km_ld;     // stage offset of this lane's ldmatrix row of the broadcast k_min operand (tile by lane & 8)
   uint32_t vs_row8;   // INT8 stages (eight tokens in natural order): V scales of token r of the stage
   uint32_t vm_ld8;    // INT8 stages: this lane's ldmatrix row of the [v_min | ones] operand (stage by lane & 16)
+  int tk0, tk1;       // MT: token of its sequence that column 2j / 2j + 1 belongs to
+  int d0, d1;         // MT: how many tokens fewer it sees than the sequence's last token (-1: no such token)
 };
 
 // This lane's ldmatrix row offset inside a stage for the K side / V side of tier BITS: lane & 7 picks the slot
@@ -690,10 +693,10 @@ __device__ __forceinline__ void enter_tier(WarpState& w, const Lane& ln, float* 
 
 // One group: NT tiles (stage bases sbk[t] for the K side, sbv[t] for the V side; they differ at INT8 only).
 // With NT == 2 both tiles are full and code-based.  With NT == 1 the tile may be partial (`n_valid` < 16) and its
-// K may come from the residual buffer.
-template <int BITS, int H, int NT>
+// K may come from the residual buffer.  `rem`: tokens of the sequence from the first tile's start on.
+template <int BITS, int H, int NT, bool MT>
 __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, const uint32_t (&sbk)[NT], const uint32_t (&sbv)[NT],
-                                              int n_valid, bool in_res, long long res_slot, int pos0, WarpState& w,
+                                              int n_valid, int rem, bool in_res, long long res_slot, int pos0, WarpState& w,
                                               float* remap, int* lock, bool& ok) {
   PROF_T(f0);
   enter_tier<BITS>(w, ln, remap, lock, P.wait_ns, ok);
@@ -713,7 +716,19 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
       for (int k = 0; k < 4; ++k) c[t][k] = fmaf(c[t][k], CODE_UNSCALE, c2[2 * (NT == 1 ? 0 : t) + (k & 1)]);
     }
   }
-  if (NT == 1 && n_valid < TILE) {  // a partial tile (the sequence's last): tokens past the end do not count
+  if constexpr (MT) {  // near the sequence's end: every column up to its own token
+    if (rem < NT * TILE + CHUNK_GROUP) {
+      const int t0 = BITS == 8 ? ln.r : 2 * ln.r, t1 = BITS == 8 ? ln.r + 8 : 2 * ln.r + 1;  // tokens of MMA rows r / r + 8
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int n0 = rem - ln.d0 - t * TILE, n1 = rem - ln.d1 - t * TILE;
+        if (t0 >= n0) c[t][0] = -INFINITY;
+        if (t0 >= n1) c[t][1] = -INFINITY;
+        if (t1 >= n0) c[t][2] = -INFINITY;
+        if (t1 >= n1) c[t][3] = -INFINITY;
+      }
+    }
+  } else if (NT == 1 && n_valid < TILE) {  // a partial tile (the sequence's last): tokens past the end do not count
     const int t0 = BITS == 8 ? ln.r : 2 * ln.r, t1 = BITS == 8 ? ln.r + 8 : 2 * ln.r + 1;  // tokens of MMA rows r / r + 8
     if (t0 >= n_valid) { c[0][0] = -INFINITY; c[0][1] = -INFINITY; }
     if (t1 >= n_valid) { c[0][2] = -INFINITY; c[0][3] = -INFINITY; }
@@ -736,18 +751,22 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
   // accumulators need no rescaling.  The result is the same softmax (the reference point cancels).
   const bool grew = (t0 > w.m0 + RESCALE_SLACK) || (t1 > w.m1 + RESCALE_SLACK);
   if (__any_sync(0xffffffffu, grew)) {
-    const float n0 = fmaxf(w.m0, t0), n1 = fmaxf(w.m1, t1);
-    const float a0 = ex2(w.m0 - n0), a1 = ex2(w.m1 - n1);
+    // a column moves only when it has outgrown its own reference: its bits do not depend on its neighbours'
+    const bool g0 = t0 > w.m0 + RESCALE_SLACK, g1 = t1 > w.m1 + RESCALE_SLACK;
+    const float n0 = g0 ? t0 : w.m0, n1 = g1 ? t1 : w.m1;
+    const float a0 = g0 ? ex2(w.m0 - n0) : 1.f, a1 = g1 ? ex2(w.m1 - n1) : 1.f;
 #pragma unroll
     for (int mt = 0; mt < 8; ++mt) { w.acc[mt][0] *= a0; w.acc[mt][1] *= a1; w.acc[mt][2] *= a0; w.acc[mt][3] *= a1; }
     w.bl[0] *= a0; w.bl[1] *= a1; w.bl[2] *= a0; w.bl[3] *= a1;
     w.m0 = n0; w.m1 = n1;
   }
   uint32_t p_lo[NT], p_hi[NT];
+  // MT: a column may have seen no token yet
+  const float m0 = MT && w.m0 == -INFINITY ? 0.f : w.m0, m1 = MT && w.m1 == -INFINITY ? 0.f : w.m1;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    p_lo[t] = pack_h2(ex2(c[t][0] - w.m0), ex2(c[t][1] - w.m1));   // token 2r
-    p_hi[t] = pack_h2(ex2(c[t][2] - w.m0), ex2(c[t][3] - w.m1));   // token 2r + 1
+    p_lo[t] = pack_h2(ex2(c[t][0] - m0), ex2(c[t][1] - m1));   // token 2r
+    p_hi[t] = pack_h2(ex2(c[t][2] - m0), ex2(c[t][3] - m1));   // token 2r + 1
   }
   PROF_T(f2);
   PROF_PHASE(1, f1, f2);
@@ -759,11 +778,12 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
 }
 
 // ---- the kernel ------------------------------------------------------------------------------
+template <bool MT>
 __device__ __forceinline__ bool item_range(const Params& P, int bps_min, int item, int& seq, int& split,
                                            int64_t& seq_len, int& b_start, int& b_end) {
   seq = item % P.num_seqs;
   split = item / P.num_seqs;
-  seq_len = P.A.lens[seq];
+  seq_len = seq_length<MT>(P.A, seq);
   return split_range(seq_len, P.L.BS, P.A.num_splits, bps_min, split, b_start, b_end);
 }
 
@@ -789,16 +809,19 @@ __device__ __forceinline__ BlockMeta load_meta(const Params& P, int64_t bt_row, 
 // running maximum and denominator to ml.  A lane's accumulator rows are neighbouring channels (INT4: 4 per V group,
 // INT2: 8 per half of the head, INT8: 2 per 16-channel tile), so they leave as 16- or 8-byte stores that the
 // eight lanes of a query head put side by side.
-template <int BITS, int H>
-__device__ __forceinline__ void write_partial(const Params& P, const WarpState& w, int seq, int split, int h, int lane) {
+template <int BITS, int H, bool MT>
+__device__ __forceinline__ void write_partial(const Params& P, const Lane& ln, const WarpState& w, int seq, int split) {
+  const int h = ln.h, lane = ln.lane;
   const int r = lane >> 2, j = lane & 3;
   const DecodeArgs& A = P.A;
   const int g0 = 2 * j, g1 = 2 * j + 1;
-  const int64_t o0 = (((int64_t)seq * A.Hq + h * A.gqa + g0) * A.num_splits + split);
-  const int64_t o1 = o0 + A.num_splits;
+  // MT: columns are (token, query head of the group) pairs
+  const int64_t r0 = MT ? ((int64_t)seq * A.tok + ln.tk0) * A.Hq + g0 - ln.tk0 * A.gqa : (int64_t)seq * A.Hq + g0;
+  const int64_t r1 = MT ? ((int64_t)seq * A.tok + ln.tk1) * A.Hq + g1 - ln.tk1 * A.gqa : (int64_t)seq * A.Hq + g1;
+  const int64_t o0 = (r0 + h * A.gqa) * A.num_splits + split, o1 = (r1 + h * A.gqa) * A.num_splits + split;
   float* dst0 = A.acc + o0 * D;
   float* dst1 = A.acc + o1 * D;
-  const bool on0 = g0 < A.gqa, on1 = g1 < A.gqa;
+  const bool on0 = MT ? ln.d0 >= 0 : g0 < A.gqa, on1 = MT ? ln.d1 >= 0 : g1 < A.gqa;
   // V min contribution of V group G: held by lane (r = bias_row(G), j)
   float bias0[NG], bias1[NG];
 #pragma unroll
@@ -856,7 +879,10 @@ template <int H> struct Teams {
   static constexpr int V_SMALL = H == 8 ? 1 : (H == 4 ? 3 : (H == 2 ? 4 : 7));
 };
 
-template <int H, int V>
+// MT: the MMAs' columns are the query heads of several consecutive tokens of a chunk (DecodeArgs::counts): the codes are unpacked, the
+// scales folded and the pages read once for all of them.  With a sequence per token, 528 tokens of 16 chunks over 1,440 stored
+// ones (32 / 8 heads, two tokens a pass) took 273 us a layer with the merge, now 158.
+template <int H, int V, bool MT>
 __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const Params P) {
   extern __shared__ __align__(128) unsigned char smem_all[];
   pdl_launch_dependents();  // the merge may take its place behind this kernel; it waits for this kernel to complete
@@ -884,7 +910,8 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
   uint64_t* sempty = sfull + MAX_NS;                     // stage ring: every consumer warp is done with the stage
   TilePlan* plan = reinterpret_cast<TilePlan*>(smem + HDR_BYTES);
   unsigned char* qs = smem + HDR_BYTES + UNIT * sizeof(TilePlan);
-  unsigned char* ring = qs + (q_copy_bytes(H, A.gqa) + 127) / 128 * 128;
+  const int cols = MT ? A.tok * A.gqa : A.gqa;  // columns of the MMAs in use
+  unsigned char* ring = qs + (q_copy_bytes(H, cols) + 127) / 128 * 128;
   const uint32_t ring_u = smem_u32(ring), full_u = smem_u32(sfull), empty_u = smem_u32(sempty);
 
   if (tid == 0) {
@@ -916,7 +943,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     const int U = tpb >= UNIT ? 1 : UNIT / tpb;      // blocks per unit
     const bool contig = L.BS == TILE && L.KG == TILE;  // a tile's four stats arrays form one run in the page
     const uint64_t policy = stream_policy();
-    if (P.q_vec16 && A.q_s1 == D) {  // the batch's query rows into L2 now: a work item's first step is to read one
+    if (!MT && P.q_vec16 && A.q_s1 == D) {  // the batch's query rows into L2 now: a work item's first step is to read one
       const int elt = 2, teams = gridDim.x * V, me = blockIdx.x * V + team;
       for (int sq = me * 32 + lane; sq < P.num_seqs; sq += teams * 32) {
         const int64_t q_row = A.q_rows ? A.q_rows[sq] : sq;
@@ -941,7 +968,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     if (A.num_splits > 1) {
       int longest = 0;
 #pragma unroll 4
-      for (int i = lane; i < P.num_seqs; i += 32) longest = max(longest, (int)A.lens[i]);
+      for (int i = lane; i < P.num_seqs / (MT ? A.sub : 1); i += 32) longest = max(longest, (int)A.lens[i]);
       longest = __reduce_max_sync(0xffffffffu, longest);
       used_max = min(A.num_splits, ((longest + L.BS - 1) / L.BS + bps_min - 1) / bps_min);
     }
@@ -953,8 +980,8 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         if (lane == 0) it = atomicAdd(P.counter, 1);
         it = __shfl_sync(0xffffffffu, it, 0) + n_teams;
         if (it >= n_items) { have = false; return false; }
-        if (item_range(P, bps_min, it, seq, split, seq_len, b_start, b_end)) {
-          base = b_start; bt_row = A.bt_rows ? A.bt_rows[seq] : seq; have = true;
+        if (item_range<MT>(P, bps_min, it, seq, split, seq_len, b_start, b_end)) {
+          base = b_start; bt_row = seq_table<MT>(A, seq); have = true;
           return true;
         }
       }
@@ -1088,8 +1115,8 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // The first item may be empty (a short sequence's last split): then its successor comes from the counter.
     bool more = false;
     if (!P.idle_producer) {
-      if (item0 < n_items && item_range(P, bps_min, item0, seq, split, seq_len, b_start, b_end)) {
-        base = b_start; bt_row = A.bt_rows ? A.bt_rows[seq] : seq; have = true;
+      if (item0 < n_items && item_range<MT>(P, bps_min, item0, seq, split, seq_len, b_start, b_end)) {
+        base = b_start; bt_row = seq_table<MT>(A, seq); have = true;
         more = true;
       } else {
         wait_once();
@@ -1138,7 +1165,8 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
           d.hdr.bits = bits; d.hdr.n_valid = nv;
           const int rt_log = 31 - __clz(rt);                // for the fills: a run's rows by shift and mask
           d.hdr.flags = (in_res ? F_RES : 0) | (u_first && lane == 0 ? F_FIRST : 0) |
-                        (u_last && lane == unit_tiles - 1 ? F_LAST : 0) | (rt_log << RT_LOG_SHIFT);
+                        (u_last && lane == unit_tiles - 1 ? F_LAST : 0) | (rt_log << RT_LOG_SHIFT) |
+                        ((int)min(u_len - ((int64_t)(u_base + kb) * L.BS + t0), (int64_t)MAX_REM) << REM_SHIFT);
           d.hdr.pos0 = t0 - grp * L.KG; d.hdr.res_slot = ks_slot; d.hdr.seq = u_seq; d.hdr.split = u_split;
           d.stats[0] = page + L.o_vs + (int64_t)t0 * H * NG * 2;
           d.stats[1] = page + L.o_vm + (int64_t)t0 * H * NG * 2;
@@ -1211,11 +1239,12 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // ===================== consumers: warp h owns KV head h =====================
     Lane ln;
     ln.h = warp; ln.lane = lane; ln.r = lane >> 2; ln.j = lane & 3;
-    unsigned char* qn = qs + ln.h * A.gqa * QN_ROW;
+    unsigned char* qn = qs + ln.h * cols * QN_ROW;
+    if constexpr (MT) { ln.tk0 = 2 * ln.j / A.gqa; ln.tk1 = (2 * ln.j + 1) / A.gqa; }
     {  // query columns >= gqa of the MMAs read the team's zero row (every warp writes the same zeros)
-      unsigned char* zero = qs + H * A.gqa * QN_ROW;
-      ln.qn_lane = smem_u32(ln.r < A.gqa ? qn + ln.r * QN_ROW : zero);
-      ln.qn_ld = smem_u32(((lane & 7) < A.gqa ? qn + (lane & 7) * QN_ROW : zero) + (lane >> 3) * 16);
+      unsigned char* zero = qs + H * cols * QN_ROW;
+      ln.qn_lane = smem_u32(ln.r < cols ? qn + ln.r * QN_ROW : zero);
+      ln.qn_ld = smem_u32(((lane & 7) < cols ? qn + (lane & 7) * QN_ROW : zero) + (lane >> 3) * 16);
       for (int i = lane; i < D / 2; i += 32) *reinterpret_cast<uint32_t*>(zero + i * 4) = 0u;
       __syncwarp();
     }
@@ -1256,7 +1285,17 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // This head's queries of sequence `seq` -> fp16 in shared memory, pre-multiplied by softmax_scale * log2(e)
     // (rows >= gqa are zero).  All global loads are issued before the first use so the item pays one memory latency.
     auto load_queries = [&]() {
-      const int64_t q_row = A.q_rows ? A.q_rows[seq] : seq;
+      const int64_t q_row = seq_query<MT>(A, seq);
+      const int n_rows = MT ? seq_tokens<MT>(A, seq) * A.gqa : A.gqa;  // columns that have a token
+      if constexpr (MT) {
+        const int last = seq_tokens<MT>(A, seq) - 1;
+        ln.d0 = ln.tk0 < A.tok && ln.tk0 <= last ? last - ln.tk0 : -1;
+        ln.d1 = ln.tk1 < A.tok && ln.tk1 <= last ? last - ln.tk1 : -1;
+      }
+      auto q_at = [&](int n) {  // element offset of column n's query row
+        const int tk = MT ? n / A.gqa : 0;
+        return (q_row + tk) * A.q_s0 + (int64_t)(ln.h * A.gqa + n - tk * A.gqa) * A.q_s1;
+      };
       __syncwarp();
       if (P.q_vec16) {  // 16-bit queries, 16-byte aligned rows: lane l loads 8 channels of rows l / 16, + 2, + 4, + 6
         const int c8 = (lane & 15) * 8;
@@ -1265,9 +1304,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         for (int k = 0; k < 4; ++k) {
           const int n = (lane >> 4) + 2 * k;
           raw[k] = make_uint4(0, 0, 0, 0);
-          if (n < A.gqa)
-            raw[k] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(A.q) + q_row * A.q_s0 +
-                                                     (int64_t)(ln.h * A.gqa + n) * A.q_s1 + c8);
+          if (n < n_rows) raw[k] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(A.q) + q_at(n) + c8);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -1281,13 +1318,14 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
             else { const __half2 hh = *reinterpret_cast<const __half2*>(&wds[e]); x = __low2float(hh); y = __high2float(hh); }
             o[e] = pack_h2(x * A.scale_log2e, y * A.scale_log2e);
           }
-          if (n < A.gqa) *reinterpret_cast<uint4*>(qn + n * QN_ROW + c8 * 2) = make_uint4(o[0], o[1], o[2], o[3]);
+          if (n < cols) *reinterpret_cast<uint4*>(qn + n * QN_ROW + c8 * 2) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       } else {
-        for (int i = lane; i < A.gqa * (D / 2); i += 32) {
+        for (int i = lane; i < cols * (D / 2); i += 32) {
           const int d2 = i % (D / 2), n = i / (D / 2);
-          const int64_t e = q_row * A.q_s0 + (int64_t)(ln.h * A.gqa + n) * A.q_s1 + 2 * d2;
-          const float x = ld_dt(A.q, A.q_dt, e) * A.scale_log2e, y = ld_dt(A.q, A.q_dt, e + 1) * A.scale_log2e;
+          const int64_t e = q_at(n) + 2 * d2;
+          const bool on = n < n_rows;
+          const float x = on ? ld_dt(A.q, A.q_dt, e) * A.scale_log2e : 0.f, y = on ? ld_dt(A.q, A.q_dt, e + 1) * A.scale_log2e : 0.f;
           *reinterpret_cast<uint32_t*>(qn + n * QN_ROW + d2 * 4) = pack_h2(x, y);
         }
       }
@@ -1339,14 +1377,14 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         const int cur_split = split;
         if constexpr (KIND == K_TILE8) {
           const uint32_t sk[1] = {sb0}, sv[1] = {sb1};
-          process_group<8, H, 1>(P, ln, sk, sv, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
+          process_group<8, H, 1, MT>(P, ln, sk, sv, n_valid, flags >> REM_SHIFT, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
         } else if constexpr (KIND == K_SINGLE) {
           const uint32_t s1[1] = {sb0};
-          if (bits == 4) process_group<4, H, 1>(P, ln, s1, s1, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
-          else process_group<2, H, 1>(P, ln, s1, s1, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
+          if (bits == 4) process_group<4, H, 1, MT>(P, ln, s1, s1, n_valid, flags >> REM_SHIFT, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
+          else process_group<2, H, 1, MT>(P, ln, s1, s1, n_valid, flags >> REM_SHIFT, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
         } else {
           const uint32_t s2[2] = {sb0, sb1};
-          process_group<BITS, H, 2>(P, ln, s2, s2, TILE, false, 0, 0, w, remap, lock, ok);
+          process_group<BITS, H, 2, MT>(P, ln, s2, s2, TILE, flags >> REM_SHIFT, false, 0, 0, w, remap, lock, ok);
         }
         __syncwarp();
         mbar_arrive(empty_u + c_st * 8);  // every lane arrives (the barrier counts threads): no branch, no warp sync needed
@@ -1359,10 +1397,10 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         }
         if (last) {
           if constexpr (KIND == K_SINGLE) {
-            if (w.bits == 4) write_partial<4, H>(P, w, seq, cur_split, ln.h, lane);
-            else write_partial<2, H>(P, w, seq, cur_split, ln.h, lane);
+            if (w.bits == 4) write_partial<4, H, MT>(P, ln, w, seq, cur_split);
+            else write_partial<2, H, MT>(P, ln, w, seq, cur_split);
           } else {
-            write_partial<BITS, H>(P, w, seq, cur_split, ln.h, lane);
+            write_partial<BITS, H, MT>(P, ln, w, seq, cur_split);
           }
         }
         PROF_T(r2);
@@ -1423,16 +1461,23 @@ struct DecodeDevice {
 template <int H>
 static cudaError_t allow_smem(int bytes) {
   using namespace mma;
-  cudaError_t e = cudaFuncSetAttribute(decode_mma_kernel<H, Teams<H>::V>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(decode_mma_kernel<H, Teams<H>::V_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  auto allow = [&](auto* kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+  cudaError_t e = allow(decode_mma_kernel<H, Teams<H>::V, false>);
+  if (e == cudaSuccess) e = allow(decode_mma_kernel<H, Teams<H>::V_SMALL, false>);
+  if (e == cudaSuccess) e = allow(decode_mma_kernel<H, Teams<H>::V, true>);
+  if (e == cudaSuccess) e = allow(decode_mma_kernel<H, Teams<H>::V_SMALL, true>);
   return e;
+}
+template <int H, bool MT>
+static void launch_teams(bool small, unsigned grid, int smem_bytes, cudaStream_t st, const mma::Params& P) {
+  using namespace mma;
+  if (small) launch_pdl(decode_mma_kernel<H, Teams<H>::V_SMALL, MT>, dim3(grid), dim3((H + 1) * 32 * Teams<H>::V_SMALL), smem_bytes, st, P);
+  else launch_pdl(decode_mma_kernel<H, Teams<H>::V, MT>, dim3(grid), dim3((H + 1) * 32 * Teams<H>::V), smem_bytes, st, P);
 }
 template <int H>
 static void launch_teams(bool small, unsigned grid, int smem_bytes, cudaStream_t st, const mma::Params& P) {
-  using namespace mma;
-  if (small) launch_pdl(decode_mma_kernel<H, Teams<H>::V_SMALL>, dim3(grid), dim3((H + 1) * 32 * Teams<H>::V_SMALL), smem_bytes, st, P);
-  else launch_pdl(decode_mma_kernel<H, Teams<H>::V>, dim3(grid), dim3((H + 1) * 32 * Teams<H>::V), smem_bytes, st, P);
+  if (P.A.counts) launch_teams<H, true>(small, grid, smem_bytes, st, P);
+  else launch_teams<H, false>(small, grid, smem_bytes, st, P);
 }
 static int decode_device(DecodeDevice** out) {
   using namespace mma;
@@ -1505,7 +1550,7 @@ int launch_decode_mma(const LayoutDev& L, const ResidualDev& R, const uint8_t* p
   *handled = false;
   if (g_decode_path == 1) return ECHOKV_OK;
   const int H = L.H;
-  if (!mma_shape_ok(H, L.D, L.VG, L.KG, L.BS, A.gqa)) return ECHOKV_OK;
+  if (!mma_shape_ok(H, L.D, L.VG, L.KG, L.BS, A.tok * A.gqa)) return ECHOKV_OK;
   if ((R.s_slot | R.s_pos | R.s_head) & 3) return ECHOKV_OK;                 // 8-byte residual loads
   if ((reinterpret_cast<uintptr_t>(R.base) & 15) != 0) return ECHOKV_OK;
   if (num_seqs * (int64_t)A.num_splits > (1 << 30)) return ECHOKV_OK;
@@ -1520,7 +1565,7 @@ int launch_decode_mma(const LayoutDev& L, const ResidualDev& R, const uint8_t* p
   P.wait_ns = g_wait_ns;
   P.idle_producer = g_idle_producer;
   TeamShape ts;
-  if (!team_shape(*dv, H, A.gqa, &ts)) return ECHOKV_OK;
+  if (!team_shape(*dv, H, A.tok * A.gqa, &ts)) return ECHOKV_OK;
   const int V = ts.V, ns = ts.ns, fixed = ts.fixed, sbytes = stage_bytes(H);
   const bool small = ts.small;
   P.NS = ns;

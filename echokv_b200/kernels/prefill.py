@@ -8,8 +8,9 @@ bottom-right causal mask.  There is no PyTorch path.
 
 Two device paths:
   * row path: every query token is handed to the split-K decode kernel as a
-    sequence whose length is its causal limit.  Each token re-reads its context,
-    so this is for short chunks (the reference's fused path has the same
+    sequence whose length is its causal limit; with up to four query heads per KV
+    head, 2 to 8 consecutive tokens of a chunk share one pass over the pages.  Every
+    such pass re-reads the context, so this is for short chunks (the reference's fused path has the same
     trade-off, kernels/prefill.py:10-13).
   * dense path: dequantize every context once into ``[total_ctx, H, D]`` in the
     model dtype, then run the tensor-core attention kernel over it.
@@ -22,7 +23,7 @@ import torch
 
 from echokv_b200 import _native as N
 from echokv_b200._util import to_device
-from echokv_b200.kernels.decode import decode_attention
+from echokv_b200.kernels.decode import CHUNK_GROUP, decode_attention
 
 ROW_PATH_MAX_CHUNK = 64  # longer chunks take the dense path when it is available
 
@@ -57,19 +58,38 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
     return k, v
 
 
+class RowPlan(tuple):
+    """What ``build_rows`` returns: a 4-tuple (query rows, block-table rows, causal limits, largest limit), with the same tokens as
+    ``groups`` of consecutive ones for ``decode_attention``."""
+
+    groups: torch.Tensor
+
+
 def build_rows(prefill, req_of, device):
-    """Row-path metadata: per query token its row, its request and its causal limit (device int64)."""
+    """Row-path metadata: per query token its row, its request and its causal limit (device int64), and the largest limit."""
     pairs = list(zip(prefill, req_of))
     start = np.array([p[0] for p, _ in pairs], dtype=np.int64)
     nq = np.array([max(p[1] - p[0], 0) for p, _ in pairs], dtype=np.int64)
     ctx = np.array([p[2] for p, _ in pairs], dtype=np.int64)
-    rows = np.empty((3, int(nq.sum())), dtype=np.int64)
-    at = np.arange(rows.shape[1]) - np.repeat(np.cumsum(nq) - nq, nq)  # place in the chunk
+    req = np.array([r for _, r in pairs], dtype=np.int64)
+    n, per = int(nq.sum()), -(-nq // CHUNK_GROUP)
+    g = int(per.sum())
+    buf = np.empty(3 * n + 4 * g, dtype=np.int64)
+    rows, groups = buf[: 3 * n].reshape(3, n), buf[3 * n:].reshape(4, g)
+    at = np.arange(n) - np.repeat(np.cumsum(nq) - nq, nq)  # place in the chunk
     rows[0] = np.repeat(start, nq) + at
-    rows[1] = np.repeat(np.array([r for _, r in pairs], dtype=np.int64), nq)
+    rows[1] = np.repeat(req, nq)
     rows[2] = np.repeat(ctx - nq + 1, nq) + at
-    packed = to_device(torch.from_numpy(rows), device)
-    return packed[0], packed[1], packed[2], int(rows[2].max(initial=0))
+    first = (np.arange(g) - np.repeat(np.cumsum(per) - per, per)) * CHUNK_GROUP  # place of a group's first token
+    groups[3] = np.minimum(CHUNK_GROUP, np.repeat(nq, per) - first)
+    groups[0] = np.repeat(start, per) + first
+    groups[1] = np.repeat(req, per)
+    groups[2] = np.repeat(ctx - nq, per) + first + groups[3]
+    dev = to_device(torch.from_numpy(buf), device)
+    packed = dev[: 3 * n].view(3, n)
+    plan = RowPlan((packed[0], packed[1], packed[2], int(rows[2].max(initial=0))))
+    plan.groups = dev[3 * n:].view(4, g)
+    return plan
 
 
 def build_dense(prefill, req_of, block_size: int, device):
@@ -133,4 +153,4 @@ def prefill_attention(store, query: torch.Tensor, output: torch.Tensor, prefill,
     q_rows, reqs, lens, max_len = rows
     # Splits of the default size: a token's split then follows from its own context, and its bits from the request alone.
     decode_attention(store, query, block_table, lens, softmax_scale, q_rows=q_rows, bt_rows=reqs, out=out3,
-                     max_len=max_len)
+                     max_len=max_len, groups=getattr(rows, "groups", None))

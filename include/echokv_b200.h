@@ -243,6 +243,21 @@ int echokv_decode_step(const echokv_layout* layout, const echokv_pages* pages, c
                        float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
                        const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream);
 
+/* echokv_decode_ex (without a run-time split size) for sequences that are the query tokens of chunks: consecutive tokens of a chunk
+ * see the same cache, one token more each, and are worked off together where the shape allows it.  `groups` int64 [4, num_groups],
+ * row after row: the query row of a group's first token, its block-table row, the cache length of its last token, its tokens
+ * (1 .. 8, on consecutive query rows; cut from each chunk's first token on, so that a token's result follows from its chunk
+ * alone).  Together the groups hold the num_seqs tokens that q_rows / bt_rows / lens list one by one, which serve the shapes that
+ * take one token at a time (more than four query heads per KV head, and those of the generic kernel).  `scratch` holds
+ * max(num_seqs, 8 * num_groups) sequences (echokv_decode_scratch_bytes). */
+int echokv_decode_chunks(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
+                         const void* query, int64_t q_s0, int64_t q_s1, int32_t q_dtype, const int64_t* q_rows,
+                         const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
+                         void* scratch, int64_t scratch_bytes,
+                         void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
+                         float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
+                         const int64_t* groups, int64_t num_groups, int64_t num_seqs, int32_t num_q_heads, void* stream);
+
 /* How many work items (sequence, split) the split kernel works on at the same time on the current device for
  * this layout and number of query heads, or 0 when the shape takes the generic kernel (one CTA per item and KV
  * head).  A host that picks the split size per step sizes the splits so that the items fill this many slots
