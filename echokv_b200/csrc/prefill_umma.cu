@@ -672,6 +672,11 @@ __global__ void __launch_bounds__(UM * G + (TMA ? 64 : 32), 1) prefill_umma_pipe
 constexpr int WN = 128;                    // keys per tile
 constexpr int WKV_BYTES = WN * UD * 2;     // one K or V tile: two panels of 128 rows x 128 bytes
 constexpr int W_STAGES = 2;
+// P of a tile is handed to the issuer in this many parts, so that the first part's O += P V runs under the rest's
+// exponentials: a group's chain (scores, softmax, O += P V) is what bounds the kernel, neither pipe is full (tensor and XU pipes
+// 45 % active each).  Two parts: 8 x 512 tokens behind 8,192, the 8-layer step 6.10 -> 5.84 ms; 12 prompts 2.32 -> 2.24 ms; four parts
+// gain nothing.  A quarter or a third of the exponentials on the FMA pipe (a polynomial) gave nothing on top.
+constexpr int P_PARTS = 2;
 constexpr int W_SCOL = 0, W_OCOL = 128, W_GCOLS = 256;
 constexpr int smem_wide() { return 2 * Q_BYTES + 2 * W_STAGES * WKV_BYTES + 1024; }
 
@@ -696,7 +701,7 @@ __device__ __forceinline__ void tmem_ld16_raw(uint32_t taddr, uint32_t (&r)[16])
 // behind 8,192: 636 -> 585 us (0.59 of the measured bf16 peak); 512 behind 1,600: 36.6 -> 29.5 us.
 __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args A, const __grid_constant__ Maps M) {
   extern __shared__ unsigned char dyn[];
-  __shared__ __align__(8) uint64_t bar_s[2], bar_p[2], bar_o[2], bar_k[W_STAGES], bar_v[W_STAGES], bar_kfree[W_STAGES],
+  __shared__ __align__(8) uint64_t bar_s[2], bar_p[2][P_PARTS], bar_o[2], bar_k[W_STAGES], bar_v[W_STAGES], bar_kfree[W_STAGES],
       bar_vfree[W_STAGES];
   __shared__ uint32_t tmem_slot;
   constexpr int NROW = 2 * UM;
@@ -767,7 +772,7 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
   };
   if (tid == NROW + 32) {  // the tile producer sets the barriers up and starts the first tiles under the copies of Q
     auto init = [](uint64_t* b, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n)); };
-    for (int g = 0; g < 2; ++g) { init(&bar_s[g], 1); init(&bar_p[g], UM); init(&bar_o[g], 1); }
+    for (int g = 0; g < 2; ++g) { init(&bar_s[g], 1); init(&bar_o[g], 1); for (int i = 0; i < P_PARTS; ++i) init(&bar_p[g][i], UM); }
     for (int i = 0; i < W_STAGES; ++i) { init(&bar_k[i], 1); init(&bar_v[i], 1); init(&bar_kfree[i], 1); init(&bar_vfree[i], 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -821,14 +826,17 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
       const bool more = tile + 1 < n_tiles;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
-        if (!bar_wait(&bar_p[g], tile & 1)) { ok = false; break; }  // the group's P is in tensor memory
         if (g == 0 && !bar_wait(&bar_v[stage], (tile / W_STAGES) & 1)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
         for (int k = 0; k < WN / 16; ++k) {  // 16 keys = 8 columns of P; V as it lies in memory (MN-major B)
+          if (k % (WN / 16 / P_PARTS) == 0) {  // the next part of the group's P is in tensor memory
+            if (!bar_wait(&bar_p[g][k / (WN / 16 / P_PARTS)], tile & 1)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+          }
           const uint64_t b = make_desc(v_s + stage * WKV_BYTES + k * 2048, WN * 128, 1024);
           mma_f16_ts(tmem + g * W_GCOLS + W_OCOL, tmem + g * W_GCOLS + W_SCOL + k * 8, b, idesc_pv, (tile > 0 || k > 0) ? 1u : 0u);
         }
+        if (!ok) break;
         mma_commit(&bar_o[g]);
         if (g == 1) mma_commit(&bar_vfree[stage]);
         if (more) {  // the group's next scores go over its P, after the MMA that reads it
@@ -920,13 +928,15 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
           w[e] = pack16(pp.x, pp.y, bf16);
         }
         tmem_st16_raw(t_row + W_SCOL + 16 * c, w);
+        if ((c + 1) % (WN / 32 / P_PARTS) == 0) {  // a part of P is complete
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          bar_arrive(&bar_p[grp][c / (WN / 32 / P_PARTS)]);
+        }
       }
       const float2 s01 = __fadd2_rn(sum2[0], sum2[1]), s23 = __fadd2_rn(sum2[2], sum2[3]);
       l_run += (s01.x + s01.y) + (s23.x + s23.y);
       PF_T(c5);
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      bar_arrive(&bar_p[grp]);
       PF_T(c6);
       PF_ADD(0, c0, c1); PF_ADD(1, c1, c2); PF_ADD(2, c2, c3); PF_ADD(3, c3, c4); PF_ADD(4, c4, c5); PF_ADD(5, c5, c6);
 #ifdef ECHOKV_PROFILE
