@@ -876,7 +876,7 @@ __device__ __forceinline__ int ring_next(int st, int NS) { return st + 1 == NS ?
 // memory (many query heads per KV head) does not fit V times.
 template <int H> struct Teams {
   static constexpr int V = H == 8 ? 2 : (H == 4 ? 4 : (H == 2 ? 6 : 10));   // 18 / 20 / 18 / 20 warps
-  static constexpr int V_SMALL = H == 8 ? 1 : (H == 4 ? 3 : (H == 2 ? 4 : 7));
+  static constexpr int V_SMALL = H == 8 ? 1 : (H == 4 ? 3 : (H == 2 ? 4 : 8));
 };
 
 // MT: the MMAs' columns are the query heads of several consecutive tokens of a chunk (DecodeArgs::counts): the codes are unpacked, the
@@ -1514,7 +1514,13 @@ static bool team_shape(const DecodeDevice& dv, int H, int gqa, TeamShape* out) {
   int V = H == 8 ? Teams<8>::V : H == 4 ? Teams<4>::V : H == 2 ? Teams<2>::V : Teams<1>::V;
   bool small = false;
   int ns = ((room / V) / 128 * 128 - fixed) / sbytes;
-  if (ns < 4) {
+  // With more than four query heads per KV head, 15 or 16 warps of 128 registers beat 20 of 96 at four KV heads and one: the query
+  // copy leaves a team of the larger count four or five stages, and the columns in use are worth the registers (4 bits: 16 x 28,000 at H 1
+  // 51.3 -> 48.7 us, 48 x 6,000 at H 4 59.4 -> 56.4; 8 x 2,000 at H 4 19.3 -> 18.0).  With four or fewer it is the other way
+  // round (64 x 4,000, block 64, at H 4: 52.6 -> 61.4), and at two KV heads it depends on the tier (4 bits 50.5 -> 47.6, 8 bits
+  // 35.9 -> 36.4).
+  const bool few = gqa > 4 && (H == 1 || H == 4);
+  if (ns < 4 || few) {
     small = true;
     V = H == 8 ? Teams<8>::V_SMALL : H == 4 ? Teams<4>::V_SMALL : H == 2 ? Teams<2>::V_SMALL : Teams<1>::V_SMALL;
     ns = ((room / V) / 128 * 128 - fixed) / sbytes;
