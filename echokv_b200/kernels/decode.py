@@ -112,15 +112,18 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
     L = store.layout
     given = (block_table, seq_lens, q_rows, bt_rows)
     N.require_cuda(query, block_table, seq_lens, out)
-    if query.dim() != 3 or query.shape[2] != L.head_size:
+    q_shape, q_s, bt_s = query.shape, query.stride(), block_table.stride()  # each in one call: this runs once per layer and step
+    if len(q_shape) != 3 or q_shape[2] != L.head_size:
         raise ValueError("query must be [T, Hq, D]")
-    if query.stride(2) != 1:
+    if q_s[2] != 1:
         query = query.contiguous()
-    hq = query.shape[1]
+        q_s = query.stride()
+    hq = q_shape[1]
     s = seq_lens.shape[0]
     dev = query.device
-    if block_table.dtype != torch.int32 or block_table.stride(1) != 1:
+    if block_table.dtype != torch.int32 or bt_s[1] != 1:
         block_table = block_table.to(torch.int32).contiguous()
+        bt_s = block_table.stride()
     lens = seq_lens if seq_lens.dtype == torch.long and seq_lens.is_contiguous() else seq_lens.long().contiguous()
     if q_rows is not None and (q_rows.dtype != torch.long or not q_rows.is_contiguous()):
         q_rows = q_rows.long().contiguous()
@@ -128,7 +131,8 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
         bt_rows = bt_rows.long().contiguous()
     if out is None:
         out = torch.empty(query.shape[0], hq, L.head_size, device=dev, dtype=torch.float32)
-    if out.stride(2) != 1:
+    o_s = out.stride()
+    if o_s[2] != 1:
         raise ValueError("out must have a contiguous last dim")
     if num_splits is None:
         width = block_table.shape[1]
@@ -149,10 +153,10 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
             raise ValueError("groups must be a contiguous int64 [4, G] tensor, without bps_dev")
         N.check(N.lib.echokv_decode_chunks(
             store.c_layout, store.c_pages, store.c_res,
-            query.data_ptr(), query.stride(0), query.stride(1), N.dtype_code(query.dtype), N.ptr(q_rows),
-            block_table.data_ptr(), block_table.stride(0), N.ptr(bt_rows), lens.data_ptr(),
+            query.data_ptr(), q_s[0], q_s[1], N.dtype_code(query.dtype), N.ptr(q_rows),
+            block_table.data_ptr(), bt_s[0], N.ptr(bt_rows), lens.data_ptr(),
             scratch.data_ptr(), scratch.numel(),
-            out.data_ptr(), out.stride(0), out.stride(1), N.dtype_code(out.dtype),
+            out.data_ptr(), o_s[0], o_s[1], N.dtype_code(out.dtype),
             float(softmax_scale), int(num_splits), int(blocks_per_split), groups.data_ptr(), groups.shape[1], s, hq,
             N.stream_ptr(dev)))
         return out
@@ -161,9 +165,9 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
     launch = N.lib.echokv_decode_step if planned else N.lib.echokv_decode_ex
     N.check(launch(
         store.c_layout, store.c_pages, store.c_res,
-        query.data_ptr(), query.stride(0), query.stride(1), N.dtype_code(query.dtype), N.ptr(q_rows),
-        block_table.data_ptr(), block_table.stride(0), N.ptr(bt_rows), lens.data_ptr(),
+        query.data_ptr(), q_s[0], q_s[1], N.dtype_code(query.dtype), N.ptr(q_rows),
+        block_table.data_ptr(), bt_s[0], N.ptr(bt_rows), lens.data_ptr(),
         scratch.data_ptr(), scratch.numel(),
-        out.data_ptr(), out.stride(0), out.stride(1), N.dtype_code(out.dtype),
+        out.data_ptr(), o_s[0], o_s[1], N.dtype_code(out.dtype),
         float(softmax_scale), int(num_splits), int(blocks_per_split), N.ptr(bps_dev), s, hq, N.stream_ptr(dev)))
     return out

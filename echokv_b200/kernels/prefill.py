@@ -49,11 +49,13 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
     v = torch.empty_like(k)
     if work.numel():
         N.require_cuda(work, block_table)
-        if block_table.dtype != torch.int32 or block_table.stride(1) != 1:
+        bt_s, k_s = block_table.stride(), k.stride()
+        if block_table.dtype != torch.int32 or bt_s[1] != 1:
             block_table = block_table.to(torch.int32).contiguous()
+            bt_s = block_table.stride()
         N.check(N.lib.echokv_dequant_dense(
             store.c_layout, store.c_pages, store.c_res, work.data_ptr(), work.shape[0],
-            block_table.data_ptr(), block_table.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
+            block_table.data_ptr(), bt_s[0], k.data_ptr(), v.data_ptr(), k_s[0], k_s[1],
             N.dtype_code(dtype), N.stream_ptr(store.device)))
     return k, v
 
@@ -111,15 +113,16 @@ def dense_attention(query: torch.Tensor, k: torch.Tensor, v: torch.Tensor, chunk
     ``query [T, Hq, D]`` and ``k``/``v [total_ctx, H, D]`` share one 16-bit dtype; ``out [T, Hq, D]``.
     ``query_rows``: the chunks' query rows together, when known (it sizes the launch)."""
     N.require_cuda(query, k, v, chunks, out)
-    if query.dtype != k.dtype or k.dtype != v.dtype or k.stride() != v.stride():
+    q_s, k_s, o_s, q_shape, k_shape = query.stride(), k.stride(), out.stride(), query.shape, k.shape
+    if query.dtype != k.dtype or k.dtype != v.dtype or k_s != v.stride():
         raise ValueError("query, K and V must share a dtype and K, V a layout")
-    if query.stride(2) != 1 or k.stride(2) != 1 or out.stride(2) != 1:
+    if q_s[2] != 1 or k_s[2] != 1 or o_s[2] != 1:
         raise ValueError("the head dimension must be contiguous")
     N.check(N.lib.echokv_prefill_ex(
-        query.data_ptr(), query.stride(0), query.stride(1), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
-        k.shape[0], N.dtype_code(query.dtype), chunks.data_ptr(), chunks.shape[0], max_chunk, query_rows,
-        out.data_ptr(), out.stride(0), out.stride(1), N.dtype_code(out.dtype), softmax_scale, query.shape[1],
-        k.shape[1], query.shape[2], N.stream_ptr(query.device)))
+        query.data_ptr(), q_s[0], q_s[1], k.data_ptr(), v.data_ptr(), k_s[0], k_s[1],
+        k_shape[0], N.dtype_code(query.dtype), chunks.data_ptr(), chunks.shape[0], max_chunk, query_rows,
+        out.data_ptr(), o_s[0], o_s[1], N.dtype_code(out.dtype), softmax_scale, q_shape[1],
+        k_shape[1], q_shape[2], N.stream_ptr(query.device)))
 
 
 def dense_supported(store, query: torch.Tensor) -> bool:

@@ -18,6 +18,14 @@ def _rows_hd(t: torch.Tensor, what: str) -> torch.Tensor:
     return t
 
 
+def _strides_hd(t: torch.Tensor, what: str) -> tuple:
+    """``_rows_hd``'s check, returning the strides: they cost 0.15 us in one call, 0.3 - 0.4 us one by one."""
+    s = t.stride()
+    if len(s) != 3 or s[2] != 1:
+        raise ValueError(f"{what} must be [rows, H, D] with a contiguous last dim")
+    return s
+
+
 def scatter_i64(dst: torch.Tensor, idx: torch.Tensor, val: torch.Tensor) -> None:
     """``dst[idx] = val`` for int64 device tensors (one tiny kernel, no host sync)."""
     n = idx.numel()
@@ -83,10 +91,11 @@ def write_step(store, key: torch.Tensor, value: torch.Tensor, meta, kref: torch.
     if meta.n_rows == 0 and n_fin == 0 and stash is None:
         return
     N.require_cuda(key, value, meta.tok, meta.fin, kref)
-    key, value = _rows_hd(key, "key"), _rows_hd(value, "value")
+    k_s, v_s = _strides_hd(key, "key"), _strides_hd(value, "value")
     if key.dtype != value.dtype:
         raise TypeError("key and value must share a dtype")
-    if kref is not None and (kref.dtype != torch.float32 or kref.stride(2) != 1):
+    r_s = (0, 0) if kref is None else kref.stride()
+    if kref is not None and (kref.dtype != torch.float32 or r_s[2] != 1):
         raise ValueError("the K_ref ring must be float32 [W, H, D] with a contiguous last dim")
     tok = meta.tok
     if stash is None:
@@ -99,9 +108,9 @@ def write_step(store, key: torch.Tensor, value: torch.Tensor, meta, kref: torch.
     launch = N.lib.echokv_write_step if meta.launched else N.lib.echokv_write_step_first
     N.check(launch(
         store.c_layout, store.c_pages,
-        key.data_ptr(), key.stride(0), key.stride(1), value.data_ptr(), value.stride(0), value.stride(1),
+        key.data_ptr(), k_s[0], k_s[1], value.data_ptr(), v_s[0], v_s[1],
         N.dtype_code(key.dtype), tok.data_ptr(), tok.stride(0), store.c_res,
-        N.ptr(kref), 0 if kref is None else kref.stride(0), 0 if kref is None else kref.stride(1),
+        N.ptr(kref), r_s[0], r_s[1],
         meta.n_rows, N.ptr(meta.fin) if n_fin else None, N.ptr(meta.fin_count) if n_fin else None, n_fin,
         *s_args, N.stream_ptr(key.device)))
     meta.launched = meta.launched or meta.n_rows > 0

@@ -175,9 +175,10 @@ class ChunkPool:
 def lru_victims(tier: np.ndarray, full: np.ndarray, last: np.ndarray, chunks_needed: int, keep: np.ndarray) -> np.ndarray:
     """The least recently written INT4/INT8 blocks (``full``: mask of full blocks, ``last``: step of the last write; ties by
     block id) without those in ``keep``, up to the one whose extra chunks make ``chunks_needed``, or all there are."""
-    ranked = np.flatnonzero((tier >= 4) & full)
+    candidate = (tier >= 4) & full
+    candidate[keep[(keep >= 0) & (keep < candidate.size)]] = False
+    ranked = np.flatnonzero(candidate)
     ranked = ranked[np.argsort(last[ranked], kind="stable")]
-    ranked = ranked[~np.isin(ranked, keep)]
     freed = np.cumsum(_NEXTRA_OF[tier[ranked]])
     return ranked[: int(np.searchsorted(freed, chunks_needed)) + 1]
 
@@ -381,6 +382,9 @@ class TieredKVCache:
         query rows).  ``capturing`` gives the group pass its full grid, masked by the device count."""
         from echokv_b200.kernels.write import write_step
 
+        if not torch.autograd._profiler_enabled():  # the range alone costs 8 us of host time a layer
+            write_step(self, key, value, meta, kref, full_grid=capturing, stash=stash)
+            return
         with record_function("echokv.write.step"):
             write_step(self, key, value, meta, kref, full_grid=capturing, stash=stash)
 
