@@ -8,7 +8,7 @@ using namespace echokv;
 namespace echokv {
 int launch_decode_mma(const LayoutDev& L, const ResidualDev& R, const uint8_t* pages, const DecodeArgs& A,
                       int64_t num_seqs, int* counter, bool zero_counter, int* status, cudaStream_t st, bool* handled);
-int decode_mma_teams(int H, int D, int VG, int KG, int BS, int gqa);
+int decode_mma_teams(int H, int D, int VG, int KG, int BS, int gqa, int chunks);
 int decode_status_take(bool clear);
 int prefill_status_take(bool clear);
 
@@ -154,7 +154,7 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
   int64_t parts = 0;
   if (groups && num_groups > 0 && gqa <= CHUNK_GROUP / 2) {
     const int tok = CHUNK_GROUP / gqa;
-    if (decode_mma_teams(L.H, L.D, L.VG, L.KG, L.BS, tok * gqa) > 0) parts = num_groups * (CHUNK_GROUP / tok);
+    if (decode_mma_teams(L.H, L.D, L.VG, L.KG, L.BS, tok * gqa, L.KC) > 0) parts = num_groups * (CHUNK_GROUP / tok);
   }
   const int64_t rows = parts ? num_groups * CHUNK_GROUP : num_seqs;
   if (scratch_bytes < echokv_decode_scratch_bytes(rows > num_seqs ? rows : num_seqs, num_q_heads, L.D, num_splits) ||
@@ -263,7 +263,7 @@ int echokv_decode(const echokv_layout* layout, const echokv_pages* pages, const 
 int32_t echokv_decode_parallelism(const echokv_layout* layout, int32_t num_q_heads) {
   if (!layout || layout->num_kv_heads <= 0 || num_q_heads <= 0 || num_q_heads % layout->num_kv_heads) return 0;
   return decode_mma_teams(layout->num_kv_heads, layout->head_size, layout->v_group, layout->k_group, layout->block_size,
-                          num_q_heads / layout->num_kv_heads);
+                          num_q_heads / layout->num_kv_heads, layout->mem_bits / 2);
 }
 
 

@@ -1506,7 +1506,7 @@ static int decode_device(DecodeDevice** out) {
 // of the SM's shared memory; false when not even the smaller team count leaves room for four stages (a group of
 // two stages in work and one in flight at the least).
 struct TeamShape { int V, ns, fixed; bool small; };
-static bool team_shape(const DecodeDevice& dv, int H, int gqa, TeamShape* out) {
+static bool team_shape(const DecodeDevice& dv, int H, int gqa, int chunks, TeamShape* out) {  // chunks: of a page
   using namespace mma;
   const int fixed = HDR_BYTES + UNIT * (int)sizeof(TilePlan) + (q_copy_bytes(H, gqa) + 127) / 128 * 128;
   const int sbytes = stage_bytes(H);
@@ -1514,12 +1514,10 @@ static bool team_shape(const DecodeDevice& dv, int H, int gqa, TeamShape* out) {
   int V = H == 8 ? Teams<8>::V : H == 4 ? Teams<4>::V : H == 2 ? Teams<2>::V : Teams<1>::V;
   bool small = false;
   int ns = ((room / V) / 128 * 128 - fixed) / sbytes;
-  // With more than four query heads per KV head, 15 or 16 warps of 128 registers beat 20 of 96 at four KV heads and one: the query
-  // copy leaves a team of the larger count four or five stages, and the columns in use are worth the registers (4 bits: 16 x 28,000 at H 1
-  // 51.3 -> 48.7 us, 48 x 6,000 at H 4 59.4 -> 56.4; 8 x 2,000 at H 4 19.3 -> 18.0).  With four or fewer it is the other way
-  // round (64 x 4,000, block 64, at H 4: 52.6 -> 61.4), and at two KV heads it depends on the tier (4 bits 50.5 -> 47.6, 8 bits
-  // 35.9 -> 36.4).
-  const bool few = gqa > 4 && (H == 1 || H == 4);
+  // One KV head, more than four query heads, pages of at most 4 bits: 16 warps of 128 registers beat 20 of 96 (16 x 28,000 tokens 51.3 ->
+  // 48.7 us, 1 x 30,000 30.9 -> 29.3).  With pages of 6 or 8 bits it depends on the step (6 bits: 48 x 3,000 30.4 -> 28.4 us, 100 x
+  // 3,000 40.4 -> 44.8), and at four KV heads the larger count is better (4 bits, block 64, 64 x 4,000: 61.7 against 52.6).
+  const bool few = gqa > 4 && H == 1 && chunks <= 2;
   if (ns < 4 || few) {
     small = true;
     V = H == 8 ? Teams<8>::V_SMALL : H == 4 ? Teams<4>::V_SMALL : H == 2 ? Teams<2>::V_SMALL : Teams<1>::V_SMALL;
@@ -1540,12 +1538,12 @@ static bool mma_shape_ok(int H, int D_, int VG, int KG, int BS, int gqa) {
 }
 
 // Teams of the tensor-core kernel on the current device for this shape (0: the generic kernel takes it, or no device).
-int decode_mma_teams(int H, int D_, int VG, int KG, int BS, int gqa) {
+int decode_mma_teams(int H, int D_, int VG, int KG, int BS, int gqa, int chunks) {
   if (g_decode_path == 1 || !mma_shape_ok(H, D_, VG, KG, BS, gqa)) return 0;
   DecodeDevice* dv = nullptr;
   if (decode_device(&dv)) return 0;
   TeamShape ts;
-  if (!team_shape(*dv, H, gqa, &ts)) return 0;
+  if (!team_shape(*dv, H, gqa, chunks, &ts)) return 0;
   return dv->num_sms * ts.V;
 }
 
@@ -1571,7 +1569,7 @@ int launch_decode_mma(const LayoutDev& L, const ResidualDev& R, const uint8_t* p
   P.wait_ns = g_wait_ns;
   P.idle_producer = g_idle_producer;
   TeamShape ts;
-  if (!team_shape(*dv, H, A.tok * A.gqa, &ts)) return ECHOKV_OK;
+  if (!team_shape(*dv, H, A.tok * A.gqa, L.KC, &ts)) return ECHOKV_OK;
   const int V = ts.V, ns = ts.ns, fixed = ts.fixed, sbytes = stage_bytes(H);
   const bool small = ts.small;
   P.NS = ns;

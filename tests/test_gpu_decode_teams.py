@@ -1,4 +1,4 @@
-"""Decode attention with more than four query heads per KV head at one and four KV heads, where the split kernel runs fewer teams an SM:
+"""Decode attention with more than four query heads per KV head; at one KV head and pages of 4 bits the split kernel runs fewer teams an SM:
 fewer work items than teams and several rounds of them, every tier, lengths around tiles, pairs and splits."""
 
 import numpy as np
@@ -18,7 +18,7 @@ def test_fewer_teams(h, gqa, bits):
     from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
 
     bs, blocks = 16, -(-TOKENS // 16)
-    layout = TieredLayout(num_kv_heads=h, head_size=D, block_size=bs, mem_bits=8, k_group=16, v_group=32)
+    layout = TieredLayout(num_kv_heads=h, head_size=D, block_size=bs, mem_bits=8 if bits == 8 else 4, k_group=16, v_group=32)
     store = TieredKVCache(layout, torch.zeros(blocks + 1, layout.page_bytes, dtype=torch.uint8, device="cuda"), residual_slots=4,
                           residual_dtype=torch.float16)
     gen = torch.Generator(device="cuda").manual_seed(h * 10 + gqa)
