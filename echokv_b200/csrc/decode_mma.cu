@@ -749,12 +749,20 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
   // The reference point of the exponentials only moves when a group's maximum exceeds it by more
   // than RESCALE_SLACK (in log2 units): until then p <= 2^RESCALE_SLACK, well inside fp16, and the
   // accumulators need no rescaling.  The result is the same softmax (the reference point cancels).
-  const bool grew = (t0 > w.m0 + RESCALE_SLACK) || (t1 > w.m1 + RESCALE_SLACK);
-  if (__any_sync(0xffffffffu, grew)) {
-    // a column moves only when it has outgrown its own reference: its bits do not depend on its neighbours'
-    const bool g0 = t0 > w.m0 + RESCALE_SLACK, g1 = t1 > w.m1 + RESCALE_SLACK;
-    const float n0 = g0 ? t0 : w.m0, n1 = g1 ? t1 : w.m1;
-    const float a0 = g0 ? ex2(w.m0 - n0) : 1.f, a1 = g1 ? ex2(w.m1 - n1) : 1.f;
+  const bool g0 = t0 > w.m0 + RESCALE_SLACK, g1 = t1 > w.m1 + RESCALE_SLACK;
+  if (__any_sync(0xffffffffu, g0 || g1)) {
+    float n0 = fmaxf(w.m0, t0), n1 = fmaxf(w.m1, t1);
+    float a0, a1;
+    if constexpr (MT) {  // the query heads of a token move together and not with another token's: its bits are those of the token alone
+      auto spread = [](uint32_t x) { return (x & 1) | (x & 2) << 1 | (x & 4) << 2 | (x & 8) << 3; };
+      const uint32_t b0 = __ballot_sync(0xffffffffu, g0), b1 = __ballot_sync(0xffffffffu, g1);
+      const uint32_t cols = spread(b0) | spread(b1) << 1, heads = (1u << P.A.gqa) - 1;  // lanes 0 .. 3 speak for the columns
+      const bool s0 = cols >> (ln.tk0 * P.A.gqa) & heads, s1 = cols >> (ln.tk1 * P.A.gqa) & heads;
+      a0 = s0 ? ex2(w.m0 - n0) : 1.f; a1 = s1 ? ex2(w.m1 - n1) : 1.f;
+      n0 = s0 ? n0 : w.m0; n1 = s1 ? n1 : w.m1;
+    } else {
+      a0 = ex2(w.m0 - n0); a1 = ex2(w.m1 - n1);
+    }
 #pragma unroll
     for (int mt = 0; mt < 8; ++mt) { w.acc[mt][0] *= a0; w.acc[mt][1] *= a1; w.acc[mt][2] *= a0; w.acc[mt][3] *= a1; }
     w.bl[0] *= a0; w.bl[1] *= a1; w.bl[2] *= a0; w.bl[3] *= a1;
