@@ -30,7 +30,7 @@ import torch
 from torch.profiler import record_function
 
 from echokv_b200 import _native as N
-from echokv_b200._util import to_device
+from echokv_b200._util import ranges_are_seen, to_device
 from echokv_b200.quant import EXTRA_CHUNKS, SUPPORTED_BITS
 from echokv_b200.write_plan import Eviction, SharedState, WriteMeta, WritePlan, stage_plan
 
@@ -382,7 +382,7 @@ class TieredKVCache:
         query rows).  ``capturing`` gives the group pass its full grid, masked by the device count."""
         from echokv_b200.kernels.write import write_step
 
-        if not torch.autograd._profiler_enabled():  # the range alone costs 8 us of host time a layer
+        if not ranges_are_seen():  # the range alone costs 8 us of host time a layer
             write_step(self, key, value, meta, kref, full_grid=capturing, stash=stash)
             return
         with record_function("echokv.write.step"):
