@@ -175,7 +175,7 @@ class ChunkPool:
 def lru_victims(tier: np.ndarray, full: np.ndarray, last: np.ndarray, chunks_needed: int, keep: np.ndarray) -> np.ndarray:
     """The least recently written INT4/INT8 blocks (``full``: mask of full blocks, ``last``: step of the last write; ties by
     block id) without those in ``keep``, up to the one whose extra chunks make ``chunks_needed``, or all there are."""
-    candidate = (tier >= 4) & full
+    candidate, keep = (tier >= 4) & full, np.asarray(keep, dtype=np.int64)
     candidate[keep[(keep >= 0) & (keep < candidate.size)]] = False
     ranked = np.flatnonzero(candidate)
     ranked = ranked[np.argsort(last[ranked], kind="stable")]

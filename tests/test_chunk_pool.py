@@ -61,6 +61,15 @@ def test_victims_are_those_of_the_sequential_loop(seed):
         assert lru_victims(tier, full, last, needed, keep).tolist() == want
 
 
+@pytest.mark.parametrize("keep", [[], [1], (1,), np.array([]), np.array([1.0]), np.array([1, -3, 99], dtype=np.int32)])
+def test_kept_blocks_take_every_form(keep):
+    """Lists, empty arrays (which are of floats) and ids outside the pool."""
+    from echokv_b200.tiered_cache import lru_victims
+
+    got = lru_victims(np.array([4, 8, 4]), np.ones(3, dtype=bool), np.arange(3), 9, keep)
+    assert got.tolist() == ([0, 2] if 1 in keep else [0, 1, 2])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", [set, list, np.array])
 def test_protected_blocks_of_every_form_stay(form):
