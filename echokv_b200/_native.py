@@ -85,7 +85,7 @@ _SIGS = {
     "echokv_decode_step": [_LP, _PP, _RP, _P, _I64, _I64, _I32, _P, _P, _I64, _P, _P, _P, _I64, _P, _I64, _I64, _I32,
                            _F, _I32, _I32, _P, _I64, _I32, _P],
     "echokv_decode_chunks": [_LP, _PP, _RP, _P, _I64, _I64, _I32, _P, _P, _I64, _P, _P, _P, _I64, _P, _I64, _I64, _I32,
-                             _F, _I32, _I32, _P, _I64, _I64, _I32, _P],
+                             _F, _I32, _I32, _P, _I64, _I32, _P, _I64, _I32, _P],
     "echokv_decode_static": [_LP, _PP, _RP, _P, _I64, _I64, _I32, _P, _P, _I64, _P, _P, _P, _I64, _I64, _I32,
                              _F, _I32, _I32, _I64, _I32, _P],
     "echokv_dequant_dense": [_LP, _PP, _RP, _P, _I64, _P, _I64, _P, _P, _I64, _I64, _I32, _P],
@@ -120,10 +120,12 @@ lib.echokv_planner_plan.argtypes = [C.c_void_p, C.c_void_p, C.c_int64] + [C.c_vo
 lib.echokv_planner_plan.restype = C.c_int
 lib.echokv_decode_parallelism.argtypes = [_LP, C.c_int32]
 lib.echokv_decode_parallelism.restype = C.c_int32
+lib.echokv_chunk_groups.argtypes = [_P, _I64, _I64, _P, _I32, _P, _P, _P, _P]
+lib.echokv_chunk_groups.restype = C.c_int64
 lib.echokv_kernel_status.argtypes = [C.c_int]
 lib.echokv_kernel_status.restype = C.c_int
 
-EXPORTS = sorted(list(_SIGS) + ["echokv_set_decode_path", "echokv_set_decode_wait_limit", "echokv_kernel_status", "echokv_set_prefill_path", "echokv_decode_static_scratch_bytes", "echokv_decode_parallelism", "echokv_planner_create", "echokv_planner_destroy", "echokv_planner_get",
+EXPORTS = sorted(list(_SIGS) + ["echokv_set_decode_path", "echokv_set_decode_wait_limit", "echokv_kernel_status", "echokv_set_prefill_path", "echokv_decode_static_scratch_bytes", "echokv_decode_parallelism", "echokv_chunk_groups", "echokv_planner_create", "echokv_planner_destroy", "echokv_planner_get",
                                 "echokv_planner_sealed_mask", "echokv_planner_plan", "echokv_abi_version", "echokv_last_error", "echokv_decode_scratch_bytes",
                                 "echokv_demote_scratch_bytes"])
 

@@ -21,18 +21,17 @@ int prefill_status_take(bool clear);
 // and a CTA per head (before) made 8,192 CTAs of a batch of 256 sequences x 32 heads: 27.8 us, now 6.7 us; one sequence x 8 splits 3.75 -> 2.5 us,
 // 528 rows x 24 splits 54 -> 11 us.
 constexpr int MERGE_HEADS = 4;
-template <int VEC, bool CHUNKS>
+template <int VEC>
 __global__ void __launch_bounds__(MERGE_HEADS * 32) decode_merge_kernel(DecodeArgs A, int BS, int D) {
   constexpr int BATCH = 8;
   using V = typename std::conditional<VEC == 4, float4, float2>::type;
-  const int row = blockIdx.x, head = blockIdx.y * MERGE_HEADS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int seq = CHUNKS ? row / A.tok : row, tk = CHUNKS ? row - seq * A.tok : 0;  // the row is token tk of its sequence
+  const int seq = blockIdx.x, head = blockIdx.y * MERGE_HEADS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int d = (blockIdx.z * 32 + lane) * VEC;  // this lane's channels
   pdl_launch_dependents();
   pdl_wait();  // the split kernel has completed
-  if (row == 0 && head == 0 && blockIdx.z == 0 && lane == 0) A.state[0] = 0;  // its item counter, for the next call
+  if (seq == 0 && head == 0 && blockIdx.z == 0 && lane == 0) A.state[0] = 0;  // its item counter, for the next call
   if (head >= A.Hq) return;
-  const int64_t base = ((int64_t)row * A.Hq + head) * A.num_splits;
+  const int64_t base = ((int64_t)seq * A.Hq + head) * A.num_splits;
   const float* src = A.acc + base * D + min(d, D - VEC);
   // The first splits' partials are read along with the length that says how many there are (the rows exist either way).
   V x[BATCH];
@@ -40,9 +39,9 @@ __global__ void __launch_bounds__(MERGE_HEADS * 32) decode_merge_kernel(DecodeAr
   if (lane < A.num_splits) ml = *reinterpret_cast<const float2*>(A.ml + (base + lane) * 2);
 #pragma unroll
   for (int k = 0; k < BATCH; ++k) x[k] = *reinterpret_cast<const V*>(src + (int64_t)min(k, A.num_splits - 1) * D);
-  const int64_t seq_len = seq_length<CHUNKS>(A, seq);
-  const int64_t o_row = seq_query<CHUNKS>(A, seq) + tk;
-  if (seq_len == 0 || tk >= seq_tokens<CHUNKS>(A, seq)) return;  // CUDA-graph padding, a group's missing tokens: leave the row alone
+  const int64_t seq_len = A.lens[seq];
+  const int64_t o_row = A.q_rows ? A.q_rows[seq] : seq;
+  if (seq_len == 0) return;  // CUDA-graph padding: leave the row alone
   const int n_blocks = (int)((seq_len + BS - 1) / BS);
   const int bps = max(bps_floor(A), (n_blocks + A.num_splits - 1) / A.num_splits);
   const int used = (n_blocks + bps - 1) / bps;
@@ -136,7 +135,8 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
                        void* scratch, int64_t scratch_bytes, void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
                        float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
                        const int32_t* blocks_per_split_dev, bool zero_state, bool planned, int64_t num_seqs,
-                       int32_t num_q_heads, void* stream, const int64_t* groups = nullptr, int64_t num_groups = 0) {
+                       int32_t num_q_heads, void* stream, const int64_t* groups = nullptr, int64_t num_groups = 0,
+                       int32_t group_tokens = 1, const int64_t* split_lens = nullptr) {
   if (num_seqs <= 0) return ECHOKV_OK;
   LayoutDev L;
   ResidualDev R;
@@ -149,16 +149,7 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
   if (num_q_heads % L.H) return set_error(ECHOKV_E_ARGUMENT, "decode: %d query heads not a multiple of %d KV heads", num_q_heads, L.H);
   if (q_dtype < 0 || q_dtype > 2 || out_dtype < 0 || out_dtype > 2) return set_error(ECHOKV_E_ARGUMENT, "decode: bad dtype");
   const int gqa = num_q_heads / L.H;
-  // Groups of consecutive tokens: where two or more tokens' query heads fit the eight columns of the tensor-core kernel's MMAs
-  // (a step of 16 chunks of 33 tokens, 32 / 8 heads: 1.72 -> 1.14 ms); with five or more there is nothing to share.
-  int64_t parts = 0;
-  if (groups && num_groups > 0 && gqa <= CHUNK_GROUP / 2) {
-    const int tok = CHUNK_GROUP / gqa;
-    if (decode_mma_teams(L.H, L.D, L.VG, L.KG, L.BS, tok * gqa, L.KC) > 0) parts = num_groups * (CHUNK_GROUP / tok);
-  }
-  const int64_t rows = parts ? num_groups * CHUNK_GROUP : num_seqs;
-  if (scratch_bytes < echokv_decode_scratch_bytes(rows > num_seqs ? rows : num_seqs, num_q_heads, L.D, num_splits) ||
-      (reinterpret_cast<uintptr_t>(scratch) & 15))
+  if (scratch_bytes < echokv_decode_scratch_bytes(num_seqs, num_q_heads, L.D, num_splits) || (reinterpret_cast<uintptr_t>(scratch) & 15))
     return set_error(ECHOKV_E_ARGUMENT, "decode: scratch too small (%lld bytes) or misaligned", (long long)scratch_bytes);
   if (gqa > 16) return set_error(ECHOKV_E_UNSUPPORTED, "decode: %d query heads per KV head (max 16)", gqa);
 
@@ -168,25 +159,25 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
   // scratch = [256 bytes of work-queue state][split partials: accumulators, then running max / sum]
   A.state = reinterpret_cast<int*>(scratch);
   A.acc = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + 256);
-  A.ml = A.acc + (rows > num_seqs ? rows : num_seqs) * num_q_heads * (int64_t)num_splits * L.D;
+  A.ml = A.acc + num_seqs * num_q_heads * (int64_t)num_splits * L.D;
   A.out = out; A.o_s0 = o_s0; A.o_s1 = o_s1; A.out_dt = out_dtype;
   A.scale_log2e = softmax_scale * 1.4426950408889634f;
   A.num_splits = num_splits; A.bps_min = blocks_per_split; A.gqa = gqa; A.Hq = num_q_heads;
   A.bps_dev = blocks_per_split_dev;
   A.planned = planned;
-  A.counts = nullptr; A.tok = A.sub = 1;
+  A.groups = nullptr; A.tok = 1;
   cudaStream_t st = (cudaStream_t)stream;
   const uint8_t* pg = (const uint8_t*)pages->base;
 
   bool handled = false;
-  int64_t merge_rows = num_seqs;
-  if (parts) {
+  // Groups of consecutive tokens, where the query heads of two or more tokens fit the columns of the tensor-core kernel's MMAs (a step
+  // of 16 chunks of 33 tokens, 32 / 8 heads: 1.72 -> 1.14 ms).  Their partials are those of the tokens one by one, so the merge is too.
+  if (num_groups > 0 && group_tokens > 1) {
     DecodeArgs G = A;
-    G.q_rows = groups; G.bt_rows = groups + num_groups; G.lens = groups + 2 * num_groups; G.counts = groups + 3 * num_groups;
-    G.tok = CHUNK_GROUP / gqa; G.sub = CHUNK_GROUP / G.tok;
-    rc = launch_decode_mma(L, R, pg, G, parts, A.state, zero_state, nullptr, st, &handled);
+    G.groups = groups; G.tok = group_tokens;
+    rc = launch_decode_mma(L, R, pg, G, num_groups, A.state, zero_state, nullptr, st, &handled);
     if (rc) return rc;
-    if (handled) { A = G; merge_rows = parts * G.tok; }
+    if (handled) A.lens = split_lens;
   }
   if (!handled) {
     rc = launch_decode_mma(L, R, pg, A, num_seqs, A.state, zero_state, nullptr, st, &handled);
@@ -203,13 +194,12 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
     rc = check_launch("decode");
     if (rc) return rc;
   }
-  dim3 mgrid((unsigned)merge_rows, (unsigned)((num_q_heads + MERGE_HEADS - 1) / MERGE_HEADS), (unsigned)((L.D + 127) / 128));
+  dim3 mgrid((unsigned)num_seqs, (unsigned)((num_q_heads + MERGE_HEADS - 1) / MERGE_HEADS), (unsigned)((L.D + 127) / 128));
   const int vec = L.D == 64 ? 2 : 4;
   A.out_vec = out_dtype != ECHOKV_DT_F32 && ((o_s0 | o_s1) % vec) == 0 && (reinterpret_cast<uintptr_t>(out) % (2 * vec)) == 0;
   cudaError_t e;
-  if (A.counts) e = launch_pdl(decode_merge_kernel<4, true>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
-  else if (L.D == 64) e = launch_pdl(decode_merge_kernel<2, false>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
-  else e = launch_pdl(decode_merge_kernel<4, false>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
+  if (L.D == 64) e = launch_pdl(decode_merge_kernel<2>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
+  else e = launch_pdl(decode_merge_kernel<4>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
   if (e != cudaSuccess) return check_launch("decode merge");
   return check_launch("decode merge");
 }
@@ -241,10 +231,13 @@ int echokv_decode_chunks(const echokv_layout* layout, const echokv_pages* pages,
                          const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
                          void* scratch, int64_t scratch_bytes, void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
                          float softmax_scale, int32_t num_splits, int32_t blocks_per_split, const int64_t* groups,
-                         int64_t num_groups, int64_t num_seqs, int32_t num_q_heads, void* stream) {
+                         int64_t num_groups, int32_t group_tokens, const int64_t* split_lens, int64_t num_seqs, int32_t num_q_heads,
+                         void* stream) {
+  if (num_groups > 0 && (!groups || !split_lens || group_tokens < 1))
+    return set_error(ECHOKV_E_ARGUMENT, "decode_chunks: groups need their records, their tokens' split lengths and a size");
   return decode_impl(layout, pages, residual, query, q_s0, q_s1, q_dtype, q_rows, block_table, bt_s0, bt_rows, lens, scratch,
                      scratch_bytes, out, o_s0, o_s1, out_dtype, softmax_scale, num_splits, blocks_per_split,
-                     nullptr, false, false, num_seqs, num_q_heads, stream, groups, num_groups);
+                     nullptr, false, false, num_seqs, num_q_heads, stream, groups, num_groups, group_tokens, split_lens);
 }
 
 int echokv_decode(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,

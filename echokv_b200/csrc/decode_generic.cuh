@@ -30,39 +30,36 @@ struct DecodeArgs {
   int planned;             // the step's metadata was final before the kernel in front of the split kernel (echokv_decode_step)
   int out_vec;             // the merge can store a lane's channels of `out` at once (its launcher sets it)
   int* state;              // work-queue state at the start of the scratch: [0] = the split kernel's item counter
-  // Chunks of query tokens (echokv_decode_chunks, tensor-core kernel only): `counts` holds the 1 .. CHUNK_GROUP consecutive query
-  // tokens of every group, `q_rows` / `lens` belong to a group's first / last token, and a "sequence" of the kernels is one of the
-  // `sub` parts of `tok` tokens that a group is worked off in.  NULL, tok = sub = 1: one token per sequence.
-  const int64_t* counts;
-  int tok, sub;
+  // Chunks of query tokens (echokv_decode_chunks, tensor-core kernel only): a "sequence" of the split kernel is a group of 1 .. `tok`
+  // consecutive tokens, described by a record of GROUP_WORDS words.  NULL, tok = 1: one token per sequence.
+  const int64_t* groups;
+  int tok;
 };
-constexpr int CHUNK_GROUP = 8;
+// A group's record: query row of its first token, block-table row, cache length of its last token, tokens, place of its first token in
+// the call's list of tokens (whose partials' rows the group's results go to).
+constexpr int GROUP_QUERY = 0, GROUP_TABLE = 1, GROUP_LEN = 2, GROUP_TOKENS = 3, GROUP_FIRST = 4, GROUP_WORDS = 5;
 
-// Tokens, cache length of the last token, first query row and block-table row of "sequence" `seq` (see DecodeArgs::counts).
+// Tokens, cache length of the last token, first query row and block-table row of "sequence" `seq`.
 template <bool CHUNKS>
 __device__ __forceinline__ int seq_tokens(const DecodeArgs& A, int seq) {
   if constexpr (!CHUNKS) return 1;
-  const int g = seq / A.sub, s = seq - g * A.sub;
-  return max(0, min(A.tok, (int)A.counts[g] - s * A.tok));
+  return min(A.tok, (int)A.groups[(int64_t)seq * GROUP_WORDS + GROUP_TOKENS]);
 }
 template <bool CHUNKS>
 __device__ __forceinline__ int64_t seq_length(const DecodeArgs& A, int seq) {
   if constexpr (!CHUNKS) return A.lens[seq];
-  const int g = seq / A.sub, s = seq - g * A.sub, left = (int)A.counts[g] - s * A.tok;  // tokens from this part on
-  return left <= 0 ? 0 : A.lens[g] - (left - min(A.tok, left));
+  return A.groups[(int64_t)seq * GROUP_WORDS + GROUP_LEN];
 }
 template <bool CHUNKS>
 __device__ __forceinline__ int64_t seq_query(const DecodeArgs& A, int seq) {
   if constexpr (!CHUNKS) return A.q_rows ? A.q_rows[seq] : seq;
-  const int g = seq / A.sub;
-  return A.q_rows[g] + (seq - g * A.sub) * A.tok;
+  return A.groups[(int64_t)seq * GROUP_WORDS + GROUP_QUERY];
 }
 template <bool CHUNKS>
 __device__ __forceinline__ int64_t seq_table(const DecodeArgs& A, int seq) {
-  const int g = CHUNKS ? seq / A.sub : seq;
-  return A.bt_rows ? A.bt_rows[g] : g;
+  if constexpr (!CHUNKS) return A.bt_rows ? A.bt_rows[seq] : seq;
+  return A.groups[(int64_t)seq * GROUP_WORDS + GROUP_TABLE];
 }
-
 // Lower bound of a split's size in blocks: the call's argument, raised by the run-time value when there is one (an
 // ordinary load: the word may have been written while a kernel launched ahead of time was already resident).
 __device__ __forceinline__ int bps_floor(const DecodeArgs& A) {

@@ -54,6 +54,7 @@ __device__ unsigned long long g_cta[1024 * 4];  // per CTA: start ns, end ns, SM
 constexpr int D = 128;          // head size of this kernel
 constexpr int NG = 4;           // V groups per head (v_group 32)
 constexpr int TILE = 16;        // tokens per tile
+constexpr int COLS = 8;         // columns of the MMAs: query heads of a token, or of consecutive tokens of a chunk
 constexpr unsigned long long WAIT_NS = 2000000000ull;  // a wait gives up after this long (echokv_set_decode_wait_limit changes it)
 
 // What the producer tells the consumers about a staged group (stored at `o_hdr` of its first stage).
@@ -376,6 +377,7 @@ struct Lane {
   uint32_t vm_ld8;    // INT8 stages: this lane's ldmatrix row of the [v_min | ones] operand (stage by lane & 16)
   int tk0, tk1;       // MT: token of its sequence that column 2j / 2j + 1 belongs to
   int d0, d1;         // MT: how many tokens fewer it sees than the sequence's last token (-1: no such token)
+  int first;          // MT: row of partials of the sequence's first token
 };
 
 // This lane's ldmatrix row offset inside a stage for the K side / V side of tier BITS: lane & 7 picks the slot
@@ -717,7 +719,7 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
     }
   }
   if constexpr (MT) {  // near the sequence's end: every column up to its own token
-    if (rem < NT * TILE + CHUNK_GROUP) {
+    if (rem < NT * TILE + COLS) {
       const int t0 = BITS == 8 ? ln.r : 2 * ln.r, t1 = BITS == 8 ? ln.r + 8 : 2 * ln.r + 1;  // tokens of MMA rows r / r + 8
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
@@ -824,8 +826,8 @@ __device__ __forceinline__ void write_partial(const Params& P, const Lane& ln, c
   const DecodeArgs& A = P.A;
   const int g0 = 2 * j, g1 = 2 * j + 1;
   // MT: columns are (token, query head of the group) pairs
-  const int64_t r0 = MT ? ((int64_t)seq * A.tok + ln.tk0) * A.Hq + g0 - ln.tk0 * A.gqa : (int64_t)seq * A.Hq + g0;
-  const int64_t r1 = MT ? ((int64_t)seq * A.tok + ln.tk1) * A.Hq + g1 - ln.tk1 * A.gqa : (int64_t)seq * A.Hq + g1;
+  const int64_t r0 = MT ? (int64_t)(ln.first + ln.tk0) * A.Hq + g0 - ln.tk0 * A.gqa : (int64_t)seq * A.Hq + g0;
+  const int64_t r1 = MT ? (int64_t)(ln.first + ln.tk1) * A.Hq + g1 - ln.tk1 * A.gqa : (int64_t)seq * A.Hq + g1;
   const int64_t o0 = (r0 + h * A.gqa) * A.num_splits + split, o1 = (r1 + h * A.gqa) * A.num_splits + split;
   float* dst0 = A.acc + o0 * D;
   float* dst1 = A.acc + o1 * D;
@@ -887,7 +889,7 @@ template <int H> struct Teams {
   static constexpr int V_SMALL = H == 8 ? 1 : (H == 4 ? 3 : (H == 2 ? 4 : 8));
 };
 
-// MT: the MMAs' columns are the query heads of several consecutive tokens of a chunk (DecodeArgs::counts): the codes are unpacked, the
+// MT: the MMAs' columns are the query heads of several consecutive tokens of a chunk (DecodeArgs::groups): the codes are unpacked, the
 // scales folded and the pages read once for all of them.  With a sequence per token, 528 tokens of 16 chunks over 1,440 stored
 // ones (32 / 8 heads, two tokens a pass) took 273 us a layer with the merge, now 158.
 template <int H, int V, bool MT>
@@ -971,12 +973,13 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     // the grid, 9 in use: a dozen round trips per team).  A sequence of n blocks uses at most min(num_splits,
     // ceil(n / bps_min)) splits, so the longest one bounds the items.  Every producer of the grid runs the loop: with
     // the split rule's divisions per sequence in it, 4,096 rows of 40 tokens at one KV head took 97 us, now 51 us, and
-    // 256 of 1,000 took 31.4, now 29.6 us.
-    int used_max = 1;
-    if (A.num_splits > 1) {
+    // 256 of 1,000 took 31.4, now 29.6 us.  The groups of chunks come in an eager call, whose grid fits its longest context: there the
+    // records, 40 bytes apart, are not looked through.
+    int used_max = MT ? A.num_splits : 1;
+    if (!MT && A.num_splits > 1) {
       int longest = 0;
 #pragma unroll 4
-      for (int i = lane; i < P.num_seqs / (MT ? A.sub : 1); i += 32) longest = max(longest, (int)A.lens[i]);
+      for (int i = lane; i < P.num_seqs; i += 32) longest = max(longest, (int)A.lens[i]);
       longest = __reduce_max_sync(0xffffffffu, longest);
       used_max = min(A.num_splits, ((longest + L.BS - 1) / L.BS + bps_min - 1) / bps_min);
     }
@@ -1297,6 +1300,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
       const int n_rows = MT ? seq_tokens<MT>(A, seq) * A.gqa : A.gqa;  // columns that have a token
       if constexpr (MT) {
         const int last = seq_tokens<MT>(A, seq) - 1;
+        ln.first = (int)A.groups[(int64_t)seq * GROUP_WORDS + GROUP_FIRST];
         ln.d0 = ln.tk0 < A.tok && ln.tk0 <= last ? last - ln.tk0 : -1;
         ln.d1 = ln.tk1 < A.tok && ln.tk1 <= last ? last - ln.tk1 : -1;
       }
@@ -1484,7 +1488,7 @@ static void launch_teams(bool small, unsigned grid, int smem_bytes, cudaStream_t
 }
 template <int H>
 static void launch_teams(bool small, unsigned grid, int smem_bytes, cudaStream_t st, const mma::Params& P) {
-  if (P.A.counts) launch_teams<H, true>(small, grid, smem_bytes, st, P);
+  if (P.A.groups) launch_teams<H, true>(small, grid, smem_bytes, st, P);
   else launch_teams<H, false>(small, grid, smem_bytes, st, P);
 }
 static int decode_device(DecodeDevice** out) {
@@ -1541,7 +1545,7 @@ static bool mma_shape_ok(int H, int D_, int VG, int KG, int BS, int gqa) {
   using namespace mma;
   // a block of a power of two of tokens: only then does a tile's run of rows never cross from one chunk to the next;
   // of at most UNIT tiles: the producer plans at least one whole block at a time
-  return D_ == D && VG == 32 && KG % TILE == 0 && BS % TILE == 0 && (BS & (BS - 1)) == 0 && BS <= UNIT * TILE && gqa <= 8 &&
+  return D_ == D && VG == 32 && KG % TILE == 0 && BS % TILE == 0 && (BS & (BS - 1)) == 0 && BS <= UNIT * TILE && gqa <= COLS &&
          (H == 1 || H == 2 || H == 4 || H == 8);
 }
 

@@ -2,6 +2,10 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <algorithm>
+#include <exception>
+#include <numeric>
+#include <vector>
 
 #include "common.cuh"
 
@@ -95,6 +99,49 @@ const char* echokv_last_error(void) { return echokv::g_err; }
 
 int echokv_layout_describe(const echokv_layout* layout, echokv_layout_info* out) {
   return echokv::describe(layout, out);
+}
+
+int64_t echokv_chunk_groups(const int64_t* chunks, int64_t num_chunks, int64_t num_tokens, const int64_t* widths, int32_t num_widths,
+                            int64_t* rows, int64_t* split_lens, int64_t* groups, int64_t* num_groups) {
+  const int64_t n = num_tokens;
+  std::vector<int64_t> order, place;  // chunks from the longest context to the shortest; where a chunk's tokens begin in the list
+  try {
+    order.resize(num_chunks);
+    place.resize(num_chunks + 1);
+  } catch (const std::exception&) {  // no memory, or a negative count
+    return echokv::set_error(ECHOKV_E_ARGUMENT, "chunk_groups: no memory for %lld chunks", (long long)num_chunks);
+  }
+  std::iota(order.begin(), order.end(), 0);
+  std::sort(order.begin(), order.end(), [&](int64_t a, int64_t b) {
+    return chunks[4 * a + 2] != chunks[4 * b + 2] ? chunks[4 * a + 2] > chunks[4 * b + 2] : a < b;
+  });
+  for (int64_t c = 0; c < num_chunks; ++c) {
+    if (chunks[4 * c + 1] < 0) return echokv::set_error(ECHOKV_E_ARGUMENT, "chunk_groups: a chunk of %lld tokens", (long long)chunks[4 * c + 1]);
+    place[c + 1] = place[c] + chunks[4 * c + 1];
+  }
+  if (place[num_chunks] != n)
+    return echokv::set_error(ECHOKV_E_ARGUMENT, "chunk_groups: %lld tokens, not %lld", (long long)place[num_chunks], (long long)n);
+  for (int64_t c = 0, at = 0; c < num_chunks; ++c)
+    for (int64_t i = 0; i < chunks[4 * c + 1]; ++i, ++at) {
+      rows[at] = chunks[4 * c] + i;
+      rows[n + at] = chunks[4 * c + 3];
+      rows[2 * n + at] = chunks[4 * c + 2] - chunks[4 * c + 1] + 1 + i;
+    }
+  int64_t total = 0;
+  for (int32_t k = 0; k < num_widths; ++k) {
+    const int64_t before = total;
+    for (const int64_t c : order)
+      for (int64_t first = place[c], end = place[c + 1]; first < end;) {
+        int64_t next = first + 1;
+        while (next < end && next - first < widths[k]) ++next;
+        int64_t* g = groups + 5 * total++;
+        g[0] = rows[first]; g[1] = rows[n + first]; g[2] = rows[2 * n + next - 1]; g[3] = next - first; g[4] = first;
+        for (int64_t i = first; i < next; ++i) split_lens[k * n + i] = g[2];
+        first = next;
+      }
+    num_groups[k] = total - before;
+  }
+  return total;
 }
 
 }  // extern "C"

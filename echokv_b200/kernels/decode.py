@@ -14,7 +14,7 @@ BLOCKS_PER_SPLIT = 16
 MAX_DECODE_SPLITS = 64  # upper bound of the split grid (backend.py:67-69 of the reference caps its fixed grid alike)
 EAGER_MAX_SPLITS = 32   # calls that size their own grid (the prefill row path): their scratch grows with rows x splits
 MIN_SPLIT_TOKENS = 64   # smallest split `choose_blocks_per_split` proposes
-CHUNK_GROUP = 8         # consecutive query tokens of a chunk that are handed to the kernels together (CHUNK_GROUP in csrc)
+MMA_COLUMNS = 8         # columns of the split kernel's MMAs: query heads of a token, or of consecutive tokens of a chunk
 ITEM_COST_TILES = 4     # fixed cost of a (sequence, split) work item in units of one 16-token tile's work
 
 
@@ -92,7 +92,7 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
                      q_rows: torch.Tensor | None = None, bt_rows: torch.Tensor | None = None,
                      out: torch.Tensor | None = None, max_len: int | None = None,
                      num_splits: int | None = None, bps_dev: torch.Tensor | None = None,
-                     planned: bool = False, groups: torch.Tensor | None = None) -> torch.Tensor:
+                     planned: bool = False, groups: dict | None = None) -> torch.Tensor:
     """Attention of one query token per sequence over each sequence's cache.
 
     Sequence ``i`` uses query row ``q_rows[i]`` and block-table row ``bt_rows[i]``
@@ -105,9 +105,9 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
     device, or the low half of an int64) raises ``blocks_per_split`` at run time: a captured graph
     keeps reading it, so the host can size the splits for every replayed step.  ``planned``: a write of the
     same step is ahead on the stream, and everything but the queries and the pages' rows was final before it, so the
-    kernel may read that while the kernel before it still runs.  ``groups`` (int64 ``[4, G]`` on the device, from
-    ``kernels.prefill.build_rows``): the sequences are tokens of chunks, listed there in runs of up to ``CHUNK_GROUP``
-    consecutive tokens (first query row, block-table row, length of the last token, tokens); it excludes ``bps_dev``.
+    kernel may read that while the kernel before it still runs.  ``groups`` (from
+    ``kernels.prefill.build_rows``): the sequences are tokens of chunks; per number of tokens that share a pass the device int64
+    tensors ``[G, 5]`` of their runs and ``[S]`` of their split lengths (``echokv_decode_chunks``); it excludes ``bps_dev``.
     """
     L = store.layout
     given = (block_table, seq_lens, q_rows, bt_rows)
@@ -140,25 +140,26 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
         num_splits = max(1, min(-(-max_blocks // blocks_per_split), EAGER_MAX_SPLITS))
     if s == 0:
         return out
-    nbytes = N.lib.echokv_decode_scratch_bytes(s if groups is None else max(s, CHUNK_GROUP * groups.shape[1]), hq, L.head_size,
-                                               num_splits)
+    nbytes = N.lib.echokv_decode_scratch_bytes(s, hq, L.head_size, num_splits)
     scratch = _scratch.get(dev, nbytes)
     if bps_dev is not None:
         N.require_cuda(bps_dev)
         if bps_dev.dtype not in (torch.int32, torch.int64) or bps_dev.numel() < 1:
             raise TypeError("bps_dev must hold one int32 / int64 on the device")
-    if groups is not None:
-        N.require_cuda(groups, q_rows, bt_rows)
-        if groups.dtype != torch.long or groups.dim() != 2 or groups.shape[0] != 4 or not groups.is_contiguous() or bps_dev is not None:
-            raise ValueError("groups must be a contiguous int64 [4, G] tensor, without bps_dev")
+    width = MMA_COLUMNS * L.num_kv_heads // hq if groups is not None else 0
+    if groups is not None and width in groups:  # two or more tokens fit
+        if bps_dev is not None:
+            raise ValueError("groups exclude bps_dev")
+        runs, split_lens = groups[width]
+        N.require_cuda(runs, split_lens)
         N.check(N.lib.echokv_decode_chunks(
             store.c_layout, store.c_pages, store.c_res,
             query.data_ptr(), q_s[0], q_s[1], N.dtype_code(query.dtype), N.ptr(q_rows),
             block_table.data_ptr(), bt_s[0], N.ptr(bt_rows), lens.data_ptr(),
             scratch.data_ptr(), scratch.numel(),
             out.data_ptr(), o_s[0], o_s[1], N.dtype_code(out.dtype),
-            float(softmax_scale), int(num_splits), int(blocks_per_split), groups.data_ptr(), groups.shape[1], s, hq,
-            N.stream_ptr(dev)))
+            float(softmax_scale), int(num_splits), int(blocks_per_split), runs.data_ptr(), runs.shape[0], width,
+            split_lens.data_ptr(), s, hq, N.stream_ptr(dev)))
         return out
     # a conversion above is itself the kernel before this one
     planned = planned and given[0] is block_table and given[1] is lens and given[2] is q_rows and given[3] is bt_rows

@@ -23,9 +23,10 @@ import torch
 
 from echokv_b200 import _native as N
 from echokv_b200._util import to_device
-from echokv_b200.kernels.decode import CHUNK_GROUP, decode_attention
+from echokv_b200.kernels.decode import decode_attention
 
 ROW_PATH_MAX_CHUNK = 64  # longer chunks take the dense path when it is available
+GROUP_WIDTHS = np.array([8, 4, 2], dtype=np.int64)  # tokens that share a pass with one, two, and three or four query heads per KV head
 
 
 def build_dequant_work(prefill, req_of, block_size: int, device) -> torch.Tensor:
@@ -61,36 +62,26 @@ def dequant_dense(store, work: torch.Tensor, total_ctx: int, block_table: torch.
 
 
 class RowPlan(tuple):
-    """What ``build_rows`` returns: a 4-tuple (query rows, block-table rows, causal limits, largest limit), with the same tokens as
-    ``groups`` of consecutive ones for ``decode_attention``."""
+    """What ``build_rows`` returns: a 4-tuple (query rows, block-table rows, causal limits, largest limit), with the same tokens in
+    runs of consecutive ones as ``groups`` for ``decode_attention``."""
 
-    groups: torch.Tensor
+    groups: dict
 
 
 def build_rows(prefill, req_of, device):
     """Row-path metadata: per query token its row, its request and its causal limit (device int64), and the largest limit."""
-    pairs = list(zip(prefill, req_of))
-    start = np.array([p[0] for p, _ in pairs], dtype=np.int64)
-    nq = np.array([max(p[1] - p[0], 0) for p, _ in pairs], dtype=np.int64)
-    ctx = np.array([p[2] for p, _ in pairs], dtype=np.int64)
-    req = np.array([r for _, r in pairs], dtype=np.int64)
-    n, per = int(nq.sum()), -(-nq // CHUNK_GROUP)
-    g = int(per.sum())
-    buf = np.empty(3 * n + 4 * g, dtype=np.int64)
-    rows, groups = buf[: 3 * n].reshape(3, n), buf[3 * n:].reshape(4, g)
-    at = np.arange(n) - np.repeat(np.cumsum(nq) - nq, nq)  # place in the chunk
-    rows[0] = np.repeat(start, nq) + at
-    rows[1] = np.repeat(req, nq)
-    rows[2] = np.repeat(ctx - nq + 1, nq) + at
-    first = (np.arange(g) - np.repeat(np.cumsum(per) - per, per)) * CHUNK_GROUP  # place of a group's first token
-    groups[3] = np.minimum(CHUNK_GROUP, np.repeat(nq, per) - first)
-    groups[0] = np.repeat(start, per) + first
-    groups[1] = np.repeat(req, per)
-    groups[2] = np.repeat(ctx - nq, per) + first + groups[3]
-    dev = to_device(torch.from_numpy(buf), device)
-    packed = dev[: 3 * n].view(3, n)
-    plan = RowPlan((packed[0], packed[1], packed[2], int(rows[2].max(initial=0))))
-    plan.groups = dev[3 * n:].view(4, g)
+    chunks = np.array([(p[0], max(p[1] - p[0], 0), p[2], r) for p, r in zip(prefill, req_of)], dtype=np.int64).reshape(-1, 4)
+    n, widths = int(chunks[:, 1].sum()), GROUP_WIDTHS.size
+    buf, counts = np.empty((3 + 6 * widths) * n, dtype=np.int64), np.empty(widths, dtype=np.int64)
+    words = [k * n for k in (0, 3, 3 + widths)]  # where the rows, the split lengths and the groups begin
+    at = [buf.ctypes.data + 8 * w for w in words]
+    total = N.lib.echokv_chunk_groups(chunks.ctypes.data, chunks.shape[0], n, GROUP_WIDTHS.ctypes.data, widths, *at, counts.ctypes.data)
+    if total < 0:
+        N.check(total)
+    dev = to_device(torch.from_numpy(buf[: words[2] + 5 * total]), device)
+    packed, lens, groups = dev[: words[1]].view(3, n), dev[words[1]: words[2]].view(widths, n), dev[words[2]:].view(-1, 5)
+    plan = RowPlan((packed[0], packed[1], packed[2], int(buf[2 * n: 3 * n].max(initial=0))))
+    plan.groups = {int(w): (g, lens[i]) for i, (w, g) in enumerate(zip(GROUP_WIDTHS, groups.split(counts.tolist())))}
     return plan
 
 

@@ -244,19 +244,28 @@ int echokv_decode_step(const echokv_layout* layout, const echokv_pages* pages, c
                        const int32_t* blocks_per_split_dev, int64_t num_seqs, int32_t num_q_heads, void* stream);
 
 /* echokv_decode_ex (without a run-time split size) for sequences that are the query tokens of chunks: consecutive tokens of a chunk
- * see the same cache, one token more each, and are worked off together where the shape allows it.  `groups` int64 [4, num_groups],
- * row after row: the query row of a group's first token, its block-table row, the cache length of its last token, its tokens
- * (1 .. 8, on consecutive query rows; cut from each chunk's first token on, so that a token's result follows from its chunk
- * alone).  Together the groups hold the num_seqs tokens that q_rows / bt_rows / lens list one by one, which serve the shapes that
- * take one token at a time (more than four query heads per KV head, and those of the generic kernel).  `scratch` holds
- * max(num_seqs, 8 * num_groups) sequences (echokv_decode_scratch_bytes). */
+ * see the same cache, one token more each, and are worked off together where the shape allows it.  q_rows / bt_rows / lens list the
+ * num_seqs tokens one by one.  `groups` int64 [num_groups, 5] lists the same tokens in runs of 1 .. group_tokens consecutive ones of
+ * a chunk, on consecutive query rows: the query row of a run's first token, its block-table row, the cache length of its last
+ * token, its tokens, and the place of its first token in the list of tokens.  `split_lens` int64 [num_seqs]: per token the cache
+ * length of its run's last token.  Where group_tokens tokens have more than eight query heads per KV head, and for the shapes of the
+ * generic kernel, the tokens are taken one by one.  `scratch` as for num_seqs sequences. */
 int echokv_decode_chunks(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
                          const void* query, int64_t q_s0, int64_t q_s1, int32_t q_dtype, const int64_t* q_rows,
                          const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
                          void* scratch, int64_t scratch_bytes,
                          void* out, int64_t o_s0, int64_t o_s1, int32_t out_dtype,
                          float softmax_scale, int32_t num_splits, int32_t blocks_per_split,
-                         const int64_t* groups, int64_t num_groups, int64_t num_seqs, int32_t num_q_heads, void* stream);
+                         const int64_t* groups, int64_t num_groups, int32_t group_tokens, const int64_t* split_lens,
+                         int64_t num_seqs, int32_t num_q_heads, void* stream);
+
+/* The host side of that: the tokens of `chunks` int64 [num_chunks, 4] (first query row, tokens, context with them, block-table row),
+ * num_tokens together, as `rows` int64 [3, num_tokens] (q_rows, bt_rows, lens) and, for every number of tokens in `widths`, as groups:
+ * `split_lens` [num_widths, num_tokens], `num_groups` [num_widths] and the widths' groups one behind the other (room for
+ * num_widths * num_tokens), the longest contexts first: the split kernel takes its work in this order, and what comes last should
+ * be short.  Returns the number of groups, or an error code (< 0).  Host memory throughout. */
+int64_t echokv_chunk_groups(const int64_t* chunks, int64_t num_chunks, int64_t num_tokens, const int64_t* widths,
+                            int32_t num_widths, int64_t* rows, int64_t* split_lens, int64_t* groups, int64_t* num_groups);
 
 /* How many work items (sequence, split) the split kernel works on at the same time on the current device for
  * this layout and number of query heads, or 0 when the shape takes the generic kernel (one CTA per item and KV
