@@ -61,8 +61,7 @@ constexpr unsigned long long WAIT_NS = 2000000000ull;  // a wait gives up after 
 constexpr int F_RES = 1, F_FIRST = 2, F_LAST = 4;  // K from the residual buffer / first / last group of a work item
 constexpr int F_PAIR = 8;                          // the next stage holds a second full tile of the same tier
 constexpr int RT_LOG_SHIFT = 8;                    // plan entries only: bits 8..11 = log2(token rows per run)
-constexpr int REM_SHIFT = 16, MAX_REM = 4095;      // bits 16 and up: tokens of the sequence from the tile's first on
-constexpr int F_MASK = 0xff | MAX_REM << REM_SHIFT;  // the flag bits a stage header carries
+constexpr int F_MASK = 0xff;                       // the flag bits a stage header carries
 struct alignas(16) StageHeader {
   int bits, n_valid, flags, pos0;   // n_valid: 1..16 tokens, -1 = no more work
   long long res_slot;
@@ -695,10 +694,10 @@ __device__ __forceinline__ void enter_tier(WarpState& w, const Lane& ln, float* 
 
 // One group: NT tiles (stage bases sbk[t] for the K side, sbv[t] for the V side; they differ at INT8 only).
 // With NT == 2 both tiles are full and code-based.  With NT == 1 the tile may be partial (`n_valid` < 16) and its
-// K may come from the residual buffer.  `rem`: tokens of the sequence from the first tile's start on.
+// K may come from the residual buffer.
 template <int BITS, int H, int NT, bool MT>
 __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, const uint32_t (&sbk)[NT], const uint32_t (&sbv)[NT],
-                                              int n_valid, int rem, bool in_res, long long res_slot, int pos0, WarpState& w,
+                                              int n_valid, bool in_res, long long res_slot, int pos0, WarpState& w,
                                               float* remap, int* lock, bool& ok) {
   PROF_T(f0);
   enter_tier<BITS>(w, ln, remap, lock, P.wait_ns, ok);
@@ -718,22 +717,13 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
       for (int k = 0; k < 4; ++k) c[t][k] = fmaf(c[t][k], CODE_UNSCALE, c2[2 * (NT == 1 ? 0 : t) + (k & 1)]);
     }
   }
-  if constexpr (MT) {  // near the sequence's end: every column up to its own token
-    if (rem < NT * TILE + COLS) {
-      const int t0 = BITS == 8 ? ln.r : 2 * ln.r, t1 = BITS == 8 ? ln.r + 8 : 2 * ln.r + 1;  // tokens of MMA rows r / r + 8
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const int n0 = rem - ln.d0 - t * TILE, n1 = rem - ln.d1 - t * TILE;
-        if (t0 >= n0) c[t][0] = -INFINITY;
-        if (t0 >= n1) c[t][1] = -INFINITY;
-        if (t1 >= n0) c[t][2] = -INFINITY;
-        if (t1 >= n1) c[t][3] = -INFINITY;
-      }
-    }
-  } else if (NT == 1 && n_valid < TILE) {  // a partial tile (the sequence's last): tokens past the end do not count
+  if (NT == 1 && n_valid < TILE) {  // a partial tile (the sequence's last): tokens past the end of the column's own token do not count
     const int t0 = BITS == 8 ? ln.r : 2 * ln.r, t1 = BITS == 8 ? ln.r + 8 : 2 * ln.r + 1;  // tokens of MMA rows r / r + 8
-    if (t0 >= n_valid) { c[0][0] = -INFINITY; c[0][1] = -INFINITY; }
-    if (t1 >= n_valid) { c[0][2] = -INFINITY; c[0][3] = -INFINITY; }
+    const int n0 = MT ? n_valid - ln.d0 : n_valid, n1 = MT ? n_valid - ln.d1 : n_valid;
+    if (t0 >= n0) c[0][0] = -INFINITY;
+    if (t0 >= n1) c[0][1] = -INFINITY;
+    if (t1 >= n0) c[0][2] = -INFINITY;
+    if (t1 >= n1) c[0][3] = -INFINITY;
   }
   PROF_T(f1);
   PROF_PHASE(0, f0, f1);
@@ -771,7 +761,7 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
     w.m0 = n0; w.m1 = n1;
   }
   uint32_t p_lo[NT], p_hi[NT];
-  // MT: a column may have seen no token yet
+  // MT: a column may see no token of the split
   const float m0 = MT && w.m0 == -INFINITY ? 0.f : w.m0, m1 = MT && w.m1 == -INFINITY ? 0.f : w.m1;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -1176,8 +1166,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
           d.hdr.bits = bits; d.hdr.n_valid = nv;
           const int rt_log = 31 - __clz(rt);                // for the fills: a run's rows by shift and mask
           d.hdr.flags = (in_res ? F_RES : 0) | (u_first && lane == 0 ? F_FIRST : 0) |
-                        (u_last && lane == unit_tiles - 1 ? F_LAST : 0) | (rt_log << RT_LOG_SHIFT) |
-                        ((int)min(u_len - ((int64_t)(u_base + kb) * L.BS + t0), (int64_t)MAX_REM) << REM_SHIFT);
+                        (u_last && lane == unit_tiles - 1 ? F_LAST : 0) | (rt_log << RT_LOG_SHIFT);
           d.hdr.pos0 = t0 - grp * L.KG; d.hdr.res_slot = ks_slot; d.hdr.seq = u_seq; d.hdr.split = u_split;
           d.stats[0] = page + L.o_vs + (int64_t)t0 * H * NG * 2;
           d.stats[1] = page + L.o_vm + (int64_t)t0 * H * NG * 2;
@@ -1389,14 +1378,14 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         const int cur_split = split;
         if constexpr (KIND == K_TILE8) {
           const uint32_t sk[1] = {sb0}, sv[1] = {sb1};
-          process_group<8, H, 1, MT>(P, ln, sk, sv, n_valid, flags >> REM_SHIFT, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
+          process_group<8, H, 1, MT>(P, ln, sk, sv, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
         } else if constexpr (KIND == K_SINGLE) {
           const uint32_t s1[1] = {sb0};
-          if (bits == 4) process_group<4, H, 1, MT>(P, ln, s1, s1, n_valid, flags >> REM_SHIFT, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
-          else process_group<2, H, 1, MT>(P, ln, s1, s1, n_valid, flags >> REM_SHIFT, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
+          if (bits == 4) process_group<4, H, 1, MT>(P, ln, s1, s1, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
+          else process_group<2, H, 1, MT>(P, ln, s1, s1, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
         } else {
           const uint32_t s2[2] = {sb0, sb1};
-          process_group<BITS, H, 2, MT>(P, ln, s2, s2, TILE, flags >> REM_SHIFT, false, 0, 0, w, remap, lock, ok);
+          process_group<BITS, H, 2, MT>(P, ln, s2, s2, TILE, false, 0, 0, w, remap, lock, ok);
         }
         __syncwarp();
         mbar_arrive(empty_u + c_st * 8);  // every lane arrives (the barrier counts threads): no branch, no warp sync needed

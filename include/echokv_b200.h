@@ -246,7 +246,7 @@ int echokv_decode_step(const echokv_layout* layout, const echokv_pages* pages, c
 /* echokv_decode_ex (without a run-time split size) for sequences that are the query tokens of chunks: consecutive tokens of a chunk
  * see the same cache, one token more each, and are worked off together where the shape allows it.  q_rows / bt_rows / lens list the
  * num_seqs tokens one by one.  `groups` int64 [num_groups, 5] lists the same tokens in runs of 1 .. group_tokens consecutive ones of
- * a chunk, on consecutive query rows: the query row of a run's first token, its block-table row, the cache length of its last
+ * a chunk, on consecutive query rows, whose caches end in the same tile (lens / 16 rounded down is the same): the query row of a run's first token, its block-table row, the cache length of its last
  * token, its tokens, and the place of its first token in the list of tokens.  `split_lens` int64 [num_seqs]: per token the cache
  * length of its run's last token.  Where group_tokens tokens have more than eight query heads per KV head, and for the shapes of the
  * generic kernel, the tokens are taken one by one.  `scratch` as for num_seqs sequences. */

@@ -36,8 +36,45 @@ def test_groups_list_every_token_once(seed, monkeypatch):
             assert first == at and 1 <= tokens <= width and len(set(chunk_of[at: at + tokens])) == 1
             assert want[at: at + tokens] == [(row + i, req, length - tokens + 1 + i) for i in range(tokens)]
             assert split_lens[at: at + tokens].tolist() == [length] * tokens
+            for ln in range(length - tokens + 2, length + 1):  # nothing about the kernels' tiles and splits changes inside a group
+                assert ln // 16 == (ln - 1) // 16 and (ln - 1) % 512
             at += tokens
         assert at == len(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,gqa,bits", [(2, 1, 4), (2, 2, 2), (2, 3, 8), (2, 4, 4), (1, 4, 4), (2, 4, 0), (8, 1, 0)])
+def test_bits_of_each_token_alone(h, gqa, bits):
+    """Contexts that pass the end of a tile, of a pair of tiles, of a split (256 tokens) and of 512 blocks, from where the split size
+    follows the context; loud queries, so that the reference moves; ``bits`` 0: blocks of all tiers.  However the chunk is cut,
+    a token has the bits of the token alone."""
+    import torch
+    from echokv_b200.kernels.decode import decode_attention
+    from echokv_b200.kernels.prefill import prefill_attention
+    from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
+
+    tokens, d = 8240, 128
+    layout = TieredLayout(num_kv_heads=h, head_size=d, block_size=16, mem_bits=8, k_group=16, v_group=32)
+    store = TieredKVCache(layout, torch.zeros(tokens // 16, layout.page_bytes, dtype=torch.uint8, device="cuda"), residual_slots=4,
+                          residual_dtype=torch.float16)
+    gen = torch.Generator(device="cuda").manual_seed(gqa)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
+    for at in range(0, tokens, 16 if bits == 0 else tokens):
+        n = 16 if bits == 0 else tokens
+        store.write(rand(n, h, d), rand(n, h, d), torch.arange(at, at + n), bits or (8, 4, 4, 2, 4, 8, 2, 2)[at // 16 % 8])
+    table = torch.arange(tokens // 16, device="cuda", dtype=torch.int32).expand(6, -1).contiguous()
+    chunks = [(40, 1050), (64, 8230), (7, 8195), (37, 290), (5, 5), (20, 4110)]
+    ends = np.cumsum([n for n, _ in chunks]).tolist()
+    q = rand(ends[-1], h * gqa, d) * 4
+    lens = torch.cat([torch.arange(ctx - n + 1, ctx + 1) for n, ctx in chunks]).cuda()
+    reqs = torch.arange(6, device="cuda").repeat_interleave(torch.tensor([n for n, _ in chunks], device="cuda"))
+    want = decode_attention(store, q, table, lens, d ** -0.5, bt_rows=reqs, max_len=8230)
+    for cut in (64, 3):
+        pieces = [(i, e - n + a, min(e - n + a + cut, e), ctx - n + min(a + cut, n)) for i, (e, (n, ctx)) in enumerate(zip(ends, chunks))
+                  for a in range(0, n, cut)]
+        out = torch.full(q.shape, 7.0, device="cuda")
+        prefill_attention(store, q, out, [(a, b, ctx, 0) for _, a, b, ctx in pieces], [i for i, *_ in pieces], table, d ** -0.5)
+        assert torch.equal(out, want)
 
 
 def test_counts_that_do_not_fit_are_refused():
