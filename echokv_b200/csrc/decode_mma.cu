@@ -374,7 +374,6 @@ struct Lane {
   uint32_t km_ld;     // stage offset of this lane's ldmatrix row of the broadcast k_min operand (tile by lane & 8)
   uint32_t vs_row8;   // INT8 stages (eight tokens in natural order): V scales of token r of the stage
   uint32_t vm_ld8;    // INT8 stages: this lane's ldmatrix row of the [v_min | ones] operand (stage by lane & 16)
-  int tk0, tk1;       // MT: token of its sequence that column 2j / 2j + 1 belongs to
   int d0, d1;         // MT: how many tokens fewer it sees than the sequence's last token (-1: no such token)
   int first;          // MT: row of partials of the sequence's first token
 };
@@ -749,7 +748,8 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
       auto spread = [](uint32_t x) { return (x & 1) | (x & 2) << 1 | (x & 4) << 2 | (x & 8) << 3; };
       const uint32_t b0 = __ballot_sync(0xffffffffu, g0), b1 = __ballot_sync(0xffffffffu, g1);
       const uint32_t cols = spread(b0) | spread(b1) << 1, heads = (1u << P.A.gqa) - 1;  // lanes 0 .. 3 speak for the columns
-      const bool s0 = cols >> (ln.tk0 * P.A.gqa) & heads, s1 = cols >> (ln.tk1 * P.A.gqa) & heads;
+      const int c0 = 2 * ln.j, c1 = c0 + 1;  // the token's first column
+      const bool s0 = cols >> (c0 - c0 % P.A.gqa) & heads, s1 = cols >> (c1 - c1 % P.A.gqa) & heads;
       a0 = s0 ? ex2(w.m0 - n0) : 1.f; a1 = s1 ? ex2(w.m1 - n1) : 1.f;
       n0 = s0 ? n0 : w.m0; n1 = s1 ? n1 : w.m1;
     } else {
@@ -761,12 +761,10 @@ __device__ __forceinline__ void process_group(const Params& P, const Lane& ln, c
     w.m0 = n0; w.m1 = n1;
   }
   uint32_t p_lo[NT], p_hi[NT];
-  // MT: a column may see no token of the split
-  const float m0 = MT && w.m0 == -INFINITY ? 0.f : w.m0, m1 = MT && w.m1 == -INFINITY ? 0.f : w.m1;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    p_lo[t] = pack_h2(ex2(c[t][0] - m0), ex2(c[t][1] - m1));   // token 2r
-    p_hi[t] = pack_h2(ex2(c[t][2] - m0), ex2(c[t][3] - m1));   // token 2r + 1
+    p_lo[t] = pack_h2(ex2(c[t][0] - w.m0), ex2(c[t][1] - w.m1));   // token 2r
+    p_hi[t] = pack_h2(ex2(c[t][2] - w.m0), ex2(c[t][3] - w.m1));   // token 2r + 1
   }
   PROF_T(f2);
   PROF_PHASE(1, f1, f2);
@@ -809,19 +807,20 @@ __device__ __forceinline__ BlockMeta load_meta(const Params& P, int64_t bt_row, 
 // running maximum and denominator to ml.  A lane's accumulator rows are neighbouring channels (INT4: 4 per V group,
 // INT2: 8 per half of the head, INT8: 2 per 16-channel tile), so they leave as 16- or 8-byte stores that the
 // eight lanes of a query head put side by side.
+// MT: of the tokens that see `lo` to `hi` - 1 tokens fewer than the sequence's last one.
 template <int BITS, int H, bool MT>
-__device__ __forceinline__ void write_partial(const Params& P, const Lane& ln, const WarpState& w, int seq, int split) {
+__device__ __forceinline__ void write_partial(const Params& P, const Lane& ln, const WarpState& w, int seq, int split, int lo, int hi) {
   const int h = ln.h, lane = ln.lane;
   const int r = lane >> 2, j = lane & 3;
   const DecodeArgs& A = P.A;
   const int g0 = 2 * j, g1 = 2 * j + 1;
   // MT: columns are (token, query head of the group) pairs
-  const int64_t r0 = MT ? (int64_t)(ln.first + ln.tk0) * A.Hq + g0 - ln.tk0 * A.gqa : (int64_t)seq * A.Hq + g0;
-  const int64_t r1 = MT ? (int64_t)(ln.first + ln.tk1) * A.Hq + g1 - ln.tk1 * A.gqa : (int64_t)seq * A.Hq + g1;
+  const int64_t r0 = MT ? (int64_t)(ln.first + g0 / A.gqa) * A.Hq + g0 % A.gqa : (int64_t)seq * A.Hq + g0;
+  const int64_t r1 = MT ? (int64_t)(ln.first + g1 / A.gqa) * A.Hq + g1 % A.gqa : (int64_t)seq * A.Hq + g1;
   const int64_t o0 = (r0 + h * A.gqa) * A.num_splits + split, o1 = (r1 + h * A.gqa) * A.num_splits + split;
   float* dst0 = A.acc + o0 * D;
   float* dst1 = A.acc + o1 * D;
-  const bool on0 = MT ? ln.d0 >= 0 : g0 < A.gqa, on1 = MT ? ln.d1 >= 0 : g1 < A.gqa;
+  const bool on0 = MT ? ln.d0 >= lo && ln.d0 < hi : g0 < A.gqa, on1 = MT ? ln.d1 >= lo && ln.d1 < hi : g1 < A.gqa;
   // V min contribution of V group G: held by lane (r = bias_row(G), j)
   float bias0[NG], bias1[NG];
 #pragma unroll
@@ -1240,7 +1239,6 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     Lane ln;
     ln.h = warp; ln.lane = lane; ln.r = lane >> 2; ln.j = lane & 3;
     unsigned char* qn = qs + ln.h * cols * QN_ROW;
-    if constexpr (MT) { ln.tk0 = 2 * ln.j / A.gqa; ln.tk1 = (2 * ln.j + 1) / A.gqa; }
     {  // query columns >= gqa of the MMAs read the team's zero row (every warp writes the same zeros)
       unsigned char* zero = qs + H * cols * QN_ROW;
       ln.qn_lane = smem_u32(ln.r < cols ? qn + ln.r * QN_ROW : zero);
@@ -1290,8 +1288,8 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
       if constexpr (MT) {
         const int last = seq_tokens<MT>(A, seq) - 1;
         ln.first = (int)A.groups[(int64_t)seq * GROUP_WORDS + GROUP_FIRST];
-        ln.d0 = ln.tk0 < A.tok && ln.tk0 <= last ? last - ln.tk0 : -1;
-        ln.d1 = ln.tk1 < A.tok && ln.tk1 <= last ? last - ln.tk1 : -1;
+        ln.d0 = max(last - 2 * ln.j / A.gqa, -1);
+        ln.d1 = max(last - (2 * ln.j + 1) / A.gqa, -1);
       }
       auto q_at = [&](int n) {  // element offset of column n's query row
         const int tk = MT ? n / A.gqa : 0;
@@ -1375,7 +1373,20 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         PROF_T(r1);
         PROF_PHASE(4, r0, r1);  // item start + wait for the second stage
         const bool last = (flags & F_LAST) != 0;
-        const int cur_split = split;
+        const int cur_split = split, cur_valid = n_valid;
+        if constexpr (MT && (KIND == K_TILE8 || KIND == K_SINGLE)) {
+          // The first token's cache may end right in front of this tile.  Its result leaves before the tile is worked off: a
+          // probability of 0 times an infinite scale, or times whatever lies behind the sequence's end, would be NaN.
+          if (last && __any_sync(0xffffffffu, ln.d0 == n_valid || ln.d1 == n_valid)) {
+            auto first_token = [&](auto bc) {
+              enter_tier<decltype(bc)::value>(w, ln, remap, lock, P.wait_ns, ok);
+              write_partial<decltype(bc)::value, H, MT>(P, ln, w, seq, split, n_valid, n_valid + 1);
+            };
+            if constexpr (KIND == K_TILE8) first_token(std::integral_constant<int, 8>{});
+            else if (bits == 4) first_token(std::integral_constant<int, 4>{});
+            else first_token(std::integral_constant<int, 2>{});
+          }
+        }
         if constexpr (KIND == K_TILE8) {
           const uint32_t sk[1] = {sb0}, sv[1] = {sb1};
           process_group<8, H, 1, MT>(P, ln, sk, sv, n_valid, (flags & F_RES) != 0, res_slot, pos0, w, remap, lock, ok);
@@ -1398,10 +1409,10 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
         }
         if (last) {
           if constexpr (KIND == K_SINGLE) {
-            if (w.bits == 4) write_partial<4, H, MT>(P, ln, w, seq, cur_split);
-            else write_partial<2, H, MT>(P, ln, w, seq, cur_split);
+            if (w.bits == 4) write_partial<4, H, MT>(P, ln, w, seq, cur_split, 0, cur_valid);
+            else write_partial<2, H, MT>(P, ln, w, seq, cur_split, 0, cur_valid);
           } else {
-            write_partial<BITS, H, MT>(P, ln, w, seq, cur_split);
+            write_partial<BITS, H, MT>(P, ln, w, seq, cur_split, 0, cur_valid);
           }
         }
         PROF_T(r2);

@@ -77,6 +77,37 @@ def test_bits_of_each_token_alone(h, gqa, bits):
         assert torch.equal(out, want)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("at", [160, 256])
+@pytest.mark.parametrize("h,gqa,bits", [(2, 1, 4), (2, 2, 8), (2, 4, 2), (1, 3, 4), (2, 4, 0)])
+def test_infinite_values_of_later_tokens(h, gqa, bits, at):
+    """A token with an infinite value, in a tile that begins where the cache of some tokens of the chunk ends (160: inside a split,
+    256: at a split's begin): those tokens do not see it.  ``bits`` 0: a tile of another tier than the ones before."""
+    import torch
+    from echokv_b200.kernels.decode import decode_attention
+    from echokv_b200.kernels.prefill import prefill_attention
+    from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
+
+    d = 128
+    layout = TieredLayout(num_kv_heads=h, head_size=d, block_size=16, mem_bits=8, k_group=16, v_group=32)
+    store = TieredKVCache(layout, torch.zeros(20, layout.page_bytes, dtype=torch.uint8, device="cuda"), residual_slots=4,
+                          residual_dtype=torch.float16)
+    gen = torch.Generator(device="cuda").manual_seed(gqa)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).half()
+    k, v = rand(320, h, d), rand(320, h, d)
+    v[at + 5] = torch.inf
+    for a, b in ((0, at), (at, 320)):
+        store.write(k[a:b], v[a:b], torch.arange(a, b), bits or (4 if a else 8))
+    table = torch.arange(20, device="cuda", dtype=torch.int32)[None]
+    n, ctx = 18, at + 9  # lengths at - 8 .. at + 9
+    q, out = rand(n, h * gqa, d), torch.full((n, h * gqa, d), 7.0, device="cuda")
+    prefill_attention(store, q, out, [(0, n, ctx, 0)], [0], table, d ** -0.5)
+    lens = torch.arange(ctx - n + 1, ctx + 1, device="cuda")
+    want = decode_attention(store, q, table, lens, d ** -0.5, bt_rows=torch.zeros_like(lens), max_len=ctx)
+    seen = lens <= at
+    assert torch.isfinite(want[seen]).all() and torch.equal(out[seen], want[seen]) and not torch.isfinite(want[~seen]).any()
+
+
 def test_counts_that_do_not_fit_are_refused():
     from echokv_b200 import _native as N
 
