@@ -872,7 +872,7 @@ __device__ __forceinline__ int ring_next(int st, int NS) { return st + 1 == NS ?
 // plans, query copy and stage ring in its slice of the CTA's shared memory.  One CTA per SM.  Registers are handed
 // out per SM sub-partition (16,384 each): with 17 to 20 warps per SM (5 on a sub-partition) a thread gets 96, so
 // V is chosen to use those 18 to 20 warps for every H.  The smaller V of each H is for shapes whose per-team shared
-// memory (many query heads per KV head) does not fit V times.
+// memory (many query heads per KV head) does not fit V times, and for one KV head where it is the faster (team_shape).
 template <int H> struct Teams {
   static constexpr int V = H == 8 ? 2 : (H == 4 ? 4 : (H == 2 ? 6 : 10));   // 18 / 20 / 18 / 20 warps
   static constexpr int V_SMALL = H == 8 ? 1 : (H == 4 ? 3 : (H == 2 ? 4 : 8));
@@ -1239,7 +1239,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
     Lane ln;
     ln.h = warp; ln.lane = lane; ln.r = lane >> 2; ln.j = lane & 3;
     unsigned char* qn = qs + ln.h * cols * QN_ROW;
-    {  // query columns >= gqa of the MMAs read the team's zero row (every warp writes the same zeros)
+    {  // columns of the MMAs that are not in use read the team's zero row (every warp writes the same zeros)
       unsigned char* zero = qs + H * cols * QN_ROW;
       ln.qn_lane = smem_u32(ln.r < cols ? qn + ln.r * QN_ROW : zero);
       ln.qn_ld = smem_u32(((lane & 7) < cols ? qn + (lane & 7) * QN_ROW : zero) + (lane >> 3) * 16);
@@ -1281,7 +1281,7 @@ __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const P
       return true;
     };
     // This head's queries of sequence `seq` -> fp16 in shared memory, pre-multiplied by softmax_scale * log2(e)
-    // (rows >= gqa are zero).  All global loads are issued before the first use so the item pays one memory latency.
+    // (rows of a group's missing tokens are zero).  All global loads are issued before the first use so the item pays one memory latency.
     auto load_queries = [&]() {
       const int64_t q_row = seq_query<MT>(A, seq);
       const int n_rows = MT ? seq_tokens<MT>(A, seq) * A.gqa : A.gqa;  // columns that have a token
@@ -1514,22 +1514,28 @@ static int decode_device(DecodeDevice** out) {
   return ECHOKV_OK;
 }
 
-// Teams per CTA and ring stages per team for H KV heads with gqa query heads each: every team gets an equal slice
+// Teams per CTA and ring stages per team for H KV heads and `cols` columns of the MMAs in use (the query heads per KV head, or those of
+// a group's tokens), pages of `chunks` x 2 bits: the larger count, or the smaller one by the rule below.  Every team gets an equal slice
 // of the SM's shared memory; false when not even the smaller team count leaves room for four stages (a group of
 // two stages in work and one in flight at the least).
 struct TeamShape { int V, ns, fixed; bool small; };
-static bool team_shape(const DecodeDevice& dv, int H, int gqa, int chunks, TeamShape* out) {  // chunks: of a page
+static bool team_shape(const DecodeDevice& dv, int H, int cols, int chunks, TeamShape* out) {
   using namespace mma;
-  const int fixed = HDR_BYTES + UNIT * (int)sizeof(TilePlan) + (q_copy_bytes(H, gqa) + 127) / 128 * 128;
+  const int fixed = HDR_BYTES + UNIT * (int)sizeof(TilePlan) + (q_copy_bytes(H, cols) + 127) / 128 * 128;
   const int sbytes = stage_bytes(H);
   const int room = dv.max_smem - CTA_SHARED_BYTES;
   int V = H == 8 ? Teams<8>::V : H == 4 ? Teams<4>::V : H == 2 ? Teams<2>::V : Teams<1>::V;
   bool small = false;
   int ns = ((room / V) / 128 * 128 - fixed) / sbytes;
-  // One KV head, more than four query heads, pages of at most 4 bits: 16 warps of 128 registers beat 20 of 96 (16 x 28,000 tokens 51.3 ->
-  // 48.7 us, 1 x 30,000 30.9 -> 29.3).  With pages of 6 or 8 bits it depends on the step (6 bits: 48 x 3,000 30.4 -> 28.4 us, 100 x
-  // 3,000 40.4 -> 44.8), and at four KV heads the larger count is better (4 bits, block 64, 64 x 4,000: 61.7 against 52.6).
-  const bool few = gqa > 4 && H == 1 && chunks <= 2;
+  // One KV head, more than four columns, pages of at most 4 bits: 16 warps of 128 registers beat 20 of 96.  Splits sized for the count
+  // (choose_blocks_per_split), 1 to 256 sequences of 900 to 30,000 tokens, blocks of 4 and 2 bits: 4 to 21 % faster throughout (1 x
+  // 30,000 31.1 -> 29.2 us, 16 x 28,000 51.9 -> 48.4, 100 x 3,000 33.3 -> 32.0).  Blocks of 8 bits, which larger pages are for, lose
+  // where the work fills all teams (100 x 3,000 41.6 -> 45.4 us in 6-bit pages, 41.0 -> 45.4 in 8-bit ones, 16 x 28,000 79.5 -> 73.4 and
+  // 69.5 -> 68.6).  Groups of a chunk's tokens, 4-bit pages: 16 x 33 behind 1,472 23.1 -> 20.8 us with one query head, 50.7 -> 46.3
+  // with four; of 48 such pairs (4- and 2-bit blocks, 1 to 128 chunks) five lose, 64 x 8 behind 2,000 with three heads 56.6 -> 61.0 the most.
+  // One to four query heads of single tokens would gain 3 to 11 % as well and keep the larger count, which their splits have been
+  // sized for.  At four KV heads the larger count is better (4 bits, block 64, 64 x 4,000: 61.7 against 52.6).
+  const bool few = cols > 4 && H == 1 && chunks <= 2;
   if (ns < 4 || few) {
     small = true;
     V = H == 8 ? Teams<8>::V_SMALL : H == 4 ? Teams<4>::V_SMALL : H == 2 ? Teams<2>::V_SMALL : Teams<1>::V_SMALL;
