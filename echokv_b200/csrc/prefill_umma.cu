@@ -929,16 +929,18 @@ __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args 
         }
         tmem_st16_raw(t_row + W_SCOL + 16 * c, w);
         if ((c + 1) % (WN / 32 / P_PARTS) == 0) {  // a part of P is complete
+          PF_T(p0);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;");
           bar_arrive(&bar_p[grp][c / (WN / 32 / P_PARTS)]);
+          PF_T(p1);
+          PF_ADD(5, p0, p1); PF_ADD(4, p1, p0);  // of phase 4's span
         }
       }
       const float2 s01 = __fadd2_rn(sum2[0], sum2[1]), s23 = __fadd2_rn(sum2[2], sum2[3]);
       l_run += (s01.x + s01.y) + (s23.x + s23.y);
       PF_T(c5);
-      PF_T(c6);
-      PF_ADD(0, c0, c1); PF_ADD(1, c1, c2); PF_ADD(2, c2, c3); PF_ADD(3, c3, c4); PF_ADD(4, c4, c5); PF_ADD(5, c5, c6);
+      PF_ADD(0, c0, c1); PF_ADD(1, c1, c2); PF_ADD(2, c2, c3); PF_ADD(3, c3, c4); PF_ADD(4, c4, c5);
 #ifdef ECHOKV_PROFILE
       pf[7] += 1;
 #endif
