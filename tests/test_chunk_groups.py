@@ -77,6 +77,60 @@ def test_bits_of_each_token_alone(h, gqa, bits):
         assert torch.equal(out, want)
 
 
+def _mixed_store(h, tokens, dtype="float16"):
+    """One context whose blocks of 16 tokens are of all tiers, and its block table (one row)."""
+    import torch
+    from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
+
+    layout = TieredLayout(num_kv_heads=h, head_size=128, block_size=16, mem_bits=8, k_group=16, v_group=32)
+    store = TieredKVCache(layout, torch.zeros(tokens // 16, layout.page_bytes, dtype=torch.uint8, device="cuda"), residual_slots=4,
+                          residual_dtype=getattr(torch, dtype))
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    kv = torch.randn(2, tokens, h, 128, device="cuda", generator=gen).to(getattr(torch, dtype))
+    for at in range(0, tokens, 16):
+        store.write(kv[0, at: at + 16], kv[1, at: at + 16], torch.arange(at, at + 16), (8, 4, 4, 2, 4, 8, 2, 2)[at // 16 % 8])
+    return store, torch.arange(tokens // 16, device="cuda", dtype=torch.int32)[None]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,gqa", [(8, 1), (2, 4), (1, 3)])
+def test_long_contexts_of_all_tiers(h, gqa):
+    """Behind more than 4,096 tokens and more than 512 blocks, against 64-bit attention over the stored values (fp16 operands: 2^-11
+    per product, 2e-3 of the norm)."""
+    import torch
+    from echokv_b200.kernels.prefill import prefill_attention
+
+    store, table = _mixed_store(h, 8208)
+    k, v = (x.transpose(0, 1).repeat_interleave(gqa, 0).double() for x in store.gather(torch.arange(8208) // 16, torch.arange(8208) % 16))
+    chunks = [(20, 8205), (9, 4101), (33, 4130)]
+    q = torch.randn(62, h * gqa, 128, device="cuda", generator=torch.Generator(device="cuda").manual_seed(h)).half()
+    out = torch.full(q.shape, 7.0, device="cuda")
+    prefill = [(0, 20, 8205, 0), (20, 29, 4101, 0), (29, 62, 4130, 0)]
+    prefill_attention(store, q, out, prefill, [0, 1, 2], table.expand(3, -1).contiguous(), 128 ** -0.5)
+    for (n, ctx), (qs, qe, _, _) in zip(chunks, prefill):
+        hidden = torch.arange(8208, device="cuda")[None] >= torch.arange(ctx - n + 1, ctx + 1, device="cuda")[:, None]
+        s = (q[qs:qe].transpose(0, 1).double() @ k.transpose(1, 2) * 128 ** -0.5).masked_fill(hidden, -torch.inf)
+        want = (torch.softmax(s, -1) @ v).transpose(0, 1)
+        assert (out[qs:qe].double() - want).norm() <= 2e-3 * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gqa,shared", [(1, True), (2, True), (3, True), (4, True), (5, False), (8, False)])
+def test_which_shapes_share_a_pass(gqa, shared):
+    """With the lengths of the tokens one by one all wrong, the result follows the groups exactly where tokens are taken together."""
+    import torch
+    from echokv_b200.kernels.decode import decode_attention
+    from echokv_b200.kernels.prefill import build_rows
+
+    store, table = _mixed_store(2, 320)
+    q = torch.randn(20, 2 * gqa, 128, device="cuda", generator=torch.Generator(device="cuda").manual_seed(gqa)).half()
+    plan = build_rows([(0, 20, 310, 0)], [0], "cuda")
+    rows, reqs, lens, longest = plan
+    attend = lambda lens, groups: decode_attention(store, q, table, lens, 128 ** -0.5, q_rows=rows, bt_rows=reqs, max_len=longest, groups=groups)
+    wrong = torch.full_like(lens, 100)
+    assert torch.equal(attend(wrong, plan.groups), attend(lens if shared else wrong, None))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("at", [160, 256])
 @pytest.mark.parametrize("h,gqa,bits", [(2, 1, 4), (2, 2, 8), (2, 4, 2), (1, 3, 4), (2, 4, 0)])

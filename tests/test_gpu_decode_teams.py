@@ -9,6 +9,20 @@ pytestmark = pytest.mark.gpu
 D, TOKENS = 128, 700
 
 
+@pytest.mark.parametrize("h,gqa,mem,teams", [(1, 5, 4, 8), (1, 8, 2, 8), (1, 4, 4, 10), (1, 8, 6, 10), (1, 8, 8, 10), (2, 8, 4, 6), (4, 8, 4, 4),
+                                             (8, 4, 8, 2)])
+def test_team_counts(h, gqa, mem, teams):
+    """Which shapes run how many teams an SM."""
+    import torch
+    from echokv_b200.kernels.decode import decode_parallelism
+    from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
+
+    layout = TieredLayout(num_kv_heads=h, head_size=D, block_size=16, mem_bits=mem, k_group=16, v_group=32)
+    store = TieredKVCache(layout, torch.zeros(2, layout.page_bytes, dtype=torch.uint8, device="cuda"), residual_slots=4,
+                          residual_dtype=torch.float16)
+    assert decode_parallelism(store, h * gqa) == teams * torch.cuda.get_device_properties("cuda").multi_processor_count
+
+
 @pytest.mark.parametrize("bits", [8, 4, 2])
 @pytest.mark.parametrize("h,gqa", [(1, 5), (1, 8), (4, 7), (4, 8)])
 def test_fewer_teams(h, gqa, bits):
