@@ -1531,7 +1531,7 @@ static bool team_shape(const DecodeDevice& dv, int H, int cols, int chunks, Team
   // (choose_blocks_per_split), 1 to 256 sequences of 900 to 30,000 tokens, blocks of 4 and 2 bits: 4 to 21 % faster throughout (1 x
   // 30,000 31.1 -> 29.2 us, 16 x 28,000 51.9 -> 48.4, 100 x 3,000 33.3 -> 32.0).  Blocks of 8 bits, which larger pages are for, lose
   // where the work fills all teams (100 x 3,000 41.6 -> 45.4 us in 6-bit pages, 41.0 -> 45.4 in 8-bit ones, 16 x 28,000 79.5 -> 73.4 and
-  // 69.5 -> 68.6).  Groups of a chunk's tokens, 4-bit pages: 16 x 33 behind 1,472 23.1 -> 20.8 us with one query head, 50.7 -> 46.3
+  // 69.5 -> 68.6); a third of them among 2-bit blocks in 4-bit pages, 44.8 -> 46.1 and 73.2 -> 68.6.  Groups of a chunk's tokens, 4-bit pages: 16 x 33 behind 1,472 23.1 -> 20.8 us with one query head, 50.7 -> 46.3
   // with four; of 48 such pairs (4- and 2-bit blocks, 1 to 128 chunks) five lose, 64 x 8 behind 2,000 with three heads 56.6 -> 61.0 the most.
   // One to four query heads of single tokens would gain 3 to 11 % as well and keep the larger count, which their splits have been
   // sized for.  At four KV heads the larger count is better (4 bits, block 64, 64 x 4,000: 61.7 against 52.6).

@@ -674,8 +674,8 @@ constexpr int WKV_BYTES = WN * UD * 2;     // one K or V tile: two panels of 128
 constexpr int W_STAGES = 2;
 // P of a tile is handed to the issuer in this many parts, so that the first part's O += P V runs under the rest's
 // exponentials: a group's chain (scores, softmax, O += P V) is what bounds the kernel, neither pipe is full (tensor and XU pipes
-// 45 % active each).  Two parts: 8 x 512 tokens behind 8,192, the 8-layer step 6.10 -> 5.84 ms; 12 prompts 2.32 -> 2.24 ms; four parts
-// gain nothing.  A quarter or a third of the exponentials on the FMA pipe (a polynomial) gave nothing on top.
+// 49 % of active cycles each with P in one part, 57 % in two).  Two parts: 8 x 512 tokens behind 8,192, the 8-layer step 6.10 ->
+// 5.84 ms; 12 prompts 2.32 -> 2.24 ms, which is what their runs spread by; four parts gain nothing.  A quarter or a third of the exponentials on the FMA pipe (a polynomial) gave nothing on top.
 constexpr int P_PARTS = 2;
 constexpr int W_SCOL = 0, W_OCOL = 128, W_GCOLS = 256;
 constexpr int smem_wide() { return 2 * Q_BYTES + 2 * W_STAGES * WKV_BYTES + 1024; }
@@ -698,7 +698,7 @@ __device__ __forceinline__ void tmem_ld16_raw(uint32_t taddr, uint32_t (&r)[16])
 // Chunks of uneven length: the row tiles of all chunks form one list, longest first, so that the launch has next to no
 // empty CTAs and what is left at its end is short; a grid of (longest chunk's tiles) x chunks launched three empty CTAs
 // of 193 KB for each working one, in no order.  12 prompts of 87 - 2,900 tokens, 32 / 8 heads: 309 -> 222 us; 8 x 512 tokens
-// behind 8,192: 636 -> 585 us (0.59 of the measured bf16 peak); 512 behind 1,600: 36.6 -> 29.5 us.
+// behind 8,192: 636 -> 585 us, 538 (0.66 of the measured bf16 peak) with P in two parts; 512 behind 1,600: 36.6 -> 29.5 us.
 __global__ void __launch_bounds__(2 * UM + 64, 1) prefill_umma_wide_kernel(Args A, const __grid_constant__ Maps M) {
   extern __shared__ unsigned char dyn[];
   __shared__ __align__(8) uint64_t bar_s[2], bar_p[2][P_PARTS], bar_o[2], bar_k[W_STAGES], bar_v[W_STAGES], bar_kfree[W_STAGES],
