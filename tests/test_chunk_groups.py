@@ -132,6 +132,24 @@ def test_which_shapes_share_a_pass(gqa, shared):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("gqa", [1, 2, 4])
+def test_tokens_that_see_nothing(gqa):
+    """A chunk longer than its context: the row of the token with a causal limit of 0 stays as it is, those behind it have the bits of
+    the token alone."""
+    import torch
+    from echokv_b200.kernels.decode import decode_attention
+    from echokv_b200.kernels.prefill import prefill_attention
+
+    store, table = _mixed_store(2, 320)
+    q = torch.randn(40, 2 * gqa, 128, device="cuda", generator=torch.Generator(device="cuda").manual_seed(gqa)).half()
+    out = torch.full(q.shape, 7.0, device="cuda")
+    prefill_attention(store, q, out, [(0, 40, 12, 0)], [0], table, 128 ** -0.5)
+    lens = torch.arange(1, 13, device="cuda")
+    want = decode_attention(store, q[28:], table, lens, 128 ** -0.5, bt_rows=torch.zeros_like(lens), max_len=12)
+    assert (out[27] == 7.0).all() and torch.equal(out[28:], want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("at", [160, 256])
 @pytest.mark.parametrize("h,gqa,bits", [(2, 1, 4), (2, 2, 8), (2, 4, 2), (1, 3, 4), (2, 4, 0)])
 def test_infinite_values_of_later_tokens(h, gqa, bits, at):
