@@ -171,7 +171,7 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
 
   bool handled = false;
   // Groups of consecutive tokens, where the query heads of two or more tokens fit the columns of the tensor-core kernel's MMAs (a step
-  // of 16 chunks of 33 tokens, 32 / 8 heads: 1.72 -> 1.14 ms).  Their partials are those of the tokens one by one, so the merge is too.
+  // of 16 chunks of 33 tokens, 32 / 8 heads: 1.72 -> 1.10 ms).  Their partials are those of the tokens one by one, so the merge is too.
   if (num_groups > 0 && group_tokens > 1) {
     DecodeArgs G = A;
     G.groups = groups; G.tok = group_tokens;

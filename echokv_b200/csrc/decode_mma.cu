@@ -880,7 +880,7 @@ template <int H> struct Teams {
 
 // MT: the MMAs' columns are the query heads of several consecutive tokens of a chunk (DecodeArgs::groups): the codes are unpacked, the
 // scales folded and the pages read once for all of them.  With a sequence per token, 528 tokens of 16 chunks over 1,440 stored
-// ones (32 / 8 heads, two tokens a pass) took 273 us a layer with the merge, now 158.
+// ones (32 / 8 heads, two tokens a pass) took 273 us a layer with the merge, now 151.
 template <int H, int V, bool MT>
 __global__ void __launch_bounds__((H + 1) * 32 * V, 1) decode_mma_kernel(const Params P) {
   extern __shared__ __align__(128) unsigned char smem_all[];

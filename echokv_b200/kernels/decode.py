@@ -146,12 +146,14 @@ def decode_attention(store, query: torch.Tensor, block_table: torch.Tensor, seq_
         N.require_cuda(bps_dev)
         if bps_dev.dtype not in (torch.int32, torch.int64) or bps_dev.numel() < 1:
             raise TypeError("bps_dev must hold one int32 / int64 on the device")
-    width = MMA_COLUMNS * L.num_kv_heads // hq if groups is not None else 0
+    if groups is not None and (bps_dev is not None or not isinstance(groups, dict)):
+        raise ValueError("groups must be those of build_rows, without bps_dev")
+    width = 0 if groups is None else MMA_COLUMNS * L.num_kv_heads // hq
     if groups is not None and width in groups:  # two or more tokens fit
-        if bps_dev is not None:
-            raise ValueError("groups exclude bps_dev")
         runs, split_lens = groups[width]
         N.require_cuda(runs, split_lens)
+        if split_lens.shape[0] != s:
+            raise ValueError("groups must list the sequences' tokens")
         N.check(N.lib.echokv_decode_chunks(
             store.c_layout, store.c_pages, store.c_res,
             query.data_ptr(), q_s[0], q_s[1], N.dtype_code(query.dtype), N.ptr(q_rows),

@@ -189,6 +189,34 @@ def test_counts_that_do_not_fit_are_refused():
         assert N.lib.echokv_chunk_groups(chunks.ctypes.data, count, tokens, np.array([2]).ctypes.data, 1, *args) < 0 and not room.any()
 
 
+@pytest.mark.parametrize("form,gqa", [("run-time split size", 4), ("run-time split size", 8), ("a tensor", 4), ("a tensor", 8),
+                                      ("another step's groups", 4)])
+def test_groups_that_do_not_fit_are_refused(form, gqa, monkeypatch):
+    """Whether or not the shape takes tokens together."""
+    import torch
+    from types import SimpleNamespace
+
+    from echokv_b200 import _native as N
+    from echokv_b200.kernels import decode, prefill
+
+    monkeypatch.setattr(prefill, "to_device", lambda t, device: t)
+    monkeypatch.setattr(N, "require_cuda", lambda *t: None)
+    monkeypatch.setattr(N, "stream_ptr", lambda dev: 0)
+    monkeypatch.setattr(decode._scratch, "get", lambda dev, n: torch.zeros(n, dtype=torch.uint8))
+    store = SimpleNamespace(c_layout=None, c_pages=None, c_res=None, layout=SimpleNamespace(num_kv_heads=2, head_size=64, block_size=16))
+    rows, reqs, lens, longest = plan = prefill.build_rows([(0, 5, 9, 0)], [0], "cpu")
+    groups, bps = plan.groups, None
+    if form == "run-time split size":
+        bps = torch.ones(1, dtype=torch.int32)
+    elif form == "another step's groups":
+        groups = prefill.build_rows([(0, 3, 9, 0)], [0], "cpu").groups
+    else:
+        groups = groups[2][0]
+    with pytest.raises(ValueError):
+        decode.decode_attention(store, torch.zeros(5, 2 * gqa, 64), torch.zeros(1, 4, dtype=torch.int32), lens, 1.0, q_rows=rows,
+                                bt_rows=reqs, max_len=longest, bps_dev=bps, groups=groups)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("h,gqa,n,chunks", [(8, 4, 2, 64), (8, 4, 3, 40), (2, 1, 1, 100), (1, 2, 3, 33), (2, 8, 2, 20)])
 def test_partials_of_the_tokens_there_are(h, gqa, n, chunks, monkeypatch):
