@@ -12,82 +12,162 @@ int decode_mma_teams(int H, int D, int VG, int KG, int BS, int gqa, int chunks);
 int decode_status_take(bool clear);
 int prefill_status_take(bool clear);
 
-// out[q_rows[seq], head] = splits merged in split order (kernels/decode.py:226-262).  One warp per (sequence, query
-// head), four heads per CTA: lane s holds split s's running maximum and denominator (further rounds when there are more
-// than 32), the weights are exchanged by shuffles and a lane sums VEC channels over the splits, with the loads of
-// eight splits in flight.  A sequence's result is a function of its own splits alone.
+// out[q_rows[seq], head] = the splits' partials weighted by their maxima and added up (kernels/decode.py:226-262).  W warps
+// share a (sequence, query head): lane s holds the running maximum and denominator of splits s and s + 32 (further rounds
+// when there are more than 64), the weights are exchanged by shuffles and a lane sums VEC channels.  The sum has one order
+// whatever W is: splits s, s + 8, s + 16, ... one after the other for each of s = 0 .. 7, then these eight as a tree; so a
+// sequence's result is a function of its own splits alone, and the batch may choose W.
 //
-// Bound by its latency (split partials just written sit in L2): launch, one round of loads, the sum.  A thread per channel
-// and a CTA per head (before) made 8,192 CTAs of a batch of 256 sequences x 32 heads: 27.8 us, now 6.7 us; one sequence x 8 splits 3.75 -> 2.5 us,
-// 528 rows x 24 splits 54 -> 11 us.
-constexpr int MERGE_HEADS = 4;
-template <int VEC>
-__global__ void __launch_bounds__(MERGE_HEADS * 32) decode_merge_kernel(DecodeArgs A, int BS, int D) {
-  constexpr int BATCH = 8;
+// Bound by its latency (split partials just written sit in L2): launch, the rounds of loads, the sum.  With a warp per head
+// 64 splits were eight rounds of loads one after the other, of more than a microsecond each.  From the merge to the next
+// layer's write in a decode step, a warp per head throughout and now: 8 sequences x 32 heads, 33 splits 7.0 -> 2.7 us;
+// 16 x 8, 62 splits 12.7 -> 3.0; 48 x 16, 11 splits 6.3 -> 3.6; 64 x 32, 9 splits 5.1 -> 3.6; 256 x 32, 1 or 2 splits 7.1 -> 6.3.
+// W is the largest with heads x W <= MERGE_WARPS (16 warps an SM) that leaves a warp more than two of the splits there may be:
+// 48 x 16 heads take 3.6 us at W = 2 and 5.0 at 4, 64 x 32 take 3.6 at 1 and 4.8 at 2.
+constexpr int MERGE_SUMS = 8;      // independent sums over the splits
+constexpr int MERGE_ROUND = 64;    // splits whose maxima and denominators a warp holds at a time
+constexpr int64_t MERGE_WARPS = 2400;
+// FEW (W = 1): calls of at most FEW_SPLITS splits, whose sums are a product each: 48 registers instead of 94, more warps (528
+// tokens x 32 heads, 2 splits: 12.9 -> 9.5 us a layer).
+constexpr int FEW_SPLITS = 4;
+template <int VEC, int W, bool FEW>
+__global__ void __launch_bounds__(W == 8 ? 256 : 128, W == 1 ? (FEW ? 8 : 5) : 1) decode_merge_kernel(DecodeArgs A, int BS, int D) {
+  constexpr int HEADS = W == 8 ? 1 : 4 / W;   // per CTA
+  constexpr int OWN = MERGE_SUMS / W;         // sums of this warp
+  constexpr int LOADS = W == 1 ? FEW_SPLITS : MERGE_SUMS;  // splits in flight; with a warp per head the heads are many and registers limit the warps
   using V = typename std::conditional<VEC == 4, float4, float2>::type;
-  const int seq = blockIdx.x, head = blockIdx.y * MERGE_HEADS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  __shared__ __align__(16) float part[W == 1 ? 1 : HEADS * W][32 * VEC];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, me = warp % W;
+  const int seq = blockIdx.x, slot = blockIdx.y * HEADS + warp / W, head = min(slot, A.Hq - 1);
   const int d = (blockIdx.z * 32 + lane) * VEC;  // this lane's channels
   pdl_launch_dependents();
+  // In a planned step the lengths were final before the step's first write (see common.cuh): they are read ahead of the wait,
+  // and only partials that exist are read behind it.  Otherwise the first splits' partials are read along with the length
+  // that says how many there are (the rows exist either way); with a warp per head, whose warps hide one another's
+  // latency, behind it.
+  int64_t seq_len = 0, o_row = seq;
+  int used = A.num_splits;
+  auto plan = [&]() {
+    seq_len = A.lens[seq];
+    if (A.q_rows) o_row = A.q_rows[seq];
+    const int n_blocks = (int)((seq_len + BS - 1) / BS);
+    const int bps = max(bps_floor(A), (n_blocks + A.num_splits - 1) / A.num_splits);
+    used = (n_blocks + bps - 1) / bps;
+  };
+  if (A.planned) plan();
   pdl_wait();  // the split kernel has completed
-  if (seq == 0 && head == 0 && blockIdx.z == 0 && lane == 0) A.state[0] = 0;  // its item counter, for the next call
-  if (head >= A.Hq) return;
+  if (W == 1 && !A.planned) plan();
+  if (seq == 0 && slot == 0 && blockIdx.z == 0 && me == 0 && lane == 0) A.state[0] = 0;  // its item counter, for the next call
   const int64_t base = ((int64_t)seq * A.Hq + head) * A.num_splits;
   const float* src = A.acc + base * D + min(d, D - VEC);
-  // The first splits' partials are read along with the length that says how many there are (the rows exist either way).
-  V x[BATCH];
-  float2 ml = make_float2(-INFINITY, 0.f);
-  if (lane < A.num_splits) ml = *reinterpret_cast<const float2*>(A.ml + (base + lane) * 2);
+  // Split of this warp's load k of the batch that starts at split s: sums me * OWN .. of W consecutive groups of eight.
+  auto split_of = [&](int s, int k) { return s + (k / OWN) * MERGE_SUMS + me * OWN + k % OWN; };
+  V x[LOADS];
+  float2 ml[2] = {make_float2(-INFINITY, 0.f), make_float2(-INFINITY, 0.f)};
 #pragma unroll
-  for (int k = 0; k < BATCH; ++k) x[k] = *reinterpret_cast<const V*>(src + (int64_t)min(k, A.num_splits - 1) * D);
-  const int64_t seq_len = A.lens[seq];
-  const int64_t o_row = A.q_rows ? A.q_rows[seq] : seq;
+  for (int r = 0; r < 2; ++r)
+    if (r * 32 + lane < used) ml[r] = *reinterpret_cast<const float2*>(A.ml + (base + r * 32 + lane) * 2);
+#pragma unroll
+  for (int k = 0; k < LOADS; ++k)
+    if (split_of(0, k) < used) x[k] = *reinterpret_cast<const V*>(src + (int64_t)split_of(0, k) * D);
+  if (W > 1 && !A.planned) plan();
   if (seq_len == 0) return;  // CUDA-graph padding: leave the row alone
-  const int n_blocks = (int)((seq_len + BS - 1) / BS);
-  const int bps = max(bps_floor(A), (n_blocks + A.num_splits - 1) / A.num_splits);
-  const int used = (n_blocks + bps - 1) / bps;
-  float m = lane < used ? ml.x : -INFINITY;
-  for (int s0 = 32; s0 < used; s0 += 32)
+  float m = fmaxf(lane < used ? ml[0].x : -INFINITY, 32 + lane < used ? ml[1].x : -INFINITY);
+  for (int s0 = MERGE_ROUND; s0 < used; s0 += 32)
     if (s0 + lane < used) m = fmaxf(m, A.ml[(base + s0 + lane) * 2]);
   m = warp_max(m);  // the overall maximum
-  float acc[VEC];
+  float lt = 0.f, sum[VEC];
+  if constexpr (FEW) {
+    const float w = lane < used ? exp2f(ml[0].x - m) : 0.f;
+    lt = lane < used ? ml[0].y * w : 0.f;
+    float t[FEW_SPLITS][VEC];
 #pragma unroll
-  for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
-  float lt = 0.f;
-  for (int s0 = 0; s0 < used; s0 += 32) {
-    const bool on = s0 + lane < used;
-    if (s0 > 0 && on) ml = *reinterpret_cast<const float2*>(A.ml + (base + s0 + lane) * 2);
-    const float w = on ? exp2f(ml.x - m) : 0.f;
-    lt += on ? ml.y * w : 0.f;
-    const int n = min(32, used - s0);
-    for (int s = 0; s < n; s += BATCH) {
-      if (s0 + s > 0) {
+    for (int k = 0; k < FEW_SPLITS; ++k) {
+      const float wk = __shfl_sync(0xffffffffu, w, k);
 #pragma unroll
-        for (int k = 0; k < BATCH; ++k) x[k] = *reinterpret_cast<const V*>(src + (int64_t)min(s0 + s + k, used - 1) * D);
+      for (int e = 0; e < VEC; ++e) t[k][e] = k < used ? __fmul_rn(reinterpret_cast<const float*>(&x[k])[e], wk) : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) sum[e] = __fadd_rn(__fadd_rn(t[0][e], t[1][e]), __fadd_rn(t[2][e], t[3][e]));
+  } else {
+    float acc[OWN][VEC];
+#pragma unroll
+    for (int i = 0; i < OWN; ++i)
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[i][e] = 0.f;
+    for (int s0 = 0; s0 < used; s0 += MERGE_ROUND) {
+      float w[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int s = s0 + r * 32 + lane;
+        if (s0 > 0 && s < used) ml[r] = *reinterpret_cast<const float2*>(A.ml + (base + s) * 2);
+        w[r] = s < used ? exp2f(ml[r].x - m) : 0.f;
+        lt += s < used ? ml[r].y * w[r] : 0.f;
       }
+      const int end = min(s0 + MERGE_ROUND, used);
+      for (int s = s0; s < end; s += MERGE_SUMS * W) {
 #pragma unroll
-      for (int k = 0; k < BATCH; ++k) {
-        const float wk = __shfl_sync(0xffffffffu, w, s + k);
-        if (s + k < n) {
+        for (int k0 = 0; k0 < MERGE_SUMS; k0 += LOADS) {
+          if (s > 0 || k0 > 0) {
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) acc[e] += reinterpret_cast<const float*>(&x[k])[e] * wk;
+            for (int k = 0; k < LOADS; ++k)
+              if (split_of(s, k0 + k) < used) x[k] = *reinterpret_cast<const V*>(src + (int64_t)split_of(s, k0 + k) * D);
+          }
+#pragma unroll
+          for (int k = 0; k < LOADS; ++k) {
+            const int sk = split_of(s, k0 + k), at = sk - s0;
+            const float wk = __shfl_sync(0xffffffffu, at < 32 ? w[0] : w[1], at & 31);
+            if (sk < used) {
+#pragma unroll
+              for (int e = 0; e < VEC; ++e) acc[(k0 + k) % OWN][e] += reinterpret_cast<const float*>(&x[k])[e] * wk;
+            }
+          }
+          if (s + k0 + LOADS >= end) break;
         }
       }
     }
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      float t[OWN];
+#pragma unroll
+      for (int i = 0; i < OWN; ++i) t[i] = acc[i][e];
+#pragma unroll
+      for (int n = OWN / 2; n >= 1; n /= 2)
+#pragma unroll
+        for (int i = 0; i < n; ++i) t[i] = t[2 * i] + t[2 * i + 1];
+      sum[e] = t[0];
+    }
   }
   lt = warp_sum(lt);
-  if (d >= D) return;
+  if constexpr (W > 1) {
+    *reinterpret_cast<V*>(&part[warp][lane * VEC]) = *reinterpret_cast<const V*>(sum);
+    __syncthreads();
+    if (me != 0) return;
+    float t[W][VEC];
+#pragma unroll
+    for (int i = 0; i < W; ++i) *reinterpret_cast<V*>(t[i]) = *reinterpret_cast<const V*>(&part[warp + i][lane * VEC]);
+#pragma unroll
+    for (int n = W / 2; n >= 1; n /= 2)
+#pragma unroll
+      for (int i = 0; i < n; ++i)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) t[i][e] = t[2 * i][e] + t[2 * i + 1][e];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) sum[e] = t[0][e];
+  }
+  if (slot >= A.Hq || d >= D) return;
   const int64_t o = o_row * A.o_s0 + (int64_t)head * A.o_s1 + d;
 #pragma unroll
-  for (int e = 0; e < VEC; ++e) acc[e] /= lt;
+  for (int e = 0; e < VEC; ++e) sum[e] /= lt;
   if (A.out_vec) {  // 16-bit rows that take a lane's channels as one store
     uint32_t w[VEC / 2];
 #pragma unroll
     for (int e = 0; e < VEC / 2; ++e) {
       if (A.out_dt == ECHOKV_DT_BF16) {
-        const __nv_bfloat162 p = __floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1]);
+        const __nv_bfloat162 p = __floats2bfloat162_rn(sum[2 * e], sum[2 * e + 1]);
         w[e] = *reinterpret_cast<const uint32_t*>(&p);
       } else {
-        const __half2 p = __floats2half2_rn(acc[2 * e], acc[2 * e + 1]);
+        const __half2 p = __floats2half2_rn(sum[2 * e], sum[2 * e + 1]);
         w[e] = *reinterpret_cast<const uint32_t*>(&p);
       }
     }
@@ -96,8 +176,24 @@ __global__ void __launch_bounds__(MERGE_HEADS * 32) decode_merge_kernel(DecodeAr
     else *reinterpret_cast<uint32_t*>(dst) = w[0];
   } else {
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) st_dt(A.out, A.out_dt, o + e, acc[e]);
+    for (int e = 0; e < VEC; ++e) st_dt(A.out, A.out_dt, o + e, sum[e]);
   }
+}
+
+template <int VEC, int W, bool FEW = false>
+static cudaError_t launch_merge_w(const DecodeArgs& A, int64_t num_seqs, int BS, int D, cudaStream_t st) {
+  constexpr int HEADS = W == 8 ? 1 : 4 / W;
+  return launch_pdl(decode_merge_kernel<VEC, W, FEW>, dim3((unsigned)num_seqs, (unsigned)((A.Hq + HEADS - 1) / HEADS), (unsigned)((D + 127) / 128)),
+                    dim3(W == 8 ? 256 : 128), 0, st, A, BS, D);
+}
+template <int VEC>
+static cudaError_t launch_merge(const DecodeArgs& A, int64_t num_seqs, int BS, int D, cudaStream_t st) {
+  const int64_t heads = num_seqs * A.Hq;
+  if (A.num_splits > 16 && heads * 8 <= MERGE_WARPS) return launch_merge_w<VEC, 8>(A, num_seqs, BS, D, st);
+  if (A.num_splits > 8 && heads * 4 <= MERGE_WARPS) return launch_merge_w<VEC, 4>(A, num_seqs, BS, D, st);
+  if (A.num_splits > 4 && heads * 2 <= MERGE_WARPS) return launch_merge_w<VEC, 2>(A, num_seqs, BS, D, st);
+  if (A.num_splits <= FEW_SPLITS) return launch_merge_w<VEC, 1, true>(A, num_seqs, BS, D, st);
+  return launch_merge_w<VEC, 1>(A, num_seqs, BS, D, st);
 }
 
 }  // namespace echokv
@@ -194,12 +290,9 @@ static int decode_impl(const echokv_layout* layout, const echokv_pages* pages, c
     rc = check_launch("decode");
     if (rc) return rc;
   }
-  dim3 mgrid((unsigned)num_seqs, (unsigned)((num_q_heads + MERGE_HEADS - 1) / MERGE_HEADS), (unsigned)((L.D + 127) / 128));
   const int vec = L.D == 64 ? 2 : 4;
   A.out_vec = out_dtype != ECHOKV_DT_F32 && ((o_s0 | o_s1) % vec) == 0 && (reinterpret_cast<uintptr_t>(out) % (2 * vec)) == 0;
-  cudaError_t e;
-  if (L.D == 64) e = launch_pdl(decode_merge_kernel<2>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
-  else e = launch_pdl(decode_merge_kernel<4>, mgrid, dim3(MERGE_HEADS * 32), 0, st, A, L.BS, L.D);
+  const cudaError_t e = L.D == 64 ? launch_merge<2>(A, num_seqs, L.BS, L.D, st) : launch_merge<4>(A, num_seqs, L.BS, L.D, st);
   if (e != cudaSuccess) return check_launch("decode merge");
   return check_launch("decode merge");
 }
