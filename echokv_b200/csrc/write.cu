@@ -162,6 +162,20 @@ static int log2_or_neg(int v) {
 }
 static Shifts make_shifts(const LayoutDev& L) { return {log2_or_neg(L.D), log2_or_neg(L.VG), log2_or_neg(L.BS), log2_or_neg(L.KG)}; }
 
+// Tier of a block and byte offset (from the pool base) of its token `off`, from the 16 bytes of its header.
+__device__ __forceinline__ int header_bits(const uint4& hd) { return (hd.x & 0xff) == 0 ? 2 : (int)(hd.x & 0xff); }
+__device__ __forceinline__ int64_t header_row(const LayoutDev& L, const Shifts& sh, const uint4& hd, int64_t blk, int off, int bits) {
+  const int sh_bits = bits == 2 ? 1 : (bits == 4 ? 2 : 3);
+  const int tpc = (2 * L.BS) >> sh_bits, j = qdiv(off, tpc, sh.BS >= 0 ? sh.BS + 1 - sh_bits : -1);
+  int64_t page = blk, slot = 0;
+  if (j > 0) {
+    const int id = j == 1 ? (int)hd.y : (j == 2 ? (int)hd.z : (int)hd.w);
+    page = id / L.KC;
+    slot = id - page * L.KC;
+  }
+  return page * L.PS + L.o_data + slot * L.CB + (int64_t)(off - j * tpc) * ((2 * L.H * L.D * bits) / 8);
+}
+
 // Byte offsets (from the pool base) of consecutive token rows of one block stored at `bits`: the chunk of a row is
 // looked up once per chunk, not once per row.
 struct RowWalk {
@@ -278,10 +292,9 @@ __device__ __forceinline__ RowMeta row_meta(const TokArgs<T>& A, int64_t row) {
   m.kidx = A.kref ? A.tok[3 * A.tok_s0 + row] : -1;
   m.blk = sh.BS >= 0 ? m.slot >> sh.BS : m.slot / L.BS;
   m.off = (int)(m.slot - m.blk * L.BS);
-  m.bits = block_bits(A.pages, L, m.blk);
-  RowWalk walk;
-  walk.start(A.pages, L, sh.BS, m.blk, m.off, m.bits);
-  m.rowoff = walk.offset();
+  const uint4 hd = *reinterpret_cast<const uint4*>(A.pages + m.blk * L.PS);
+  m.bits = header_bits(hd);
+  m.rowoff = header_row(L, sh, hd, m.blk, m.off, m.bits);
   return m;
 }
 
@@ -302,10 +315,10 @@ struct RowRaw {
   }
 };
 
-// One token row that is stored (its slot is not negative).  `skip_residual`: the row's open-group key is stored by
-// someone else (see write_step_kernel).
-template <typename T, int MODE>
-__device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, const RowMeta& M, const RowRaw& raw, bool skip_residual) {
+// One token row that is stored (its slot is not negative).  `skip_residual()`, asked behind the value: the row's open-group key
+// is stored by someone else (see write_step_kernel).
+template <typename T, int MODE, class Skip>
+__device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, const RowMeta& M, const RowRaw& raw, Skip&& skip_residual) {
   const LayoutDev& L = A.L;
   uint8_t* __restrict__ pages = A.pages;
   const T* __restrict__ value = A.value;
@@ -321,9 +334,6 @@ __device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, cons
   uint8_t* page = pages + M.blk * L.PS;
   const int units = (L.H * L.D) / 8;  // 8-channel pieces of a row
   const int first = MODE == 2 ? threadIdx.x : lane, step = MODE == 2 ? WT_WARPS * 32 : 32;
-  int64_t rslot = skip_residual ? -1 : M.rslot;
-  const bool key_early = MODE == 2 && rslot >= 0 && A.res_raw && A.vec_in && units <= step;  // the whole key row is in `raw`
-
   if constexpr (MODE != 0) {
     // V: per token, groups of VG along head_dim; VG / 8 neighbouring threads share a group.
     const int upg = L.VG / 8;
@@ -386,7 +396,8 @@ __device__ __forceinline__ void token_row(const TokArgs<T>& A, int64_t row, cons
   }
 
   // K: residual row (open group), codes under stored stats (sealed group), K_ref ring row.
-  if (key_early) {
+  int64_t rslot = skip_residual() ? -1 : M.rslot;
+  if (MODE == 2 && rslot >= 0 && A.res_raw && A.vec_in && units <= step) {  // the whole key row is in `raw`
     if (raw.on) {
       const int h = qdiv(first * 8, L.D, sh.D), d0 = qmod(first * 8, L.D, sh.D);
       const int64_t ro = rslot * A.r_s0 + (int64_t)qmod(off, L.KG, sh.KG) * A.r_s1 + h * A.r_s2 + d0;
@@ -475,7 +486,7 @@ __global__ void __launch_bounds__(WT_WARPS * 32) write_tokens_kernel(const TokAr
   RowRaw raw;
   raw.on = false;
   if constexpr (MODE == 2) raw.load<T>(A, row);
-  token_row<T, MODE>(A, row, row_meta<T>(A, row), raw, false);
+  token_row<T, MODE>(A, row, row_meta<T>(A, row), raw, [] { return false; });
 }
 
 // One CTA per completed K group; each thread owns 8 channels of one head over the KG tokens
@@ -626,14 +637,27 @@ __global__ void __launch_bounds__(256, 4) finalize_k_kernel(const FinArgs<T> A) 
 // the chain list -> rows -> statistics -> codes, and with a thread walking all KG tokens twice (finalize_group) that
 // chain had 2 KG loads in a row.  350 groups of 32 x 8 heads x 128: 20 us, 24 us before; in a decode step see
 // write_step_kernel.
-template <typename T> struct SplitArgs { int n_take; const int* take; const TokArgs<T>* tok; };
+template <typename T> struct SplitArgs { int *n_take, *take; const TokArgs<T>* tok; };  // tok NULL: nobody takes a slot over
+
+// Token rows of the step whose open group takes residual slot `slot` over: their number to *n_take, the rows to take[].
+template <typename T>
+__device__ __forceinline__ void find_takers(const TokArgs<T>& TA, int64_t slot, int* n_take, int* take) {
+  __syncthreads();  // the list of the group before is no longer read
+  if (threadIdx.x == 0) *n_take = 0;
+  __syncthreads();
+  if (slot >= 0) {
+    for (int r = threadIdx.x; r < (int)TA.n_rows; r += blockDim.x)
+      if (TA.tok[r] >= 0 && TA.tok[TA.tok_s0 + r] == slot) take[atomicAdd(n_take, 1)] = r;
+  }
+  __syncthreads();
+}
 
 template <typename T, int SL, int TPL>
 __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
   const LayoutDev& L = A.L;
   const Shifts sh = A.sh;
   const int64_t* line = A.fin + f * (3 + L.KG);
-  const int64_t blk = line[0], rs = max(line[2], (int64_t)0);
+  const int64_t blk = line[0], slot = line[2], rs = max(slot, (int64_t)0);
   const int grp = (int)line[1];
   const int sub = threadIdx.x % SL, per = blockDim.x / SL;  // token lane, 8-channel pieces at a time
   int rows[TPL];
@@ -641,22 +665,11 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
   for (int i = 0; i < TPL; ++i) rows[i] = (int)line[3 + sub + SL * i];
   uint8_t* page = A.pages + blk * L.PS;
   const uint4 hd = *reinterpret_cast<const uint4*>(page);
-  const int bits = (hd.x & 0xff) == 0 ? 2 : (int)(hd.x & 0xff);
+  const int bits = header_bits(hd);
   const float levels = (float)((1 << bits) - 1);
-  const int row_bytes = (2 * L.H * L.D * bits) / 8;
   int64_t dst_row[TPL];  // byte offsets of this lane's token rows from the pool base
 #pragma unroll
-  for (int i = 0; i < TPL; ++i) {
-    const int t = grp * L.KG + sub + SL * i, sh_bits = bits == 2 ? 1 : (bits == 4 ? 2 : 3);
-    const int tpc = (2 * L.BS) >> sh_bits, j = qdiv(t, tpc, sh.BS >= 0 ? sh.BS + 1 - sh_bits : -1);
-    int64_t pg = blk, slot = 0;
-    if (j > 0) {
-      const int id = j == 1 ? (int)hd.y : (j == 2 ? (int)hd.z : (int)hd.w);
-      pg = id / L.KC;
-      slot = id - pg * L.KC;
-    }
-    dst_row[i] = pg * L.PS + L.o_data + slot * L.CB + (int64_t)(t - j * tpc) * row_bytes;
-  }
+  for (int i = 0; i < TPL; ++i) dst_row[i] = header_row(L, sh, hd, blk, grp * L.KG + sub + SL * i, bits);
   const int units = (L.H * L.D) / 8;
   for (int base = part * per; base < units; base += parts * per) {
     const int u = base + threadIdx.x / SL;
@@ -671,6 +684,7 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
       const T* src = rows[i] >= 0 ? kcol + (int64_t)rows[i] * (int)A.k_s0 : rcol + (int64_t)(sub + SL * i) * (int)A.r_s1;
       raw[i] = *reinterpret_cast<const uint4*>(src);
     }
+    if (S.tok && base == part * per) find_takers<T>(*S.tok, slot, S.n_take, S.take);  // while the rows are on their way
     MinMax8<T> acc;
     acc.init();
 #pragma unroll
@@ -688,15 +702,15 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
     float mn[8], mx[8];
     acc.finish(mn, mx);
     // The SL lanes hold the same minima and maxima: each works out the statistics of 8 / SL channels for all.
-    constexpr int CH = 8 / SL;
+    constexpr int CH = SL < 8 ? 8 / SL : 1;  // (with more than eight lanes, lanes sub and sub + 8 the same one)
     uint32_t own[CH];  // scale, min as fp16 pair
     float own_r[CH];
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
       float lo = mn[i], hi = mx[i];
 #pragma unroll
-      for (int l = 1; l < SL; ++l) {
-        if (sub == l) { lo = mn[l * CH + i]; hi = mx[l * CH + i]; }
+      for (int l = 1; l < 8 / CH; ++l) {
+        if ((sub & (8 / CH - 1)) == l) { lo = mn[l * CH + i]; hi = mx[l * CH + i]; }
       }
       __half s, z;
       group_stats(lo, hi, levels, s, z);
@@ -728,7 +742,8 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
       quant_store8<true>(bits, col + dst_row[i], x, m, sc, rsc);
     }
     // Keys of a group that takes the slot over (write_step_kernel): every lane of these channels has its rows in registers.
-    for (int i = sub; i < S.n_take; i += SL) {
+    const int n_take = S.tok ? *S.n_take : 0;
+    for (int i = sub; i < n_take; i += SL) {
       const TokArgs<T>& TA = *S.tok;
       const int64_t row = S.take[i], tslot = TA.tok[row];
       const int off = (int)(tslot - (sh.BS >= 0 ? tslot >> sh.BS : tslot / L.BS) * L.BS);
@@ -738,48 +753,59 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
     }
   }
 }
-// The group sizes finalize_split is instantiated for (split_group_ok says which).
+// The group sizes finalize_split is instantiated for (split_group_ok says which).  FINE: half the tokens per lane.
+template <typename T, int KG, bool FINE>
+__device__ __forceinline__ void finalize_split_kg(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
+  constexpr int SL = (KG == 16 ? 4 : 8) * (FINE ? 2 : 1);
+  finalize_split<T, SL, KG / SL>(A, f, part, parts, S);
+}
 template <typename T>
 __device__ __forceinline__ void finalize_split_any(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
   if constexpr (sizeof(T) == 2) {
-    if (A.L.KG == 16) finalize_split<T, 4, 4>(A, f, part, parts, S);
-    else if (A.L.KG == 32) finalize_split<T, 8, 4>(A, f, part, parts, S);
-    else finalize_split<T, 8, 8>(A, f, part, parts, S);
+    if (A.L.KG == 16) finalize_split_kg<T, 16, false>(A, f, part, parts, S);
+    else if (A.L.KG == 32) finalize_split_kg<T, 32, false>(A, f, part, parts, S);
+    else finalize_split_kg<T, 64, false>(A, f, part, parts, S);
   }
+}
+// CTAs that a group's channels fill.
+__host__ __device__ __forceinline__ int split_need(const LayoutDev& L, bool fine) {
+  const int per = WT_WARPS * 32 / ((L.KG == 16 ? 4 : 8) * (fine ? 2 : 1));
+  return (L.H * L.D / 8 + per - 1) / per;
 }
 static bool split_group_ok(const LayoutDev& L, bool raw16) { return raw16 && (L.KG == 16 || L.KG == 32 || L.KG == 64); }
 // CTAs per group: as many as the group's pieces fill, while the launch stays within about one round of the chip
 // (a captured step launches a group per row, and nearly all of them have nothing to do).
 static int split_parts(const LayoutDev& L, int64_t n_groups) {
-  const int per = 128 / (L.KG == 16 ? 4 : 8), need = (L.H * L.D / 8 + per - 1) / per;
+  const int need = split_need(L, false);
   const int64_t room = 1024 / (n_groups > 0 ? n_groups : 1);
   return room < 1 ? 1 : (room < need ? (int)room : need);
 }
 
-// CTAs per group of write_step_kernel, or 0: a thread owns 8 channels over the group's tokens (finalize_group), which keeps more
+// Whether write_step_kernel spreads a group over lanes and CTAs; if not, a thread owns 8 channels over the group's tokens (finalize_group), which keeps more
 // CTAs on an SM.  That is the better route where a launch has far more groups than the chip works on at once: captured steps of
 // 1,024 rows x 8 heads x 128, us a layer, split / not: no group of 32 tokens complete 5.1 / 4.4, 62 complete 22.7 / 25.2,
 // all 54 / 43; at 512 rows 3.1 / 3.8, 10.2 / 19.7, 28 / 25.  At 64 tokens per group (all of 1,024: 88 / 94) and with short rows
 // (two heads of 64, 62 of 1,024: 10.6 / 18.6) the split is ahead throughout.
 constexpr int64_t SPLIT_MAX_GROUPS = 512;
-static int step_split(const LayoutDev& L, bool raw16, int64_t n_groups) {
-  return n_groups > 0 && split_group_ok(L, raw16) && (n_groups <= SPLIT_MAX_GROUPS || L.KG == 64 || L.H * L.D < 512) ? split_parts(L, n_groups) : 0;
+constexpr int64_t STEP_GROUP_CTAS = 592;  // CTAs of the split pass on the chip at once
+static bool step_split(const LayoutDev& L, bool raw16, int64_t n_groups) {
+  return n_groups > 0 && split_group_ok(L, raw16) && (n_groups <= SPLIT_MAX_GROUPS || L.KG == 64 || L.H * L.D < 512);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(WT_WARPS * 32) finalize_split_kernel(const FinArgs<T> A, int parts) {
   const int64_t f = blockIdx.x / parts;
   if (f >= *A.fin_count) return;
-  const SplitArgs<T> none = {0, nullptr, nullptr};
+  const SplitArgs<T> none = {nullptr, nullptr, nullptr};
   finalize_split_any<T>(A, f, (int)(blockIdx.x - f * parts), parts, none);
 }
 
-// A step's writes of one layer in one launch: CTAs [0, n_rows) store the token rows, the next n_fin_launch CTAs
-// quantize the completed K groups (masked by the device-side count), the rest copy `stash_n` rows of `stash_src`
-// (the canary's query rows) to `stash_dst`.  Run one after the other, the group pass comes first because a
-// residual slot a completing group gives up may be taken by a new group in the same step; here the two run at
-// once, so the CTA of a token row whose slot a completing group still reads leaves that key alone, and the
-// group's CTA stores it after its own last read of the slot.
+// A step's writes of one layer in one launch: the first n_fin_ctas CTAs quantize the completed K groups (masked by the
+// device-side count; with SPLIT a group is several pieces of work, which the CTAs take in turn), the next n_rows store
+// the token rows, the rest copy `stash_n` rows of `stash_src` (the canary's query rows) to `stash_dst`.  Run one after the other,
+// the group pass comes first because a residual slot a completing group gives up may be taken by a new group in the same
+// step; here the two run at once, so the CTA of a token row whose slot a completing group still reads leaves that key
+// alone, and the group's CTA stores it after its own last read of the slot.
 struct StashArgs {
   const uint4* src; int64_t src_stride16;
   const int64_t* rows; int64_t n;
@@ -792,75 +818,79 @@ constexpr int STEP_MAX_ROWS = 1024;
 // group's tokens are spread over lanes and CTAs (finalize_split).  Per layer: 12.4 -> 6.3 us at 64 sequences x 8 heads, 10.1 -> 5.6 us
 // at 16 sequences x 1 head, 20 -> 10 us at 575 rows.  Four CTAs of the split pass fit an SM (with the 168 registers it would
 // take it is three: 512 groups of 32 tokens complete 35 us, now 28).
-template <typename T, bool SPLIT>
-__global__ void __launch_bounds__(WT_WARPS * 32, SPLIT ? 4 : (sizeof(T) == 2 ? 7 : 6))
-write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, int parts, const StashArgs SA) {
+// In a decode step most launches complete a few groups, and those are the end of the launch: a group's CTAs are chains of some
+// 1,500 instructions with a warp per scheduler.  So they go first, with half the tokens per lane while the CTAs suffice for that,
+// and on a bounded number of CTAs (a captured step of 256 rows launched 1,024 for its 8 groups).  From the write to the layer's
+// split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 7.0 -> 5.9 us, 256 x 8, groups of 32 13.4 -> 6.2,
+// 16 x 1 6.5 -> 5.3, 48 x 2 8.1 -> 5.6; a launch of empty CTAs takes 1.1.
+// SPLIT_KG: tokens of a group that is spread over lanes and CTAs (finalize_split), 0: a thread walks a group's tokens.  One group
+// size per instance, to keep the code short.
+template <typename T, int SPLIT_KG>
+__global__ void __launch_bounds__(WT_WARPS * 32, SPLIT_KG ? 4 : (sizeof(T) == 2 ? 7 : 6))
+write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, int64_t n_fin_ctas, const StashArgs SA) {
   __shared__ int take[STEP_MAX_ROWS];
   __shared__ int n_take;
   pdl_launch_dependents();
-  pdl_wait();
   const LayoutDev& L = TA.L;
-  const int64_t b = blockIdx.x, n_fin_ctas = n_fin_launch * (SPLIT ? parts : 1);
+  const int64_t b = blockIdx.x, row = b - n_fin_ctas;
   const int w = 3 + L.KG;
-  if (b < TA.n_rows) {
-    if (TA.tok[b] < 0) return;  // padding, or a token that is not stored
+  pdl_wait();
+  if (row >= 0 && row < TA.n_rows) {  // ahead of the group passes' long code, which is fetched anew in every launch: 0.7 us at one sequence
+    const int64_t n_fin = n_fin_launch > 0 ? min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
+    if (TA.tok[row] < 0) return;  // padding, or a token that is not stored
     RowRaw raw;
-    raw.load<T>(TA, b);
-    const RowMeta M = row_meta<T>(TA, b);
-    bool skip = false;
-    if (M.rslot >= 0) {
-      const int64_t n_fin = n_fin_launch > 0 ? min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
-      int hit = 0;
+    raw.load<T>(TA, row);
+    const RowMeta M = row_meta<T>(TA, row);
+    int hit = 0;
+    if (M.rslot >= 0)
       for (int64_t f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[f * w + 2] == M.rslot;
-      skip = __syncthreads_or(hit) != 0;
-    }
-    token_row<T, 2>(TA, b, M, raw, skip);
+    token_row<T, 2>(TA, row, M, raw, [&] { return M.rslot >= 0 && __syncthreads_or(hit) != 0; });
     return;
   }
-  if (b < TA.n_rows + n_fin_ctas) {
-    const int64_t g = b - TA.n_rows, f = SPLIT ? g / parts : g;
-    if (f >= *FA.fin_count) return;
-    const int64_t slot = FA.fin[f * w + 2];
-    if (threadIdx.x == 0) n_take = 0;
-    __syncthreads();
-    if (slot >= 0) {
-      for (int r = threadIdx.x; r < (int)TA.n_rows; r += blockDim.x)
-        if (TA.tok[r] >= 0 && TA.tok[TA.tok_s0 + r] == slot) take[atomicAdd(&n_take, 1)] = r;
+  if (row >= TA.n_rows) {
+    const int64_t i = (row - TA.n_rows) * blockDim.x + threadIdx.x;
+    if (i >= SA.n * SA.row16) return;
+    const int64_t r = i / SA.row16;
+    SA.dst[i] = SA.src[SA.rows[r] * SA.src_stride16 + (i - r * SA.row16)];
+    return;
+  }
+  if constexpr (SPLIT_KG != 0) {
+    const int64_t count = min(*FA.fin_count, n_fin_launch);
+    const int fine = split_need(L, true);
+    const SplitArgs<T> S = {&n_take, take, &TA};
+    if (count * fine <= n_fin_ctas) {  // a piece is a chain of a warp or two per scheduler: the shorter, the better
+      if (b < count * fine) finalize_split_kg<T, SPLIT_KG, true>(FA, b / fine, (int)(b % fine), fine, S);
+    } else {
+      const int parts = (int)max((int64_t)1, min((int64_t)split_need(L, false), n_fin_ctas / count));
+      for (int64_t g = b; g < count * parts; g += n_fin_ctas) finalize_split_kg<T, SPLIT_KG, false>(FA, g / parts, (int)(g % parts), parts, S);
     }
-    __syncthreads();
-    if constexpr (SPLIT) {
-      const SplitArgs<T> S = {n_take, take, &TA};
-      finalize_split_any<T>(FA, f, (int)(g - f * parts), parts, S);
-      return;
-    }
-    finalize_group<T, false>(FA, f);
-    // Keys of the group that takes the slot over: each thread stores the channels it has just read for the last time.
-    const int units = (L.H * L.D) / 8;
-    for (int i = 0; i < n_take; ++i) {
-      const int64_t row = take[i];
-      const int64_t tslot = TA.tok[row];
-      const int off = (int)(tslot - (TA.sh.BS >= 0 ? tslot >> TA.sh.BS : tslot / L.BS) * L.BS);
-      const int gpos = qmod(off, L.KG, TA.sh.KG);
-      for (int c = threadIdx.x; c < units; c += blockDim.x) {
-        const int h = qdiv(c * 8, L.D, TA.sh.D), d0 = qmod(c * 8, L.D, TA.sh.D);
-        const int64_t src = row * TA.k_s0 + h * TA.k_s1 + d0;
-        const int64_t ro = slot * TA.r_s0 + (int64_t)gpos * TA.r_s1 + h * TA.r_s2 + d0;
-        if (TA.res_raw) {
-          *reinterpret_cast<uint4*>(reinterpret_cast<T*>(TA.res) + ro) = *reinterpret_cast<const uint4*>(TA.key + src);
-        } else {
-          float x[8];
-          ld8<T>(TA.key, src, TA.vec_in, x);
+    return;
+  }
+  if (b >= *FA.fin_count) return;
+  const int64_t slot = FA.fin[b * w + 2];
+  find_takers<T>(TA, slot, &n_take, take);
+  finalize_group<T, false>(FA, b);
+  // Keys of the group that takes the slot over: each thread stores the channels it has just read for the last time.
+  const int units = (L.H * L.D) / 8;
+  for (int i = 0; i < n_take; ++i) {
+    const int64_t row = take[i];
+    const int64_t tslot = TA.tok[row];
+    const int off = (int)(tslot - (TA.sh.BS >= 0 ? tslot >> TA.sh.BS : tslot / L.BS) * L.BS);
+    const int gpos = qmod(off, L.KG, TA.sh.KG);
+    for (int c = threadIdx.x; c < units; c += blockDim.x) {
+      const int h = qdiv(c * 8, L.D, TA.sh.D), d0 = qmod(c * 8, L.D, TA.sh.D);
+      const int64_t src = row * TA.k_s0 + h * TA.k_s1 + d0;
+      const int64_t ro = slot * TA.r_s0 + (int64_t)gpos * TA.r_s1 + h * TA.r_s2 + d0;
+      if (TA.res_raw) {
+        *reinterpret_cast<uint4*>(reinterpret_cast<T*>(TA.res) + ro) = *reinterpret_cast<const uint4*>(TA.key + src);
+      } else {
+        float x[8];
+        ld8<T>(TA.key, src, TA.vec_in, x);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) st_dt(TA.res, TA.res_dt, ro + k, x[k]);
-        }
+        for (int k = 0; k < 8; ++k) st_dt(TA.res, TA.res_dt, ro + k, x[k]);
       }
     }
-    return;
   }
-  const int64_t i = (b - TA.n_rows - n_fin_ctas) * blockDim.x + threadIdx.x;
-  if (i >= SA.n * SA.row16) return;
-  const int64_t r = i / SA.row16;
-  SA.dst[i] = SA.src[SA.rows[r] * SA.src_stride16 + (i - r * SA.row16)];
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -926,16 +956,26 @@ static FinArgs<T> fin_args(const LayoutDev& L, const echokv_pages* pages, const 
 
 using namespace echokv;
 
+template <typename T, int SPLIT_KG>
+static void launch_write_split(bool first, int64_t rest, cudaStream_t st, const TokArgs<T>& TA, const FinArgs<T>& FA, int64_t n_fin, const StashArgs& SA) {
+  // A captured step launches room for a group per row, and nearly all of it has nothing to do: the pieces go round on no more
+  // CTAs than fit the chip beside the rows'.
+  const int64_t room = std::max<int64_t>(STEP_GROUP_CTAS - rest, STEP_GROUP_CTAS / 2);
+  const int64_t ctas = std::min(n_fin * split_need(TA.L, true), room);
+  launch_after(!first, write_step_kernel<T, SPLIT_KG>, dim3((unsigned)(ctas + rest)), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, ctas, SA);
+}
 template <typename T>
-static void launch_write_step(bool first, int parts, unsigned grid, cudaStream_t st, const TokArgs<T>& TA, const FinArgs<T>& FA,
+static void launch_write_step(bool first, bool split, int64_t rest, cudaStream_t st, const TokArgs<T>& TA, const FinArgs<T>& FA,
                               int64_t n_fin, const StashArgs& SA) {
   if constexpr (sizeof(T) == 2) {
-    if (parts > 0) {
-      launch_after(!first, write_step_kernel<T, true>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, parts, SA);
+    if (split) {
+      if (TA.L.KG == 16) launch_write_split<T, 16>(first, rest, st, TA, FA, n_fin, SA);
+      else if (TA.L.KG == 32) launch_write_split<T, 32>(first, rest, st, TA, FA, n_fin, SA);
+      else launch_write_split<T, 64>(first, rest, st, TA, FA, n_fin, SA);
       return;
     }
   }
-  launch_after(!first, write_step_kernel<T, false>, dim3(grid), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, 0, SA);
+  launch_after(!first, write_step_kernel<T, 0>, dim3((unsigned)(n_fin + rest)), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, n_fin, SA);
 }
 
 extern "C" {
@@ -1131,9 +1171,8 @@ static int write_step_impl(const echokv_layout* layout, const echokv_pages* page
     const TokArgs<T> TA = tok_args<T>(L, pages, R, key, k_s0, k_s1, value, v_s0, v_s1, tok, tok_s0, kref, kref_s0, \
                                       kref_s1, n_rows);                                                            \
     const FinArgs<T> FA = fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count);                               \
-    const int parts = step_split(L, FA.raw16 && TA.res_raw, n_fin_launch);                                         \
-    const unsigned grid = (unsigned)(n_rows + n_fin_launch * (parts > 0 ? parts : 1) + stash_ctas);                \
-    launch_write_step<T>(first, parts, grid, st, TA, FA, n_fin_launch, SA);                                        \
+    const bool split = step_split(L, FA.raw16 && TA.res_raw, n_fin_launch);                                        \
+    launch_write_step<T>(first, split, n_rows + stash_ctas, st, TA, FA, n_fin_launch, SA);                         \
   }
   switch (kv_dtype) {
     case ECHOKV_DT_F32: LAUNCH(float); break;
