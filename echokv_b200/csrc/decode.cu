@@ -27,8 +27,8 @@ int prefill_status_take(bool clear);
 constexpr int MERGE_SUMS = 8;      // independent sums over the splits
 constexpr int MERGE_ROUND = 64;    // splits whose maxima and denominators a warp holds at a time
 constexpr int64_t MERGE_WARPS = 2400;
-// FEW (W = 1): calls of at most FEW_SPLITS splits, whose sums are a product each: 48 registers instead of 94, more warps (528
-// tokens x 32 heads, 2 splits: 12.9 -> 9.5 us a layer).
+// FEW (W = 1): calls of at most FEW_SPLITS splits, whose sums are a product each: 48 registers instead of 94, more warps
+// (528 tokens x 32 heads, 2 splits: 13.1 us before, 10.2 now, under ncu).
 constexpr int FEW_SPLITS = 4;
 template <int VEC, int W, bool FEW>
 __global__ void __launch_bounds__(W == 8 ? 256 : 128, W == 1 ? (FEW ? 8 : 5) : 1) decode_merge_kernel(DecodeArgs A, int BS, int D) {
