@@ -759,25 +759,17 @@ __device__ __forceinline__ void finalize_split_kg(const FinArgs<T>& A, int64_t f
   constexpr int SL = (KG == 16 ? 4 : 8) * (FINE ? 2 : 1);
   finalize_split<T, SL, KG / SL>(A, f, part, parts, S);
 }
-template <typename T>
-__device__ __forceinline__ void finalize_split_any(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
-  if constexpr (sizeof(T) == 2) {
-    if (A.L.KG == 16) finalize_split_kg<T, 16, false>(A, f, part, parts, S);
-    else if (A.L.KG == 32) finalize_split_kg<T, 32, false>(A, f, part, parts, S);
-    else finalize_split_kg<T, 64, false>(A, f, part, parts, S);
-  }
-}
 // CTAs that a group's channels fill.
 __host__ __device__ __forceinline__ int split_need(const LayoutDev& L, bool fine) {
   const int per = WT_WARPS * 32 / ((L.KG == 16 ? 4 : 8) * (fine ? 2 : 1));
   return (L.H * L.D / 8 + per - 1) / per;
 }
 static bool split_group_ok(const LayoutDev& L, bool raw16) { return raw16 && (L.KG == 16 || L.KG == 32 || L.KG == 64); }
-// CTAs per group: as many as the group's pieces fill, while the launch stays within about one round of the chip
-// (a captured step launches a group per row, and nearly all of them have nothing to do).
+// CTAs per group: as many as the group's pieces fill, while the launch stays within a few rounds of the chip (a CTA that walks
+// several pieces waits for the rows of each: with at most 1,024 CTAs 325 groups of 32 took three pieces a CTA).
 static int split_parts(const LayoutDev& L, int64_t n_groups) {
   const int need = split_need(L, false);
-  const int64_t room = 1024 / (n_groups > 0 ? n_groups : 1);
+  const int64_t room = 4096 / (n_groups > 0 ? n_groups : 1);
   return room < 1 ? 1 : (room < need ? (int)room : need);
 }
 
@@ -792,12 +784,21 @@ static bool step_split(const LayoutDev& L, bool raw16, int64_t n_groups) {
   return n_groups > 0 && split_group_ok(L, raw16) && (n_groups <= SPLIT_MAX_GROUPS || L.KG == 64 || L.H * L.D < 512);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(WT_WARPS * 32) finalize_split_kernel(const FinArgs<T> A, int parts) {
-  const int64_t f = blockIdx.x / parts;
+template <typename T, int KG>
+__global__ void __launch_bounds__(WT_WARPS * 32, KG == 64 ? 4 : 6) finalize_split_kernel(const FinArgs<T> A, int parts) {
+  const int f = blockIdx.x / parts;
   if (f >= *A.fin_count) return;
   const SplitArgs<T> none = {nullptr, nullptr, nullptr};
-  finalize_split_any<T>(A, f, (int)(blockIdx.x - f * parts), parts, none);
+  finalize_split_kg<T, KG, false>(A, f, (int)blockIdx.x - f * parts, parts, none);
+}
+template <typename T>
+static void launch_finalize_split(const FinArgs<T>& A, int64_t n, int parts, cudaStream_t st) {
+  if constexpr (sizeof(T) == 2) {
+    const dim3 grid((unsigned)(n * parts)), block(WT_WARPS * 32);
+    if (A.L.KG == 16) finalize_split_kernel<T, 16><<<grid, block, 0, st>>>(A, parts);
+    else if (A.L.KG == 32) finalize_split_kernel<T, 32><<<grid, block, 0, st>>>(A, parts);
+    else finalize_split_kernel<T, 64><<<grid, block, 0, st>>>(A, parts);
+  }
 }
 
 // A step's writes of one layer in one launch: the first n_fin_ctas CTAs quantize the completed K groups (masked by the
@@ -1097,8 +1098,7 @@ int echokv_finalize_k(const echokv_layout* layout, const echokv_pages* pages, co
 #define LAUNCH(T)                                                                                              \
   {                                                                                                            \
     const FinArgs<T> A = fin_args<T>(L, pages, R, key, k_s0, k_s1, fin, fin_count);                            \
-    if (split_group_ok(L, A.raw16))                                                                            \
-      finalize_split_kernel<T><<<(unsigned)(n_launch * parts), WT_WARPS * 32, 0, st>>>(A, parts);              \
+    if (split_group_ok(L, A.raw16)) launch_finalize_split<T>(A, n_launch, parts, st);                          \
     else finalize_k_kernel<T, false><<<(unsigned)n_launch, threads, 0, st>>>(A);                               \
   }
   switch (kv_dtype) {
