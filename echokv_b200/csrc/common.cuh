@@ -42,9 +42,9 @@ int check_launch(const char* what);
 // kernel has completed and its writes are visible.  `pdl_launch_dependents()` lets the next such kernel start being
 // scheduled; a kernel that does not call it lets its dependents start as its last CTAs exit, which says nothing about
 // the visibility of its writes.  Every CTA calls `pdl_wait()` before it writes anything another kernel touches (so
-// completion of this kernel implies completion of the one before it).  One kernel reads ahead of its wait: the split
-// kernel of a planned decode step (echokv_decode_step), whose lengths, rows, block table, page headers and residual map
-// were written by kernels and copies ahead of the step's first write.  All kernels of a step trigger at their start, so
+// completion of this kernel implies completion of the one before it).  Two kernels read ahead of their wait: the split
+// kernel and the merge of a planned decode step (echokv_decode_step), whose lengths, rows, block table, split size, page headers
+// and residual map were written by kernels and copies ahead of the step's first write.  All kernels of a step trigger at their start, so
 // nothing in their chain would hold the split kernel back until those writers have completed, were it not that the
 // step's first write (echokv_write_step_first) is launched the ordinary way: it starts
 // when everything before it has completed and is visible, and what follows starts after it.  A trigger after the

@@ -20,6 +20,11 @@ EAGER_MAX_SPLITS = 32   # calls that size their own grid (the prefill row path):
 # splits of a step that leaves the chip idle shortens it: 1 x 500 tokens x 32 layers 0.519 -> 0.444 ms, 4 x 678 in blocks of 32
 # 0.561 -> 0.546; larger steps choose the sizes they chose with 64.
 MIN_SPLIT_TOKENS = 32
+# Split size of a step whose shape takes the CUDA-core kernel: a CTA's four warps take a block each, and a batch that leaves the chip
+# idle wants more CTAs.  8 heads of 64 channels, blocks of 32, ms a step with 16 and with 4 blocks: 1 x 6,000 tokens 0.341 -> 0.172,
+# 4 x 900 0.344 -> 0.191, 32 x 1,500 0.623 -> 0.576, 128 x 700 0.530 -> 0.523, 8 x 12,000 0.525 -> 0.527; in blocks of 16 4 blocks are too
+# few (32 x 1,500: 0.773 with 16, 0.690 with 8, 0.724 with 4), in blocks of 64 2 are (0.575, 0.584 with 4, 0.755 with 2).
+GENERIC_SPLIT_BLOCKS, GENERIC_SPLIT_TOKENS = 4, 128
 MMA_COLUMNS = 8         # columns of the split kernel's MMAs: query heads of a token, or of consecutive tokens of a chunk
 ITEM_COST_TILES = 4     # fixed cost of a (sequence, split) work item in units of one 16-token tile's work
 
@@ -27,6 +32,11 @@ ITEM_COST_TILES = 4     # fixed cost of a (sequence, split) work item in units o
 def decode_parallelism(store, num_q_heads: int) -> int:
     """Work items the split kernel has in work at once on the current device (0: generic kernel)."""
     return int(N.lib.echokv_decode_parallelism(store.c_layout, int(num_q_heads)))
+
+
+def generic_blocks_per_split(block_size: int) -> int:
+    """Blocks per split for a step on the CUDA-core kernel, whatever the lengths."""
+    return max(GENERIC_SPLIT_BLOCKS, GENERIC_SPLIT_TOKENS // block_size)
 
 
 def choose_blocks_per_split(lens, block_size: int, num_splits: int, slots: int) -> int:

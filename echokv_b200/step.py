@@ -26,7 +26,7 @@ from echokv_b200.canary import canary_kl_ring, tp_mean
 from echokv_b200.controller import LayerController
 from echokv_b200.quant import SUPPORTED_BITS
 from echokv_b200.kernels.decode import (BLOCKS_PER_SPLIT, MAX_DECODE_SPLITS, MIN_SPLIT_TOKENS, choose_blocks_per_split,
-                                        decode_attention, decode_parallelism)
+                                        decode_attention, decode_parallelism, generic_blocks_per_split)
 from echokv_b200.kernels.write import gather_rows
 from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
 from echokv_b200.write_plan import SharedState, WriteMeta
@@ -214,8 +214,9 @@ class GroupRunner:
         dec = decode if decode is not None else (empty, empty, empty)
         can = np.zeros(self.canary_max_q, dtype=np.int64) if canary is None else canary
         bps = BLOCKS_PER_SPLIT
-        if self.decode_slots and dec[2].size:
-            bps = choose_blocks_per_split(dec[2], self.layout.block_size, self.num_splits, self.decode_slots)
+        if dec[2].size:
+            bps = (choose_blocks_per_split(dec[2], self.layout.block_size, self.num_splits, self.decode_slots) if self.decode_slots
+                   else generic_blocks_per_split(self.layout.block_size))
         fin_count, canary_rows, dviews, tok, fin, views, bps_dev = self.staging.stage(
             plan.n_fin, can, dec, (plan.tok_slot, plan.tok_res, plan.tok_sealed, plan.tok_kref), plan.fin, tail, bps)
         shared.apply_res_map(*views[:4])

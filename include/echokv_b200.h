@@ -233,8 +233,8 @@ int echokv_decode_ex(const echokv_layout* layout, const echokv_pages* pages, con
 
 /* echokv_decode_ex behind an echokv_write_step_first of the same step (any layer's) on the same stream, where lens, q_rows,
  * bt_rows, block_table, the split-size word, the page headers and the residual map were all written ahead of that
- * write and nothing has changed them since.  The split kernel then resolves its first work items while the kernel
- * before it still runs.  Call echokv_decode_ex otherwise. */
+ * write and nothing has changed them since.  The split kernel then resolves its first work items, and the merge reads
+ * the lengths, rows and split size, while the kernel before it still runs.  Call echokv_decode_ex otherwise. */
 int echokv_decode_step(const echokv_layout* layout, const echokv_pages* pages, const echokv_residual* residual,
                        const void* query, int64_t q_s0, int64_t q_s1, int32_t q_dtype, const int64_t* q_rows,
                        const int32_t* block_table, int64_t bt_s0, const int64_t* bt_rows, const int64_t* lens,
