@@ -819,8 +819,8 @@ constexpr int STEP_MAX_ROWS = 1024;
 // group's tokens are spread over lanes and CTAs (finalize_split).  Per layer: 12.4 -> 6.3 us at 64 sequences x 8 heads, 10.1 -> 5.6 us
 // at 16 sequences x 1 head, 20 -> 10 us at 575 rows.  Four CTAs of the split pass fit an SM (with the 168 registers it would
 // take it is three: 512 groups of 32 tokens complete 35 us, now 28).
-// In a decode step most launches complete a few groups, and those are the end of the launch: a group's CTAs are chains of some
-// 1,500 instructions with a warp per scheduler.  So they go first, with half the tokens per lane while the CTAs suffice for that,
+// In a decode step most launches complete a few groups, and those are the end of the launch: a group's CTAs are long chains
+// with a warp per scheduler (256 rows x 8 heads: 3.9 us without the groups, 10.3 with them alone).  So they go first, with half the tokens per lane while the CTAs suffice for that,
 // and on a bounded number of CTAs (a captured step of 256 rows launched 1,024 for its 8 groups).  From the write to the layer's
 // split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 7.0 -> 5.9 us, 256 x 8, groups of 32 13.4 -> 6.2,
 // 16 x 1 6.5 -> 5.3, 48 x 2 8.1 -> 5.6; a launch of empty CTAs takes 1.1.
