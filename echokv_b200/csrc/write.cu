@@ -652,8 +652,9 @@ __device__ __forceinline__ void find_takers(const TokArgs<T>& TA, int64_t slot, 
   __syncthreads();
 }
 
+// Pieces [first, last) of group `f`: a piece is the blockDim.x / SL 8-channel units that a CTA takes at a time.
 template <typename T, int SL, int TPL>
-__device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
+__device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, int first, int last, const SplitArgs<T>& S) {
   const LayoutDev& L = A.L;
   const Shifts sh = A.sh;
   const int64_t* line = A.fin + f * (3 + L.KG);
@@ -671,8 +672,8 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
 #pragma unroll
   for (int i = 0; i < TPL; ++i) dst_row[i] = header_row(L, sh, hd, blk, grp * L.KG + sub + SL * i, bits);
   const int units = (L.H * L.D) / 8;
-  for (int base = part * per; base < units; base += parts * per) {
-    const int u = base + threadIdx.x / SL;
+  for (int piece = first; piece < last; ++piece) {
+    const int u = piece * per + threadIdx.x / SL;
     const bool on = u < units;
     const int c = on ? u : 0;
     const int h = qdiv(c * 8, L.D, sh.D), d0 = qmod(c * 8, L.D, sh.D);
@@ -684,7 +685,7 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
       const T* src = rows[i] >= 0 ? kcol + (int64_t)rows[i] * (int)A.k_s0 : rcol + (int64_t)(sub + SL * i) * (int)A.r_s1;
       raw[i] = *reinterpret_cast<const uint4*>(src);
     }
-    if (S.tok && base == part * per) find_takers<T>(*S.tok, slot, S.n_take, S.take);  // while the rows are on their way
+    if (S.tok && piece == first) find_takers<T>(*S.tok, slot, S.n_take, S.take);  // while the rows are on their way
     MinMax8<T> acc;
     acc.init();
 #pragma unroll
@@ -755,11 +756,11 @@ __device__ __forceinline__ void finalize_split(const FinArgs<T>& A, int64_t f, i
 }
 // The group sizes finalize_split is instantiated for (split_group_ok says which).  FINE: half the tokens per lane.
 template <typename T, int KG, bool FINE>
-__device__ __forceinline__ void finalize_split_kg(const FinArgs<T>& A, int64_t f, int part, int parts, const SplitArgs<T>& S) {
+__device__ __forceinline__ void finalize_split_kg(const FinArgs<T>& A, int64_t f, int first, int last, const SplitArgs<T>& S) {
   constexpr int SL = (KG == 16 ? 4 : 8) * (FINE ? 2 : 1);
-  finalize_split<T, SL, KG / SL>(A, f, part, parts, S);
+  finalize_split<T, SL, KG / SL>(A, f, first, last, S);
 }
-// CTAs that a group's channels fill.
+// Pieces that a group's channels make.
 __host__ __device__ __forceinline__ int split_need(const LayoutDev& L, bool fine) {
   const int per = WT_WARPS * 32 / ((L.KG == 16 ? 4 : 8) * (fine ? 2 : 1));
   return (L.H * L.D / 8 + per - 1) / per;
@@ -774,10 +775,10 @@ static int split_parts(const LayoutDev& L, int64_t n_groups) {
 }
 
 // Whether write_step_kernel spreads a group over lanes and CTAs; if not, a thread owns 8 channels over the group's tokens (finalize_group), which keeps more
-// CTAs on an SM.  That is the better route where a launch has far more groups than the chip works on at once: captured steps of
-// 1,024 rows x 8 heads x 128, us a layer, split / not: no group of 32 tokens complete 5.1 / 4.4, 62 complete 22.7 / 25.2,
-// all 54 / 43; at 512 rows 3.1 / 3.8, 10.2 / 19.7, 28 / 25.  At 64 tokens per group (all of 1,024: 88 / 94) and with short rows
-// (two heads of 64, 62 of 1,024: 10.6 / 18.6) the split is ahead throughout.
+// CTAs on an SM.  That is the better route where a launch has far more groups than the chip works on at once and all or none of them
+// complete: captured steps of 1,000 rows x 8 heads x 128, us a layer, split / not: no group of 32 tokens complete 5.9 / 4.4,
+// all 53 / 48; groups of 16 5.9 / 4.4, 30 / 27; but 62 of the 1,000 complete 12.7 / 25.6 and 9.2 / 15.8.  At 64 tokens per group (15 of
+// 1,000 9.7, all 81) and with short rows (two heads of 64: 6.9, 13.3) the split is ahead throughout.
 constexpr int64_t SPLIT_MAX_GROUPS = 512;
 constexpr int64_t STEP_GROUP_CTAS = 592;  // CTAs of the split pass on the chip at once
 static bool step_split(const LayoutDev& L, bool raw16, int64_t n_groups) {
@@ -786,10 +787,10 @@ static bool step_split(const LayoutDev& L, bool raw16, int64_t n_groups) {
 
 template <typename T, int KG>
 __global__ void __launch_bounds__(WT_WARPS * 32, KG == 64 ? 4 : 6) finalize_split_kernel(const FinArgs<T> A, int parts) {
-  const int f = blockIdx.x / parts;
+  const int f = blockIdx.x / parts, part = (int)blockIdx.x - f * parts, need = split_need(A.L, false);
   if (f >= *A.fin_count) return;
   const SplitArgs<T> none = {nullptr, nullptr, nullptr};
-  finalize_split_kg<T, KG, false>(A, f, (int)blockIdx.x - f * parts, parts, none);
+  finalize_split_kg<T, KG, false>(A, f, part * need / parts, (part + 1) * need / parts, none);
 }
 template <typename T>
 static void launch_finalize_split(const FinArgs<T>& A, int64_t n, int parts, cudaStream_t st) {
@@ -801,8 +802,8 @@ static void launch_finalize_split(const FinArgs<T>& A, int64_t n, int parts, cud
   }
 }
 
-// A step's writes of one layer in one launch: the first n_fin_ctas CTAs quantize the completed K groups (masked by the
-// device-side count; with SPLIT a group is several pieces of work, which the CTAs take in turn), the next n_rows store
+// A step's writes of one layer in one launch: the first CTAs quantize the completed K groups (masked by the
+// device-side count; groups that are spread over lanes are several pieces of work each, see GroupCtas), the next n_rows store
 // the token rows, the rest copy `stash_n` rows of `stash_src` (the canary's query rows) to `stash_dst`.  Run one after the other,
 // the group pass comes first because a residual slot a completing group gives up may be taken by a new group in the same
 // step; here the two run at once, so the CTA of a token row whose slot a completing group still reads leaves that key
@@ -814,39 +815,56 @@ struct StashArgs {
 };
 constexpr int STEP_MAX_ROWS = 1024;
 
+// CTAs of write_step_kernel that work on its groups.
+struct GroupCtas {
+  int ctas;     // launched for them
+  int enough;   // completed groups for whose pieces these suffice
+  int workers;  // if more have completed: with the CTAs of the first token rows, as many as are on the chip at once
+};
+
 // A step's rows are a few hundred kilobytes: the time is the chain of dependent reads (token list -> page header ->
 // rows -> statistics -> codes), so a row's value and key are on their way while the header is looked up, and a
 // group's tokens are spread over lanes and CTAs (finalize_split).  Per layer: 12.4 -> 6.3 us at 64 sequences x 8 heads, 10.1 -> 5.6 us
-// at 16 sequences x 1 head, 20 -> 10 us at 575 rows.  Four CTAs of the split pass fit an SM (with the 168 registers it would
-// take it is three: 512 groups of 32 tokens complete 35 us, now 28).
+// at 16 sequences x 1 head, 20 -> 10 us at 575 rows.  Four CTAs of the split pass fit an SM (it would
+// take 168 registers, which is three).
 // In a decode step most launches complete a few groups, and those are the end of the launch: a group's CTAs are long chains
 // with a warp per scheduler (256 rows x 8 heads: 3.9 us without the groups, 10.3 with them alone).  So they go first, with half the tokens per lane while the CTAs suffice for that,
 // and on a bounded number of CTAs (a captured step of 256 rows launched 1,024 for its 8 groups).  From the write to the layer's
 // split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 7.0 -> 5.9 us, 256 x 8, groups of 32 13.4 -> 6.2,
 // 16 x 1 6.5 -> 5.3, 48 x 2 8.1 -> 5.6; a launch of empty CTAs takes 1.1.
+// Sequences in lock step (equal prompts) complete their groups together, once every KG steps.  Then there are several times as many
+// pieces as CTAs were launched for groups: the CTAs of the first rows join in behind their row, up to as many workers as the chip
+// holds, and every worker takes one run of consecutive pieces.  us a layer, 8 heads x 128, all groups complete, with a
+// group per CTA of the bounded number / with 1,024 CTAs for the groups alone / now: 128 rows, groups of 32 12.1 / 10.9 / 9.5; 256 rows
+// 25.8 / 18.2 / 15.4; 300 rows 35.5 / 22.1 / 18.4; 512 rows 44 / 32 / 28; 512 rows, groups of 16 23.4 / 19.1 / 16.0, of 64 67 / 51 / 43.
+// Equal single pieces taken in turn instead of runs: 27.9 at 256 rows without the rows' CTAs, 18.0 with them.  More CTAs launched for
+// groups would do it too, but cost the steps that complete few or none (64 rows 2.8 -> 3.5 us); that the rows' CTAs look at the
+// count costs 0.1 us there at 128 to 256 rows.
 // SPLIT_KG: tokens of a group that is spread over lanes and CTAs (finalize_split), 0: a thread walks a group's tokens.  One group
 // size per instance, to keep the code short.
 template <typename T, int SPLIT_KG>
 __global__ void __launch_bounds__(WT_WARPS * 32, SPLIT_KG ? 4 : (sizeof(T) == 2 ? 7 : 6))
-write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, int64_t n_fin_ctas, const StashArgs SA) {
+write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, const GroupCtas G, const StashArgs SA) {
   __shared__ int take[STEP_MAX_ROWS];
   __shared__ int n_take;
   pdl_launch_dependents();
   const LayoutDev& L = TA.L;
-  const int64_t b = blockIdx.x, row = b - n_fin_ctas;
+  const int64_t b = blockIdx.x, row = b - G.ctas;
   const int w = 3 + L.KG;
   pdl_wait();
   if (row >= 0 && row < TA.n_rows) {  // ahead of the group passes' long code, which is fetched anew in every launch: 0.7 us at one sequence
     const int64_t n_fin = n_fin_launch > 0 ? min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
-    if (TA.tok[row] < 0) return;  // padding, or a token that is not stored
-    RowRaw raw;
-    raw.load<T>(TA, row);
-    const RowMeta M = row_meta<T>(TA, row);
-    int hit = 0;
-    if (M.rslot >= 0)
-      for (int64_t f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[f * w + 2] == M.rslot;
-    token_row<T, 2>(TA, row, M, raw, [&] { return M.rslot >= 0 && __syncthreads_or(hit) != 0; });
-    return;
+    const bool help = SPLIT_KG != 0 && n_fin > G.enough && b < G.workers;
+    if (TA.tok[row] >= 0) {  // not padding, nor a token that is not stored
+      RowRaw raw;
+      raw.load<T>(TA, row);
+      const RowMeta M = row_meta<T>(TA, row);
+      int hit = 0;
+      if (M.rslot >= 0)
+        for (int64_t f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[f * w + 2] == M.rslot;
+      token_row<T, 2>(TA, row, M, raw, [&] { return M.rslot >= 0 && __syncthreads_or(hit) != 0; });
+    }
+    if (!help) return;
   }
   if (row >= TA.n_rows) {
     const int64_t i = (row - TA.n_rows) * blockDim.x + threadIdx.x;
@@ -857,13 +875,20 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
   }
   if constexpr (SPLIT_KG != 0) {
     const int64_t count = min(*FA.fin_count, n_fin_launch);
-    const int fine = split_need(L, true);
+    const int fine = split_need(L, true), need = split_need(L, false);
     const SplitArgs<T> S = {&n_take, take, &TA};
-    if (count * fine <= n_fin_ctas) {  // a piece is a chain of a warp or two per scheduler: the shorter, the better
-      if (b < count * fine) finalize_split_kg<T, SPLIT_KG, true>(FA, b / fine, (int)(b % fine), fine, S);
-    } else {
-      const int parts = (int)max((int64_t)1, min((int64_t)split_need(L, false), n_fin_ctas / count));
-      for (int64_t g = b; g < count * parts; g += n_fin_ctas) finalize_split_kg<T, SPLIT_KG, false>(FA, g / parts, (int)(g % parts), parts, S);
+    if (count * fine <= G.ctas) {  // a piece is a chain of a warp or two per scheduler: the shorter, the better
+      if (b < count * fine) finalize_split_kg<T, SPLIT_KG, true>(FA, b / fine, (int)(b % fine), (int)(b % fine) + 1, S);
+      return;
+    }
+    // A run of consecutive pieces for every worker, one more for the first few; pieces of one group share what is looked up for it.
+    const int workers = count > G.enough ? G.workers : G.ctas, pieces = (int)count * need;
+    const int share = pieces / workers, more = pieces % workers;
+    int at = (int)b * share + min((int)b, more);
+    for (const int end = at + share + ((int)b < more); at < end;) {
+      const int f = at / need, first = at - f * need, last = min(need, first + end - at);
+      finalize_split_kg<T, SPLIT_KG, false>(FA, f, first, last, S);
+      at += last - first;
     }
     return;
   }
@@ -959,11 +984,12 @@ using namespace echokv;
 
 template <typename T, int SPLIT_KG>
 static void launch_write_split(bool first, int64_t rest, cudaStream_t st, const TokArgs<T>& TA, const FinArgs<T>& FA, int64_t n_fin, const StashArgs& SA) {
-  // A captured step launches room for a group per row, and nearly all of it has nothing to do: the pieces go round on no more
-  // CTAs than fit the chip beside the rows'.
+  // A captured step launches room for a group per row, and nearly all of it has nothing to do: no more CTAs than fit the chip beside
+  // the rows', but half the chip's in any case.
   const int64_t room = std::max<int64_t>(STEP_GROUP_CTAS - rest, STEP_GROUP_CTAS / 2);
   const int64_t ctas = std::min(n_fin * split_need(TA.L, true), room);
-  launch_after(!first, write_step_kernel<T, SPLIT_KG>, dim3((unsigned)(ctas + rest)), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, ctas, SA);
+  const GroupCtas G = {(int)ctas, (int)(ctas / split_need(TA.L, false)), (int)std::max(ctas, std::min(ctas + TA.n_rows, STEP_GROUP_CTAS))};
+  launch_after(!first, write_step_kernel<T, SPLIT_KG>, dim3((unsigned)(ctas + rest)), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, G, SA);
 }
 template <typename T>
 static void launch_write_step(bool first, bool split, int64_t rest, cudaStream_t st, const TokArgs<T>& TA, const FinArgs<T>& FA,
@@ -976,7 +1002,7 @@ static void launch_write_step(bool first, bool split, int64_t rest, cudaStream_t
       return;
     }
   }
-  launch_after(!first, write_step_kernel<T, 0>, dim3((unsigned)(n_fin + rest)), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, n_fin, SA);
+  launch_after(!first, write_step_kernel<T, 0>, dim3((unsigned)(n_fin + rest)), dim3(WT_WARPS * 32), 0, st, TA, FA, n_fin, GroupCtas{(int)n_fin, 0, 0}, SA);
 }
 
 extern "C" {
