@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(W == 8 ? 256 : 128, W == 1 ? (FEW ? 8 : 5) : 1
   for (int s0 = MERGE_ROUND; s0 < used; s0 += 32)
     if (s0 + lane < used) m = fmaxf(m, A.ml[(base + s0 + lane) * 2]);
   m = warp_max(m);  // the overall maximum
-  float lt = 0.f, sum[VEC];
+  __align__(16) float sum[VEC];
+  float lt = 0.f;
   if constexpr (FEW) {
     const float w = lane < used ? exp2f(ml[0].x - m) : 0.f;
     lt = lane < used ? ml[0].y * w : 0.f;
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(W == 8 ? 256 : 128, W == 1 ? (FEW ? 8 : 5) : 1
     *reinterpret_cast<V*>(&part[warp][lane * VEC]) = *reinterpret_cast<const V*>(sum);
     __syncthreads();
     if (me != 0) return;
-    float t[W][VEC];
+    __align__(16) float t[W][VEC];
 #pragma unroll
     for (int i = 0; i < W; ++i) *reinterpret_cast<V*>(t[i]) = *reinterpret_cast<const V*>(&part[warp + i][lane * VEC]);
 #pragma unroll
