@@ -20,6 +20,11 @@ EAGER_MAX_SPLITS = 32   # calls that size their own grid (the prefill row path):
 # splits of a step that leaves the chip idle shortens it: 1 x 500 tokens x 32 layers 0.519 -> 0.444 ms, 4 x 678 in blocks of 32
 # 0.561 -> 0.546; larger steps choose the sizes they chose with 64.
 MIN_SPLIT_TOKENS = 32
+# The scratch of a runner grows with its split grid, which is fixed: one for models of 2,048 tokens in blocks of 16 that allows splits
+# of 32 tokens everywhere would take 273 MB at 256 sequences x 32 heads x 128, twice that of splits of 64, for batches that fill the
+# chip with far fewer splits.  So only a runner whose batches are small gets it (64 sequences of the same: 68 MB with 64 splits, 18 MB
+# for 528 tokens); the others still cut sequences of up to half their longest into splits of 32 tokens.
+GRID_SPLIT_TOKENS, FINE_GRID_BYTES = 64, 72 << 20
 # Split size of a step whose shape takes the CUDA-core kernel: a CTA's four warps take a block each, and a batch that leaves the chip
 # idle wants more CTAs.  8 heads of 64 channels, blocks of 32, ms a step with 16 and with 4 blocks: 1 x 6,000 tokens 0.341 -> 0.172,
 # 4 x 900 0.344 -> 0.191, 32 x 1,500 0.623 -> 0.576, 128 x 700 0.530 -> 0.523, 8 x 12,000 0.525 -> 0.527; in blocks of 16 4 blocks are too
@@ -32,6 +37,17 @@ ITEM_COST_TILES = 4     # fixed cost of a (sequence, split) work item in units o
 def decode_parallelism(store, num_q_heads: int) -> int:
     """Work items the split kernel has in work at once on the current device (0: generic kernel)."""
     return int(N.lib.echokv_decode_parallelism(store.c_layout, int(num_q_heads)))
+
+
+def split_grid(max_model_len: int, block_size: int, split_bytes: int, slots: int) -> int:
+    """Splits of the fixed split grid of a runner whose largest batch writes ``split_bytes`` of partials per split.
+
+    ``slots``: ``decode_parallelism``.  Where the tensor-core kernel runs the grid allows splits of ``MIN_SPLIT_TOKENS`` for sequences
+    of ``max_model_len``, as long as its scratch stays within ``FINE_GRID_BYTES``; otherwise splits of ``GRID_SPLIT_TOKENS``."""
+    blocks = -(-max_model_len // block_size)
+    fine, coarse = (max(1, min(-(-blocks // max(1, tokens // block_size)), MAX_DECODE_SPLITS))
+                    for tokens in (MIN_SPLIT_TOKENS, GRID_SPLIT_TOKENS))
+    return fine if slots and fine * split_bytes <= FINE_GRID_BYTES else coarse
 
 
 def generic_blocks_per_split(block_size: int) -> int:

@@ -25,8 +25,8 @@ from echokv_b200 import _native as N
 from echokv_b200.canary import canary_kl_ring, tp_mean
 from echokv_b200.controller import LayerController
 from echokv_b200.quant import SUPPORTED_BITS
-from echokv_b200.kernels.decode import (BLOCKS_PER_SPLIT, MAX_DECODE_SPLITS, MIN_SPLIT_TOKENS, choose_blocks_per_split,
-                                        decode_attention, decode_parallelism, generic_blocks_per_split)
+from echokv_b200.kernels.decode import (BLOCKS_PER_SPLIT, MIN_SPLIT_TOKENS, choose_blocks_per_split, decode_attention,
+                                        decode_parallelism, generic_blocks_per_split, split_grid)
 from echokv_b200.kernels.write import gather_rows
 from echokv_b200.tiered_cache import TieredKVCache, TieredLayout
 from echokv_b200.write_plan import SharedState, WriteMeta
@@ -181,11 +181,11 @@ class GroupRunner:
         self.staging = Staging(cap, canary_max_q, 3 + g, tail, dev)
         # The split grid is fixed (a graph replays it); how many of its splits a step uses follows from the
         # blocks per split chosen for that step in `plan_step`, never less than `split_floor` blocks.
-        max_blocks = -(-max_model_len // layout.block_size)
         self.split_floor = max(1, MIN_SPLIT_TOKENS // layout.block_size)
-        self.num_splits = max(1, min(-(-max_blocks // self.split_floor), MAX_DECODE_SPLITS))
         with torch.cuda.device(dev):
             self.decode_slots = decode_parallelism(self.stores[0], num_q_heads)
+        self.num_splits = split_grid(max_model_len, layout.block_size,
+                                     N.lib.echokv_decode_scratch_bytes(cap, num_q_heads, layout.head_size, 1), self.decode_slots)
 
     # -- host side, once per step ---------------------------------------------------------
     def plan_step(self, slots_cpu, decode=None, canary: np.ndarray | None = None) -> StepMeta:

@@ -30,3 +30,19 @@ def test_split_sizes_of_the_cuda_core_kernel(block_size, blocks):
     from echokv_b200.kernels.decode import generic_blocks_per_split
 
     assert generic_blocks_per_split(block_size) == blocks
+
+
+def test_the_split_grid_of_short_models_is_fine_only_where_its_scratch_is_small():
+    """2,048 tokens in blocks of 16, 32 heads of 128: a runner of 256 sequences keeps the 136 MB of splits of 64 tokens, one of 64
+    sequences has splits of 32 throughout; the CUDA-core kernel never cuts so fine."""
+    from echokv_b200.kernels.decode import FINE_GRID_BYTES, split_grid
+
+    row = 32 * (128 + 2) * 4
+    assert split_grid(2048, 16, 256 * row, 296) == 32 and 32 * 256 * row < 137 << 20
+    assert split_grid(2048, 16, 64 * row, 296) == 64 and 64 * 64 * row <= FINE_GRID_BYTES
+    assert split_grid(2048, 16, 64 * row, 0) == 32
+    assert split_grid(528, 16, 64 * row, 296) == 17 and split_grid(528, 16, 512 * row, 296) == 9
+    for slots in (0, 296):  # blocks of 64 tokens and more, and long models: one answer
+        assert split_grid(2048, 64, row, slots) == split_grid(2048, 64, 512 * row, slots) == 32
+        assert split_grid(100000, 16, row, slots) == split_grid(100000, 16, 512 * row, slots) == 64
+        assert split_grid(1, 16, row, slots) == 1
