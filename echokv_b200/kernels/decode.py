@@ -30,6 +30,13 @@ GRID_SPLIT_TOKENS, FINE_GRID_BYTES = 64, 72 << 20
 # 4 x 900 0.344 -> 0.191, 32 x 1,500 0.623 -> 0.576, 128 x 700 0.530 -> 0.523, 8 x 12,000 0.525 -> 0.527; in blocks of 16 4 blocks are too
 # few (32 x 1,500: 0.773 with 16, 0.690 with 8, 0.724 with 4), in blocks of 64 2 are (0.575, 0.584 with 4, 0.755 with 2).
 GENERIC_SPLIT_BLOCKS, GENERIC_SPLIT_TOKENS = 4, 128
+# A batch that fills the chip many times over only pays for finer splits, in partials written and read again: from so many CTAs
+# times query heads per KV head on they have twice the tokens, and in blocks of up to 32 BLOCKS_PER_SPLIT blocks where more than
+# eight heads' partials are as long as the pages they come from.  us a layer at 128 / 256 / 512 tokens: 256 x 900, 8 heads of 64, 4 query
+# heads each, blocks of 16 342 / 328 / 348, of 32 269 / 257 / 268; 128 x 700 of the same 139 / 142 / 150, 118 / 118 / 119; 16 query heads each of
+# 128 channels, blocks of 32, 128 x 700 565 / 525 / 507, 8 x 3,000 116 / 106 / 124 and, one KV head, 32 x 1,500 44 / 50 / 74; in blocks of
+# 64 32 x 1,500 - / 282 / 295, 128 x 700 - / 547 / 533.
+GENERIC_MANY, GENERIC_MANY_TOKENS = 12000, 256
 MMA_COLUMNS = 8         # columns of the split kernel's MMAs: query heads of a token, or of consecutive tokens of a chunk
 ITEM_COST_TILES = 4     # fixed cost of a (sequence, split) work item in units of one 16-token tile's work
 
@@ -50,9 +57,19 @@ def split_grid(max_model_len: int, block_size: int, split_bytes: int, slots: int
     return fine if slots and fine * split_bytes <= FINE_GRID_BYTES else coarse
 
 
-def generic_blocks_per_split(block_size: int) -> int:
-    """Blocks per split for a step on the CUDA-core kernel, whatever the lengths."""
-    return max(GENERIC_SPLIT_BLOCKS, GENERIC_SPLIT_TOKENS // block_size)
+def generic_blocks_per_split(block_size: int, lens=None, num_splits: int = MAX_DECODE_SPLITS, num_kv_heads: int = 1, gqa: int = 1) -> int:
+    """Blocks per split for a step on the CUDA-core kernel: the smallest, or those for sequences of cache lengths ``lens``."""
+    b = max(GENERIC_SPLIT_BLOCKS, GENERIC_SPLIT_TOKENS // block_size)
+    if lens is None:
+        return b
+    blocks = -(-np.asarray(lens) // block_size)
+    # The kernel itself would fit longer sequences into the grid with splits of any number of blocks, five of which keep four warps busy
+    # as long as eight: 16 x 12,000, 2 heads of 64, 8 query heads each, blocks of 32 100 us a layer with 3 to 6 blocks, 74 with 8.
+    longest = -(-int(blocks.max(initial=0)) // num_splits)
+    b = max(b, -(-longest // GENERIC_SPLIT_BLOCKS) * GENERIC_SPLIT_BLOCKS)
+    if num_kv_heads * gqa * int((-(-blocks // b)).sum()) < GENERIC_MANY:
+        return b
+    return max(b, BLOCKS_PER_SPLIT if gqa > MMA_COLUMNS and block_size <= 32 else GENERIC_MANY_TOKENS // block_size)
 
 
 def choose_blocks_per_split(lens, block_size: int, num_splits: int, slots: int) -> int:

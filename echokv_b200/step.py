@@ -216,7 +216,8 @@ class GroupRunner:
         bps = BLOCKS_PER_SPLIT
         if dec[2].size:
             bps = (choose_blocks_per_split(dec[2], self.layout.block_size, self.num_splits, self.decode_slots) if self.decode_slots
-                   else generic_blocks_per_split(self.layout.block_size))
+                   else generic_blocks_per_split(self.layout.block_size, dec[2], self.num_splits, self.layout.num_kv_heads,
+                                                 self.num_q_heads // self.layout.num_kv_heads))
         fin_count, canary_rows, dviews, tok, fin, views, bps_dev = self.staging.stage(
             plan.n_fin, can, dec, (plan.tok_slot, plan.tok_res, plan.tok_sealed, plan.tok_kref), plan.fin, tail, bps)
         shared.apply_res_map(*views[:4])

@@ -46,3 +46,20 @@ def test_the_split_grid_of_short_models_is_fine_only_where_its_scratch_is_small(
         assert split_grid(2048, 64, row, slots) == split_grid(2048, 64, 512 * row, slots) == 32
         assert split_grid(100000, 16, row, slots) == split_grid(100000, 16, 512 * row, slots) == 64
         assert split_grid(1, 16, row, slots) == 1
+
+
+def test_split_sizes_of_the_cuda_core_kernel_follow_the_batch():
+    """Whole rounds of a CTA's four warps for sequences that need the whole grid; twice the tokens, and for wide query groups 16
+    blocks, where the batch fills the chip many times over."""
+    from echokv_b200.kernels.decode import generic_blocks_per_split as size
+
+    assert [size(bs, np.array([500]), 64, 8, 4) for bs in (16, 32, 48, 64, 256)] == [8, 4, 4, 4, 4]
+    assert size(32, np.full(16, 12000), 64, 2, 1) == 8 and size(16, np.full(3, 20000), 64, 1, 1) == 20 and size(16, np.array([20001]), 64, 1, 1) == 20
+    assert size(16, np.array([500, 0, 0]), 2, 1, 1) == 16 and size(16, np.zeros(4, dtype=np.int64), 64, 8, 16) == 8
+    assert size(32, np.full(256, 900), 64, 8, 4) == 8 and size(16, np.full(256, 900), 64, 8, 4) == 16
+    assert size(32, np.full(128, 700), 64, 8, 16) == 16 and size(16, np.full(8, 3000), 64, 8, 16) == 16 and size(64, np.full(128, 700), 64, 8, 16) == 4
+    assert size(32, np.full(32, 1500), 64, 1, 16) == 4
+    for gqa in (1, 4, 8, 16):  # any length fits the grid
+        for top in (1, 63, 64, 65, 4097, 100000):
+            for splits in (1, 3, 64):
+                assert size(16, np.array([top, 1]), splits, 8, gqa) * splits * 16 >= top
