@@ -97,7 +97,7 @@ def choose_blocks_per_split(lens, block_size: int, num_splits: int, slots: int) 
     return int(b[cost == cost.min()].max())
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=16)
 def _split_counts(num_splits: int):
     """1 .. num_splits, read-only."""
     counts = np.arange(1, max(1, num_splits) + 1)
