@@ -83,6 +83,87 @@ def test_split_kernel_waits_first_unless_the_step_was_planned():
     assert "if (warp != H) pdl_wait();" in ahead
 
 
+def test_merge_waits_first_unless_the_step_was_planned():
+    """Of the step's metadata, which one function reads, the merge sees nothing ahead of its wait unless the step was planned; the splits'
+    partials, its item counter and the output row are touched behind the wait."""
+    body = _body("decode.cu", "decode_merge_kernel")
+    ahead, behind = body.split("pdl_wait();", 1)
+    plan = ahead[ahead.index("auto plan = [&]()"): ahead.index("};")]
+    metadata, results = r"A\.(lens|q_rows|bps_dev)\b|bps_floor", r"A\.(ml|acc|state|out)\["
+    assert re.search(metadata, plan) and not re.search(metadata, ahead.replace(plan, "")) and not re.search(metadata, behind)
+    assert re.findall(r".*plan\(\);", ahead.replace(plan, "")) == ["  if (A.planned) plan();"]
+    assert re.findall(r".*plan\(\);", behind) == ["  if (W == 1 && !A.planned) plan();", "  if (W > 1 && !A.planned) plan();"]
+    assert not re.search(results, ahead)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n", [2, 60, 150, 400])
+def test_merges_of_planned_steps(n, d):
+    """Steps of 2 to 400 sequences of eight query heads over a grid of 64 splits, all the numbers of warps a head, padding rows among them:
+    eager and as one replayed graph whose lengths, rows and split sizes change, the bits of a decode that plans nothing."""
+    import torch
+    from echokv_b200.controller import ControllerParams, LayerController
+    from echokv_b200.kernels.decode import decode_attention
+    from echokv_b200.step import GroupRunner
+    from echokv_b200.tiered_cache import TieredLayout
+
+    h, bs, layers, held = 2, 16, 2, 4  # four sequences are stored, the step's read them over and over
+    layout = TieredLayout(num_kv_heads=h, head_size=d, block_size=bs, mem_bits=8, k_group=16, v_group=32)
+    per = 4096 // bs
+    caches = [torch.zeros(held * per + n, layout.page_bytes, dtype=torch.uint8, device="cuda") for _ in range(layers)]
+    runner = GroupRunner(layout, caches, 4 * h, d ** -0.5, [LayerController(ControllerParams(fixed_bits=b)) for b in (4, 8)],
+                         residual_slots=n + held, model_dtype=torch.bfloat16, cap=512, max_model_len=4096)
+    assert runner.num_splits == 64
+    gen = torch.Generator(device="cuda").manual_seed(n + d)
+    draw = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).bfloat16()
+    for at in range(0, held * 4096, 8192):
+        meta = runner.plan_step(np.arange(at, at + 8192))
+        for i in range(layers):
+            runner.write(i, draw(8192, h, d), draw(8192, h, d), meta)
+    table = torch.arange(held * per, device="cuda", dtype=torch.int32).view(held, per)
+    kv, q, out = draw(2, layers, n, h, d), draw(layers, n, 4 * h, d), torch.zeros(layers, n, 4 * h, d, device="cuda")
+    own = held * 4096 + np.arange(n) * bs  # the tokens that the step itself stores, in blocks of their own
+    rng = np.random.default_rng(n)
+
+    def plan(step):
+        top = (4096, 1000, 150, 20)[step % 4]
+        lens = np.maximum(1, (top * rng.random(n)).astype(np.int64))
+        lens[0], lens[1:: 7] = top, 0
+        rows = rng.permutation(n)
+        return runner.plan_step(own + step % bs, decode=(rows, rng.integers(0, held, n), lens)), lens
+
+    def layers_of(meta, capturing):
+        for i in range(layers):
+            runner.write(i, kv[0, i], kv[1, i], meta, capturing=capturing)
+            runner.decode(i, q[i], table, out[i], meta)
+
+    graph, sizes, used = None, set(), set()
+    for step in range(16):
+        meta, lens = plan(step)
+        if step == 8:
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                layers_of(meta, True)
+        out.fill_(7.0)
+        if graph is None:
+            layers_of(meta, False)
+            assert meta.write.launched
+        else:
+            graph.replay()
+        size = int(meta.bps_dev[0])
+        sizes.add(size)
+        used.update(-(-(-(-lens // bs)) // max(size, runner.split_floor)))
+        for i in range(layers):
+            want = torch.full_like(out[i], 7.0)
+            decode_attention(runner.stores[i], q[i], table, meta.decode_lens, d ** -0.5, runner.split_floor, q_rows=meta.decode_rows,
+                             bt_rows=meta.decode_reqs, out=want, num_splits=64, bps_dev=meta.bps_dev)
+            assert torch.equal(out[i], want)
+            assert bool((out[i][meta.decode_rows[torch.from_numpy(lens == 0).cuda()]] == 7.0).all())
+    assert len(used) > 3 and (d == 64 or len(sizes) > 1)  # the CUDA-core kernel has one size here
+
+
 @pytest.mark.gpu
 def test_metadata_written_by_the_kernel_right_before():
     """Lengths, rows, tables and split sizes that a kernel just produced, or that the call itself converts, give the bits of
