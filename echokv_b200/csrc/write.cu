@@ -841,7 +841,10 @@ struct GroupCtas {
 // groups would do it too, but cost the steps that complete few or none (64 rows 2.8 -> 3.5 us); that the rows' CTAs look at the
 // count costs 0.1 us there at 128 to 256 rows.
 // SPLIT_KG: tokens of a group that is spread over lanes and CTAs (finalize_split), 0: a thread walks a group's tokens.  One group
-// size per instance, to keep the code short.
+// size per instance, to keep the code short.  Without the spread the groups' CTAs are one per row of a captured step, nearly all of them with
+// nothing to do, and in front of the rows they held these up: us a layer with the groups / the rows first, 1,000 rows x 8 heads, groups
+// of 32, none complete 4.9 / 4.4, 62 27.4 / 25.6, all 47.8 / 48.7; 256 rows in blocks of 48 with groups of 48, 8 complete 27.7 / 25.4, all
+// 40.8 / 38.7; 600 rows, groups of 32, 37 complete 20.0 / 22.2, all 36.0 / 38.0.
 template <typename T, int SPLIT_KG>
 __global__ void __launch_bounds__(WT_WARPS * 32, SPLIT_KG ? 4 : (sizeof(T) == 2 ? 7 : 6))
 write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch, const GroupCtas G, const StashArgs SA) {
@@ -849,7 +852,9 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
   __shared__ int n_take;
   pdl_launch_dependents();
   const LayoutDev& L = TA.L;
-  const int64_t b = blockIdx.x, row = b - G.ctas;
+  // This CTA's place among the groups' and among the rows' CTAs (from n_rows on: copies).  Groups that are not spread come behind the rows.
+  const int64_t b = SPLIT_KG ? (int64_t)blockIdx.x : blockIdx.x - TA.n_rows;
+  const int64_t row = SPLIT_KG ? b - G.ctas : (b < 0 ? (int64_t)blockIdx.x : (b < G.ctas ? -1 : blockIdx.x - (int64_t)G.ctas));
   const int w = 3 + L.KG;
   pdl_wait();
   if (row >= 0 && row < TA.n_rows) {  // ahead of the group passes' long code, which is fetched anew in every launch: 0.7 us at one sequence
