@@ -839,7 +839,7 @@ struct GroupCtas {
 // 25.8 / 18.2 / 15.4; 300 rows 35.5 / 22.1 / 18.4; 512 rows 44 / 32 / 28; 512 rows, groups of 16 23.4 / 19.1 / 16.0, of 64 67 / 51 / 43.
 // Equal single pieces taken in turn instead of runs: 27.9 at 256 rows without the rows' CTAs, 18.0 with them.  More CTAs launched for
 // groups would do it too, but cost the steps that complete few or none (64 rows 2.8 -> 3.5 us); that the rows' CTAs look at the
-// count costs 0.1 us there at 128 to 256 rows.
+// count costs these nothing (0.1 us with the count in 64 bits).
 // SPLIT_KG: tokens of a group that is spread over lanes and CTAs (finalize_split), 0: a thread walks a group's tokens.  One group
 // size per instance, to keep the code short.  Without the spread the groups' CTAs are one per row of a captured step, nearly all of them with
 // nothing to do, and in front of the rows they held these up: us a layer with the groups / the rows first, 1,000 rows x 8 heads, groups
@@ -858,7 +858,7 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
   const int w = 3 + L.KG;
   pdl_wait();
   if (row >= 0 && row < TA.n_rows) {  // ahead of the group passes' long code, which is fetched anew in every launch: 0.7 us at one sequence
-    const int64_t n_fin = n_fin_launch > 0 ? min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
+    const int n_fin = n_fin_launch > 0 ? (int)min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
     const bool help = SPLIT_KG != 0 && n_fin > G.enough && b < G.workers;
     if (TA.tok[row] >= 0) {  // not padding, nor a token that is not stored
       RowRaw raw;
@@ -866,7 +866,7 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
       const RowMeta M = row_meta<T>(TA, row);
       int hit = 0;
       if (M.rslot >= 0)
-        for (int64_t f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[f * w + 2] == M.rslot;
+        for (int f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[(int64_t)f * w + 2] == M.rslot;
       token_row<T, 2>(TA, row, M, raw, [&] { return M.rslot >= 0 && __syncthreads_or(hit) != 0; });
     }
     if (!help) return;
