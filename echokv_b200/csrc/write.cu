@@ -830,8 +830,8 @@ struct GroupCtas {
 // In a decode step most launches complete a few groups, and those are the end of the launch: a group's CTAs are long chains
 // with a warp per scheduler (256 rows x 8 heads: 3.9 us without the groups, 10.3 with them alone).  So they go first, with half the tokens per lane while the CTAs suffice for that,
 // and on a bounded number of CTAs (a captured step of 256 rows launched 1,024 for its 8 groups).  From the write to the layer's
-// split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 7.0 -> 5.9 us, 256 x 8, groups of 32 13.4 -> 6.2,
-// 16 x 1 6.5 -> 5.3, 48 x 2 8.1 -> 5.6; a launch of empty CTAs takes 1.1.
+// split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 6.9 -> 5.5 us, 256 x 8, groups of 32 13.4 -> 6.5,
+// 16 x 1 6.5 -> 5.2, 48 x 2 8.1 -> 5.3; a launch of empty CTAs takes 1.1.
 // Sequences in lock step (equal prompts) complete their groups together, once every KG steps.  Then there are several times as many
 // pieces as CTAs were launched for groups: the CTAs of the first rows join in behind their row, up to as many workers as the chip
 // holds, and every worker takes one run of consecutive pieces.  us a layer, 8 heads x 128, all groups complete, with a
