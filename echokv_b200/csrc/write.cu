@@ -853,12 +853,16 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
   pdl_launch_dependents();
   const LayoutDev& L = TA.L;
   // This CTA's place among the groups' and among the rows' CTAs (from n_rows on: copies).  Groups that are not spread come behind the rows.
-  const int64_t b = SPLIT_KG ? (int64_t)blockIdx.x : blockIdx.x - TA.n_rows;
-  const int64_t row = SPLIT_KG ? b - G.ctas : (b < 0 ? (int64_t)blockIdx.x : (b < G.ctas ? -1 : blockIdx.x - (int64_t)G.ctas));
+  // In 64 bits the instances with the spread are 0.1 to 0.7 us a layer slower (16 sequences x 1 KV head: 4.4 -> 5.1, from the write to the
+  // split kernel); without it 32 bits are (1,000 rows x 8 heads, 62 groups of 32 complete: 25.8 -> 32.4).
+  using Place = typename std::conditional<SPLIT_KG != 0, int, int64_t>::type;
+  const Place cta = blockIdx.x, n_rows = (Place)TA.n_rows;
+  const Place b = SPLIT_KG ? cta : cta - n_rows;
+  const Place row = SPLIT_KG ? b - G.ctas : (b < 0 ? cta : (b < G.ctas ? -1 : cta - G.ctas));
   const int w = 3 + L.KG;
   pdl_wait();
-  if (row >= 0 && row < TA.n_rows) {  // ahead of the group passes' long code, which is fetched anew in every launch: 0.7 us at one sequence
-    const int n_fin = n_fin_launch > 0 ? (int)min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
+  if (row >= 0 && row < n_rows) {  // ahead of the group passes' long code, which is fetched anew in every launch: 0.7 us at one sequence
+    const Place n_fin = n_fin_launch > 0 ? (Place)min(*FA.fin_count, n_fin_launch) : 0;  // no list, no pointer
     const bool help = SPLIT_KG != 0 && n_fin > G.enough && b < G.workers;
     if (TA.tok[row] >= 0) {  // not padding, nor a token that is not stored
       RowRaw raw;
@@ -866,31 +870,31 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
       const RowMeta M = row_meta<T>(TA, row);
       int hit = 0;
       if (M.rslot >= 0)
-        for (int f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[(int64_t)f * w + 2] == M.rslot;
+        for (Place f = threadIdx.x; f < n_fin; f += blockDim.x) hit |= FA.fin[(int64_t)f * w + 2] == M.rslot;
       token_row<T, 2>(TA, row, M, raw, [&] { return M.rslot >= 0 && __syncthreads_or(hit) != 0; });
     }
     if (!help) return;
   }
-  if (row >= TA.n_rows) {
-    const int64_t i = (row - TA.n_rows) * blockDim.x + threadIdx.x;
+  if (row >= n_rows) {
+    const int64_t i = (int64_t)(row - n_rows) * blockDim.x + threadIdx.x;
     if (i >= SA.n * SA.row16) return;
     const int64_t r = i / SA.row16;
     SA.dst[i] = SA.src[SA.rows[r] * SA.src_stride16 + (i - r * SA.row16)];
     return;
   }
   if constexpr (SPLIT_KG != 0) {
-    const int64_t count = min(*FA.fin_count, n_fin_launch);
+    const int count = (int)min(*FA.fin_count, n_fin_launch);
     const int fine = split_need(L, true), need = split_need(L, false);
     const SplitArgs<T> S = {&n_take, take, &TA};
     if (count * fine <= G.ctas) {  // a piece is a chain of a warp or two per scheduler: the shorter, the better
-      if (b < count * fine) finalize_split_kg<T, SPLIT_KG, true>(FA, b / fine, (int)(b % fine), (int)(b % fine) + 1, S);
+      if (b < count * fine) finalize_split_kg<T, SPLIT_KG, true>(FA, b / fine, b % fine, b % fine + 1, S);
       return;
     }
     // A run of consecutive pieces for every worker, one more for the first few; pieces of one group share what is looked up for it.
-    const int workers = count > G.enough ? G.workers : G.ctas, pieces = (int)count * need;
+    const int workers = count > G.enough ? G.workers : G.ctas, pieces = count * need;
     const int share = pieces / workers, more = pieces % workers;
-    int at = (int)b * share + min((int)b, more);
-    for (const int end = at + share + ((int)b < more); at < end;) {
+    int at = b * share + min(b, more);
+    for (const int end = at + share + (b < more); at < end;) {
       const int f = at / need, first = at - f * need, last = min(need, first + end - at);
       finalize_split_kg<T, SPLIT_KG, false>(FA, f, first, last, S);
       at += last - first;
@@ -898,7 +902,7 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
     return;
   }
   if (b >= *FA.fin_count) return;
-  const int64_t slot = FA.fin[b * w + 2];
+  const int64_t slot = FA.fin[(int64_t)b * w + 2];
   find_takers<T>(TA, slot, &n_take, take);
   finalize_group<T, false>(FA, b);
   // Keys of the group that takes the slot over: each thread stores the channels it has just read for the last time.
