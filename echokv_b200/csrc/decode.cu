@@ -20,8 +20,8 @@ int prefill_status_take(bool clear);
 //
 // Bound by its latency (split partials just written sit in L2): launch, the rounds of loads, the sum.  With a warp per head
 // 64 splits were eight rounds of loads one after the other, of more than a microsecond each.  From the merge to the next
-// layer's write in a decode step, a warp per head throughout and now: 8 sequences x 32 heads, 33 splits 7.0 -> 2.6 us;
-// 16 x 8, 62 splits 12.7 -> 3.0; 48 x 16, 11 splits 6.3 -> 3.5; 64 x 32, 9 splits 5.1 -> 3.7; 256 x 32, 1 or 2 splits 7.1 -> 6.8.
+// layer's write in a decode step, a warp per head throughout and now: 8 sequences x 32 heads, 33 splits 7.0 -> 2.7 us;
+// 16 x 8, 62 splits 12.7 -> 3.1; 48 x 16, 11 splits 6.3 -> 3.5; 64 x 32, 9 splits 5.1 -> 3.7; 256 x 32, 1 or 2 splits 7.1 -> 6.8.
 // W is the largest with heads x W <= MERGE_WARPS (16 warps an SM) that leaves a warp more than two of the splits there may be:
 // 48 x 16 heads take 3.6 us at W = 2 and 5.0 at 4, 64 x 32 take 3.6 at 1 and 4.8 at 2.
 // The rule sees the grid, not the splits in use: a layer's step of two sequences x 32 heads in blocks of 64 takes 18.9 us at 3,000 tokens

@@ -830,8 +830,8 @@ struct GroupCtas {
 // In a decode step most launches complete a few groups, and those are the end of the launch: a group's CTAs are long chains
 // with a warp per scheduler (256 rows x 8 heads: 3.9 us without the groups, 10.3 with them alone).  So they go first, with half the tokens per lane while the CTAs suffice for that,
 // and on a bounded number of CTAs (a captured step of 256 rows launched 1,024 for its 8 groups).  From the write to the layer's
-// split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 6.9 -> 5.5 us, 256 x 8, groups of 32 13.4 -> 6.5,
-// 16 x 1 6.5 -> 5.2, 48 x 2 8.1 -> 5.3; a launch of empty CTAs takes 1.1.
+// split kernel, before and now: 64 sequences x 8 heads, groups of 16 tokens 6.9 -> 5.4 us, 256 x 8, groups of 32 13.4 -> 6.4,
+// 16 x 1 6.5 -> 5.0, 48 x 2 8.1 -> 5.2; a launch of empty CTAs takes 1.1.
 // Sequences in lock step (equal prompts) complete their groups together, once every KG steps.  Then there are several times as many
 // pieces as CTAs were launched for groups: the CTAs of the first rows join in behind their row, up to as many workers as the chip
 // holds, and every worker takes one run of consecutive pieces.  us a layer, 8 heads x 128, all groups complete, with a
@@ -853,8 +853,8 @@ write_step_kernel(const TokArgs<T> TA, const FinArgs<T> FA, int64_t n_fin_launch
   pdl_launch_dependents();
   const LayoutDev& L = TA.L;
   // This CTA's place among the groups' and among the rows' CTAs (from n_rows on: copies).  Groups that are not spread come behind the rows.
-  // In 64 bits the instances with the spread are 0.1 to 0.7 us a layer slower (16 sequences x 1 KV head: 4.4 -> 5.1, from the write to the
-  // split kernel); without it 32 bits are (1,000 rows x 8 heads, 62 groups of 32 complete: 25.8 -> 32.4).
+  // In 64 bits the instances with the spread are 0.1 to 0.8 us a layer slower (16 layers of 16 sequences x 1 KV head 693 -> 706 us a pass);
+  // without it 32 bits are (1,000 rows x 8 heads, 62 groups of 32 complete: 25.8 -> 32.4).
   using Place = typename std::conditional<SPLIT_KG != 0, int, int64_t>::type;
   const Place cta = blockIdx.x, n_rows = (Place)TA.n_rows;
   const Place b = SPLIT_KG ? cta : cta - n_rows;
